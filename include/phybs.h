@@ -43,7 +43,7 @@ extern "C" {
 #define PBS_E_OUT_OF_MEMORY (-7)
 #define PBS_E_CAPACITY (-8)    /* a size beyond a documented fixed maximum      */
 #define PBS_E_DEVICE_TIMEOUT (-9) /* a kernel's bounded wait on its own copies,
-                                     or of the frame engine on a grid barrier,
+                                     or of the frame kernel for another CTA,
                                      ran out (the step's results are invalid)   */
 
 /* Pass engines of pbs_step (pbs_set_pass_engine). */
@@ -123,8 +123,9 @@ typedef struct pbs_step_params {
 
 typedef struct pbs_stats {
     int passes;               /* iterations executed, including redone ones (max over instances); the
-                                 graph engine also counts a pass that carried the state over
-                                 unchanged because a non-finite residual forced an energy check */
+                                 graph engine's pass kernels also count a pass that carried the
+                                 state over unchanged because a non-finite residual forced an
+                                 energy check */
     int iterations;           /* accepted iterations k at exit (max over instances) */
     int rejections;           /* line-search rejections (sum over instances)      */
     int converged;            /* instances that met tol                          */
@@ -134,7 +135,7 @@ typedef struct pbs_stats {
     double energy;            /* instance 0 energy at its last check             */
     double residual_ratio;    /* instance 0 |g_k| / |g_0|                         */
     double device_ms;         /* device time of the last pbs_step (CUDA events)   */
-    int graph_launches;       /* 16-pass bodies the last step's graph ran */
+    int graph_launches;       /* 16-pass bodies the last step ran (0: PBS_ENGINE_FRAME) */
     int warm_start_used;      /* instances whose step started from the learned guess */
     int guess_fallbacks;      /* RESTART control: instances whose inertial guess inverted a
                                  tet, started from the step's start positions instead */
@@ -293,7 +294,7 @@ typedef struct pbs_tune_result {
     int node_npt;            /* nodes per thread of the node kernel (1 or 2)      */
     int n_tried;             /* shapes timed                                      */
     double pass_ms;          /* per-tet + per-node kernel time of one pass, kept shape */
-    double default_pass_ms;  /* the same for the default shape (256, 1024, 448)   */
+    double default_pass_ms;  /* the same for the first shape tried (256, 1024, 448) */
 } pbs_tune_result;
 /* Autotuner of the pass kernels' block and tile shapes: rebuilds the pass
  * layout for each candidate chunk shape (threads per CTA, tets per chunk,
@@ -315,18 +316,23 @@ int pbs_autotune(pbs_handle *h, int passes, pbs_tune_result *out);
  * steps. */
 int pbs_set_chunk_shape(pbs_handle *h, int threads, int chunk_tets, int chunk_nodes, int staged, int node_npt);
 /* Pass engine of pbs_step.  PBS_ENGINE_GRAPH (the default): each pass is a
- * per-tet and a per-node kernel, 16 passes to a captured CUDA graph, and the
- * host reads the count of running instances between graphs.
+ * per-tet and a per-node kernel, 16 passes to the body of a captured CUDA
+ * graph's loop.  A handle whose caller set neither an engine (this call) nor a
+ * chunk shape (pbs_set_chunk_shape, pbs_autotune) runs the frame kernel
+ * instead where every chunk has a resident CTA (up to ~155,000 tets; any
+ * number of instances), which is faster there; its steps report
+ * graph_launches as the 16-pass bodies the passes fill.
  * PBS_ENGINE_FRAME: one cooperative launch runs all the passes of a step; its
- * CTAs stay resident for the whole step, grid barriers separate the tet and
- * node phases of a pass, and every CTA takes the line-search and stop
- * decisions from the same sums.  For one-instance handles whose chunk shape
+ * CTAs stay resident for the whole step and hand each other the node words
+ * and force sums of a pass as tagged 16-byte words, and every CTA takes the
+ * line-search and stop decisions from the same sums.  For one-instance handles whose chunk shape
  * is unstaged (staged 0) with 128 or 256 threads; PBS_E_INVALID_ARG
  * otherwise, and from pbs_step when a later shape or parameter change leaves
  * the handle outside that set.  The instance's energy and residual sums are
  * grouped per CTA instead of per chunk, so results agree with the graph
- * engine's to rounding; they are bit-reproducible run to run.  A barrier wait
- * that runs out (0.5 s) ends the step with PBS_E_DEVICE_TIMEOUT.
+ * engine's to rounding; they are bit-reproducible run to run.  A wait for
+ * another CTA's words that runs out (2 s) ends the step with
+ * PBS_E_DEVICE_TIMEOUT.
  * pbs_stats.graph_launches is 0 for a frame-engine step.  No counterpart in
  * the reference, which launches each kernel from the host. */
 int pbs_set_pass_engine(pbs_handle *h, int engine);

@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(BLOCK / NPT, NPT == 2 ? 6 : 0) k_node(DevMesh 
         NodeConst nc;
         nc.ch = s_c[0][l];
         nc.cl = s_c[1][l];
-        r2 += node_update<NPRE>(m, p, st, b * BLOCK + l, nc, in[j], fp[j], ctx);
+        r2 += node_update(p, st, b * BLOCK + l, nc, in[j], ctx, [&] { return node_sums<NPRE>(st, in[j], fp[j], do_h); });
     }
     const float sr = block_sum_f(r2, sh);
     if (threadIdx.x == 0) st.npartf[b] = sr;

@@ -41,15 +41,49 @@ struct PassCtx {
     size_t cur, nxt;
 };
 
-// Jacobi step with Chebyshev extrapolation (or restore / save) of node i;
-// returns its |g|^2 (FP32: three positive squares).
+// A node's per-chunk partial sums added in chunk order, and of the
+// Jacobi-diagonal terms on refresh passes (else zero).
+struct NodeSums {
+    float3 f, h;
+};
+
 // NPRE: partials of the node loaded together with its state words (a node of
 // the 1M box touches 2-4 chunks of 256 tets; the rest cost one more round
 // trip).
 template <int NPRE>
-__device__ __forceinline__ float node_update(const DevMesh &m, const DevParams &p, const DevState &st, int i,
-                                             const NodeConst &in, const NodeIn &nn, const float4 (&f)[NPRE],
-                                             const PassCtx &c) {
+__device__ __forceinline__ NodeSums node_sums(const DevState &st, const NodeIn &nn, const float4 (&f)[NPRE],
+                                              bool do_h) {
+    float3 s = make_float3(0.f, 0.f, 0.f), h = make_float3(0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < NPRE; ++j) {
+        s.x += f[j].x;
+        s.y += f[j].y;
+        s.z += f[j].z;
+    }
+    for (int j = nn.pa + NPRE; j < nn.pe; ++j) {
+        const float4 q = st.part[j];
+        s.x += q.x;
+        s.y += q.y;
+        s.z += q.z;
+    }
+    if (do_h) {
+        for (int j = nn.pa; j < nn.pe; ++j) {
+            const float4 q = st.parth[j];
+            h.x += q.x;
+            h.y += q.y;
+            h.z += q.z;
+        }
+    }
+    return NodeSums{s, h};
+}
+
+// Jacobi step with Chebyshev extrapolation (or restore / save) of node i;
+// returns its |g|^2 (FP32: three positive squares).  *out (when not null): the
+// new state words (hi, lo).  sums(): the node's NodeSums, asked for only by a
+// free node that takes a step.
+template <class Sums>
+__device__ __forceinline__ float node_update(const DevParams &p, const DevState &st, int i, const NodeConst &in,
+                                             const NodeIn &nn, const PassCtx &c, Sums sums, float4 *out = nullptr) {
     float r2 = 0.f;
     const float state = in.cl.w;
     if (state == 2.f) return r2;
@@ -71,33 +105,12 @@ __device__ __forceinline__ float node_update(const DevMesh &m, const DevParams &
             st.ol[i] = ul;
         }
         if (state == 0.f) {
-            float fx = 0.f, fy = 0.f, fz = 0.f, hx = 0.f, hy = 0.f, hz = 0.f;
-            // this node's per-chunk partial sums, in chunk order (the first
-            // NPRE loaded with the state words, the rest here)
-#pragma unroll
-            for (int j = 0; j < NPRE; ++j) {
-                fx += f[j].x;
-                fy += f[j].y;
-                fz += f[j].z;
-            }
-            for (int j = nn.pa + NPRE; j < nn.pe; ++j) {
-                const float4 q = st.part[j];
-                fx += q.x;
-                fy += q.y;
-                fz += q.z;
-            }
-            if (c.do_h) {
-                for (int j = nn.pa; j < nn.pe; ++j) {
-                    const float4 q = st.parth[j];
-                    hx += q.x;
-                    hy += q.y;
-                    hz += q.z;
-                }
-            }
+            const NodeSums ns = sums();
+            const float fx = ns.f.x, fy = ns.f.y, fz = ns.f.z;
             const float mh = in.ch.w;  // M / h^2
             float4 D;
             if (c.do_h) {
-                D = make_float4(hx + mh, hy + mh, hz + mh, 0.f);
+                D = make_float4(ns.h.x + mh, ns.h.y + mh, ns.h.z + mh, 0.f);
                 st.diag[i] = D;
             } else {
                 D = nn.diag;
@@ -131,6 +144,10 @@ __device__ __forceinline__ float node_update(const DevMesh &m, const DevParams &
     st.uh[nxt + i] = nh;
     st.ul[nxt + i] = nl;
     st.dd[nxt + i] = nd;
+    if (out) {
+        out[0] = nh;
+        out[1] = nl;
+    }
     return r2;
 }
 

@@ -4,7 +4,7 @@
 // graph path takes the line search in the last CTA of the pass's tet kernel
 // and the pass decision in the first chunk CTA of the next pass's tet kernel
 // (settle_pass, chunks.cu) or in k_settle after the last pass of a run
-// (kernels.cu); the persistent frame kernel (chunks.cu) takes them in every
+// (kernels.cu); the persistent frame kernel (frame.cu) takes them in every
 // CTA from the same sums, so every CTA's copy stays the same.
 #pragma once
 #include <math.h>
@@ -22,7 +22,10 @@ __device__ __forceinline__ void decide_line_search(InstCtl &ci, const DevParams 
     ci.energy = E;
     // rounding-noise allowance: the FP64 sum of FP32 terms e_i carries a random
     // error of order 2^-24 sqrt(sum e_i^2); slack 0 is the reference's strict test
-    const double tau = (double)p.energy_slack * 5.9604644775390625e-8 * sqrt(E2);
+    // (no FP64 square root for a slack of 0, where only a non-finite E2 matters)
+    const double tau = p.energy_slack == 0.f && isfinite(E2)
+                           ? 0.0
+                           : (double)p.energy_slack * 5.9604644775390625e-8 * sqrt(E2);
     // RESTART control also treats a non-finite energy (a step that inverted
     // tets) as a rejection; the reference control accepts it (NaN > E_old is
     // false), and the step then ends with PBS_E_NONFINITE below
@@ -64,8 +67,14 @@ __device__ __forceinline__ void decide_pass(InstCtl &ci, const DevParams &p, int
     } else {
         if (k == 0 && !ci.g0_fixed) g0 = sqrt(R2);
         ci.r2 = R2;
-        const double lim = (double)p.tol * g0;
-        if (p.tol > 0.f && k > 0 && R2 <= lim * lim) {
+        // (no FP64 arithmetic without a tolerance: each operation is some 200
+        // cycles of this decision's latency)
+        bool met = false;
+        if (p.tol > 0.f && k > 0) {
+            const double lim = (double)p.tol * g0;
+            met = R2 <= lim * lim;
+        }
+        if (met) {
             converged = 1;  // keep x_k (the current parity)
             done = 1;
         } else {

@@ -212,13 +212,15 @@ __device__ __forceinline__ bool pass_forces_c(const float4 &x0, const float4 &x1
         disp_gradient<float>(z, f4add(f4sub(x1, x0), f4sub(l1, l0)), f4add(f4sub(x2, x0), f4sub(l2, l0)),
                              f4add(f4sub(x3, x0), f4sub(l3, l0)), dinv, kin.G);
         kinematics(kin);
-        // near inversion (det F < 1e-3, or a stretch-material tet whose FP32
-        // spectrum has sigma_3 < 0.3): the FP64 stress from the absolute positions
-        exact = 1.0f + kin.d < 1e-3f;
-        if (!exact) {
-            if (MATERIAL == PBS_MATERIAL_STRETCH) exact = !stretch_pk1<float>(kin.G, mu, lambda, P);
-            else pk1_neohookean<float>(kin, mu, lambda, P);
-        }
+        // near inversion (det F < 1e-3): the FP64 stress from the absolute
+        // positions.  The stretch-based material is the same energy, so an
+        // uninverted tet takes its stress from the invariants too, without an
+        // SVD, unless its smallest singular value may be below 0.3
+        // (stretch_needs_svd)
+        exact = 1.0f + kin.d < 1e-3f || (MATERIAL == PBS_MATERIAL_STRETCH && stretch_needs_svd(kin));
+        if (!exact) pk1_neohookean<float>(kin, mu, lambda, P);
+        if (MATERIAL == PBS_MATERIAL_STRETCH && !DEFER && exact && 1.0f + kin.d >= 1e-3f)
+            exact = !stretch_pk1<float>(kin.G, mu, lambda, P);
         if (exact && !DEFER)
             pk1_exact_fp64(MATERIAL, cr, x0, x1, x2, x3, l0, l1, l2, l3,
                            make_float4(dinv[0], dinv[1], dinv[2], 0.f), make_float4(dinv[3], dinv[4], dinv[5], 0.f),

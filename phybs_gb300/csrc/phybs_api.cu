@@ -52,7 +52,7 @@ struct pbs_handle {
     DevBuf<float4> row0, row1, row2, info, rest4;
     DevBuf<int> inc_ptr, inc, tblk_inst, nblk_inst, pad2user, tet_user, node_state, bad, staging_ids;
     // pass layout (chunks of tets) and the host copies it is rebuilt from
-    int n_chunks = 0, chunk_tets = CHUNK_TETS, chunk_nodes = CHUNK_NODES, chunk_threads = CHUNK_THREADS;
+    int n_chunks = 0, chunk_tets = 0, chunk_nodes = 0, chunk_threads = 0;
     int chunk_stage = 0;
     int node_npt = NODE_NPT_DEFAULT;
     std::vector<int4> h_tets_pad;
@@ -135,11 +135,17 @@ struct pbs_handle {
     cudaEvent_t ev_start = nullptr, ev_end = nullptr, ev_chunk[2] = {nullptr, nullptr};
     cudaGraphExec_t graph = nullptr;
     bool graph_valid = false;
+    bool shape_auto = true;   // no caller set the chunk shape (pbs_set_chunk_shape, pbs_autotune)
+    bool engine_auto = true;  // nor the pass engine (pbs_set_pass_engine)
+    bool plan_valid = false;  // fplan describes the current layout, material and stress
+    FramePlan fplan;
     bool graph_loop = false;  // graph is the WHILE node over the pass body (else the body alone)
-    // persistent frame kernel: its barrier words and per-CTA sums
+    // persistent frame kernel: its exchanged words
     int engine = PBS_ENGINE_GRAPH;
-    DevBuf<FrameSync> fsync;
-    DevBuf<double2> fce, fcr;
+    DevBuf<float4> fxh, fxl, fce;
+    DevBuf<uint2> fcr;
+    unsigned frame_tag = 0;     // the last tag any word may hold
+    bool frame_clean = false;   // false: the words are cleared before the next launch
     double last_ms = 0.0;
     pbs_stats stats{};
 
@@ -189,7 +195,7 @@ struct pbs_handle {
         DevBuf<float4> *cf[] = {&qrows, &part, &parth};
         for (auto b : cf) b->release();
         tf.release(); hd.release(); staging.release(); staging2.release(); tpart.release(); npart.release(); npartf.release(); ctl.release(); ctl2.release(); tcount.release();
-        fsync.release(); fce.release(); fcr.release();
+        fxh.release(); fxl.release(); fce.release(); fcr.release();
         faces_pad.release(); ring_pad.release(); pick_id.release(); pick_d2.release(); drag_ext.release();
         bsr_ptr.release(); bsr_col.release(); bsr_val.release(); cg_dinv.release(); cg_part.release(); cg_state.release();
         pbd_grp.release(); pbd_lvl.release(); pbd_tet.release(); pbd_d0.release(); pbd_d1.release(); pbd_d2.release();
@@ -221,9 +227,10 @@ struct pbs_handle {
         }                                                       \
     } while (0)
 
-// (Re)builds the pass layout with the given chunk shape: host chunking of the
-// padded mesh, the device arrays, the chunk-ordered copy of the per-tet rows
-// (when they exist) and the instances' chunk ranges.  host_ctl: the control
+// (Re)builds the pass layout: host chunking of the padded mesh, the device
+// arrays, the chunk-ordered copy of the per-tet rows (when they exist) and the
+// instances' chunk ranges.  threads > 0: that chunk shape for every instance;
+// threads = 0: each instance's automatic limits.  host_ctl: the control
 // blocks still on the host (creation), else those on the device are updated.
 static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage, std::vector<InstCtl> *host_ctl) {
     std::vector<InstCtl> ctl;
@@ -233,8 +240,19 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
         ctl.resize(h->B);
         CK(cudaMemcpy(ctl.data(), h->ctl.p, sizeof(InstCtl) * h->B, cudaMemcpyDeviceToHost));
     }
+    std::vector<ChunkLimits> limits(h->B, ChunkLimits{ct, cn});
+    h->shape_auto = threads == 0;
+    if (threads == 0) {
+        ct = cn = 0;
+        for (int b = 0; b < h->B; ++b) {
+            limits[b] = auto_chunk_limits(ctl[b].tet_end - ctl[b].tet_begin, h->sms);
+            ct = std::max(ct, limits[b].tets);
+            cn = std::max(cn, limits[b].nodes);
+        }
+        threads = ct > 256 ? 256 : 128;  // one or two tets a thread
+    }
     ChunkLayout cl;
-    build_chunks(h->Np, h->h_tets_pad, h->h_rest_pad, ctl, ct, cn, cl);
+    build_chunks(h->Np, h->h_tets_pad, h->h_rest_pad, ctl, limits, cl);
     const int nc = (int)cl.chunk.size();
     const size_t L = cl.lmeta.size(), T = (size_t)h->T;
     h->chunk.release(); h->chunk_inst.release(); h->cpart.release(); h->qperm.release();
@@ -266,7 +284,7 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
                             h->qrow2));
     }
     CK(cudaStreamSynchronize(s));
-    h->graph_valid = false;
+    h->graph_valid = h->plan_valid = false;
     return PBS_OK;
 }
 
@@ -324,7 +342,7 @@ const char *pbs_error_string(int code) {
         case PBS_E_NO_DEVICE: return "no compute capability 10.3 CUDA device";
         case PBS_E_OUT_OF_MEMORY: return "out of device memory";
         case PBS_E_CAPACITY: return "size beyond the fixed maximum";
-        case PBS_E_DEVICE_TIMEOUT: return "a kernel's bounded wait (its own copies, a grid barrier) ran out";
+        case PBS_E_DEVICE_TIMEOUT: return "a kernel's bounded wait (its own copies, another CTA's words) ran out";
         default: return "unknown error";
     }
 }
@@ -537,7 +555,7 @@ int pbs_create(const pbs_mesh_desc *d, pbs_handle **out) {
     CKC(prepare_chunk_kernels());
     cudaStream_t s = h->stream;
     {
-        const int rc = set_pass_layout(h, CHUNK_THREADS, CHUNK_TETS, CHUNK_NODES, 0, &ctl);
+        const int rc = set_pass_layout(h, 0, 0, 0, 0, &ctl);
         if (rc != PBS_OK) return fail(rc);
     }
     CKC(cudaMemcpyAsync(h->tets.p, tets_pad.data(), sizeof(int4) * Tp, cudaMemcpyHostToDevice, s));
@@ -616,7 +634,7 @@ int pbs_set_l2_residency(pbs_handle *h, int enable) {
     if (enable && !h->l2_setaside) return PBS_E_INVALID_ARG;  // the device offers no persisting L2
     if ((enable != 0) != h->l2_use) {
         h->l2_use = enable != 0;
-        h->graph_valid = false;  // the captured launches carry the window
+        h->graph_valid = h->plan_valid = false;  // the captured launches carry the window
         if (!enable) cudaCtxResetPersistingL2Cache();
     }
     return PBS_OK;
@@ -640,7 +658,7 @@ int pbs_set_material(pbs_handle *h, int model, const float *mu, const float *lam
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     buf.release();
     CK(e);
-    if (h->material != model) h->graph_valid = false;
+    if (h->material != model) h->graph_valid = h->plan_valid = false;
     h->material = model;
     h->dparams.incremental = model == PBS_MATERIAL_NEOHOOKEAN && h->params.incremental_stress ? 1 : 0;
     return PBS_OK;
@@ -653,7 +671,7 @@ int pbs_set_params(pbs_handle *h, const pbs_step_params *p) {
     h->params = *p;
     to_dev_params(h->params, h->dparams);
     h->dparams.incremental = h->material == PBS_MATERIAL_NEOHOOKEAN && h->params.incremental_stress ? 1 : 0;
-    h->graph_valid = false;
+    h->graph_valid = h->plan_valid = false;
     return PBS_OK;
 }
 
@@ -733,42 +751,79 @@ static int ensure_graph(pbs_handle *h) {
     return PBS_OK;
 }
 
-// CTAs of the frame kernel for the handle's current layout; 0 when the frame
-// engine does not apply to it.
-static int frame_ctas(const pbs_handle *h) {
-    return frame_grid(h->mesh(), h->material, h->material == PBS_MATERIAL_NEOHOOKEAN && h->dparams.incremental,
-                      h->sms);
+// How the frame kernel runs the handle's current layout.
+static const FramePlan &handle_frame_plan(pbs_handle *h) {
+    if (!h->plan_valid) {
+        h->fplan = frame_plan(h->mesh(), h->material,
+                              h->material == PBS_MATERIAL_NEOHOOKEAN && h->dparams.incremental, h->sms);
+        h->plan_valid = true;
+    }
+    return h->fplan;
 }
 
-// Enqueues one frame-kernel launch of at most max_passes passes with params p
-// (the barrier words zeroed first).  PBS_E_INVALID_ARG when the frame engine
-// does not apply to the handle's layout.
+// The frame engine as the caller selects it: one instance.
+static bool frame_applies(pbs_handle *h) { return h->B == 1 && handle_frame_plan(h).grid > 0; }
+
+// Enqueues one frame-kernel launch of at most max_passes passes with params p;
+// frame_done must follow once the launch has ended.  PBS_E_INVALID_ARG when
+// the frame kernel does not apply to the handle's layout.
 static int launch_frame_step(pbs_handle *h, const DevParams &p, int max_passes) {
-    const int G = frame_ctas(h);
-    if (G <= 0) return PBS_E_INVALID_ARG;
+    const FramePlan &plan = handle_frame_plan(h);
+    if (plan.grid <= 0) return PBS_E_INVALID_ARG;
     cudaStream_t s = h->stream;
-    if (!h->fsync.p) CK(h->fsync.alloc(1));
-    if (h->fce.n < (size_t)G) {
+    if (!h->fxh.p) {
+        CK(h->fxh.alloc(h->Np));
+        CK(h->fxl.alloc(h->Np));
+        h->frame_clean = false;
+    }
+    if (h->fce.n < (size_t)plan.grid) {
         h->fce.release();
         h->fcr.release();
-        CK(h->fce.alloc(G));
-        CK(h->fcr.alloc(G));
+        CK(h->fce.alloc(plan.grid));
+        CK(h->fcr.alloc(2 * (size_t)plan.grid));
+        h->frame_clean = false;
     }
-    CK(cudaMemsetAsync(h->fsync.p, 0, sizeof(FrameSync), s));
+    // tags only grow, so the words of earlier launches need no clearing; they
+    // are cleared after a launch whose passes are not known, and long before
+    // the tags would wrap
+    if (!h->frame_clean || h->frame_tag > 0x40000000u) {
+        CK(cudaMemsetAsync(h->fxh.p, 0, sizeof(float4) * h->fxh.n, s));
+        CK(cudaMemsetAsync(h->fxl.p, 0, sizeof(float4) * h->fxl.n, s));
+        CK(cudaMemsetAsync(h->fce.p, 0, sizeof(float4) * h->fce.n, s));
+        CK(cudaMemsetAsync(h->fcr.p, 0, sizeof(uint2) * h->fcr.n, s));
+        CK(cudaMemsetAsync(h->part.p, 0, sizeof(float4) * h->part.n, s));
+        CK(cudaMemsetAsync(h->parth.p, 0, sizeof(float4) * h->parth.n, s));
+        h->frame_tag = 0;
+    }
     FrameAux fx;
-    fx.sync = h->fsync.p;
+    fx.xh = h->fxh.p;
+    fx.xl = h->fxl.p;
     fx.ce = h->fce.p;
     fx.cr = h->fcr.p;
+    fx.tag0 = h->frame_tag;
     fx.max_passes = max_passes;
-    CK(launch_frame(s, h->mesh(), p, h->state(), h->material, fx, G));
+    h->frame_clean = false;
+    CK(launch_frame(s, h->mesh(), p, h->state(), h->material, fx, plan));
     return PBS_OK;
+}
+
+// After a frame launch that ended with at most `passes` passes of any
+// instance: the tags it used are spent.
+static void frame_done(pbs_handle *h, int passes) {
+    h->frame_tag += (unsigned)passes + 2u;
+    h->frame_clean = true;
 }
 
 int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     if (!h) return PBS_E_INVALID_ARG;
     PBS_DEVICE_SCOPE(h->device);
-    const bool frame = h->engine == PBS_ENGINE_FRAME;
-    if (frame && frame_ctas(h) <= 0) return PBS_E_INVALID_ARG;
+    bool frame = h->engine == PBS_ENGINE_FRAME;
+    if (frame && !frame_applies(h)) return PBS_E_INVALID_ARG;
+    // the caller chose neither an engine nor a shape: the frame kernel where
+    // every chunk has a resident CTA of its own (auto_chunk_limits), which
+    // spares a pass its two launches and its trips to memory
+    const bool auto_frame = !frame && h->engine_auto && h->shape_auto && handle_frame_plan(h).resident;
+    frame |= auto_frame;
     int rc = frame ? PBS_OK : ensure_graph(h);
     if (rc != PBS_OK) return rc;
     cudaStream_t s = h->stream;
@@ -845,8 +900,10 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     S.energy = h->h_ctl[0].energy;
     S.residual_ratio = residual_ratio(h->h_ctl[0]);
     S.device_ms = ms;
-    S.graph_launches = launched;
+    // the default engine counts in bodies whichever kernel ran its passes
+    S.graph_launches = auto_frame ? std::max(1, (S.passes + CHUNK_PASSES - 1) / CHUNK_PASSES) : launched;
     h->stats = S;
+    if (frame) frame_done(h, S.passes);
     if (iters_out) *iters_out = S.iterations;
     return S.status;
 }
@@ -1073,6 +1130,7 @@ static int time_frame(pbs_handle *h, int passes, double *pass_ms) {
     if (rc != PBS_OK) return rc;
     InstCtl c;
     CK(cudaMemcpy(&c, h->ctl.p, sizeof(InstCtl), cudaMemcpyDeviceToHost));
+    frame_done(h, passes);
     if (c.status != PBS_OK || c.passes < passes) {
         pbs_stats S{};
         S.passes = c.passes; S.iterations = c.k; S.rejections = c.rejections; S.converged = c.converged;
@@ -1090,8 +1148,9 @@ extern "C" {
 int pbs_set_pass_engine(pbs_handle *h, int engine) {
     if (!h || (engine != PBS_ENGINE_GRAPH && engine != PBS_ENGINE_FRAME)) return PBS_E_INVALID_ARG;
     PBS_DEVICE_SCOPE(h->device);
-    if (engine == PBS_ENGINE_FRAME && frame_ctas(h) <= 0) return PBS_E_INVALID_ARG;
+    if (engine == PBS_ENGINE_FRAME && !frame_applies(h)) return PBS_E_INVALID_ARG;
     h->engine = engine;
+    h->engine_auto = false;
     return PBS_OK;
 }
 
@@ -1140,7 +1199,8 @@ int pbs_autotune(pbs_handle *h, int passes, pbs_tune_result *out) {
                                     {128, 192, 128, 0},  {256, 256, 160, 0}};
     const int n = (int)(sizeof(shapes) / sizeof(shapes[0]));
     const bool can_stage = h->material == PBS_MATERIAL_NEOHOOKEAN;
-    const int t0 = h->chunk_threads, c0 = h->chunk_tets, n0 = h->chunk_nodes, s0 = h->chunk_stage;
+    // threads 0: the automatic shape
+    const int t0 = h->shape_auto ? 0 : h->chunk_threads, c0 = h->chunk_tets, n0 = h->chunk_nodes, s0 = h->chunk_stage;
     double best = 1e300, first = -1.0;
     int bi = -1, tried = 0;
     for (int i = 0; i < n; ++i) {
@@ -1180,7 +1240,7 @@ int pbs_autotune(pbs_handle *h, int passes, pbs_tune_result *out) {
         node_ms[npt - 1] = b;
     }
     h->node_npt = node_ms[1] < node_ms[0] ? 2 : 1;
-    h->graph_valid = false;
+    h->graph_valid = h->plan_valid = false;
     if (out) {
         out->node_npt = h->node_npt;
         out->chunk_threads = shapes[bi][0];

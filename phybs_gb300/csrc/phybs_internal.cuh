@@ -29,8 +29,8 @@
 //                                  node i owns slots inc_ptr[i] .. inc_ptr[i+1]-1
 //   tpart       double2[n_tblk]    per tet-block {sum e, sum e^2} of the energy
 // Pass layout (the per-tet kernel of a descent pass works on chunks: runs of
-// at most CHUNK_TETS tets of one instance, in Morton order of their centroids,
-// touching at most CHUNK_NODES nodes):
+// at most chunk_tets tets of one instance, in Morton order of their centroids,
+// touching at most chunk_nodes nodes):
 //   chunk       int4[n_chunks]     {first pass tet, tet count, first local entry, local count}
 //   qrow0..2    float4[T] each     row0..2 of the pass tets, in pass (chunk) order
 //   qcor        uint4[T]           corner ids of a pass tet, two 16-bit fields a word:
@@ -60,12 +60,6 @@ constexpr int BLOCK = 256;  // threads per block of the step kernels (nodes per 
 // nodes per thread of the node kernel (BLOCK / npt threads per CTA): 1 or 2,
 // picked by pbs_autotune
 constexpr int NODE_NPT_DEFAULT = 1;
-// Default chunk shape of the per-tet pass kernel (pbs_autotune may pick
-// another): at most CHUNK_TETS tets touching at most CHUNK_NODES nodes, one
-// CTA of CHUNK_THREADS threads per chunk.
-constexpr int CHUNK_TETS = 1024;
-constexpr int CHUNK_NODES = 448;
-constexpr int CHUNK_THREADS = 256;
 constexpr int CHUNK_MAX_SMEM = 200 * 1024;
 // Dynamic shared memory of the per-tet pass kernel for a chunk shape and a
 // staging mode: 0 = node words (u hi, u lo, and the force base with
@@ -238,8 +232,16 @@ struct ChunkLayout {
     std::vector<int4> lmeta;
     int max_local = 0;
 };
+// At most so many tets and nodes a chunk.
+struct ChunkLimits {
+    int tets, nodes;
+};
+// The chunk limits of an instance whose shape no caller set, from its own tet
+// count only: a packed batch then chunks an instance as it is chunked alone.
+ChunkLimits auto_chunk_limits(int tets, int sms);
+// limits: per instance
 void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<double> &rest, std::vector<InstCtl> &ctl,
-                  int chunk_tets, int chunk_nodes, ChunkLayout &out);
+                  const std::vector<ChunkLimits> &limits, ChunkLayout &out);
 cudaError_t launch_pass_rows(cudaStream_t s, int T, const int *qperm, const float4 *row0, const float4 *row1,
                              const float4 *row2, float4 *q0, float4 *q1, float4 *q2);
 cudaError_t prepare_chunk_kernels();
@@ -247,26 +249,28 @@ cudaError_t prepare_chunk_kernels();
 // and stress mode on a device with `sms` SMs; 0 when it does not apply.
 int stream_grid(const DevMesh &m, int material, bool inc, int sms);
 
-// The persistent frame kernel (chunks.cu): one cooperative launch runs a
-// step's passes of a one-instance handle, with grid barriers between its tet
-// and node phases.  FrameSync: the barrier's words (zeroed before a launch);
-// ce / cr: per-CTA {sum e, sum e^2} of a check pass and {|g|^2, 0} of a pass.
-struct FrameSync {
-    unsigned int count, gen;
-    int err;  // a barrier wait ran out: the step ends with PBS_E_DEVICE_TIMEOUT
-    int pad;
-};
+// The persistent frame kernel (frame.cu): one cooperative launch runs a
+// step's passes; its CTAs hand each other words tagged with the pass they
+// belong to.  xh / xl: the state words by padded node; ce: per-CTA {sum e
+// (FP64), sum e^2} of a check pass; cr: per-CTA |g|^2, two buffers of grid
+// pairs; the partials part / parth carry tags in .w.  A launch uses the tags
+// tag0 + 1 .. tag0 + 1 + passes; no word may hold one of them before it.
 struct FrameAux {
-    FrameSync *sync;
-    double2 *ce, *cr;
+    float4 *xh, *xl, *ce;
+    uint2 *cr;
+    unsigned tag0;
     int max_passes;
 };
-// Co-resident CTAs of the frame kernel for this mesh and shape (at most one
-// per chunk); 0 when the kernel does not apply (several instances, a staged
-// chunk shape, a thread count without an instantiation).
-int frame_grid(const DevMesh &m, int material, bool inc, int sms);
+// How the frame kernel runs a mesh: grid CTAs (0: it does not apply), each
+// with a chunk of its own (resident) or walking several (one instance only).
+struct FramePlan {
+    int grid = 0;
+    bool resident = false;
+    int per_sm = 0;  // resident: the register class, CTAs a SM it is built for
+};
+FramePlan frame_plan(const DevMesh &m, int material, bool inc, int sms);
 cudaError_t launch_frame(cudaStream_t s, const DevMesh &m, const DevParams &p, DevState st, int material,
-                         const FrameAux &fx, int grid);
+                         const FrameAux &fx, const FramePlan &plan);
 
 // Launchers (kernels.cu, warmstart.cu)
 cudaError_t launch_ref_force(cudaStream_t s, const DevMesh &m, const DevParams &p, DevState st);

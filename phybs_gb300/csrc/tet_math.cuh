@@ -380,6 +380,24 @@ template <typename T> __device__ __forceinline__ bool stretch_pk1(const T G[9], 
     return true;
 }
 
+// Whether a stretch-material tet's stress has to come from its singular
+// values: an FP32 spectrum with sigma_3 < 0.3 takes the FP64 route, so a tet
+// is spared the SVD only where sigma_3 >= 0.3 is certain.  sigma_1 sigma_2 <=
+// (sigma_1^2 + sigma_2^2) / 2 <= |F|^2 / 2, hence sigma_3 = det F / (sigma_1
+// sigma_2) >= 2 det F / |F|^2, and 0.31 leaves 3% for rounding.  At rest the
+// bound is 0.67; a tet stretched by 2 along one axis at constant volume has 0.4.
+// P = mu (F - F^-T) + lambda ln J F^-T is U diag(P^) V^T exactly, and its
+// cancellation-free form (pk1_neohookean) carries less rounding than the
+// rotations; four Jacobi sweeps and the QR of every tet were 80% of a
+// stretch-material pass.
+__device__ __forceinline__ bool stretch_needs_svd(const Kin<float> &k) {
+    float g2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) g2 += k.G[i] * k.G[i];
+    // |F|^2 = 3 + 2 tr G + |G|^2; a NaN needs the SVD
+    return !(2.f * (1.f + k.d) >= 0.31f * (3.f + 2.f * k.tr + g2));
+}
+
 // Where a tet's four rest positions are: rest[meta[id[c]].x] (chunk-local
 // ids) or rest[id[c]] (padded node ids, meta null).
 struct CornerRest {

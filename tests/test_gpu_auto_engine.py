@@ -1,0 +1,121 @@
+"""The default engine's choice between the frame kernel and the pass kernels,
+and the stretch material's stress without an SVD.
+
+A handle whose caller chose neither an engine nor a chunk shape runs the frame
+kernel where every chunk has a resident CTA.  Its trajectories are the pass
+kernels' (set_pass_engine("graph") on the same automatic chunks) bit for bit:
+the residual stop is off and the regrouped energy sums do not flip a
+line-search test on these meshes.
+"""
+import numpy as np
+import pytest
+
+from oracle import restated as O
+from phybs_gb300 import _lib as L
+from phybs_gb300 import meshes as M
+from phybs_gb300.solver import DescentSolver, make_params
+
+pytestmark = pytest.mark.gpu
+
+KEYS = ("passes", "iterations", "rejections", "converged", "status", "alpha", "rho", "omega", "graph_launches")
+
+
+@pytest.fixture(scope="module", autouse=True)
+def built():
+    from phybs_gb300.build import build
+    build()
+
+
+def _box(nx, ny, nz):
+    return M.box_mesh(nx, ny, nz, edge=0.25 / max(nx, ny), seed=nx, young=1e5)
+
+
+# one tet; one cube (5); one chunk and a few more (120, 130, 180); around the 128 / 256 line
+# (7,680, 8,320); one, two, three CTAs a SM of 256 tets (38,440, 60,000, 115,200); the 512-tet
+# class (119,000, 155,000); past the resident sizes (161,700: the pass kernels either way)
+BOXES = [(1, 1, 1), (2, 3, 4), (2, 1, 13), (3, 3, 4), (8, 8, 24), (8, 8, 26), (31, 31, 8), (20, 20, 30),
+         (24, 24, 40), (28, 25, 34), (31, 25, 40), (33, 28, 35)]
+
+
+@pytest.mark.parametrize("dims", BOXES, ids=[f"{5 * a * b * c}" for a, b, c in BOXES])
+@pytest.mark.parametrize("material,inc", [(0, 1), (0, 0), (1, 0)], ids=["incremental", "full", "stretch"])
+def test_default_engine_equals_pass_kernels(dims, material, inc):
+    m = _box(*dims)
+    p = make_params("gpu_reference", h=1 / 30, max_iters=40, incremental_stress=inc)
+    a = DescentSolver(m, params=p, material=material)
+    b = DescentSolver(m, params=p, material=material)
+    b.set_pass_engine("graph")
+    for f in range(2):
+        a.step()
+        b.step()
+        sa, sb = a.stats(), b.stats()
+        assert [sa[k] for k in KEYS] == [sb[k] for k in KEYS], f
+        assert np.array_equal(a.positions(), b.positions(), equal_nan=True), f
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("n", [2, 5, 24])
+def test_default_engine_packed(n):
+    """Packed uneven boxes: resident (2, 5) and beyond (24); the iteration
+    budget ends instances at different passes, some of them non-finite."""
+    m = M.batch_of_boxes(n, seed=n, nxy=(4, 16), nz=(8, 32))
+    p = make_params("gpu_reference", h=1 / 30, max_iters=64, alpha0=0.6, profile=((10, 0.9999),))
+    a, b = DescentSolver(m, params=p), DescentSolver(m, params=p)
+    b.set_pass_engine("graph")
+    for f in range(2):
+        a.step(raise_on_error=False)
+        b.step(raise_on_error=False)
+        for i in range(n):
+            sa, sb = a.instance_stats(i), b.instance_stats(i)
+            assert [sa[k] for k in KEYS[:8]] == [sb[k] for k in KEYS[:8]], (f, i)
+        assert np.array_equal(a.positions(), b.positions(), equal_nan=True), f
+    a.close()
+    b.close()
+
+
+def test_single_tet_and_loose_nodes():
+    """One tet, and nodes that no tet touches (more than a CTA has threads)."""
+    x = np.random.default_rng(0).uniform(0, 1, (400, 3)).astype(np.float32)
+    x[:4] = [[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1]]
+    m = M.TetMeshData(x, np.array([[0, 1, 2, 3]]), np.array([0]), 1e4, 0.3)
+    p = make_params("gpu_reference", h=1 / 30, max_iters=24)
+    a, b = DescentSolver(m, params=p), DescentSolver(m, params=p)
+    b.set_pass_engine("graph")
+    # a loose node has no mass: its update is 0 / 0, and the step ends non-finite
+    ra, rb = a.step(raise_on_error=False), b.step(raise_on_error=False)
+    assert (ra, a.last_status) == (rb, b.last_status)
+    assert np.array_equal(a.positions(), b.positions(), equal_nan=True)
+    a.close()
+    b.close()
+
+
+# principal stretches on both sides of the 2 det F >= 0.31 |F|^2 line, and of
+# sigma_3 = 0.3 beyond it
+STRETCHES = [(1.0, 1.0, 1.0), (2.2, 0.7, 0.7), (3.0, 0.6, 0.6), (0.95, 0.95, 0.32), (0.95, 0.95, 0.36), (1.5, 1.5, 0.25),
+             (0.5, 0.5, 0.5), (2.0, 2.0, 2.0)]
+
+
+@pytest.mark.parametrize("s", STRETCHES)
+def test_stretch_stress_without_svd(s):
+    """One iteration of the stretch material from a stretched, wobbling state
+    against the FP64 restatement (the SVD of every tet).  The velocity after it
+    is 0.99 alpha g / (H h): g within the 1e-5 bar of assembled forces, H's
+    closed form within another 1e-5, so 3e-5 of the largest velocity."""
+    m = M.box_mesh(5, 4, 6, edge=0.05, seed=3, young=1e5, pin="bottom")
+    x = m.rest.astype(np.float64)
+    x = x * np.array(s) + 0.002 * np.sin(40 * x[:, [1, 2, 0]])
+    x[m.pins] = m.rest[m.pins] * np.array(s, np.float32)
+    x = x.astype(np.float32)
+    p = make_params("gpu_reference", h=1 / 30, max_iters=1, alpha0=0.05)
+    a = DescentSolver(m, positions=x, material=L.PBS_MATERIAL_STRETCH, params=p)
+    a.step()
+    mu, lam = O.lame(m.young, m.poisson)
+    pm = m.pin_mask()
+    r64 = O.rest(m.rest, m.tets, pm, prec=64)
+    st = O.StepState(x)
+    O.step(st, O.make_params(h=1 / 30, max_iters=1, alpha0=0.05, body_force_scale=1.0, energy_clamp=1, material=1,
+                             hessian_closed=1), m.tets, r64, mu, lam, pm, prec=64)
+    v = a.velocities()[0]
+    assert np.abs(v - st.v).max() <= 3e-5 * np.abs(st.v).max(), np.abs(v - st.v).max() / np.abs(st.v).max()
+    a.close()
