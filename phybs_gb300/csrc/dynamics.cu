@@ -6,10 +6,11 @@
 // one more than the highest level of the earlier tets that share one of its
 // nodes, so a level's tets share no node and each reads exactly the updates of
 // the tets before it in the serial order.  One thread-block cluster sweeps an
-// instance level by level (16 CTAs when the handle holds few instances, else
-// 8), the cluster barrier ordering the levels (its arrive/wait carry
-// release/acquire semantics for the global positions):
-// 2,320 levels of ~430 tets for the 1M-tet box, 920 for the 24K bar.  The
+// instance step by step (16 CTAs when the handle holds few instances, else
+// 8), a step being one level of each sweep in flight (PbdStep), the cluster
+// barrier ordering the steps (its arrive/wait carry release/acquire semantics
+// for the positions): 2,496 steps of up to 2,150 tets for five sweeps of the
+// 1M-tet box (2,320 levels), 636 for the 24K bar (348 levels).  The
 // arithmetic is FP32 with every product and sum rounded separately (no
 // contraction) in Eigen 3.2's order, so a sweep is the CPU's bit for bit.
 //
@@ -38,7 +39,10 @@ namespace {
 // CTAs a PBD cluster sweeps an instance with: 16 (the non-portable maximum,
 // opted into at launch) when a handle holds few instances, else 8
 constexpr int kPbdClusterMax = 16;
-constexpr int kPbdThreads = 128;
+// worker threads of a CTA, and the scheduler warp: the eighth, whose warp
+// scheduler the first seven leave to at most one other
+constexpr int kPbdWorkers = 224;
+constexpr int kPbdThreads = kPbdWorkers + 32;
 
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
@@ -175,55 +179,144 @@ __device__ __forceinline__ void pbd_apply(const PbdView &v, const PbdTet &t, con
         v.px[id[c]] = make_float4(fadd(p[c].x, dp[c][0]), fadd(p[c].y, dp[c][1]), fadd(p[c].z, dp[c][2]), p[c].w);
 }
 
-// One cluster per group of levels (an instance): `iterations` sweeps over its
-// levels; a level's tets are split into one contiguous run per CTA of the
-// cluster.  Positions are read through L2 (ld.global.cg); the cluster barrier
-// orders one level's writes before the next level's reads.  A thread's first
-// static record of the next level is loaded before the barrier, so a level's
-// dependent chain starts at the position loads.
-__global__ void __launch_bounds__(kPbdThreads) k_pbd_sweep(PbdView v, int iterations, PbdConst k) {
-    cg::cluster_group cl = cg::this_cluster();
-    const int csize = (int)cl.num_blocks();
-    const int g = blockIdx.x / csize;
-    const int rank = (int)cl.block_rank();
-    const int l0 = v.grp[g], l1 = v.grp[g + 1];
-    if (l0 == l1 || iterations <= 0) return;  // uniform over the cluster
-    // this thread's run [j, b1) of level l
-    auto run_of = [&](int l, int &j, int &b1) {
-        const int a = v.lvl[l], e = v.lvl[l + 1];
+// The sweeps' schedule.  Sweep q runs level l of its group at step l + q D: with
+// D larger than any level difference between tets that share a node (the
+// group's delay), a tet comes after every earlier tet of its own sweep that
+// shares a node (their levels are lower), after all such tets of the sweep
+// before (their levels are at most its own + D - 1, D steps earlier) and before
+// those of the next one, so it reads what the serial order gives it; and tets
+// of one step share no node.  L + (sweeps - 1) D steps instead of L sweeps:
+// the dependent chain of a level, which bounds a step, then serves several
+// sweeps at once.  On structured meshes D is 2-20% of L (the 1M-tet box: L
+// 2,320, D 44; the 24,000-tet bar 348 and 72), on meshes in arbitrary order up
+// to L, where the sweeps simply follow one another.
+struct PbdStep {
+    int l0, L, D, sweeps, steps;
+    __device__ PbdStep(const PbdView &v, int g, int iterations) {
+        l0 = v.grp[g];
+        L = v.grp[g + 1] - l0;
+        D = v.delay[g];
+        sweeps = iterations;
+        steps = L > 0 && iterations > 0 ? L + (iterations - 1) * D : 0;
+    }
+    // the sweeps that are on at step t: q0 .. q1
+    __device__ __forceinline__ void on(int t, int &q0, int &q1) const {
+        q0 = t < L ? 0 : (t - L) / D + 1;
+        q1 = min(sweeps - 1, t / D);
+    }
+    // CTA `rank`'s run of the level of sweep q at step t: its first tet, count
+    __device__ __forceinline__ void run(const PbdView &v, int t, int q, int rank, int csize, int &b0, int &n) const {
+        const int l = l0 + t - q * D;
+        const int a = __ldg(v.lvl + l), e = __ldg(v.lvl + l + 1);
         const int chunk = (e - a + csize - 1) / csize;
-        const int b0 = a + rank * chunk;
-        b1 = min(b0 + chunk, e);
-        j = b0 + (int)threadIdx.x;
-    };
-    int j, b1;
-    run_of(l0, j, b1);
-    PbdTet cur = pbd_load(v, j < b1 ? j : v.lvl[l0]);
-    const int total = iterations * (l1 - l0);
-    for (int s = 0; s < total; ++s) {
-        const int l = l0 + s % (l1 - l0);
-        // next level's first record (for the last level of the last sweep: none)
-        int jn = 0, bn = 0;
-        PbdTet nxt = cur;
-        if (s + 1 < total) {
-            const int ln = l + 1 < l1 ? l + 1 : l0;
-            run_of(ln, jn, bn);
-            if (jn < bn) nxt = pbd_load(v, jn);
+        b0 = a + rank * chunk;
+        n = max(0, min(chunk, e - b0));
+    }
+    // the tet at place `pos` of CTA `rank`'s runs of step t, -1 past their end
+    __device__ __forceinline__ int tet(const PbdView &v, int t, int rank, int csize, int pos) const {
+        int q0, q1;
+        on(t, q0, q1);
+        for (int q = q0; q <= q1; ++q) {
+            int b0, n;
+            run(v, t, q, rank, csize, b0, n);
+            if (pos < n) return b0 + pos;
+            pos -= n;
         }
-        if (j < b1) pbd_apply(v, cur, k);
-        for (int jj = j + kPbdThreads; jj < b1; jj += kPbdThreads) pbd_apply(v, pbd_load(v, jj), k);
+        return -1;
+    }
+};
+
+// Scheduler warp: the first kPbdWorkers tets of CTA `rank`'s runs of step t
+// into idx (-1 past their end).
+__device__ __forceinline__ void pbd_schedule(const PbdStep &sch, const PbdView &v, int t, int rank, int csize, int *idx) {
+    const int lane = threadIdx.x & 31;
+    int q0, q1, base = 0;
+    sch.on(t, q0, q1);
+    for (int qa = q0; qa <= q1 && base < kPbdWorkers; qa += 32) {
+        int b0 = 0, n = 0;
+        if (qa + lane <= q1) sch.run(v, t, qa + lane, rank, csize, b0, n);
+        int end = n;  // inclusive prefix sum over the lanes
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += x;
+        }
+        const int cnt = min(32, q1 - qa + 1);
+        for (int i = 0; i < cnt; ++i) {
+            const int ni = __shfl_sync(0xffffffffu, n, i), bi = __shfl_sync(0xffffffffu, b0, i);
+            const int at = base + __shfl_sync(0xffffffffu, end, i) - ni;
+            for (int x = lane; x < ni && at + x < kPbdWorkers; x += 32) idx[at + x] = bi + x;
+        }
+        base += __shfl_sync(0xffffffffu, end, 31);
+    }
+    for (int x = base + lane; x < kPbdWorkers; x += 32) idx[x] = -1;
+}
+
+// One cluster per group of levels (an instance); a step's tets are split into
+// one contiguous run per level and CTA of the cluster.  The cluster barrier
+// orders one step's position writes before the next one's reads.  A scheduler
+// warp beside the workers lists the CTA's tets of the step after next, so that
+// a worker loads the next step's static record before this step's chain and
+// a step is that chain alone: position loads, the projections, the barrier.
+// (Looked up by every worker between the barrier's arrive and wait, five
+// sweeps of the 1M-tet box took 13.2 instead of 10.2 ms, of the 24,000-tet
+// bar 2.31 instead of 1.28.)
+template <class Load, class Apply>
+__device__ __forceinline__ void pbd_run(cg::cluster_group &cl, const PbdView &v, int g, int iterations, Load load,
+                                        Apply apply) {
+    __shared__ int s_idx[2][kPbdWorkers];
+    const int csize = (int)cl.num_blocks(), rank = (int)cl.block_rank(), tid = (int)threadIdx.x;
+    const PbdStep sch(v, g, iterations);
+    const bool worker = tid < kPbdWorkers;
+    if (sch.steps == 0) return;  // uniform over the cluster
+    if (!worker) {
+        pbd_schedule(sch, v, 0, rank, csize, s_idx[0]);
+        if (sch.steps > 1) pbd_schedule(sch, v, 1, rank, csize, s_idx[1]);
+    }
+    __syncthreads();
+    int j = worker ? s_idx[0][tid] : -1;
+    bool full = s_idx[0][kPbdWorkers - 1] >= 0;  // the step may have more tets than workers
+    PbdTet cur;
+    if (j >= 0) cur = load(j);
+    __syncthreads();
+    for (int t = 0; t < sch.steps; ++t) {
+        if (worker) {
+            const int jn = t + 1 < sch.steps ? s_idx[(t + 1) & 1][tid] : -1;
+            const bool fulln = t + 1 < sch.steps && s_idx[(t + 1) & 1][kPbdWorkers - 1] >= 0;
+            PbdTet nxt = cur;
+            if (jn >= 0) nxt = load(jn);
+            if (j >= 0) {
+                apply(cur);
+                // (levels wider than the cluster's workers)
+                if (full)
+                    for (int pos = tid + kPbdWorkers, x; (x = sch.tet(v, t, rank, csize, pos)) >= 0; pos += kPbdWorkers)
+                        apply(load(x));
+            }
+            cur = nxt;
+            j = jn;
+            full = fulln;
+        } else if (t + 2 < sch.steps) {
+            pbd_schedule(sch, v, t + 2, rank, csize, s_idx[t & 1]);
+        }
         cl.sync();
-        cur = nxt;
-        j = jn;
-        b1 = bn;
     }
 }
 
+// Positions in global memory, read through L2 (ld.global.cg).
+__global__ void __launch_bounds__(kPbdThreads) k_pbd_sweep(PbdView v, int iterations, PbdConst k) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int g = blockIdx.x / (int)cl.num_blocks();
+    pbd_run(cl, v, g, iterations, [&](int j) { return pbd_load(v, j); }, [&](const PbdTet &t) { pbd_apply(v, t, k); });
+}
+
 // The same sweep with the instance's positions held in the cluster's
-// distributed shared memory: CTA r of the 16 keeps nodes [r S, (r + 1) S) of
-// the instance, and a tet corner is addressed by its code (owner CTA << 16 |
-// offset), so every level's position loads and stores go SM to SM instead of
+// distributed shared memory: CTA r of the 16 keeps nodes r, r + 16, ... of the
+// instance, and a tet corner is addressed by its code (owner CTA << 16 |
+// offset), so every step's position loads and stores go SM to SM instead of
 // through L2, and the cluster barrier releases shared-memory writes only.
+// Interleaved, because a level's tets lie near one another: with contiguous
+// slices one or two CTAs served a level's whole traffic (10.3 instead of 8.7
+// ms for five sweeps of the 1M-tet box).
 // Used when an instance's nodes fit (S * 16 B of dynamic shared memory a CTA).
 __device__ __forceinline__ float4 *dsm_node(cg::cluster_group &cl, float4 *s_px, int code) {
     return cl.map_shared_rank(s_px, (unsigned)code >> 16) + (code & 0xffff);
@@ -233,64 +326,35 @@ __global__ void __launch_bounds__(kPbdThreads)
     k_pbd_sweep_dsmem(PbdView v, const int4 *codes, const int4 *gnode, int iterations, PbdConst k) {
     extern __shared__ float4 s_px[];
     cg::cluster_group cl = cg::this_cluster();
-    const int csize = (int)cl.num_blocks();
-    const int g = blockIdx.x / csize;
+    const int g = blockIdx.x / (int)cl.num_blocks();
     const int rank = (int)cl.block_rank();
     const int4 gn = gnode[g];  // {first padded node, slice S, node count}
     const int nb = gn.x, S = gn.y, cnt = gn.z;
-    for (int j = threadIdx.x; j < S; j += kPbdThreads) {
-        const int n = rank * S + j;
+    for (int j = threadIdx.x; j < S; j += blockDim.x) {
+        const int n = j * kPbdClusterMax + rank;
         if (n < cnt) s_px[j] = v.px[nb + n];
     }
     cl.sync();
-    const int l0 = v.grp[g], l1 = v.grp[g + 1];
-    const int total = iterations > 0 ? iterations * (l1 - l0) : 0;
-    auto run_of = [&](int l, int &j, int &b1) {
-        const int a = v.lvl[l], e = v.lvl[l + 1];
-        const int chunk = (e - a + csize - 1) / csize;
-        const int b0 = a + rank * chunk;
-        b1 = min(b0 + chunk, e);
-        j = b0 + (int)threadIdx.x;
-    };
-    auto apply = [&](const PbdTet &t) {
-        const float D[9] = {t.r0.x, t.r0.y, t.r0.z, t.r1.x, t.r1.y, t.r1.z, t.r2.x, t.r2.y, t.r2.z};
-        float4 *ptr[4] = {dsm_node(cl, s_px, t.q.x), dsm_node(cl, s_px, t.q.y), dsm_node(cl, s_px, t.q.z),
-                          dsm_node(cl, s_px, t.q.w)};
-        float4 p[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) p[c] = *ptr[c];
-        float dp[4][3];
-        pbd_project(p, D, k, dp);
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-            *ptr[c] = make_float4(fadd(p[c].x, dp[c][0]), fadd(p[c].y, dp[c][1]), fadd(p[c].z, dp[c][2]), p[c].w);
-    };
     PbdView vc = v;  // the static records with corner codes in place of node ids
     vc.tet = codes;
-    int j = 0, b1 = 0;
-    PbdTet cur;
-    if (total > 0) {
-        run_of(l0, j, b1);
-        cur = pbd_load(vc, j < b1 ? j : v.lvl[l0]);
-    }
-    for (int st = 0; st < total; ++st) {
-        const int l = l0 + st % (l1 - l0);
-        // the next level's first record before this level's chain
-        int jn = 0, bn = 0;
-        PbdTet nxt = cur;
-        if (st + 1 < total) {
-            run_of(l + 1 < l1 ? l + 1 : l0, jn, bn);
-            if (jn < bn) nxt = pbd_load(vc, jn);
-        }
-        if (j < b1) apply(cur);
-        for (int jj = j + kPbdThreads; jj < b1; jj += kPbdThreads) apply(pbd_load(vc, jj));
-        cl.sync();
-        cur = nxt;
-        j = jn;
-        b1 = bn;
-    }
-    for (int j = threadIdx.x; j < S; j += kPbdThreads) {
-        const int n = rank * S + j;
+    pbd_run(
+        cl, vc, g, iterations, [&](int j) { return pbd_load(vc, j); },
+        [&](const PbdTet &t) {
+            const float D[9] = {t.r0.x, t.r0.y, t.r0.z, t.r1.x, t.r1.y, t.r1.z, t.r2.x, t.r2.y, t.r2.z};
+            float4 *ptr[4] = {dsm_node(cl, s_px, t.q.x), dsm_node(cl, s_px, t.q.y), dsm_node(cl, s_px, t.q.z),
+                              dsm_node(cl, s_px, t.q.w)};
+            float4 p[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) p[c] = *ptr[c];
+            float dp[4][3];
+            pbd_project(p, D, k, dp);
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                *ptr[c] = make_float4(fadd(p[c].x, dp[c][0]), fadd(p[c].y, dp[c][1]), fadd(p[c].z, dp[c][2]), p[c].w);
+        });
+    // (the last barrier ordered every position before the copy out)
+    for (int j = threadIdx.x; j < S; j += blockDim.x) {
+        const int n = j * kPbdClusterMax + rank;
         if (n < cnt) v.px[nb + n] = s_px[j];
     }
 }

@@ -118,7 +118,7 @@ struct pbs_handle {
     std::vector<int> h_inst_nodes;  // per instance: first, end padded node
     bool pbd_ready = false;
     int pbd_groups = 0;
-    DevBuf<int> pbd_grp, pbd_lvl;
+    DevBuf<int> pbd_grp, pbd_lvl, pbd_delay;
     DevBuf<int4> pbd_tet;
     DevBuf<float4> pbd_d0, pbd_d1, pbd_d2;
     DevBuf<float2> pbd_node;  // {1 / mass, gravity_y} of the PBD rest data
@@ -198,7 +198,7 @@ struct pbs_handle {
         fxh.release(); fxl.release(); fce.release(); fcr.release();
         faces_pad.release(); ring_pad.release(); pick_id.release(); pick_d2.release(); drag_ext.release();
         bsr_ptr.release(); bsr_col.release(); bsr_val.release(); cg_dinv.release(); cg_part.release(); cg_state.release();
-        pbd_grp.release(); pbd_lvl.release(); pbd_tet.release(); pbd_d0.release(); pbd_d1.release(); pbd_d2.release();
+        pbd_grp.release(); pbd_lvl.release(); pbd_delay.release(); pbd_tet.release(); pbd_d0.release(); pbd_d1.release(); pbd_d2.release();
         pbd_node.release(); pbd_codes.release(); pbd_gnode.release();
         pd_val.release(); pd_dinv.release(); dyn_px.release(); dyn_x0.release(); dyn_s.release();
         pbd_ready = pd_ready = false;
@@ -1513,7 +1513,7 @@ int pbs_backward_euler_step(pbs_handle *h, float dt, float alpha, float beta, co
 static int ensure_pbd(pbs_handle *h) {
     if (h->pbd_ready) return PBS_OK;
     const int B = h->B, Tp = h->Tp;
-    std::vector<int> level(Tp, -1), last(h->Np, -1), grp(B + 1, 0), nlev(B, 0);
+    std::vector<int> level(Tp, -1), last(h->Np, -1), grp(B + 1, 0), nlev(B, 0), delay(B, 1);
     for (int b = 0; b < B; ++b) {
         int top = -1;
         for (int tp = h->h_inst_tets[2 * b]; tp < h->h_inst_tets[2 * b + 1]; ++tp) {
@@ -1526,6 +1526,13 @@ static int ensure_pbd(pbs_handle *h) {
         }
         nlev[b] = top + 1;
         grp[b + 1] = grp[b] + nlev[b];
+        // the delay between sweeps (last: the highest level at each node)
+        for (int tp = h->h_inst_tets[2 * b]; tp < h->h_inst_tets[2 * b + 1]; ++tp) {
+            const int4 q = h->h_tets_pad[tp];
+            if (q.x < 0) continue;
+            const int up = std::max(std::max(last[q.x], last[q.y]), std::max(last[q.z], last[q.w]));
+            delay[b] = std::max(delay[b], up - level[tp] + 1);
+        }
     }
     const int L = grp[B];
     std::vector<int> lvl(L + 1, 0);
@@ -1541,9 +1548,10 @@ static int ensure_pbd(pbs_handle *h) {
     std::vector<int4> tet(std::max(n, 1));
     for (int j = 0; j < n; ++j) tet[j] = h->h_tets_pad[order[j]];
     const size_t nn = (size_t)std::max(n, 1);
-    CK(h->pbd_grp.alloc(B + 1)); CK(h->pbd_lvl.alloc(L + 1)); CK(h->pbd_tet.alloc(nn));
+    CK(h->pbd_grp.alloc(B + 1)); CK(h->pbd_delay.alloc(B)); CK(h->pbd_lvl.alloc(L + 1)); CK(h->pbd_tet.alloc(nn));
     CK(h->pbd_d0.alloc(nn)); CK(h->pbd_d1.alloc(nn)); CK(h->pbd_d2.alloc(nn)); CK(h->pbd_node.alloc(h->Np));
     CK(cudaMemcpy(h->pbd_grp.p, grp.data(), sizeof(int) * (B + 1), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(h->pbd_delay.p, delay.data(), sizeof(int) * B, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(h->pbd_lvl.p, lvl.data(), sizeof(int) * (L + 1), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(h->pbd_tet.p, tet.data(), sizeof(int4) * n, cudaMemcpyHostToDevice));
     DevBuf<int> ord;  // level order -> padded tet, needed only here
@@ -1577,7 +1585,7 @@ static int ensure_pbd(pbs_handle *h) {
                     int c[4];
                     for (int k = 0; k < 4; ++k) {
                         const int loc = q[k] - gn[b].x;
-                        c[k] = ((loc / gn[b].y) << 16) | (loc % gn[b].y);
+                        c[k] = ((loc % 16) << 16) | (loc / 16);
                     }
                     codes[j] = make_int4(c[0], c[1], c[2], c[3]);
                 }
@@ -1620,7 +1628,7 @@ int pbs_pbd_step(pbs_handle *h, float dt, int iterations, const float *stretch, 
     CK(launch_pbd_begin(s, m, st, h->pbd_node.p, ext ? h->ext.p : nullptr, dt, h->dyn_px.p, h->dyn_x0.p));
     if (iterations > 0) {
         PbdView v;
-        v.grp = h->pbd_grp.p; v.lvl = h->pbd_lvl.p; v.tet = h->pbd_tet.p;
+        v.grp = h->pbd_grp.p; v.lvl = h->pbd_lvl.p; v.delay = h->pbd_delay.p; v.tet = h->pbd_tet.p;
         v.d0 = h->pbd_d0.p; v.d1 = h->pbd_d1.p; v.d2 = h->pbd_d2.p; v.px = h->dyn_px.p;
         if (h->pbd_smem > 0)
             CK(launch_pbd_sweeps_dsmem(s, v, h->pbd_codes.p, h->pbd_gnode.p, h->pbd_groups, h->pbd_smem, iterations,

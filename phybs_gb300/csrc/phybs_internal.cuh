@@ -418,9 +418,11 @@ cudaError_t launch_be_finish(cudaStream_t s, const DevMesh &m, const DevState &s
 
 // Strain-based PBD schedule: levels of mutually node-disjoint tets in the
 // caller's order; group g (an instance) sweeps levels grp[g] .. grp[g+1]-1,
-// level l holds tets lvl[l] .. lvl[l+1]-1 of the level-ordered copies.
+// level l holds tets lvl[l] .. lvl[l+1]-1 of the level-ordered copies.  delay:
+// one more than the largest level difference of two tets that share a node.
 struct PbdView {
     const int *grp, *lvl;
+    const int *delay;             // per group: a level's steps between two sweeps
     const int4 *tet;              // padded node ids
     const float4 *d0, *d1, *d2;   // rows of Dm^-1
     float4 *px;                   // positions; .w = inverse mass

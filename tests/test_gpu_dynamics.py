@@ -243,3 +243,43 @@ def test_pbd_handles_of_different_sizes_interleave():
     assert np.array_equal(a.positions(), x)
     a.close()
     b.close()
+
+
+def _soup(n_tets, n_nodes, seed):
+    """Tets of random corners: every pair may share a node, levels as they come."""
+    r = np.random.default_rng(seed)
+    x = r.uniform(0, 1, (n_nodes, 3)).astype(np.float32)
+    t = np.stack([r.permutation(n_nodes)[:4] for _ in range(n_tets)])
+    t = M.orient_positive(x, t)
+    keep = M.signed_volumes(x, t) > 1e-3
+    return M.TetMeshData(x, t[keep], np.array([0]), 1e5, 0.4)
+
+
+def _meshes():
+    box = M.box_mesh(9, 8, 13, edge=0.01, seed=2)
+    shuffled = M.TetMeshData(box.rest, np.random.default_rng(1).permutation(box.tets), box.pins, 1e5, 0.4)
+    # 6,000 disjoint tets: one level, far wider than the cluster's workers
+    r = np.random.default_rng(3).uniform(0, 1, (6000, 4, 3)) * 0.1 + np.arange(6000)[:, None, None]
+    r = r.astype(np.float32).reshape(-1, 3)
+    t = M.orient_positive(r, np.arange(24000).reshape(-1, 4))
+    apart = M.TetMeshData(r, t, np.array([0, 5]), 1e5, 0.4)
+    return {"box": box, "shuffled": shuffled, "apart": apart, "soup": _soup(60, 24, 5),
+            "four nodes": _soup(40, 4, 1)}
+
+
+@pytest.mark.parametrize("iterations", [1, 2, 7, 40])
+@pytest.mark.parametrize("name", ["box", "shuffled", "apart", "soup", "four nodes"])
+def test_pbd_overlapped_sweeps_bitwise(name, iterations):
+    """Several sweeps in flight, each a delay behind the one before: meshes
+    whose delay is small (box), nearly all levels (shuffled, soup) and one
+    (apart: a single level wider than the cluster's workers), with more sweeps
+    than are ever in flight, against the serial restatement."""
+    m = _meshes()[name]
+    x = (m.rest * np.float32(1.05)).astype(np.float32)
+    s = DescentSolver(m, positions=x)
+    dinv, w, grav = pbd_rest(m)
+    want, v = P.pbd_step(x, np.zeros_like(x), w, m.tets, dinv, grav, 1 / 60, iterations=iterations)
+    s.pbd_step(1 / 60, iterations=iterations)
+    assert np.array_equal(s.positions(), want, equal_nan=True)
+    assert np.array_equal(s.velocities()[0], v, equal_nan=True)
+    s.close()
