@@ -419,7 +419,7 @@ int pbs_stiffness_pattern(int n_nodes, int n_tets, const int *tets, int *nnz, in
  * Hessian, which the stretch-based material shares).  The reference uses
  * dt = 0.03, alpha = beta = 0.02.  K is assembled per 3x3 block row in a
  * fixed order (no atomics) and the system solved by block-Jacobi
- * preconditioned conjugate gradients from v, FP64 dot products, until
+ * preconditioned conjugate gradients from v, double-float dot products, until
  * |r| <= tol |b| (the reference: a cuSOLVER sparse Cholesky).  Returns
  * PBS_E_ITER_CAP (state advanced with the last iterate) when max_iters did
  * not reach tol, PBS_E_NONFINITE (state unchanged) on a non-finite residual;

@@ -47,19 +47,6 @@
 namespace pbs {
 
 // ------------------------------------------------------------ host: layout
-namespace {
-
-uint32_t spread10(uint32_t v) {  // 10 bits -> every third bit of 30
-    v &= 0x3ffu;
-    v = (v | (v << 16)) & 0x030000ffu;
-    v = (v | (v << 8)) & 0x0300f00fu;
-    v = (v | (v << 4)) & 0x030c30c3u;
-    v = (v | (v << 2)) & 0x09249249u;
-    return v;
-}
-
-}  // namespace
-
 void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<double> &rest, std::vector<InstCtl> &ctl,
                   const std::vector<ChunkLimits> &limits, ChunkLayout &out) {
     out = ChunkLayout();

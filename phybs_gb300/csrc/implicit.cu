@@ -19,8 +19,8 @@
 //     adds its incident (tet, corner) terms in the incidence order (ascending
 //     tet): no atomics, bit-reproducible;
 //   * block-Jacobi preconditioned conjugate gradients (3x3 diagonal blocks
-//     inverted in FP64), FP32 vectors as float4, FP64 dot products reduced in
-//     a fixed order; the solve stops on |r| <= tol |b|.
+//     inverted in FP64), FP32 vectors, one launch a solve (cg.cu); the solve
+//     stops on |r| <= tol |b|.
 #include <cuda_runtime.h>
 
 #include "../../include/phybs.h"
@@ -30,8 +30,6 @@
 namespace pbs {
 
 namespace {
-
-constexpr int kThreads = 256;
 
 __device__ __forceinline__ float4 f4(float x, float y, float z) { return make_float4(x, y, z, 0.f); }
 
@@ -162,170 +160,6 @@ __global__ void __launch_bounds__(128) k_be_assemble(DevMesh m, DevState st, Bsr
         for (int cl = 0; cl < 3; ++cl) dinv9[9 * (size_t)i + 3 * r + cl] = (float)(C[3 * cl + r] / det);
 }
 
-__device__ __forceinline__ float4 bsr_row_mul(const BsrView &A, int i, const float4 *p) {
-    float sx = 0.f, sy = 0.f, sz = 0.f;
-    if (A.scalar) {  // blocks a I3: one value a block
-        for (int k = A.ptr[i]; k < A.ptr[i + 1]; ++k) {
-            const float a = A.val[k];
-            const float4 v = p[A.col[k]];
-            sx += a * v.x;
-            sy += a * v.y;
-            sz += a * v.z;
-        }
-        return f4(sx, sy, sz);
-    }
-    for (int k = A.ptr[i]; k < A.ptr[i + 1]; ++k) {
-        const float *a = A.val + 9 * (size_t)k;
-        const float4 v = p[A.col[k]];
-        sx += a[0] * v.x + a[1] * v.y + a[2] * v.z;
-        sy += a[3] * v.x + a[4] * v.y + a[5] * v.z;
-        sz += a[6] * v.x + a[7] * v.y + a[8] * v.z;
-    }
-    return f4(sx, sy, sz);
-}
-
-__device__ __forceinline__ float4 block_apply(const float *D, const float4 &r) {
-    return f4(D[0] * r.x + D[1] * r.y + D[2] * r.z, D[3] * r.x + D[4] * r.y + D[5] * r.z,
-              D[6] * r.x + D[7] * r.y + D[8] * r.z);
-}
-
-__device__ __forceinline__ double dot4(const float4 &a, const float4 &b) {
-    return (double)a.x * b.x + (double)a.y * b.y + (double)a.z * b.z;
-}
-
-// Fixed-order block sums of up to three doubles into part[k * nblk + block].
-__device__ __forceinline__ void block_sums(double a0, double a1, double a2, int nv, double *part, int nblk) {
-    __shared__ double sh[3][kThreads / 32];
-    double v[3] = {a0, a1, a2};
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int k = 0; k < nv; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-        if (lane == 0) sh[k][w] = v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x < nv) {
-        double s = 0.0;
-        for (int j = 0; j < (int)(blockDim.x >> 5); ++j) s += sh[threadIdx.x][j];
-        part[threadIdx.x * nblk + blockIdx.x] = s;
-    }
-}
-
-// r = b - A x, z = D^-1 r, p = z; partial r.z, r.r and b.b (pnorm = 0) or
-// b.D^-1 b (pnorm = 1, the preconditioned norm)
-__global__ void __launch_bounds__(kThreads) k_cg_init(int Np, BsrView A, const float *dinv9, const float4 *b,
-                                                      const float4 *x, float4 *r, float4 *z, float4 *p,
-                                                      double *part, int pnorm) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double rz = 0.0, rr = 0.0, bb = 0.0;
-    if (i < Np) {
-        const float4 ax = bsr_row_mul(A, i, x), bi = b[i];
-        const float4 ri = f4(bi.x - ax.x, bi.y - ax.y, bi.z - ax.z);
-        const float4 zi = block_apply(dinv9 + 9 * (size_t)i, ri);
-        r[i] = ri;
-        z[i] = zi;
-        p[i] = zi;
-        rz = dot4(ri, zi);
-        rr = dot4(ri, ri);
-        bb = pnorm ? dot4(bi, block_apply(dinv9 + 9 * (size_t)i, bi)) : dot4(bi, bi);
-    }
-    block_sums(rz, rr, bb, 3, part, gridDim.x);
-}
-
-// q = A p; partial p.q
-__global__ void __launch_bounds__(kThreads) k_cg_spmv(int Np, BsrView A, const float4 *p, float4 *q, double *part,
-                                                      const CgState *cs) {
-    if (cs->done) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double pq = 0.0;
-    if (i < Np) {
-        const float4 qi = bsr_row_mul(A, i, p);
-        q[i] = qi;
-        pq = dot4(p[i], qi);
-    }
-    block_sums(pq, 0.0, 0.0, 1, part, gridDim.x);
-}
-
-// x += alpha p, r -= alpha q, z = D^-1 r; partial r.z, r.r
-__global__ void __launch_bounds__(kThreads) k_cg_update(int Np, const float *dinv9, const float4 *p, const float4 *q,
-                                                        float4 *x, float4 *r, float4 *z, double *part,
-                                                        const CgState *cs) {
-    if (cs->done) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double rz = 0.0, rr = 0.0;
-    if (i < Np) {
-        const float a = (float)cs->alpha;
-        const float4 pi = p[i], qi = q[i], xi = x[i], ri0 = r[i];
-        x[i] = f4(xi.x + a * pi.x, xi.y + a * pi.y, xi.z + a * pi.z);
-        const float4 ri = f4(ri0.x - a * qi.x, ri0.y - a * qi.y, ri0.z - a * qi.z);
-        const float4 zi = block_apply(dinv9 + 9 * (size_t)i, ri);
-        r[i] = ri;
-        z[i] = zi;
-        rz = dot4(ri, zi);
-        rr = dot4(ri, ri);
-    }
-    block_sums(rz, rr, 0.0, 2, part, gridDim.x);
-}
-
-// p = z + beta p
-__global__ void __launch_bounds__(kThreads) k_cg_direction(int Np, const float4 *z, float4 *p, const CgState *cs) {
-    if (cs->done) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Np) return;
-    const float bt = (float)cs->beta;
-    const float4 zi = z[i], pi = p[i];
-    p[i] = f4(zi.x + bt * pi.x, zi.y + bt * pi.y, zi.z + bt * pi.z);
-}
-
-// The scalars of one CG stage from the block partials, summed in block order
-// by one CTA.  stage 0: after init; 1: alpha = rz / pq; 2: beta, convergence
-// (|r|^2 <= tol2 |b|^2, or r.D^-1 r <= tol2 b.D^-1 b when pnorm).
-__global__ void __launch_bounds__(kThreads) k_cg_scalars(int nblk, const double *part, CgState *cs, int stage,
-                                                         double tol2, int max_iters, int pnorm) {
-    __shared__ double sh[3][kThreads / 32];
-    const int nv = stage == 1 ? 1 : (stage == 0 ? 3 : 2);
-    if (cs->done && stage != 0) return;
-    double v[3] = {0.0, 0.0, 0.0};
-    for (int k = 0; k < nv; ++k)
-        for (int j = threadIdx.x; j < nblk; j += blockDim.x) v[k] += part[k * nblk + j];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int k = 0; k < nv; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-        if (lane == 0) sh[k][w] = v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    double s[3] = {0.0, 0.0, 0.0};
-    for (int k = 0; k < nv; ++k)
-        for (int j = 0; j < (int)(blockDim.x >> 5); ++j) s[k] += sh[k][j];
-    CgState &c = *cs;
-    if (stage == 0) {
-        c.rz = s[0];
-        c.rr = s[1];
-        c.bb = s[2];
-        c.iters = 0;
-        c.status = PBS_OK;
-        c.done = 0;
-        if (!((pnorm ? s[0] : s[1]) <= tol2 * s[2])) {
-            if (!isfinite(s[1])) { c.status = PBS_E_NONFINITE; c.done = 1; }
-        } else {
-            c.done = 1;  // the initial guess already solves it
-        }
-    } else if (stage == 1) {
-        c.alpha = s[0] != 0.0 ? c.rz / s[0] : 0.0;
-        if (!isfinite(c.alpha) || s[0] <= 0.0) { c.status = PBS_E_NONFINITE; c.done = 1; }
-    } else {
-        c.iters += 1;
-        c.beta = c.rz != 0.0 ? s[0] / c.rz : 0.0;
-        c.rz = s[0];
-        c.rr = s[1];
-        if (!isfinite(s[1])) { c.status = PBS_E_NONFINITE; c.done = 1; }
-        else if ((pnorm ? s[0] : s[1]) <= tol2 * c.bb) c.done = 1;
-        else if (c.iters >= max_iters) { c.status = PBS_E_ITER_CAP; c.done = 1; }
-    }
-}
-
 // v_old <- v, v <- v', u += dt v' (compensated)
 __global__ void k_be_finish(DevMesh m, DevState st, const float4 *x, float dt) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -343,8 +177,6 @@ __global__ void k_be_finish(DevMesh m, DevState st, const float4 *x, float dt) {
 
 }  // namespace
 
-int cg_blocks(int Np) { return (Np + kThreads - 1) / kThreads; }
-
 cudaError_t launch_be_assemble(cudaStream_t s, const DevMesh &m, const DevState &st, int material, const BsrView &A,
                                float dt, float alpha, float beta, const float4 *ext, float4 *b, float4 *x,
                                float *dinv9) {
@@ -353,27 +185,6 @@ cudaError_t launch_be_assemble(cudaStream_t s, const DevMesh &m, const DevState 
         k_be_assemble<PBS_MATERIAL_STRETCH><<<g, 128, 0, s>>>(m, st, A, dt, alpha, beta, ext, b, x, dinv9);
     else
         k_be_assemble<PBS_MATERIAL_NEOHOOKEAN><<<g, 128, 0, s>>>(m, st, A, dt, alpha, beta, ext, b, x, dinv9);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_cg_init(cudaStream_t s, int Np, const BsrView &A, const float *dinv9, const float4 *b,
-                           const float4 *x, float4 *r, float4 *z, float4 *p, double *part, CgState *cs, double tol2,
-                           int pnorm) {
-    const int g = cg_blocks(Np);
-    k_cg_init<<<g, kThreads, 0, s>>>(Np, A, dinv9, b, x, r, z, p, part, pnorm);
-    k_cg_scalars<<<1, kThreads, 0, s>>>(g, part, cs, 0, tol2, 0, pnorm);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_cg_iteration(cudaStream_t s, int Np, const BsrView &A, const float *dinv9, float4 *x, float4 *r,
-                                float4 *z, float4 *p, float4 *q, double *part, CgState *cs, double tol2,
-                                int max_iters, int pnorm) {
-    const int g = cg_blocks(Np);
-    k_cg_spmv<<<g, kThreads, 0, s>>>(Np, A, p, q, part, cs);
-    k_cg_scalars<<<1, kThreads, 0, s>>>(g, part, cs, 1, tol2, max_iters, pnorm);
-    k_cg_update<<<g, kThreads, 0, s>>>(Np, dinv9, p, q, x, r, z, part, cs);
-    k_cg_scalars<<<1, kThreads, 0, s>>>(g, part, cs, 2, tol2, max_iters, pnorm);
-    k_cg_direction<<<g, kThreads, 0, s>>>(Np, z, p, cs);
     return cudaGetLastError();
 }
 

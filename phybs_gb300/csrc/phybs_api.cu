@@ -18,6 +18,7 @@ using namespace pbs;
 namespace {
 
 constexpr int CHUNK_PASSES = 16;  // passes per body of the step graph
+constexpr int CG_SOLVES = 64;     // solves of a step between two reads of their states
 
 template <typename T> struct DevBuf {
     T *p = nullptr;
@@ -90,21 +91,20 @@ struct pbs_handle {
     DevBuf<int> ring_pad, pick_id;
     DevBuf<float> pick_d2;
     DevBuf<float4> drag_ext;
-    // backward-Euler step: block-CSR pattern (built on first use), values,
-    // block-Jacobi inverses, CG vectors and reductions
+    // backward-Euler and projective-dynamics steps: block-CSR pattern and the
+    // solve's plan (built on first use), values, block-Jacobi inverses, CG
+    // vectors and exchanged words
     bool bsr_ready = false;
     DevBuf<int> bsr_ptr, bsr_col;
-    DevBuf<float> bsr_val, cg_dinv;
-    DevBuf<float4> cg_b, cg_x, cg_r, cg_z, cg_p, cg_q;
-    DevBuf<double> cg_part;
-    DevBuf<CgState> cg_state;
-    CgState *h_cg = nullptr;
-    // 16 CG iterations captured as one graph, for the system and stop rule of
-    // the key (rebuilt when they change)
-    cudaGraphExec_t cg_exec = nullptr;
-    const void *cg_key[3] = {nullptr, nullptr, nullptr};
-    double cg_key_tol2 = -1.0;
-    int cg_key_int[3] = {-1, -1, -1};
+    DevBuf<float> bsr_val, cg_dinv, cg_val;
+    DevBuf<float4> cg_b, cg_x, cg_xp, cg_red, cg_ws;
+    DevBuf<int> cg_plan;
+    DevBuf<unsigned char> cg_col;
+    CgPlanView cgp[2]{};        // of the two matrix kinds: nine values a block, one value
+    size_t cg_entries = 0, cg_rows_pad = 0, cg_halo = 0;
+    DevBuf<CgState> cg_state;   // of the solves of a step
+    DevBuf<unsigned> cg_ctl;    // [0] the last tag of the exchanged words, [1] a wait gave up
+    CgState *h_cg = nullptr;    // pinned, CG_SOLVES of them, and the two control words
     DevBuf<double2> tpart;
     DevBuf<double> npart;
     DevBuf<float> npartf;
@@ -127,7 +127,7 @@ struct pbs_handle {
     DevBuf<int4> pbd_codes, pbd_gnode;
     bool pd_ready = false;
     float pd_dtm = 0.f, pd_k = 0.f;
-    DevBuf<float> pd_val, pd_dinv;
+    DevBuf<float> pd_val, pd_dinv, pd_cgval;
     DevBuf<float4> dyn_px, dyn_x0, dyn_s;
     // host pinned
     int *h_active = nullptr;   // 2 slots: running counts of the host loop, or the bodies the loop ran
@@ -197,17 +197,16 @@ struct pbs_handle {
         tf.release(); hd.release(); staging.release(); staging2.release(); tpart.release(); npart.release(); npartf.release(); ctl.release(); ctl2.release(); tcount.release();
         fxh.release(); fxl.release(); fce.release(); fcr.release();
         faces_pad.release(); ring_pad.release(); pick_id.release(); pick_d2.release(); drag_ext.release();
-        bsr_ptr.release(); bsr_col.release(); bsr_val.release(); cg_dinv.release(); cg_part.release(); cg_state.release();
+        bsr_ptr.release(); bsr_col.release(); bsr_val.release(); cg_dinv.release(); cg_state.release();
+        cg_val.release(); cg_plan.release(); cg_col.release(); cg_ctl.release();
         pbd_grp.release(); pbd_lvl.release(); pbd_delay.release(); pbd_tet.release(); pbd_d0.release(); pbd_d1.release(); pbd_d2.release();
         pbd_node.release(); pbd_codes.release(); pbd_gnode.release();
-        pd_val.release(); pd_dinv.release(); dyn_px.release(); dyn_x0.release(); dyn_s.release();
+        pd_val.release(); pd_dinv.release(); pd_cgval.release(); dyn_px.release(); dyn_x0.release(); dyn_s.release();
         pbd_ready = pd_ready = false;
-        DevBuf<float4> *cv[] = {&cg_b, &cg_x, &cg_r, &cg_z, &cg_p, &cg_q};
+        DevBuf<float4> *cv[] = {&cg_b, &cg_x, &cg_xp, &cg_red, &cg_ws};
         for (auto b : cv) b->release();
         if (h_cg) cudaFreeHost(h_cg);
         h_cg = nullptr;
-        if (cg_exec) cudaGraphExecDestroy(cg_exec);
-        cg_exec = nullptr;
         bsr_ready = false;
         if (h_active) cudaFreeHost(h_active);
         if (h_ctl) cudaFreeHost(h_ctl);
@@ -1398,68 +1397,239 @@ int pbs_drag_face_ring(pbs_handle *h, int face, const float *drag, float *ext) {
     return download_user(h, h->drag_ext.p, ext);
 }
 
-// Block-CSR pattern of the padded mesh: per padded node, itself and every node
-// sharing a tet with it, ascending; plus the CG buffers.
+// Block-CSR pattern of the padded mesh (per padded node, itself and every node
+// sharing a tet with it, ascending) and the conjugate-gradient solve's plan:
+// real nodes in the Morton order of their rest positions, instance by
+// instance, split evenly over the CTAs; each CTA's halo (the other CTAs' nodes
+// that its rows multiply) and the rows of its own that are in others' halos.
 static int ensure_bsr(pbs_handle *h) {
     if (h->bsr_ready) return PBS_OK;
-    std::vector<std::vector<int>> nb(h->Np);
-    for (const int4 &q : h->h_tets_pad) {
-        if (q.x < 0) continue;
-        const int n[4] = {q.x, q.y, q.z, q.w};
-        for (int a = 0; a < 4; ++a)
-            for (int b = 0; b < 4; ++b) nb[n[a]].push_back(n[b]);
+    cudaStream_t s = h->stream;
+    const size_t np = (size_t)h->Np;
+    std::vector<int> ptr(np + 1, 0);
+    CK(h->bsr_ptr.alloc(np + 1));
+    CK(launch_bsr_count(s, h->mesh(), h->bsr_ptr.p + 1));
+    CK(cudaMemcpyAsync(ptr.data() + 1, h->bsr_ptr.p + 1, sizeof(int) * np, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    for (size_t i = 0; i < np; ++i) ptr[i + 1] += ptr[i];
+    const size_t nnzb = (size_t)ptr[np];
+    std::vector<int> col(nnzb);
+    CK(h->bsr_col.alloc(nnzb));
+    CK(cudaMemcpyAsync(h->bsr_ptr.p, ptr.data(), sizeof(int) * (np + 1), cudaMemcpyHostToDevice, s));
+    CK(launch_bsr_fill(s, h->mesh(), h->bsr_ptr.p, h->bsr_col.p));
+    CK(cudaMemcpyAsync(col.data(), h->bsr_col.p, sizeof(int) * nnzb, cudaMemcpyDeviceToHost, s));
+    // rows: (instance, Morton code) order, on the host meanwhile
+    std::vector<std::pair<uint64_t, int>> order;
+    order.reserve(h->N);
+    for (int b = 0; b < h->B; ++b) {
+        const int n0 = h->h_inst_nodes[2 * b], n1 = h->h_inst_nodes[2 * b + 1];
+        double lo[3], inv[3];
+        for (int d = 0; d < 3; ++d) {
+            double mn = 1e300, mx = -1e300;
+            for (int i = n0; i < n1; ++i) {
+                mn = std::min(mn, h->h_rest_pad[3 * (size_t)i + d]);
+                mx = std::max(mx, h->h_rest_pad[3 * (size_t)i + d]);
+            }
+            lo[d] = mn;
+            inv[d] = mx > mn ? 1023.0 / (mx - mn) : 0.0;
+        }
+        for (int i = n0; i < n1; ++i) {
+            uint32_t code = 0;
+            for (int d = 0; d < 3; ++d)
+                code |= spread10((uint32_t)((h->h_rest_pad[3 * (size_t)i + d] - lo[d]) * inv[d])) << d;
+            order.emplace_back(((uint64_t)b << 32) | code, i);
+        }
     }
-    std::vector<int> ptr(h->Np + 1, 0), col;
-    for (int i = 0; i < h->Np; ++i) {
-        auto &v = nb[i];
-        v.push_back(i);
-        std::sort(v.begin(), v.end());
-        v.erase(std::unique(v.begin(), v.end()), v.end());
-        col.insert(col.end(), v.begin(), v.end());
-        ptr[i + 1] = (int)col.size();
-        std::vector<int>().swap(v);
+    std::sort(order.begin(), order.end());
+    CK(cudaStreamSynchronize(s));
+    const int n = (int)order.size();
+    // one CTA a SM, but no fewer than CG_MIN_ROWS rows each: more CTAs shorten
+    // the row loops, fewer the sums every CTA waits for
+    const int G = std::max(1, std::min(h->sms, (n + CG_MIN_ROWS - 1) / CG_MIN_ROWS));
+    std::vector<int> cta_slice(G + 1, 0), cta_rows(G), cta_halo(G + 1, 0), cta_send(G + 1, 0);
+    std::vector<int> srow, rlen, soff(1, 0), soff_local, halo, send;
+    std::vector<int> place_of(np, -1), owner(np, -1), stamp(np, -1), lidx(np, 0), key;
+    std::vector<char> sent(np, 0);
+    auto row_len = [&](int i) { return ptr[i + 1] - ptr[i]; };
+    // each CTA's rows, longest first, then by node: a slice's rows end together,
+    // and on a mesh with rows of a few lengths in turn (a 5-tet box) a warp's
+    // rows multiply runs of neighbouring words
+    for (int c = 0; c < G; ++c) {
+        const int a = (int)((int64_t)n * c / G), e = (int)((int64_t)n * (c + 1) / G), nr = e - a;
+        std::sort(order.begin() + a, order.begin() + e, [&](const auto &x, const auto &y) {
+            const int lx = row_len(x.second), ly = row_len(y.second);
+            return lx != ly ? lx > ly : x.second < y.second;
+        });
+        for (int r0 = 0; r0 < nr; r0 += 32)
+            for (int l = 0; l < 32; ++l) {
+                const int i = r0 + l < nr ? order[a + r0 + l].second : -1;
+                if (i >= 0) {
+                    place_of[i] = (int)srow.size();
+                    owner[i] = c;
+                }
+                srow.push_back(i);
+                rlen.push_back(i < 0 ? 0 : row_len(i));
+            }
+        cta_rows[c] = nr;
+        cta_slice[c + 1] = (int)srow.size() / 32;
     }
-    const size_t nnzb = col.size(), np = (size_t)h->Np;
-    const int g = cg_blocks(h->Np);
-    CK(h->bsr_ptr.alloc(np + 1)); CK(h->bsr_col.alloc(nnzb)); CK(h->bsr_val.alloc(9 * nnzb));
-    CK(h->cg_dinv.alloc(9 * np)); CK(h->cg_part.alloc(3 * (size_t)g)); CK(h->cg_state.alloc(1));
-    DevBuf<float4> *cv[] = {&h->cg_b, &h->cg_x, &h->cg_r, &h->cg_z, &h->cg_p, &h->cg_q};
-    for (auto b : cv) CK(b->alloc(np));
-    if (!h->h_cg) CK(cudaMallocHost(&h->h_cg, sizeof(CgState)));
-    CK(cudaMemcpyAsync(h->bsr_ptr.p, ptr.data(), sizeof(int) * (np + 1), cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->bsr_col.p, col.data(), sizeof(int) * nnzb, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    // the halos, in the order of the words (the places of their rows)
+    std::vector<int> lcol;  // by entry and lane
+    int max_rows = 0, max_local = 0, max_halo = 0, max_entries = 0;
+    for (int c = 0; c < G; ++c) {
+        const int s0 = cta_slice[c], s1 = cta_slice[c + 1], nr = cta_rows[c], entry0 = soff.back();
+        key.clear();
+        for (int lr = 0; lr < nr; ++lr) {
+            const int i = srow[32 * (size_t)s0 + lr];
+            lidx[i] = lr;
+            for (int k = ptr[i]; k < ptr[i + 1]; ++k) {
+                const int j = col[k];
+                if (owner[j] == c || stamp[j] == c) continue;
+                stamp[j] = c;
+                sent[j] = 1;
+                key.push_back(place_of[j]);
+            }
+        }
+        std::sort(key.begin(), key.end());
+        const int nh = (int)key.size();
+        for (int j = 0; j < nh; ++j) lidx[srow[key[j]]] = nr + j;
+        halo.insert(halo.end(), key.begin(), key.end());
+        for (int sl = s0; sl < s1; ++sl) {
+            const int e0 = soff.back(), len = rlen[32 * (size_t)sl];
+            soff_local.push_back(e0 - entry0);
+            soff.push_back(e0 + len);
+            lcol.resize((size_t)(e0 + len) * 32, 0);
+            for (int l = 0; l < 32; ++l) {
+                const int i = srow[32 * (size_t)sl + l], m = rlen[32 * (size_t)sl + l];
+                for (int k = 0; k < m; ++k) lcol[(size_t)(e0 + k) * 32 + l] = lidx[col[ptr[i] + k]];
+            }
+        }
+        cta_halo[c + 1] = cta_halo[c] + nh;
+        max_rows = std::max(max_rows, nr);
+        max_local = std::max(max_local, nr + nh);
+        max_halo = std::max(max_halo, nh);
+        max_entries = std::max(max_entries, soff.back() - entry0);
+    }
+    // the local rows whose words other CTAs read
+    int max_send = 0;
+    for (int c = 0; c < G; ++c) {
+        const size_t base = 32 * (size_t)cta_slice[c];
+        for (int lr = 0; lr < cta_rows[c]; ++lr)
+            if (sent[srow[base + lr]]) send.push_back(lr);
+        cta_send[c + 1] = (int)send.size();
+        max_send = std::max(max_send, cta_send[c + 1] - cta_send[c]);
+    }
+    const int ns = (int)soff.size() - 1;
+    // one allocation for the plan's index arrays
+    struct Part {
+        const std::vector<int> *v;
+        size_t at;
+    } part[] = {{&cta_slice, 0}, {&cta_rows, 0}, {&cta_halo, 0}, {&srow, 0}, {&rlen, 0}, {&soff, 0}, {&soff_local, 0},
+                {&halo, 0}, {&cta_send, 0}, {&send, 0}};
+    size_t total = 0;
+    for (auto &p : part) {
+        p.at = total;
+        total += (p.v->size() + 31) / 32 * 32;  // (16-byte copies of srow and rlen)
+    }
+    CK(h->cg_plan.alloc(total));
+    for (auto &p : part)
+        CK(cudaMemcpyAsync(h->cg_plan.p + p.at, p.v->data(), sizeof(int) * p.v->size(), cudaMemcpyHostToDevice, s));
+    const bool col32 = max_local > 0xffff;
+    std::vector<uint16_t> lcol16;
+    if (!col32) lcol16.assign(lcol.begin(), lcol.end());
+    const void *src = col32 ? (const void *)lcol.data() : (const void *)lcol16.data();
+    const size_t cbytes = lcol.size() * (col32 ? 4 : 2);
+    CK(h->cg_col.alloc(cbytes));
+    CK(cudaMemcpyAsync(h->cg_col.p, src, cbytes, cudaMemcpyHostToDevice, s));
+    CgPlanView v{};
+    v.grid = G;
+    v.threads = max_rows > 256 ? 512 : 256;
+    v.n_slices = ns;
+    const int *base = h->cg_plan.p;
+    v.cta_slice = base + part[0].at; v.cta_rows = base + part[1].at; v.cta_halo = base + part[2].at;
+    v.srow = base + part[3].at; v.rlen = base + part[4].at; v.soff = base + part[5].at;
+    v.soff_local = base + part[6].at; v.halo = base + part[7].at;
+    v.cta_send = base + part[8].at; v.send = base + part[9].at;
+    v.scol = h->cg_col.p;
+    v.col32 = col32;
+    for (int kind = 0; kind < 2; ++kind) {
+        // what fits shared memory, the most often read first
+        CgPlanView &w = h->cgp[kind];
+        w = v;
+        w.smem = 0;
+        auto place = [&](size_t bytes) {
+            bytes = (bytes + 127) / 128 * 128;
+            if (w.smem + bytes > (size_t)CG_MAX_SMEM) return -1;
+            const int at = w.smem;
+            w.smem += (int)bytes;
+            return at;
+        };
+        const size_t pad = 128 * (size_t)((max_rows + 31) / 32), nv = kind == 0 ? 9 : 1;  // 4 B a row, padded
+        w.off_node = place(pad);
+        w.off_rlen = place(pad);
+        w.off_small = place(sizeof(int) * ((max_rows + 31) / 32 + (size_t)max_halo + max_send));
+        w.off_p = place(sizeof(float4) * max_local);
+        w.off_q = place(sizeof(float4) * max_rows);
+        w.off_r = place(sizeof(float4) * max_rows);
+        w.off_val = w.off_col = -1;
+        const size_t vb = (size_t)max_entries * 128 * nv, cb = (size_t)max_entries * 32 * (col32 ? 4 : 2);
+        if (w.smem + vb + cb + 256 <= (size_t)CG_MAX_SMEM) {
+            w.off_val = place(vb);
+            w.off_col = place(cb);
+        }
+        w.off_dinv = place(pad * nv);
+        w.off_x = place(sizeof(float4) * max_rows);
+    }
+    h->cg_entries = (size_t)soff.back();
+    h->cg_rows_pad = 32 * (size_t)ns;
+    h->cg_halo = (size_t)cta_halo[G];
+    CK(h->bsr_val.alloc(9 * nnzb)); CK(h->cg_dinv.alloc(9 * np));
+    CK(h->cg_b.alloc(np)); CK(h->cg_x.alloc(np)); CK(h->cg_xp.alloc(h->cg_rows_pad));
+    CK(h->cg_red.alloc(2 * 3 * (size_t)CG_COPIES * G));
+    CK(h->cg_ws.alloc(4 * h->cg_rows_pad + h->cg_halo));
+    CK(h->cg_state.alloc(CG_SOLVES)); CK(h->cg_ctl.alloc(2));
+    CK(cudaMemsetAsync(h->cg_xp.p, 0, sizeof(float4) * h->cg_xp.n, s));
+    CK(cudaMemsetAsync(h->cg_red.p, 0, sizeof(float4) * h->cg_red.n, s));
+    CK(cudaMemsetAsync(h->cg_ctl.p, 0, 2 * sizeof(unsigned), s));
+    if (!h->h_cg) CK(cudaMallocHost(&h->h_cg, sizeof(CgState) * CG_SOLVES + 2 * sizeof(unsigned)));
+    CK(cudaStreamSynchronize(s));
     h->bsr_ready = true;
     return PBS_OK;
 }
 
-// Launches 16 CG iterations on A x = b (state in cg_state) as one graph; the
-// kernels of a finished solve return at once, so a group may overrun the cap.
-static int cg_group(pbs_handle *h, const BsrView &A, const float *dinv9, float4 *x, double tol2, int max_iters,
-                    int pnorm) {
-    const void *key[3] = {A.val, dinv9, x};
-    const int ki[3] = {max_iters, pnorm, A.scalar};
-    bool same = h->cg_exec && h->cg_key_tol2 == tol2;
-    for (int k = 0; k < 3; ++k) same = same && key[k] == h->cg_key[k] && ki[k] == h->cg_key_int[k];
-    if (!same) {
-        if (h->cg_exec) cudaGraphExecDestroy(h->cg_exec);
-        h->cg_exec = nullptr;
-        cudaStream_t s = h->stream;
-        CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e = cudaSuccess;
-        for (int k = 0; k < 16 && e == cudaSuccess; ++k)
-            e = launch_cg_iteration(s, h->Np, A, dinv9, x, h->cg_r.p, h->cg_z.p, h->cg_p.p, h->cg_q.p, h->cg_part.p,
-                                    h->cg_state.p, tol2, max_iters, pnorm);
-        cudaGraph_t g = nullptr;
-        const cudaError_t e2 = cudaStreamEndCapture(s, &g);
-        if (e == cudaSuccess) e = e2;
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&h->cg_exec, g, 0);
-        if (g) cudaGraphDestroy(g);
-        CK(e);
-        for (int k = 0; k < 3; ++k) { h->cg_key[k] = key[k]; h->cg_key_int[k] = ki[k]; }
-        h->cg_key_tol2 = tol2;
+// Enqueues one solve A x = b (slot: where its state goes).
+static cudaError_t enqueue_solve(pbs_handle *h, bool scalar, const float *val, const float *dinv, double tol2,
+                                 int max_iters, int pnorm, int slot) {
+    CgArgs a{};
+    a.val = val;
+    a.dinv = dinv;
+    a.b = h->cg_b.p; a.x = h->cg_x.p; a.xp = h->cg_xp.p; a.red = h->cg_red.p;
+    a.ws_p = h->cg_ws.p;
+    a.ws_r = a.ws_p + h->cg_rows_pad + h->cg_halo;
+    a.ws_q = a.ws_r + h->cg_rows_pad;
+    a.ws_x = a.ws_q + h->cg_rows_pad;
+    a.cs = h->cg_state.p + slot;
+    a.tag = h->cg_ctl.p;
+    a.err = (int *)(h->cg_ctl.p + 1);
+    a.tol2 = tol2;
+    a.max_iters = max_iters;
+    a.pnorm = pnorm;
+    return launch_cg_solve(h->stream, h->cgp[scalar ? 1 : 0], a, scalar);
+}
+
+// The states of the last `count` solves on the host, and the exchanged words'
+// tags kept from wrapping (or, after a wait that gave up, made clean again).
+static int read_solves(pbs_handle *h, int count) {
+    cudaStream_t s = h->stream;
+    unsigned *ctl = (unsigned *)(h->h_cg + CG_SOLVES);
+    CK(cudaMemcpyAsync(h->h_cg, h->cg_state.p, sizeof(CgState) * count, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(ctl, h->cg_ctl.p, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    if (ctl[0] > 0x40000000u || ctl[1]) {
+        CK(cudaMemsetAsync(h->cg_xp.p, 0, sizeof(float4) * h->cg_xp.n, s));
+        CK(cudaMemsetAsync(h->cg_red.p, 0, sizeof(float4) * h->cg_red.n, s));
+        CK(cudaMemsetAsync(h->cg_ctl.p, 0, 2 * sizeof(unsigned), s));
     }
-    CK(cudaGraphLaunch(h->cg_exec, h->stream));
     return PBS_OK;
 }
 
@@ -1482,27 +1652,23 @@ int pbs_backward_euler_step(pbs_handle *h, float dt, float alpha, float beta, co
     A.col = h->bsr_col.p;
     A.val = h->bsr_val.p;
     const double tol2 = (double)tol * (double)tol;
+    if (!h->cg_val.p) CK(h->cg_val.alloc(9 * (32 * h->cg_entries + h->cg_rows_pad)));
+    float *cgd = h->cg_val.p + 9 * 32 * h->cg_entries;  // the inverses by row
     CK(launch_be_assemble(s, m, st, h->material, A, dt, alpha, beta, ext ? h->ext.p : nullptr, h->cg_b.p, h->cg_x.p,
                           h->cg_dinv.p));
-    CK(launch_cg_init(s, h->Np, A, h->cg_dinv.p, h->cg_b.p, h->cg_x.p, h->cg_r.p, h->cg_z.p, h->cg_p.p,
-                      h->cg_part.p, h->cg_state.p, tol2));
-    // iterations in groups of 16; every kernel of a finished solve returns at
-    // once, and the host reads the state once per group
-    for (int it = 0; it < max_iters; it += 16) {
-        rc = cg_group(h, A, h->cg_dinv.p, h->cg_x.p, tol2, max_iters, 0);
-        if (rc != PBS_OK) return rc;
-        CK(cudaMemcpyAsync(h->h_cg, h->cg_state.p, sizeof(CgState), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        if (h->h_cg->done) break;
-    }
-    const CgState c = *h->h_cg;
+    CK(launch_cg_pack(s, h->cgp[0], A, h->cg_dinv.p, h->cg_val.p, cgd));
+    CK(enqueue_solve(h, false, h->cg_val.p, cgd, tol2, max_iters, 0, 0));
+    rc = read_solves(h, 1);
+    if (rc != PBS_OK) return rc;
+    const CgState c = h->h_cg[0];
     if (iters_out) *iters_out = c.iters;
     if (residual_out) *residual_out = c.bb > 0.0 ? std::sqrt(c.rr / c.bb) : 0.0;
-    if (c.status == PBS_E_NONFINITE) return PBS_E_NONFINITE;  // the state is left as it was
+    // the state is left as it was
+    if (c.status == PBS_E_NONFINITE || c.status == PBS_E_DEVICE_TIMEOUT) return c.status;
     CK(launch_be_finish(s, m, st, h->cg_x.p, dt));
     CK(cudaStreamSynchronize(s));
     h->guess_pending = false;
-    return c.done ? c.status : PBS_E_ITER_CAP;
+    return c.status;
 }
 
 // ---- strain-based PBD and projective dynamics
@@ -1664,11 +1830,13 @@ int pbs_pd_step(pbs_handle *h, float dt, float dt_matrix, float stiffness, int i
         int nnzb = 0;
         CK(cudaMemcpy(&nnzb, h->bsr_ptr.p + h->Np, sizeof(int), cudaMemcpyDeviceToHost));
         CK(h->pd_val.alloc((size_t)nnzb));
+        CK(h->pd_cgval.alloc(32 * h->cg_entries + h->cg_rows_pad));
         CK(h->pd_dinv.alloc(9 * (size_t)h->Np));
     }
     A.val = h->pd_val.p;
     if (!h->pd_ready || h->pd_dtm != dtm || h->pd_k != stiffness) {
         CK(launch_pd_assemble(s, m, A, dtm, stiffness, h->pd_dinv.p));
+        CK(launch_cg_pack(s, h->cgp[1], A, h->pd_dinv.p, h->pd_cgval.p, h->pd_cgval.p + 32 * h->cg_entries));
         h->pd_ready = true;
         h->pd_dtm = dtm;
         h->pd_k = stiffness;
@@ -1676,26 +1844,28 @@ int pbs_pd_step(pbs_handle *h, float dt, float dt_matrix, float stiffness, int i
     CK(launch_pd_begin(s, m, st, ext ? h->ext.p : nullptr, dt, h->dyn_s.p, h->dyn_px.p, h->dyn_x0.p));
     const double tol2 = (double)tol * (double)tol;
     int total = 0, status = PBS_OK;
-    for (int it = 0; it < iterations; ++it) {
-        CK(launch_pd_residual(s, m, h->dyn_px.p, stiffness, dt, dtm, reinterpret_cast<float4 *>(h->tf.p),
-                              h->dyn_s.p, h->dyn_x0.p, h->cg_b.p, h->cg_x.p));
-        CK(launch_cg_init(s, h->Np, A, h->pd_dinv.p, h->cg_b.p, h->cg_x.p, h->cg_r.p, h->cg_z.p, h->cg_p.p,
-                          h->cg_part.p, h->cg_state.p, tol2, 1));
-        for (int k0 = 0; k0 < max_cg; k0 += 16) {
-            rc = cg_group(h, A, h->pd_dinv.p, h->cg_x.p, tol2, max_cg, 1);
-            if (rc != PBS_OK) return rc;
-            CK(cudaMemcpyAsync(h->h_cg, h->cg_state.p, sizeof(CgState), cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
-            if (h->h_cg->done) break;
+    // the solves follow one another on the stream; their states are read once
+    // (a solve that ends non-finite leaves the rest nothing to do, and the
+    // handle's state is only written after the last)
+    for (int it = 0; it < iterations; it += CG_SOLVES) {
+        const int count = std::min(CG_SOLVES, iterations - it);
+        for (int k = 0; k < count; ++k) {
+            CK(launch_pd_residual(s, m, h->dyn_px.p, stiffness, dt, dtm, reinterpret_cast<float4 *>(h->tf.p),
+                                  h->dyn_s.p, h->dyn_x0.p, h->cg_b.p, h->cg_x.p));
+            CK(enqueue_solve(h, true, h->pd_cgval.p, h->pd_cgval.p + 32 * h->cg_entries, tol2, max_cg, 1, k));
+            CK(launch_pd_apply(s, h->Np, h->dyn_px.p, h->cg_x.p));
         }
-        const CgState c = *h->h_cg;
-        total += c.iters;
-        if (c.status == PBS_E_NONFINITE) {
-            if (cg_iters_out) *cg_iters_out = total;
-            return PBS_E_NONFINITE;  // the state is left as it was
+        rc = read_solves(h, count);
+        if (rc != PBS_OK) return rc;
+        for (int k = 0; k < count; ++k) {
+            const CgState &c = h->h_cg[k];
+            total += c.iters;
+            if (c.status == PBS_E_NONFINITE || c.status == PBS_E_DEVICE_TIMEOUT) {
+                if (cg_iters_out) *cg_iters_out = total;
+                return c.status;  // the state is left as it was
+            }
+            if (c.status == PBS_E_ITER_CAP) status = PBS_E_ITER_CAP;
         }
-        if (!c.done || c.status == PBS_E_ITER_CAP) status = PBS_E_ITER_CAP;
-        CK(launch_pd_apply(s, h->Np, h->dyn_px.p, h->cg_x.p));
     }
     CK(launch_dyn_end(s, m, st, h->dyn_px.p, h->dyn_x0.p, dt, 1));
     CK(cudaStreamSynchronize(s));

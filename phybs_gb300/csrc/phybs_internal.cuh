@@ -222,6 +222,16 @@ __device__ __forceinline__ int node_ctl_ws(const DevMesh &m, const DevState &st,
     return st.ctl[m.nblk_inst[i / BLOCK]].ws_used;
 }
 
+// 10 bits -> every third bit of 30 (Morton codes).
+inline uint32_t spread10(uint32_t v) {
+    v &= 0x3ffu;
+    v = (v | (v << 16)) & 0x030000ffu;
+    v = (v | (v << 8)) & 0x0300f00fu;
+    v = (v | (v << 4)) & 0x030c30c3u;
+    v = (v | (v << 2)) & 0x09249249u;
+    return v;
+}
+
 // Host: the pass layout of a packed mesh (chunks.cu).  tets: padded corner ids
 // (-1 rows are padding); rest: padded rest positions (3 per node); ctl: the
 // instances' node / tet ranges, whose cblk ranges are filled in.
@@ -398,22 +408,50 @@ struct BsrView {
     int scalar = 0;
 };
 struct CgState {
-    double rz, rr, bb, alpha, beta;
-    int iters, status, done, pad;
+    double rz, rr, bb;
+    int iters, status;
 };
-int cg_blocks(int Np);
+// The conjugate-gradient solve (cg.cu): rows of the matrix by CTA, in slices
+// of 32 (a CTA's last one padded with rows -1).
+struct CgPlanView {
+    int grid, threads, smem;  // CTAs, threads and dynamic shared memory of a CTA
+    int n_slices;
+    const int *cta_slice, *cta_rows, *cta_halo, *cta_send;  // grid + 1 (rows: grid)
+    const int *srow, *rlen;    // 32 a slice: padded node (-1: none), row length
+    const int *soff, *soff_local;  // a slice's first entry, overall (n_slices + 1) and from its CTA's first
+    const int *halo;           // places in srow, ascending
+    const int *send;           // local rows that other CTAs' halos hold
+    const void *scol;          // columns by entry and lane: own rows, then the halo (16 bits, or 32 with col32)
+    bool col32;
+    // byte offsets into the CTA's shared memory, -1: in global memory
+    int off_p, off_r, off_q, off_x, off_val, off_col, off_node, off_rlen, off_small, off_dinv;
+};
+constexpr int CG_MIN_ROWS = 128;
+constexpr int CG_MAX_SMEM = 225 * 1024;
+constexpr int CG_COPIES = 8;  // places a CTA writes its share of a sum to
+struct CgArgs {
+    const float *val, *dinv;  // by entry, and the diagonal blocks' inverses by row (launch_cg_pack)
+    const float4 *b;
+    float4 *x;           // initial guess in, solution out
+    float4 *xp;          // direction words by place in srow
+    float4 *red;         // words of the sums: 2 x 3 x CG_COPIES x grid
+    float4 *ws_p, *ws_r, *ws_q, *ws_x;  // workspace of what does not fit shared memory
+    CgState *cs;
+    unsigned *tag;       // the last tag used, carried from launch to launch
+    int *err;            // a wait gave up
+    double tol2;
+    int max_iters;
+    int pnorm;  // stop on r.D^-1 r <= tol2 b.D^-1 b instead of |r|^2 <= tol2 |b|^2 (rows of very
+                // different scale, e.g. pinned nodes' 1e8 masses)
+};
+cudaError_t launch_bsr_count(cudaStream_t s, const DevMesh &m, int *cnt);
+cudaError_t launch_bsr_fill(cudaStream_t s, const DevMesh &m, const int *ptr, int *col);
+cudaError_t launch_cg_pack(cudaStream_t s, const CgPlanView &pl, const BsrView &A, const float *dinv9, float *out,
+                           float *dinv);
+cudaError_t launch_cg_solve(cudaStream_t s, const CgPlanView &pl, const CgArgs &a, bool scalar);
 cudaError_t launch_be_assemble(cudaStream_t s, const DevMesh &m, const DevState &st, int material, const BsrView &A,
                                float dt, float alpha, float beta, const float4 *ext, float4 *b, float4 *x,
                                float *dinv9);
-// pnorm: stop on the preconditioned norm r.D^-1 r <= tol2 b.D^-1 b instead
-// of |r|^2 <= tol2 |b|^2 (rows of very different scale, e.g. pinned nodes'
-// 1e8 masses)
-cudaError_t launch_cg_init(cudaStream_t s, int Np, const BsrView &A, const float *dinv9, const float4 *b,
-                           const float4 *x, float4 *r, float4 *z, float4 *p, double *part, CgState *cs, double tol2,
-                           int pnorm = 0);
-cudaError_t launch_cg_iteration(cudaStream_t s, int Np, const BsrView &A, const float *dinv9, float4 *x, float4 *r,
-                                float4 *z, float4 *p, float4 *q, double *part, CgState *cs, double tol2,
-                                int max_iters, int pnorm = 0);
 cudaError_t launch_be_finish(cudaStream_t s, const DevMesh &m, const DevState &st, const float4 *x, float dt);
 
 // Strain-based PBD schedule: levels of mutually node-disjoint tets in the

@@ -89,3 +89,54 @@ def test_bitwise_reproducible_and_iteration_cap():
     with pytest.raises(L.PhybsError):
         s.backward_euler_step(dt=-1.0)
     s.close()
+
+
+# rows about the slice and CTA lines: 4 nodes; 12; 32 rows to a slice; 126,
+# 128, 135 (a second CTA); 3,000 over two dozen CTAs; rows of 27 columns
+# (6-tet split) and of 7 and 19 in turn (5-tet)
+GRIDS = [(5, 1, 1, 1), (5, 1, 1, 2), (5, 1, 3, 3), (6, 2, 5, 6), (5, 3, 3, 7), (6, 2, 4, 8), (5, 9, 14, 19)]
+
+
+def _moving(split, nx, ny, nz):
+    """A twisted mesh held at its untwisted end, and its velocities: states
+    whose matrix is positive definite (checked on the CPU for the small ones)."""
+    if split == 6:
+        m, axis = M.bar_mesh(nx, ny, nz, edge=0.03, young=5e4, poisson=0.4), 0
+    else:
+        m, axis = M.box_mesh(nx, ny, nz, edge=0.03, young=5e4, poisson=0.4, pin="bottom"), 2
+    x0 = M.twist_positions(m.rest, 0.15, axis=axis)
+    v0 = (0.1 * np.sin(20 * m.rest[:, [1, 2, 0]])).astype(np.float32)
+    v0[m.pins] = 0.0
+    return m, x0, v0
+
+
+@pytest.mark.parametrize("split,nx,ny,nz", GRIDS)
+def test_solve_sizes_match_restatement(split, nx, ny, nz):
+    """One backward-Euler step of meshes of every row count near the solve's
+    lines, twisted and moving, against the FP64 restatement."""
+    m, x0, v0 = _moving(split, nx, ny, nz)
+    mu, lam = O.lame(m.young, m.poisson)
+    s = DescentSolver(m, positions=x0, mu=mu, lam=lam)
+    s.write_velocities(v0, v0)
+    xo, vo, _, _ = I.backward_euler_step(s.positions(), v0, m.rest, m.tets, m.pin_mask(), mu, lam)
+    it, res = s.backward_euler_step(tol=1e-6)
+    assert res <= 1e-6
+    assert np.abs(s.positions() - xo).max() / m.bbox_diagonal() < POS_TOL
+    assert np.abs(s.velocities()[0] - vo).max() <= 1e-3 * np.abs(vo).max()
+    s.close()
+
+
+@pytest.mark.parametrize("scale", [1e-4, 1e3])
+def test_solve_scales(scale):
+    """The same bar a ten-thousandth and a thousand times its size (masses and
+    residuals by the cube): the sums' scaling keeps the solve's tolerance."""
+    m = M.bar_mesh(6, 3, 3, edge=0.025 * scale, young=5e4, poisson=0.4)
+    x0 = M.twist_positions(m.rest, 0.4, axis=0)
+    x0[m.pins] = m.rest[m.pins]
+    mu, lam = O.lame(m.young, m.poisson)
+    s = DescentSolver(m, positions=x0, mu=mu, lam=lam)
+    xo, vo, _, _ = I.backward_euler_step(s.positions(), np.zeros_like(x0), m.rest, m.tets, m.pin_mask(), mu, lam)
+    it, res = s.backward_euler_step(tol=1e-6)
+    assert res <= 1e-6 and it > 0
+    assert np.abs(s.positions() - xo).max() / m.bbox_diagonal() < POS_TOL
+    s.close()
