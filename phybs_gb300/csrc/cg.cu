@@ -13,8 +13,9 @@
 // multiply (the halo), its residual, q and x, and its share of the matrix.
 // An iteration exchanges words through L2 (exchange.cuh):
 //   p     each row's direction, read by the CTAs whose halo it is in;
-//   p.q   and  r.z (r.r)   one word a sum and CTA, read by every CTA, which
-//         adds them in the same order and so takes the same decisions.
+//   p.q   and  r.z (r.r)   one word a sum and CTA, {hi, lo, check, tag}, read
+//         by every CTA, which adds them in the same order and so takes the
+//         same decisions.
 // A direction word is overwritten after a sum that its readers contribute to
 // once they have read it.  The words of two sums in a row alternate between
 // two buffers: a CTA writes a buffer again after the sum between, which every
@@ -152,8 +153,8 @@ __device__ __forceinline__ bool all_reduce(DFloat (&v)[K], Reduce &sh, const CgA
 #pragma unroll
             for (int o = kMaxWarps / 2; o > 0; o >>= 1) x = step(x, o);
             x = DFloat{__shfl_sync(full, x.hi, 0), __shfl_sync(full, x.lo, 0)};
-            if (lane < CG_COPIES)
-                st_word(words + ((size_t)k * CG_COPIES + lane) * G + c, make_float3(x.hi, x.lo, 0.f), tag);
+            const unsigned hi = __float_as_uint(x.hi), lo = __float_as_uint(x.lo);
+            if (lane < CG_COPIES) st_word(words + ((size_t)k * CG_COPIES + lane) * G + c, hi, lo, hi ^ lo ^ tag, tag);
         }
         DFloat acc[K];
 #pragma unroll
@@ -167,14 +168,18 @@ __device__ __forceinline__ bool all_reduce(DFloat (&v)[K], Reduce &sh, const CgA
 #pragma unroll
                 for (int k = 0; k < K; ++k)
                     x[u][k] = j0 + 32 * u < G ? ld_word(red + (size_t)k * CG_COPIES * G + j0 + 32 * u)
-                                              : make_uint4(0u, 0u, 0u, tag);
+                                              : make_uint4(0u, 0u, tag, tag);
+            // (the check word ties the value to its tag: a sum that used a part
+            // of the words only was compiled into narrower loads, and a maximum
+            // paired a new tag with the last solve's value)
+            auto whole = [&](const uint4 &v) { return v.w == tag && v.z == (v.x ^ v.y ^ tag); };
             Spin spin;
             for (;;) {
                 bool ready = true;
 #pragma unroll
                 for (int u = 0; u < U; ++u)
 #pragma unroll
-                    for (int k = 0; k < K; ++k) ready &= x[u][k].w == tag;
+                    for (int k = 0; k < K; ++k) ready &= whole(x[u][k]);
                 if (ready) break;
                 if (spin.expired(a.err)) {
                     ok = false;
@@ -184,7 +189,7 @@ __device__ __forceinline__ bool all_reduce(DFloat (&v)[K], Reduce &sh, const CgA
                 for (int u = 0; u < U; ++u)
 #pragma unroll
                     for (int k = 0; k < K; ++k)
-                        if (x[u][k].w != tag) x[u][k] = ld_word(red + (size_t)k * CG_COPIES * G + j0 + 32 * u);
+                        if (!whole(x[u][k])) x[u][k] = ld_word(red + (size_t)k * CG_COPIES * G + j0 + 32 * u);
             }
 #pragma unroll
             for (int u = 0; u < U; ++u)

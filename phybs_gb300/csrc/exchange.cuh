@@ -16,7 +16,9 @@ namespace pbs {
 // spinning on.
 constexpr unsigned long long EXCHANGE_WAIT_NS = 2000000000ull;
 
-// A word of the exchange: three floats and a tag, one 128-bit access.
+// A word of the exchange: three floats and a tag, one 128-bit access.  A caller
+// uses all four: a load of which a part goes unused may be compiled into
+// narrower ones, and a tag loaded by itself says nothing about the value.
 __device__ __forceinline__ uint4 ld_word(const float4 *p) {
     uint4 v;
     asm volatile(

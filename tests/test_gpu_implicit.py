@@ -140,3 +140,20 @@ def test_solve_scales(scale):
     assert res <= 1e-6 and it > 0
     assert np.abs(s.positions() - xo).max() / m.bbox_diagonal() < POS_TOL
     s.close()
+
+
+@pytest.mark.parametrize("split,nx,ny,nz", [(6, 10, 4, 4), (5, 9, 9, 9), (6, 10, 10, 12)])
+def test_solves_repeat_bitwise(split, nx, ny, nz):
+    """The same two steps forty times over (3, 8 and 13 CTAs; the second solve
+    of a handle finds the first one's words): one result, bit for bit."""
+    m, x0, v0 = _moving(split, nx, ny, nz)
+    mu, lam = O.lame(m.young, m.poisson)
+    first = None
+    for _ in range(40):
+        s = DescentSolver(m, positions=x0, mu=mu, lam=lam)
+        s.write_velocities(v0, v0)
+        its = [s.backward_euler_step(tol=1e-6) for _ in range(2)]
+        out = (its, s.positions().tobytes(), s.velocities()[0].tobytes())
+        s.close()
+        first = first or out
+        assert out == first
