@@ -35,7 +35,8 @@ def _f32(a, shape=None):
 
 
 def _ptr(a):
-    return C.c_void_p(a.ctypes.data) if a is not None else None
+    # (data_as keeps the array alive: it may be a converted copy that nothing else holds)
+    return a.ctypes.data_as(C.c_void_p) if a is not None else None
 
 
 def make_params(preset: str = "cpu_reference", **kw) -> L.StepParams:

@@ -45,7 +45,8 @@ N_OUT = 3
 
 
 def _ptr(a):
-    return C.c_void_p(a.ctypes.data) if a is not None else None
+    # (data_as keeps the array alive: it may be a converted copy that nothing else holds)
+    return a.ctypes.data_as(C.c_void_p) if a is not None else None
 
 
 def _f32(a):

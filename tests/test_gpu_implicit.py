@@ -157,3 +157,19 @@ def test_solves_repeat_bitwise(split, nx, ny, nz):
         s.close()
         first = first or out
         assert out == first
+
+
+def test_converted_inputs_outlive_the_call():
+    """Arrays that have to be converted (other order, 64 bits) are copied for
+    the call: what arrives is their values."""
+    m, x0, _ = _moving(5, 3, 3, 7)
+    s = DescentSolver(m, positions=x0)
+    rng = np.random.default_rng(3)
+    for k in range(50):
+        v = rng.standard_normal((m.n_nodes, 3))
+        s.write_velocities(np.asfortranarray(v), (2 * v)[:, ::1])
+        got, old = s.velocities()
+        assert np.array_equal(got, v.astype(np.float32)) and np.array_equal(old, (2 * v).astype(np.float32)), k
+        s.update_positions(np.asfortranarray(x0.astype(np.float64)))
+        assert np.array_equal(s.positions(), x0)
+    s.close()
