@@ -31,7 +31,18 @@ __device__ __forceinline__ void unpack_cor(const uint4 &w, int loc[4], int slot[
 // One chunk as its tet loop reads it: node words staged in shared memory;
 // per-tet rows and corner records in shared memory or at the chunk's place in
 // the pass arrays.
+//
+// A local node's words are two vectors: its displacement u (hi, lo; full
+// stress), or its increment relative to the chunk's reference node and its
+// base (incremental stress).  PACK: the six floats as {v0, v1.x} in wa and
+// {v1.y, v1.z} in wb, 24 bytes: the tet loop is bound by its shared-memory
+// wavefronts (64% of the active cycles on the 512,000-tet box), and two
+// 128-bit words a node, a quarter of them unused, were a third of those.
+// Otherwise (rows staged by asynchronous copies, which bring 16-byte words) as
+// float4 in uh / ul / ub.
 struct ChunkView {
+    float4 *wa;
+    float2 *wb;
     const float4 *uh, *ul, *ub;
     const float4 *r0, *r1, *r2;
     const uint4 *cor;
@@ -39,29 +50,44 @@ struct ChunkView {
     const float4 *rest;  // rest positions, for the FP64 stress of a near-inverted tet
 };
 
-// Corner forces of the chunk's tets into the slots; on line-search passes
-// returns the thread's sum of clamped tet energies.
-// The node words of a tet's four corners from the chunk's shared-memory
-// staging (one 128-bit access each): x = u hi (full stress) or nothing (the
-// incremental form), l = u lo or the increment relative to the chunk's
+// Stores local node j's words (PACK): v0 = u hi or the increment, v1 = u lo or
+// the base.
+__device__ __forceinline__ void pack_words(float4 *wa, float2 *wb, int j, const float4 &v0, const float4 &v1) {
+    wa[j] = make_float4(v0.x, v0.y, v0.z, v1.x);
+    wb[j] = make_float2(v1.y, v1.z);
+}
+
+// The node words of a tet's four corners: x = u hi (full stress) or nothing
+// (the incremental form), l = u lo or the increment relative to the chunk's
 // reference node, a = the base (incremental).
-template <bool INC>
+template <bool INC, bool PACK>
 __device__ __forceinline__ void corner_words(const ChunkView &v, const int lc[4], float4 x[4], float4 l[4],
                                              float4 a[4]) {
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-        x[c] = INC ? z4 : lds128(v.uh + lc[c]);
-        l[c] = lds128(v.ul + lc[c]);
-        a[c] = INC ? lds128(v.ub + lc[c]) : z4;
+        if (PACK) {
+            const float4 p = lds128(v.wa + lc[c]);
+            const float2 q = lds64(v.wb + lc[c]);
+            const float4 v0 = make_float4(p.x, p.y, p.z, 0.f), v1 = make_float4(p.w, q.x, q.y, 0.f);
+            x[c] = INC ? z4 : v0;
+            l[c] = INC ? v0 : v1;
+            a[c] = INC ? v1 : z4;
+        } else {
+            x[c] = INC ? z4 : lds128(v.uh + lc[c]);
+            l[c] = lds128(v.ul + lc[c]);
+            a[c] = INC ? lds128(v.ub + lc[c]) : z4;
+        }
     }
 }
 
+// Corner forces of the chunk's tets into the slots; on line-search passes
+// returns the thread's sum of clamped tet energies.
 // A near-inverted tet (full stress) gets its FP32 forces here and a mark in
 // its corner-0 slot's .w; *any_exact tells whether the thread marked one.
 // CHECK: a line-search pass (the tet energies too); the loop is compiled once
 // with and once without them.
-template <int MATERIAL, int THREADS, bool INC, bool CHECK>
+template <int MATERIAL, int THREADS, bool INC, bool PACK, bool CHECK>
 __device__ __forceinline__ DFloat chunk_forces(const DevParams &p, const ChunkView &v, int nt, float4 *sf,
                                                bool *any_exact) {
     DFloat e{0.f, 0.f};
@@ -74,7 +100,7 @@ __device__ __forceinline__ DFloat chunk_forces(const DevParams &p, const ChunkVi
         Kin<float> kin;
         float f[12];
         float4 x[4], l[4], a[4];
-        corner_words<INC>(v, lc, x, l, a);
+        corner_words<INC, PACK>(v, lc, x, l, a);
         const bool ex = pass_forces_c<MATERIAL, INC, true, CHECK>(
             x[0], x[1], x[2], x[3], l[0], l[1], l[2], l[3], a[0], a[1], a[2], a[3], dinv, r0.w, r1.w, r2.w, kin, f,
             CornerRest{v.rest, v.meta, {lc[0], lc[1], lc[2], lc[3]}});
@@ -106,7 +132,7 @@ static __device__ __noinline__ bool chunk_stretch_svd(const float4 x[4], const f
 // The FP64 stress of the chunk's marked (near-inverted) tets, into their
 // slots.  After the tet loop rather than inside it: the loop then carries no
 // call, and keeps its registers.
-template <int MATERIAL, int THREADS>
+template <int MATERIAL, int THREADS, bool PACK>
 __device__ __forceinline__ void chunk_exact(const ChunkView &v, int nt, float4 *sf) {
     for (int lt = threadIdx.x; lt < nt; lt += THREADS) {
         int lc[4], sl[4];
@@ -115,7 +141,7 @@ __device__ __forceinline__ void chunk_exact(const ChunkView &v, int nt, float4 *
         const float4 r0 = v.r0[lt], r1 = v.r1[lt], r2 = v.r2[lt];
         const float dinv[9] = {r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r2.x, r2.y, r2.z};
         float4 x[4], l[4], a[4];
-        corner_words<false>(v, lc, x, l, a);
+        corner_words<false, PACK>(v, lc, x, l, a);
         float P[9], f[12];
         // a stretch-material tet that only may be ill-conditioned: the FP32
         // SVD decides
@@ -148,23 +174,37 @@ template <int THREADS, bool PART> __device__ __forceinline__ bool chunk_sync_or(
 
 // chunk_forces, then the FP64 stress of a chunk that has a near-inverted tet;
 // every (participating) thread sees the finished slots on return.
-template <int MATERIAL, int THREADS, bool INC, bool PART = false>
+template <int MATERIAL, int THREADS, bool INC, bool PACK, bool PART = false>
 __device__ __forceinline__ DFloat chunk_forces_all(const DevParams &p, const ChunkView &v, int nt, bool check,
                                                    float4 *sf) {
     bool ex;
-    const DFloat e = check ? chunk_forces<MATERIAL, THREADS, INC, true>(p, v, nt, sf, &ex)
-                           : chunk_forces<MATERIAL, THREADS, INC, false>(p, v, nt, sf, &ex);
+    const DFloat e = check ? chunk_forces<MATERIAL, THREADS, INC, PACK, true>(p, v, nt, sf, &ex)
+                           : chunk_forces<MATERIAL, THREADS, INC, PACK, false>(p, v, nt, sf, &ex);
     if (INC) {
         chunk_sync<THREADS, PART>();
     } else if (chunk_sync_or<THREADS, PART>(ex)) {
-        chunk_exact<MATERIAL, THREADS>(v, nt, sf);
+        chunk_exact<MATERIAL, THREADS, PACK>(v, nt, sf);
         chunk_sync<THREADS, PART>();
     }
     return e;
 }
 
+// A thread's share of the line search's noise scale, from the sum e of its tet
+// energies: the scale adds the squares of the sums of m.noise_tets tets (four,
+// whose threads' sums are grouped by neighbouring lanes; 0: of each thread's
+// own), so that a line search rejects by the same allowance at every automatic
+// chunk size.  With each thread's own at one or two tets a thread the allowance
+// was half as large, and one pull in ten to a residual of 1e-4 took another
+// rejection.  Called by whole warps.
+template <int THREADS> __device__ __forceinline__ float noise_square(const DevMesh &m, int nt, float e) {
+    const int lanes = m.noise_tets == 0 ? 1 : nt > THREADS ? m.noise_tets / 2 : m.noise_tets;
+    if (lanes > 1) e += __shfl_xor_sync(0xffffffffu, e, 1);
+    if (lanes > 2) e += __shfl_xor_sync(0xffffffffu, e, 2);
+    return e * e / (float)lanes;
+}
+
 // Jacobi-diagonal refresh: the same slots carry the 12 diagonal terms.
-template <int MATERIAL, int THREADS, bool INC>
+template <int MATERIAL, int THREADS, bool INC, bool PACK>
 __device__ __forceinline__ void chunk_hdiag(const ChunkView &v, int nt, float4 *sf) {
     for (int lt = threadIdx.x; lt < nt; lt += THREADS) {
         const float4 r0 = v.r0[lt], r1 = v.r1[lt], r2 = v.r2[lt];
@@ -174,7 +214,7 @@ __device__ __forceinline__ void chunk_hdiag(const ChunkView &v, int nt, float4 *
         Kin<float> kin;
         float f[12], kd[12];
         float4 x[4], l[4], a[4];
-        corner_words<INC>(v, lc, x, l, a);
+        corner_words<INC, PACK>(v, lc, x, l, a);
         // only the kinematics are used here (no FP64 stress needed)
         pass_forces_c<MATERIAL, INC, true>(x[0], x[1], x[2], x[3], l[0], l[1], l[2], l[3], a[0], a[1], a[2], a[3],
                                            dinv, r0.w, r1.w, r2.w, kin, f,

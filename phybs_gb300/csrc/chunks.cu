@@ -4,8 +4,9 @@
 // the Morton order of their centroids, that touches at most chunk_nodes nodes
 // (the instance's automatic limits, auto_chunk_limits, or the chunk shape that
 // the caller or pbs_autotune set).  One CTA per chunk:
-//   1. stages the chunk's nodes (u hi, u lo and the force base) in shared
-//      memory: each node is read once per chunk instead of once per corner;
+//   1. stages the chunk's nodes (displacements hi and lo, or increments and
+//      force base) in shared memory: each node is read once per chunk instead
+//      of once per corner;
 //   2. evaluates its tets (one thread per tet, chunk tets / CTA threads tets
 //      a thread), streaming the per-tet rows in chunk order, and writes the 12
 //      corner forces to shared-memory slots, where a node's slots are
@@ -48,15 +49,17 @@ namespace pbs {
 
 // ------------------------------------------------------------ host: layout
 void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<double> &rest, std::vector<InstCtl> &ctl,
-                  const std::vector<ChunkLimits> &limits, ChunkLayout &out) {
+                  const std::vector<ChunkLimits> &limits, bool grouped, bool pad_slots, ChunkLayout &out) {
     out = ChunkLayout();
     std::vector<int> stamp(Np, -1), lidx(Np, 0), n_part(Np, 0);
+    int mark = -1;
     std::vector<std::pair<uint32_t, int>> order;
-    std::vector<int> ctets, lnodes, scount, lnode_all, lsptr_all, lsend_all;
+    std::vector<int> ctets, lnodes, scount, first, by_count, run_of, lnode_all, lrun_all, lsptr_all, lsend_all;
     int tq = 0;
     for (size_t b = 0; b < ctl.size(); ++b) {
         InstCtl &C = ctl[b];
         const int chunk_tets = limits[b].tets, chunk_nodes = limits[b].nodes;
+        const int group_tets = grouped ? CHUNK_GROUP_TETS : 0, group_nodes = CHUNK_GROUP_NODES;
         C.cblk_begin = (int)out.chunk.size();
         double lo[3], hi[3];
         for (int d = 0; d < 3; ++d) {
@@ -95,52 +98,85 @@ void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<doubl
             out.chunk.push_back(make_int4(tq, 0, (int)lnode_all.size(), 0));
             out.chunk_inst.push_back((int)b);
         }
-        size_t pos = 0;
-        while (pos < order.size()) {
-            const int cid = (int)out.chunk.size();
+        // the tets from pos on, up to end, that fit the limits -> ctets; their
+        // nodes -> lnodes
+        auto take = [&](size_t pos, size_t end, int max_tets, int max_nodes, int ref) {
             ctets.clear();
             lnodes.clear();
-            while (pos < order.size() && (int)ctets.size() < chunk_tets) {
+            ++mark;
+            if (ref >= 0) {
+                stamp[ref] = mark;
+                lnodes.push_back(ref);
+            }
+            for (; pos < end && (int)ctets.size() < max_tets; ++pos) {
                 const int t = order[pos].second;
                 const int *q = &tets[t].x;
                 int add = 0;
                 for (int c = 0; c < 4; ++c) {
-                    bool seen = stamp[q[c]] == cid;
+                    bool seen = stamp[q[c]] == mark;
                     for (int c2 = 0; c2 < c && !seen; ++c2) seen = q[c2] == q[c];
                     add += !seen;
                 }
-                if ((int)lnodes.size() + add > chunk_nodes) break;
+                if ((int)lnodes.size() + add > max_nodes) break;
                 for (int c = 0; c < 4; ++c)
-                    if (stamp[q[c]] != cid) {
-                        stamp[q[c]] = cid;
+                    if (stamp[q[c]] != mark) {
+                        stamp[q[c]] = mark;
                         lnodes.push_back(q[c]);
                     }
                 ctets.push_back(t);
-                ++pos;
             }
+        };
+        size_t pos = 0, group_end = 0;
+        int ref = -1, piece = chunk_tets;
+        while (pos < order.size()) {
+            if (group_tets && pos == group_end) {
+                // a new group, cut into pieces of even size
+                take(pos, order.size(), group_tets, group_nodes, -1);
+                group_end = pos + ctets.size();
+                ref = *std::min_element(lnodes.begin(), lnodes.end());
+                const int n = (int)ctets.size(), k = (n + chunk_tets - 1) / chunk_tets;
+                piece = (n + k - 1) / k;
+            }
+            take(pos, group_tets ? group_end : order.size(), piece, chunk_nodes, ref);
+            pos += ctets.size();
             // local nodes in ascending id order: a warp's node gathers then
-            // share sectors (ordering them by corner count, which evens out the
-            // partial-sum loops, measured slower)
+            // share sectors
             std::sort(lnodes.begin(), lnodes.end());
             const int nl = (int)lnodes.size(), nt = (int)ctets.size();
             for (int j = 0; j < nl; ++j) lidx[lnodes[j]] = j;
             scount.assign(nl + 1, 0);
+            first.resize(nl);
             for (int t : ctets)
                 for (int c = 0; c < 4; ++c) scount[lidx[(&tets[t].x)[c]] + 1]++;
-            for (int j = 0; j < nl; ++j) scount[j + 1] += scount[j];
             const int l0 = (int)lnode_all.size();
-            for (int j = 0; j < nl; ++j) {
-                lnode_all.push_back(lnodes[j]);
-                lsptr_all.push_back(scount[j]);
-                lsend_all.push_back(scount[j + 1]);
-                n_part[lnodes[j]]++;
+            // slot runs: the nodes with the most corners first (a counting sort),
+            // so that a warp's partial-sum loops end together; runs of even
+            // length padded to odd, so that eight neighbouring lanes read eight
+            // different bank groups (1M-tet box, full / incremental stress: 39.6
+            // / 44.3 us a pass with the runs in node order, 36.6 / 42.0 so; with
+            // the packed node words 35.3 / 41.1)
+            by_count.assign(nt + 2, 0);
+            for (int j = 0; j < nl; ++j) by_count[nt - scount[j + 1] + 1]++;
+            for (int k = 0; k <= nt; ++k) by_count[k + 1] += by_count[k];
+            run_of.resize(nl);
+            for (int j = 0; j < nl; ++j) run_of[by_count[nt - scount[j + 1]]++] = j;
+            int slot = 0;
+            for (int r = 0; r < nl; ++r) {
+                const int j = run_of[r], cnt = scount[j + 1];
+                first[j] = slot;
+                slot += pad_slots ? cnt | 1 : cnt;
+                lnode_all.push_back(lnodes[r]);
+                lrun_all.push_back(lnodes[j]);
+                lsptr_all.push_back(first[j]);
+                lsend_all.push_back(first[j] + cnt);
+                n_part[lnodes[r]]++;
             }
             for (int lt = 0; lt < nt; ++lt) {
                 const int *q = &tets[ctets[lt]].x;
                 unsigned loc[4], sl[4];
                 for (int c = 0; c < 4; ++c) {
                     loc[c] = (unsigned)lidx[q[c]];
-                    sl[c] = (unsigned)scount[loc[c]]++;
+                    sl[c] = (unsigned)first[loc[c]]++;
                 }
                 out.qcor.push_back(make_uint4(loc[0] | loc[1] << 16, loc[2] | loc[3] << 16, sl[0] | sl[1] << 16,
                                               sl[2] | sl[3] << 16));
@@ -149,6 +185,7 @@ void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<doubl
             out.chunk.push_back(make_int4(tq, nt, l0, nl));
             out.chunk_inst.push_back((int)b);
             out.max_local = std::max(out.max_local, nl);
+            out.max_slots = std::max(out.max_slots, slot);
             tq += nt;
         }
         C.cblk_end = (int)out.chunk.size();
@@ -158,14 +195,16 @@ void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<doubl
     for (int i = 0; i < Np; ++i) out.pptr[i + 1] = out.pptr[i] + n_part[i];
     std::vector<int> fill(out.pptr.begin(), out.pptr.end() - 1);
     out.lmeta.resize(lnode_all.size());
+    // (a chunk's runs are of its own nodes: each node's places go up by chunk)
     for (size_t j = 0; j < lnode_all.size(); ++j)
-        out.lmeta[j] = make_int4(lnode_all[j], lsptr_all[j], lsend_all[j], fill[lnode_all[j]]++);
+        out.lmeta[j] = make_int4(lnode_all[j], lsptr_all[j], lsend_all[j], fill[lrun_all[j]]++);
 }
 
 // Where the lines lie (96 passes of a 5-tet box, full / incremental stress, us;
 // "graph" the pass kernels at their best shape, "frame" the frame kernel):
-//   up to 8,192 tets: 128 a chunk (2,340 tets: 409 / 444, 256 a chunk 473 /
-//     507, graph 1003 / 1050);
+//   up to 4,096 tets: 128 a chunk (2,340 tets: 409 / 444, 256 a chunk 473 /
+//     507, graph 1003 / 1050; up to 8,192 a single instance gained 7% and the
+//     batch below lost 4%);
 //   up to 3 * sms * 256 (116,736): 256, up to three CTAs a SM of the frame
 //     kernel (24,500 tets: 501 / 548, 192 a chunk 493 / 540, graph 1059 / 1119;
 //     59,940: 631 / 673, graph 1122 / 1197; 100,800: 939 / 832, graph 1245 /
@@ -177,11 +216,14 @@ void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<doubl
 //     (149,445: 1183 / 1236, graph 1301 / 1387);
 //   beyond, the pass kernels: 384 tets up to 250,000 (203,205: 1463 / 1596,
 //     512 tets 1622 / 1731), then 512 (311,040: 1602 / 1770, 384 tets 1829 /
-//     2058).
+//     2058; 1M tets, us a pass of the tet kernel: 35.0 / 40.9, 1,024 tets and
+//     512 threads 36.7 / 43.8).
+// (Measured with chunks of exactly these sizes; the pieces of a group of 1,024
+// are of 342 where this says 384.)
 // The node limit leaves room for meshes with more nodes a tet than a box.
 ChunkLimits auto_chunk_limits(int tets, int sms) {
     int n;
-    if (tets <= 8192) n = 128;
+    if (tets <= 4096) n = 128;
     else if (tets <= 3 * 256 * sms) n = 256;
     else if (tets > 2 * 512 * sms && tets <= 250000) n = 384;
     else n = 512;
@@ -217,7 +259,7 @@ __device__ __forceinline__ void chunk_line_search(const DevMesh &m, const DevPar
     InstCtl *dst = ctl_buf(st, par ^ 1) + inst;
     unsigned int *cnt = st.tcount + inst;
     __shared__ float shs[THREADS / 32];
-    float e2 = e.hi * e.hi;
+    float e2 = noise_square<THREADS>(m, m.chunk[c].y, e.hi);
     const int cb = src->cblk_begin, ce = src->cblk_end;
     {
         const int nb = ce - cb;
@@ -277,16 +319,16 @@ __device__ __forceinline__ void chunk_line_search(const DevMesh &m, const DevPar
 // The whole of one chunk once its node words (and, with STAGE, its rows and
 // records) are in shared memory: forces, partials, the Jacobi diagonal every
 // hd_every passes, and the line-search tail.
-template <int MATERIAL, int THREADS, bool INC>
+template <int MATERIAL, int THREADS, bool INC, bool PACK>
 __device__ __forceinline__ void chunk_body(const DevMesh &m, const DevParams &p, const DevState &st, int c,
                                            int inst, int par, const PassView &pv, size_t cur, const ChunkView &v,
                                            const int4 *meta, int nt, int nl, float4 *sf, double *sh,
                                            int *is_last) {
-    const DFloat e = chunk_forces_all<MATERIAL, THREADS, INC>(p, v, nt, pv.check, sf);
+    const DFloat e = chunk_forces_all<MATERIAL, THREADS, INC, PACK>(p, v, nt, pv.check, sf);
     chunk_partials<THREADS>(meta, nl, sf, st.part);
     if (pv.do_h) {
         __syncthreads();
-        chunk_hdiag<MATERIAL, THREADS, INC>(v, nt, sf);
+        chunk_hdiag<MATERIAL, THREADS, INC, PACK>(v, nt, sf);
         __syncthreads();
         chunk_partials<THREADS>(meta, nl, sf, st.parth);
     }
@@ -316,11 +358,14 @@ __global__ void __launch_bounds__(THREADS, PBS_INC_THREADS_PER_SM / THREADS)
     k_tchunk(DevMesh m, DevParams p, DevState st, int par) {
     extern __shared__ float4 smem4[];
     const int CN = m.chunk_nodes, CT = m.chunk_tets;
-    // node words: u hi, u lo (without INC) or the increment (with INC), base
-    // (INC only); corner slots; with STAGE the rows and records
+    // node words: 24 bytes a node, or with STAGE u hi, u lo (without INC) or the
+    // increment (with INC), base (INC only); corner slots; with STAGE the rows
+    // and records
     float4 *s_uh = smem4, *s_ul = smem4 + CN, *s_ub = smem4 + 2 * CN;
-    float4 *s_f = smem4 + (INC ? 3 : 2) * CN;  // corner slots, 4 a tet
-    float4 *s_r0 = s_f + 4 * CT, *s_r1 = s_r0 + CT, *s_r2 = s_r1 + CT;  // STAGE only
+    float4 *s_wa = smem4;
+    float2 *s_wb = reinterpret_cast<float2 *>(smem4 + CN);
+    float4 *s_f = smem4 + node_words(CN, INC, STAGE ? 1 : 0);  // corner slots
+    float4 *s_r0 = s_f + m.chunk_slots, *s_r1 = s_r0 + CT, *s_r2 = s_r1 + CT;  // STAGE only
     uint4 *s_cor = reinterpret_cast<uint4 *>(s_r2 + CT);
     int4 *s_meta = reinterpret_cast<int4 *>(s_cor + CT);
     __shared__ double sh[THREADS / 32];
@@ -388,18 +433,14 @@ __global__ void __launch_bounds__(THREADS, PBS_INC_THREADS_PER_SM / THREADS)
         for (int j = threadIdx.x; j < nl; j += THREADS) {
             const int g = meta[j].x;
             const float4 uh = st.uh[cur + g], ul = st.ul[cur + g];
-            if (INC) {
-                const float4 ub = st.ub[g];
-                s_ul[j] = increment_rel(uh, ul, r);
-                s_ub[j] = ub;
-            } else {
-                s_uh[j] = uh;
-                s_ul[j] = ul;
-            }
+            if (INC) pack_words(s_wa, s_wb, j, increment_rel(uh, ul, r), st.ub[g]);
+            else pack_words(s_wa, s_wb, j, uh, ul);
         }
     }
     __syncthreads();
     ChunkView v;
+    v.wa = s_wa;
+    v.wb = s_wb;
     v.uh = s_uh;
     v.ul = s_ul;
     v.ub = s_ub;
@@ -409,7 +450,7 @@ __global__ void __launch_bounds__(THREADS, PBS_INC_THREADS_PER_SM / THREADS)
     v.cor = STAGE ? s_cor : m.qcor + tq0;
     v.meta = meta;
     v.rest = m.rest;
-    chunk_body<MATERIAL, THREADS, INC>(m, p, st, c, inst, par, pv, cur, v, meta, nt, nl, s_f, sh, &is_last);
+    chunk_body<MATERIAL, THREADS, INC, !STAGE>(m, p, st, c, inst, par, pv, cur, v, meta, nt, nl, s_f, sh, &is_last);
 }
 
 // ------------------------------------------------------------ persistent, TMA-fed variant
@@ -624,7 +665,7 @@ __global__ void __launch_bounds__(THREADS, 768 / THREADS) k_tstream(DevMesh m, D
             v.cor = sb.cor;
             v.meta = sb.meta;
             v.rest = m.rest;
-            chunk_body<MATERIAL, THREADS, INC>(m, p, st, c, cur.inst, par, cur.pv, cur.cur, v, sb.meta, cur.nt,
+            chunk_body<MATERIAL, THREADS, INC, false>(m, p, st, c, cur.inst, par, cur.pv, cur.cur, v, sb.meta, cur.nt,
                                                cur.nl, s_f, sh, &is_last);
         }
         __syncthreads();  // buffer b and the slots are free again
@@ -711,7 +752,7 @@ static cudaError_t launch_tchunk_t(cudaStream_t s, const DevMesh &m, const DevPa
                                    bool pdl) {
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = chunk_config(s, m.n_chunks, THREADS,
-                                          chunk_smem(m.chunk_tets, m.chunk_nodes, INC, STAGE ? 1 : 0), pdl, at, m);
+                                          chunk_smem(m.chunk_tets, m.chunk_nodes, m.chunk_slots, INC, STAGE ? 1 : 0), pdl, at, m);
     return cudaLaunchKernelEx(&cfg, k_tchunk<MATERIAL, THREADS, INC, STAGE>, m, p, st, par);
 }
 
@@ -721,7 +762,7 @@ static cudaError_t launch_tstream_t(cudaStream_t s, const DevMesh &m, const DevP
     if (m.stream_grid <= 0) return cudaErrorInvalidConfiguration;
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg =
-        chunk_config(s, m.stream_grid, THREADS, chunk_smem(m.chunk_tets, m.chunk_nodes, INC, 2), pdl, at, m);
+        chunk_config(s, m.stream_grid, THREADS, chunk_smem(m.chunk_tets, m.chunk_nodes, m.chunk_slots, INC, 2), pdl, at, m);
     return cudaLaunchKernelEx(&cfg, k_tstream<MATERIAL, THREADS, INC>, m, p, st, par);
 }
 
@@ -765,7 +806,7 @@ cudaError_t launch_tet_only(cudaStream_t s, const DevMesh &m, const DevParams &p
 template <int MATERIAL, int THREADS, bool INC> static int stream_fit(const DevMesh &m, int sms) {
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tstream<MATERIAL, THREADS, INC>, THREADS,
-                                                      chunk_smem(m.chunk_tets, m.chunk_nodes, INC, 2)) != cudaSuccess)
+                                                      chunk_smem(m.chunk_tets, m.chunk_nodes, m.chunk_slots, INC, 2)) != cudaSuccess)
         return 0;
     return std::min(m.n_chunks, per_sm * sms);
 }

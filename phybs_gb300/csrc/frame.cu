@@ -235,10 +235,12 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
     extern __shared__ float4 smem4[];
     constexpr int WARPS = THREADS / 32;
     const int CN = m.chunk_nodes, CT = m.chunk_tets;
-    float4 *s_uh = smem4, *s_ul = smem4 + CN, *s_ub = smem4 + 2 * CN;
-    float4 *s_f = smem4 + (INC ? 3 : 2) * CN;  // corner slots, 4 a tet
-    // resident: the chunk's rows and records, in chunk_smem's staged order
-    float4 *s_r0 = s_f + 4 * CT, *s_r1 = s_r0 + CT, *s_r2 = s_r1 + CT;
+    // node words (24 bytes a node), corner slots
+    float4 *s_wa = smem4;
+    float2 *s_wb = reinterpret_cast<float2 *>(smem4 + CN);
+    float4 *s_f = smem4 + node_words(CN, INC, 0);
+    // resident: the chunk's rows and records
+    float4 *s_r0 = s_f + m.chunk_slots, *s_r1 = s_r0 + CT, *s_r2 = s_r1 + CT;
     uint4 *s_cor = reinterpret_cast<uint4 *>(s_r2 + CT);
     int4 *s_meta = reinterpret_cast<int4 *>(s_cor + CT);
     __shared__ InstCtl sc;  // this CTA's copy of the instance's control block (the control warp's)
@@ -260,7 +262,7 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
         for (int j = tid; j < cd.w; j += THREADS) {
             const int4 md = m.lmeta[cd.z + j];
             s_meta[j] = md;
-            if (INC) s_ub[j] = st.ub[md.x];
+            if (INC) pack_words(s_wa, s_wb, j, st.ub[md.x], st.ub[md.x]);  // (the base; the increment follows)
         }
         cp_async_commit();
         cp_async_wait_all();
@@ -338,37 +340,39 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
                     const int g = meta[j].x;
                     float4 uh, ul, r;  // (the increments relative to the chunk's local node 0)
                     ok = poll_state(fx.xh, fx.xl, g, INC ? g0 : g, tag, uh, ul, r, err) && ok;
-                    if (INC) {
-                        s_ul[j] = increment_rel(uh, ul, r);
-                        if (!RES) s_ub[j] = st.ub[g];
+                    if (!INC) {
+                        pack_words(s_wa, s_wb, j, uh, ul);
+                    } else if (RES) {  // the base is there already
+                        const float4 d = increment_rel(uh, ul, r);
+                        s_wa[j].x = d.x;
+                        s_wa[j].y = d.y;
+                        s_wa[j].z = d.z;
                     } else {
-                        s_uh[j] = uh;
-                        s_ul[j] = ul;
+                        pack_words(s_wa, s_wb, j, increment_rel(uh, ul, r), st.ub[g]);
                     }
                 }
                 if (c == b && pend) asm volatile("barrier.cta.arrive 2, %0;" ::"n"(THREADS + 32) : "memory");
                 chunk_sync<THREADS, true>();
                 ChunkView v;
-                v.uh = s_uh;
-                v.ul = s_ul;
-                v.ub = s_ub;
+                v.wa = s_wa;
+                v.wb = s_wb;
                 v.r0 = RES ? s_r0 : m.qrow0 + cd.x;
                 v.r1 = RES ? s_r1 : m.qrow1 + cd.x;
                 v.r2 = RES ? s_r2 : m.qrow2 + cd.x;
                 v.cor = RES ? s_cor : m.qcor + cd.x;
                 v.meta = meta;
                 v.rest = m.rest;
-                const DFloat ec = chunk_forces_all<MATERIAL, THREADS, INC, true>(p, v, nt, check, s_f);
+                const DFloat ec = chunk_forces_all<MATERIAL, THREADS, INC, true, true>(p, v, nt, check, s_f);
                 publish_partials<THREADS>(meta, nl, s_f, st.part, tag);
                 if (do_h) {
                     chunk_sync<THREADS, true>();
-                    chunk_hdiag<MATERIAL, THREADS, INC>(v, nt, s_f);
+                    chunk_hdiag<MATERIAL, THREADS, INC, true>(v, nt, s_f);
                     chunk_sync<THREADS, true>();
                     publish_partials<THREADS>(meta, nl, s_f, st.parth, tag);
                 }
                 if (check) {
                     e = df_add(e, ec);
-                    e2 = fmaf(ec.hi, ec.hi, e2);
+                    e2 += noise_square<THREADS>(m, nt, ec.hi);
                 }
                 // the slots and node words are free for the next chunk (or pass)
                 if (!RES) chunk_sync<THREADS, true>();
@@ -503,13 +507,18 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
     }
 }
 
-// Co-resident CTAs of a variant on a device with `sms` SMs.  Shared memory of
-// a CTA: the pass kernel's node words and slots, with the resident layout also
-// the rows and records (chunk_smem's staged size).
+// Shared memory of a CTA: the pass kernel's node words and slots, with the
+// resident layout also the rows and records.
+static size_t frame_smem(const DevMesh &m, bool inc, bool resident) {
+    return chunk_smem(m.chunk_tets, m.chunk_nodes, m.chunk_slots, inc, 0) +
+           (resident ? 64 * (size_t)m.chunk_tets + sizeof(int4) * (size_t)m.chunk_nodes : 0);
+}
+
+// Co-resident CTAs of a variant on a device with `sms` SMs.
 template <int MATERIAL, int THREADS, bool INC, bool RES, int PER_SM>
 static int frame_fit(const DevMesh &m, int sms) {
     const auto kernel = k_frame<MATERIAL, THREADS, INC, RES, PER_SM>;
-    const size_t smem = chunk_smem(m.chunk_tets, m.chunk_nodes, INC, RES ? 1 : 0);
+    const size_t smem = frame_smem(m, INC, RES);
     int per_sm = 0;
     if (smem > (size_t)CHUNK_MAX_SMEM ||
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CHUNK_MAX_SMEM) != cudaSuccess ||
@@ -529,7 +538,7 @@ static cudaError_t launch_frame_v(cudaStream_t s, const DevMesh &m, const DevPar
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(THREADS + 32);
-    cfg.dynamicSmemBytes = chunk_smem(m.chunk_tets, m.chunk_nodes, INC, RES ? 1 : 0);
+    cfg.dynamicSmemBytes = frame_smem(m, INC, RES);
     cfg.stream = s;
     cfg.attrs = at;
     cfg.numAttrs = 1;

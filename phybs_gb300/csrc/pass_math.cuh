@@ -43,6 +43,13 @@ __device__ __forceinline__ void sts128(float4 *p, float x, float y, float z, flo
                  : "memory");
 }
 
+__device__ __forceinline__ float2 lds64(const float2 *p) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
+        : "=f"(v.x), "=f"(v.y)
+        : "r"((unsigned)__cvta_generic_to_shared(p)));
+    return v;
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 

@@ -53,7 +53,7 @@ struct pbs_handle {
     DevBuf<float4> row0, row1, row2, info, rest4;
     DevBuf<int> inc_ptr, inc, tblk_inst, nblk_inst, pad2user, tet_user, node_state, bad, staging_ids;
     // pass layout (chunks of tets) and the host copies it is rebuilt from
-    int n_chunks = 0, chunk_tets = 0, chunk_nodes = 0, chunk_threads = 0;
+    int n_chunks = 0, chunk_tets = 0, chunk_nodes = 0, chunk_slots = 0, chunk_threads = 0;
     int chunk_stage = 0;
     int node_npt = NODE_NPT_DEFAULT;
     std::vector<int4> h_tets_pad;
@@ -157,6 +157,8 @@ struct pbs_handle {
         m.tblk_inst = tblk_inst.p; m.nblk_inst = nblk_inst.p;
         m.n_chunks = n_chunks; m.chunk = chunk.p; m.chunk_inst = chunk_inst.p;
         m.chunk_tets = chunk_tets; m.chunk_nodes = chunk_nodes; m.chunk_threads = chunk_threads;
+        m.chunk_slots = chunk_slots;
+        m.noise_tets = shape_auto ? CHUNK_NOISE_TETS : 0;
         m.chunk_stage = chunk_stage;
         m.node_npt = node_npt;
         m.qrow0 = qrow0; m.qrow1 = qrow1; m.qrow2 = qrow2; m.qcor = qcor; m.lmeta = lmeta.p;
@@ -250,8 +252,14 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
         }
         threads = ct > 256 ? 256 : 128;  // one or two tets a thread
     }
+    const bool grouped = h->shape_auto;  // (a caller's own shape keeps a reference node a chunk)
     ChunkLayout cl;
-    build_chunks(h->Np, h->h_tets_pad, h->h_rest_pad, ctl, limits, cl);
+    const std::vector<InstCtl> ctl0 = ctl;
+    build_chunks(h->Np, h->h_tets_pad, h->h_rest_pad, ctl, limits, grouped, true, cl);
+    if (chunk_smem(ct, cn, cl.max_slots, true, stage) > (size_t)CHUNK_MAX_SMEM) {  // no room to pad slot runs
+        ctl = ctl0;
+        build_chunks(h->Np, h->h_tets_pad, h->h_rest_pad, ctl, limits, grouped, false, cl);
+    }
     const int nc = (int)cl.chunk.size();
     const size_t L = cl.lmeta.size(), T = (size_t)h->T;
     h->chunk.release(); h->chunk_inst.release(); h->cpart.release(); h->qperm.release();
@@ -273,6 +281,7 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
     h->n_chunks = nc;
     h->chunk_threads = threads;
     h->chunk_tets = ct;
+    h->chunk_slots = cl.max_slots;
     h->chunk_nodes = cn;
     h->chunk_stage = stage;
     if (host_ctl) {
@@ -1176,7 +1185,9 @@ int pbs_set_chunk_shape(pbs_handle *h, int threads, int chunk_tets, int chunk_no
         (node_npt != 1 && node_npt != 2) ||
         4 * (size_t)chunk_tets > 65536 || chunk_nodes > 65536 || staged < 0 || staged > 2 ||
         (staged && threads == 512) ||
-        chunk_smem(chunk_tets, chunk_nodes, true, staged) > (size_t)CHUNK_MAX_SMEM)
+        // (48 B a node without staging too: the packed words' 24 leave room to pad every run of slots)
+        chunk_smem(chunk_tets, chunk_nodes, 4 * chunk_tets, true, staged) + (staged ? 0 : 24 * (size_t)chunk_nodes) >
+            (size_t)CHUNK_MAX_SMEM)
         return PBS_E_INVALID_ARG;
     PBS_DEVICE_SCOPE(h->device);
     h->node_npt = node_npt;

@@ -38,8 +38,10 @@
 //                                  slot2 | slot3 << 16}; loc = local node of the tet's chunk,
 //                                  slot = its shared-memory slot (a local node's slots are
 //                                  contiguous, in (tet, corner) order)
-//   lmeta       int4[L]            per local node {padded node id (ascending per chunk), first
-//                                  slot, end slot, where the chunk's partial for the node goes}
+//   lmeta       int4[L]            per local node, .x its padded node id (ascending per chunk);
+//                                  per slot run of the chunk (as many, in order of length), .y the
+//                                  first slot, .z the end slot, .w where the partial of the run's
+//                                  node goes
 //   pptr        int[Np+1]          node i's partials: part[pptr[i] .. pptr[i+1]-1], by chunk
 //   part, parth float4[L]          per (node, chunk) partial force / Jacobi-diagonal sums
 //   cpart       double2[n_chunks]  per chunk {sum e, sum e^2}
@@ -62,16 +64,21 @@ constexpr int BLOCK = 256;  // threads per block of the step kernels (nodes per 
 constexpr int NODE_NPT_DEFAULT = 1;
 constexpr int CHUNK_MAX_SMEM = 200 * 1024;
 // Dynamic shared memory of the per-tet pass kernel for a chunk shape and a
-// staging mode: 0 = node words (u hi, u lo, and the force base with
-// incremental stress, 16 B each) and one float4 per corner slot (written and
-// read with one 128-bit access each); 1 = also the chunk's per-tet rows and
-// corner records (64 B per tet) and local-node records (16 B per node); 2 =
-// the persistent kernel, two buffers of rows, records and node words plus one
-// set of slots.
-__host__ __device__ constexpr size_t chunk_smem(int tets, int nodes, bool inc, int stage = 0) {
+// staging mode: 0 = node words (24 B a node) and one float4 per corner slot
+// (written and read with one 128-bit access each; slots: the most of any chunk,
+// its corners and the padding of its runs); 1 = the node words as u hi, u lo,
+// and with incremental stress the force base, 16 B each, and the chunk's
+// per-tet rows and corner records (64 B per tet) and local-node records (16 B
+// per node); 2 = the persistent kernel, two buffers of rows, records and node
+// words plus one set of slots.
+// node_words: the float4 words of the node words of a chunk.
+__host__ __device__ constexpr int node_words(int nodes, bool inc, int stage) {
+    return stage ? (inc ? 3 : 2) * nodes : nodes + (nodes + 1) / 2;
+}
+__host__ __device__ constexpr size_t chunk_smem(int tets, int nodes, int slots, bool inc, int stage = 0) {
     return stage == 2 ? 2 * ((inc ? 4 : 3) * sizeof(float4) * (size_t)nodes + 64 * (size_t)tets) +
-                            sizeof(float4) * 4 * (size_t)tets
-                      : (inc ? 3 : 2) * sizeof(float4) * (size_t)nodes + sizeof(float4) * 4 * (size_t)tets +
+                            sizeof(float4) * (size_t)slots
+                      : sizeof(float4) * (size_t)node_words(nodes, inc, stage) + sizeof(float4) * (size_t)slots +
                             (stage ? 64 * (size_t)tets + sizeof(int4) * (size_t)nodes : 0);
 }
 
@@ -141,7 +148,8 @@ struct DevMesh {
     const float4 *info, *rest;
     const int *tblk_inst, *nblk_inst;
     // pass layout
-    int n_chunks, chunk_tets, chunk_nodes, chunk_threads, chunk_stage;
+    int n_chunks, chunk_tets, chunk_nodes, chunk_slots, chunk_threads, chunk_stage;
+    int noise_tets;  // tets whose energies the noise scale adds before squaring (noise_square)
     int node_npt;
     const int4 *chunk;
     const int *chunk_inst;
@@ -240,7 +248,7 @@ struct ChunkLayout {
     std::vector<int> chunk_inst, qperm, pptr;
     std::vector<uint4> qcor;
     std::vector<int4> lmeta;
-    int max_local = 0;
+    int max_local = 0, max_slots = 0;
 };
 // At most so many tets and nodes a chunk.
 struct ChunkLimits {
@@ -249,9 +257,18 @@ struct ChunkLimits {
 // The chunk limits of an instance whose shape no caller set, from its own tet
 // count only: a packed batch then chunks an instance as it is chunked alone.
 ChunkLimits auto_chunk_limits(int tets, int sms);
-// limits: per instance
+// limits: per instance.  grouped: the chunks are even pieces of groups of at
+// most CHUNK_GROUP_TETS tets and CHUNK_GROUP_NODES nodes, and every chunk of a
+// group holds the group's lowest node (without corners, where it has none of
+// them), which so is its local node 0, the reference node of the incremental
+// stress: the tet forces then have the same bits at every chunk limit, and an
+// iteration to a tolerance takes the same path.  With a reference node a chunk
+// the count of passes to a residual of 1e-4 moved by up to 1%, and the
+// velocities with it by up to 5e-5.  pad_slots: see the slot runs.
+constexpr int CHUNK_GROUP_TETS = 1024, CHUNK_GROUP_NODES = 448;
+constexpr int CHUNK_NOISE_TETS = 4;
 void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<double> &rest, std::vector<InstCtl> &ctl,
-                  const std::vector<ChunkLimits> &limits, ChunkLayout &out);
+                  const std::vector<ChunkLimits> &limits, bool grouped, bool pad_slots, ChunkLayout &out);
 cudaError_t launch_pass_rows(cudaStream_t s, int T, const int *qperm, const float4 *row0, const float4 *row1,
                              const float4 *row2, float4 *q0, float4 *q1, float4 *q2);
 cudaError_t prepare_chunk_kernels();

@@ -119,3 +119,52 @@ def test_stretch_stress_without_svd(s):
     v = a.velocities()[0]
     assert np.abs(v - st.v).max() <= 3e-5 * np.abs(st.v).max(), np.abs(v - st.v).max() / np.abs(st.v).max()
     a.close()
+
+
+PULLS = [(3, 3, 5), (8, 7, 12), (12, 9, 13), (20, 17, 31), (31, 23, 46)]
+
+
+@pytest.mark.parametrize("dims", PULLS, ids=[f"{5 * a * b * c}" for a, b, c in PULLS])
+def test_pull_takes_one_path_at_every_chunk_size(dims):
+    """Two frames of a pull to a residual of 1e-4 on the automatic chunks (one
+    group and less, pieces of 128, 256, 342 tets) and on whole groups of 1,024:
+    the tets' forces have the same bits, so that the passes and rejections are
+    the same, and the positions to the sums' rounding."""
+    m = M.box_mesh(*dims, edge=0.25 / max(dims[:2]), jitter=0.1, seed=7, young=1e5, pin="both")
+    p = make_params("gpu_reference", h=1 / 30, tol=1e-4, max_iters=20000, control=L.PBS_CONTROL_RESTART,
+                    energy_slack=16.0, alpha0=0.45, alpha_grow=1.2,
+                    profile=((5, 0.99), (25, 0.999), (100, 0.9999)))
+    z = m.rest[:, 2]
+    bottom = np.nonzero(z <= z.min() + 1e-9)[0].astype(np.int32)
+    down = np.float32([0, 0, 0.5 * float(z.max() - z.min()) / 30])
+    out = []
+    for shape in (None, (256, 1024, 448)):
+        s = DescentSolver(m, params=p)
+        if shape:
+            s.set_chunk_shape(*shape)
+        its = []
+        for f in range(2):
+            s.set_node_positions(bottom, m.rest[bottom] - (f + 1) * down)
+            its.append((s.step(), s.stats()["rejections"]))
+        out.append((its, s.positions()))
+        s.close()
+    assert out[0][0] == out[1][0]
+    assert np.abs(out[0][1] - out[1][1]).max() <= 1e-6 * m.bbox_diagonal()
+
+
+@pytest.mark.parametrize("staged,threads,tets,nodes", [(1, 256, 1388, 420), (2, 256, 866, 300), (0, 512, 2400, 1066)])
+@pytest.mark.parametrize("inc", [0, 1])
+def test_shapes_without_room_for_padding(staged, threads, tets, nodes, inc):
+    """Shapes at the shared-memory limit, whose slot runs stay unpadded (or, not
+    staged, just fit padded), against the same chunks at the limits' other side
+    of the choice: bit for bit."""
+    m = _box(20, 20, 30)
+    p = make_params("gpu_reference", h=1 / 30, max_iters=24, incremental_stress=inc)
+    x = []
+    for st, th in ((staged, threads), (0, 256)):
+        s = DescentSolver(m, params=p)
+        s.set_chunk_shape(th, tets, nodes, st)
+        s.step()
+        x.append(s.positions())
+        s.close()
+    assert np.array_equal(x[0], x[1])
