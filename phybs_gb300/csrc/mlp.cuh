@@ -7,7 +7,7 @@
 //   sW1 [64][32]  (inputs padded 24 -> 32 with zeros)
 //   sW2 [64][64], sW3 [64][64]
 //   sW4 [8][64]   (outputs padded 3 -> 8 with zeros)
-// and, for the backward pass, the transposes sW2T, sW3T ([in][out]).
+// (training keeps its own copies, mlp_train.cu).
 //
 // Tensor-core tile: mma.sync m16n8k16 (row-major A = activations, col-major
 // B = weights, FP32 C).  A warp owns 16 rows (nodes); a layer's FP32

@@ -2,17 +2,26 @@
 // hand-written BF16 tensor-core kernels (mma.sync m16n8k16, FP32 accumulate).
 //
 //   k_mlp_forward   rows -> 3 outputs; each warp runs 16-row tiles.
-//   k_mlp_grad      forward + backward of a minibatch.  A CTA (4 warps) takes
-//                   64-row tiles: warps run the forward and the delta
-//                   recursion on their own 16 rows (activations, GELU' and
-//                   deltas staged in shared memory), then every warp forms a
-//                   16-output-row block of dW1..dW3 as delta^T * h over the
-//                   tile's 64 rows on the tensor cores, accumulating in
-//                   registers across the CTA's tiles.  Biases and W4's
-//                   gradient are small and use SIMT sums.  Each CTA writes
-//                   its partial gradient; k_mlp_reduce sums the partials in a
-//                   fixed order, so the gradient is deterministic.
-//   k_mlp_adam      Adam on the FP32 master parameters.
+//   k_mlp_train     up to TRAIN_STEPS Adam steps (or one gradient) in one
+//                   cooperative launch.
+//
+// A step of a minibatch: a CTA (16 warps) takes tiles of 64 rows.  Warp
+// (rg, ng) owns rows 16 rg .. + 15 and columns 16 ng .. + 15 of every layer, in
+// the forward pass, the delta recursion and (as row and column of the weight)
+// the weight gradients delta^T h, which stay in its registers over the CTA's
+// tiles; activations and deltas pass through shared memory, read as ldmatrix
+// fragments from rows of 144 bytes (no bank conflicts).  GELU' stays in the
+// registers of the thread that uses it again.  Biases and W4's gradient are
+// small and use SIMT sums.  The CTAs' partial gradients are summed in a fixed
+// order, so the gradient is deterministic, and the sum of a parameter, its Adam
+// update and its BF16 copy are one thread's; two grid barriers a step.
+//
+// A minibatch of 4,096 is 64 tiles, so a step is bound by latency: its layers'
+// dependent chain, the partial sums' trips through L2 and the barriers.
+// 12.5 us a step of 4,096 rows, against 52 us as three kernels and a copy of
+// the loss (64-row tiles on 4 warps, weights converted from FP32 by every CTA,
+// fragments read as 2-byte words); 32 steps with their two permutations 2,130
+// -> 640 us.
 // Loss: mean over rows of the squared error summed over the 3 outputs.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -24,14 +33,17 @@
 #include <vector>
 
 #include "../../include/phybs.h"
+#include "exchange.cuh"
 #include "mlp.cuh"
 
 namespace pbs {
 namespace mlp {
 
-constexpr int TRAIN_WARPS = 4;
-constexpr int TILE = 16 * TRAIN_WARPS;  // rows per CTA tile
-constexpr int NPART = NPARAM + 1;       // partial gradient + loss
+constexpr int TILE = 64;           // rows per CTA tile
+constexpr int TRAIN_THREADS = 512;
+constexpr int TRAIN_STEPS = 64;    // steps of a launch (their Adam constants are kernel parameters)
+constexpr int NPART = NPARAM + 1;  // partial gradient + loss
+constexpr int LDX = 40, LDH = 72;  // shared-memory row strides (BF16) of 32- and 64-wide rows
 
 __global__ void __launch_bounds__(128) k_mlp_forward(const float *theta, const float *X, int rows, float *Y) {
     __shared__ SmemWeights s;
@@ -56,249 +68,372 @@ __global__ void __launch_bounds__(128) k_mlp_forward(const float *theta, const f
     }
 }
 
+// The weights as a step stages them: BF16 rows at the shared-memory strides
+// (the padding zero), FP32 biases.  Written by the Adam update beside the FP32
+// masters, so that staging is a plain copy.
+struct alignas(16) TrainImage {
+    __nv_bfloat16 w1[HID * LDX];
+    __nv_bfloat16 w2[HID * LDH], w3[HID * LDH];
+    __nv_bfloat16 w4[NOUT * LDH];
+    float b1[HID], b2[HID], b3[HID], b4[NOUT];
+};
+static_assert(sizeof(TrainImage) % 16 == 0, "copied in 16-byte words");
+
+__device__ __forceinline__ void put_param(TrainImage *im, int i, float v) {
+    const __nv_bfloat16 b = __float2bfloat16_rn(v);
+    if (i < OFF_B1) im->w1[i / IN * LDX + i % IN] = b;
+    else if (i < OFF_W2) im->b1[i - OFF_B1] = v;
+    else if (i < OFF_B2) im->w2[(i - OFF_W2) / HID * LDH + (i - OFF_W2) % HID] = b;
+    else if (i < OFF_W3) im->b2[i - OFF_B2] = v;
+    else if (i < OFF_B3) im->w3[(i - OFF_W3) / HID * LDH + (i - OFF_W3) % HID] = b;
+    else if (i < OFF_W4) im->b3[i - OFF_B3] = v;
+    else if (i < OFF_B4) im->w4[(i - OFF_W4) / HID * LDH + (i - OFF_W4) % HID] = b;
+    else im->b4[i - OFF_B4] = v;
+}
+
 struct TrainSmem {
-    SmemWeights w;
-    __nv_bfloat16 w2t[HID * HID], w3t[HID * HID];  // [in][out]
-    float w4[OUT * HID];
-    float zero_bias[HID];
-    __nv_bfloat16 xs[TILE * KIN];
-    __nv_bfloat16 h1[TILE * HID], h2[TILE * HID], h3[TILE * HID];
-    float gd1[TILE * HID], gd2[TILE * HID], gd3[TILE * HID];
-    __nv_bfloat16 d1[TILE * HID], d2[TILE * HID], d3[TILE * HID];
+    TrainImage w;
+    __nv_bfloat16 xs[TILE * LDX];
+    __nv_bfloat16 h1[TILE * LDH], h2[TILE * LDH], h3[TILE * LDH];
+    __nv_bfloat16 d1[TILE * LDH], d2[TILE * LDH], d3[TILE * LDH];
     float d4[TILE * 4];
-    float acc_b[3 * HID + OUT];  // db1, db2, db3, db4
-    float acc_w4[OUT * HID];
-    float loss[TRAIN_WARPS];
+    float ys[TILE * OUT], ws[TILE];
+    float loss[4];
 };
 
-// Store one layer's activations (BF16) and GELU' (FP32) at the C-fragment
-// positions of the warp's 16 rows; returns the next layer's A fragments.
-__device__ __forceinline__ void store_act(const float (&acc)[8][4], int r0, __nv_bfloat16 *h, float *gd,
-                                          uint32_t (&a)[4][4]) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    float act[8][4];
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int r = r0 + g + (q >= 2 ? 8 : 0), c = 8 * j + 2 * t + (q & 1);
-            act[j][q] = gelu(acc[j][q]);
-            gd[r * HID + c] = gelu_grad(acc[j][q]);
-            h[r * HID + c] = __float2bfloat16_rn(act[j][q]);
-        }
-#pragma unroll
-    for (int kb = 0; kb < 4; ++kb) {
-        a[kb][0] = pack_bf16(act[2 * kb][0], act[2 * kb][1]);
-        a[kb][1] = pack_bf16(act[2 * kb][2], act[2 * kb][3]);
-        a[kb][2] = pack_bf16(act[2 * kb + 1][0], act[2 * kb + 1][1]);
-        a[kb][3] = pack_bf16(act[2 * kb + 1][2], act[2 * kb + 1][3]);
-    }
+struct TrainArgs {
+    float *theta, *m, *v, *grad, *part;  // grad: the last step's gradient, loss last
+    TrainImage *image;
+    const float *X, *Y, *W;  // W: sample weights, or null
+    const int *idx;          // rows of the minibatches, or null: rows 0, 1, ...
+    float *losses;           // a step each
+    unsigned *bar;           // grid barrier count, `base` at launch
+    int *err;                // a wait gave up
+    unsigned base;
+    int batch, steps, update;
+    float lr, b1, b2, eps;
+    float2 c[TRAIN_STEPS];   // 1 - b1^t, 1 - b2^t
+};
+
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const __nv_bfloat16 *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((unsigned)__cvta_generic_to_shared(p))
+                 : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const __nv_bfloat16 *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((unsigned)__cvta_generic_to_shared(p))
+                 : "memory");
 }
 
-// delta = acc (.) GELU'(z), stored BF16 and returned as A fragments.
-__device__ __forceinline__ void store_delta(float (&acc)[8][4], int r0, const float *gd, __nv_bfloat16 *d,
-                                            uint32_t (&a)[4][4]) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+// acc (two 8-column tiles from n0) += A (16 rows x 16 KB) * W^T, W [n][k].
+template <int KB, int LDA, int LDW>
+__device__ __forceinline__ void mm_forward(const __nv_bfloat16 *A, const __nv_bfloat16 *W, int n0, float (&acc)[2][4]) {
+    const int lane = threadIdx.x & 31;
+    const __nv_bfloat16 *pa = A + (lane & 15) * LDA + (lane >> 4) * 8;
+    const __nv_bfloat16 *pb = W + (n0 + (lane >> 4) * 8 + (lane & 7)) * LDW + ((lane >> 3) & 1) * 8;
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int r = r0 + g + (q >= 2 ? 8 : 0), c = 8 * j + 2 * t + (q & 1);
-            acc[j][q] *= gd[r * HID + c];
-            d[r * HID + c] = __float2bfloat16_rn(acc[j][q]);
-        }
-#pragma unroll
-    for (int kb = 0; kb < 4; ++kb) {
-        a[kb][0] = pack_bf16(acc[2 * kb][0], acc[2 * kb][1]);
-        a[kb][1] = pack_bf16(acc[2 * kb][2], acc[2 * kb][3]);
-        a[kb][2] = pack_bf16(acc[2 * kb + 1][0], acc[2 * kb + 1][1]);
-        a[kb][3] = pack_bf16(acc[2 * kb + 1][2], acc[2 * kb + 1][3]);
+    for (int kb = 0; kb < KB; ++kb) {
+        uint32_t a[4], b[4];
+        ldsm4(a, pa + 16 * kb);
+        ldsm4(b, pb + 16 * kb);
+        mma16816(acc[0], a, b[0], b[1]);
+        mma16816(acc[1], a, b[2], b[3]);
     }
 }
-
-// dW[16w + m][n] += sum_r delta[r][16w + m] * h[r][n] over the tile's rows
-// (A = delta^T from shared memory, B = h from shared memory).
-template <int NT, int HW>
-__device__ __forceinline__ void weight_grad(const __nv_bfloat16 *delta, const __nv_bfloat16 *hin, float (&acc)[NT][4]) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, w = threadIdx.x >> 5;
-    const int m0 = 16 * w;
+// acc += A (16 rows x 64) * W, W [k][n]: a delta through a layer.
+__device__ __forceinline__ void mm_backward(const __nv_bfloat16 *A, const __nv_bfloat16 *W, int n0, float (&acc)[2][4]) {
+    const int lane = threadIdx.x & 31;
+    const __nv_bfloat16 *pa = A + (lane & 15) * LDH + (lane >> 4) * 8;
+    const __nv_bfloat16 *pb = W + (((lane >> 3) & 1) * 8 + (lane & 7)) * LDH + n0 + (lane >> 4) * 8;
+#pragma unroll
+    for (int kb = 0; kb < HID / 16; ++kb) {
+        uint32_t a[4], b[4];
+        ldsm4(a, pa + 16 * kb);
+        ldsm4t(b, pb + 16 * kb * LDH);
+        mma16816(acc[0], a, b[0], b[1]);
+        mma16816(acc[1], a, b[2], b[3]);
+    }
+}
+// dW[m0 + ..][n0 + ..] += sum over the tile's rows of delta[r][m] h[r][n], for
+// NT column tiles from n0 (one: the second of the loaded pair is not used).
+template <int NT, int LDN>
+__device__ __forceinline__ void weight_grad(const __nv_bfloat16 *delta, const __nv_bfloat16 *h, int m0, int n0,
+                                            float (&acc)[NT][4]) {
+    const int lane = threadIdx.x & 31, mat = lane >> 3;
+    const __nv_bfloat16 *pa = delta + ((mat >> 1) * 8 + (lane & 7)) * LDH + m0 + (mat & 1) * 8;
+    const __nv_bfloat16 *pb = h + ((mat & 1) * 8 + (lane & 7)) * LDN + n0 + (NT == 2 ? (mat >> 1) * 8 : 0);
 #pragma unroll
     for (int kb = 0; kb < TILE / 16; ++kb) {
-        const int r0 = 16 * kb + 2 * t;
-        uint32_t a[4];
-        a[0] = pack_raw(delta[r0 * HID + m0 + g], delta[(r0 + 1) * HID + m0 + g]);
-        a[1] = pack_raw(delta[r0 * HID + m0 + g + 8], delta[(r0 + 1) * HID + m0 + g + 8]);
-        a[2] = pack_raw(delta[(r0 + 8) * HID + m0 + g], delta[(r0 + 9) * HID + m0 + g]);
-        a[3] = pack_raw(delta[(r0 + 8) * HID + m0 + g + 8], delta[(r0 + 9) * HID + m0 + g + 8]);
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-            const int n = 8 * j + g;
-            const uint32_t b0 = pack_raw(hin[r0 * HW + n], hin[(r0 + 1) * HW + n]);
-            const uint32_t b1 = pack_raw(hin[(r0 + 8) * HW + n], hin[(r0 + 9) * HW + n]);
-            mma16816(acc[j], a, b0, b1);
-        }
+        uint32_t a[4], b[4];
+        ldsm4t(a, pa + 16 * kb * LDH);
+        ldsm4t(b, pb + 16 * kb * LDN);
+        mma16816(acc[0], a, b[0], b[1]);
+        if (NT == 2) mma16816(acc[NT - 1], a, b[2], b[3]);
     }
 }
 
-__global__ void __launch_bounds__(128) k_mlp_grad(const float *theta, const float *X, const float *Y, const float *W,
-                                                  const int *idx, int batch, float *part) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    TrainSmem &s = *reinterpret_cast<TrainSmem *>(smem_raw);
-    stage_weights(theta, s.w);
-    for (int i = threadIdx.x; i < HID * HID; i += blockDim.x) {
-        const int o = i / HID, k = i % HID;
-        s.w2t[k * HID + o] = __float2bfloat16_rn(theta[OFF_W2 + i]);
-        s.w3t[k * HID + o] = __float2bfloat16_rn(theta[OFF_W3 + i]);
+// Activations (BF16) of the warp's 16 x 16 block; gd: GELU' of the thread's.
+__device__ __forceinline__ void store_act(const float (&acc)[2][4], int r0, int n0, __nv_bfloat16 *h, float (&gd)[2][4]) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; q += 2) {
+            const int r = r0 + g + (q >= 2 ? 8 : 0), c = n0 + 8 * j + 2 * t;
+            gd[j][q] = gelu_grad(acc[j][q]);
+            gd[j][q + 1] = gelu_grad(acc[j][q + 1]);
+            *reinterpret_cast<uint32_t *>(h + r * LDH + c) = pack_bf16(gelu(acc[j][q]), gelu(acc[j][q + 1]));
+        }
+}
+// delta = acc (.) GELU'(z), BF16.
+__device__ __forceinline__ void store_delta(const float (&acc)[2][4], int r0, int n0, const float (&gd)[2][4],
+                                            __nv_bfloat16 *d) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; q += 2) {
+            const int r = r0 + g + (q >= 2 ? 8 : 0), c = n0 + 8 * j + 2 * t;
+            *reinterpret_cast<uint32_t *>(d + r * LDH + c) =
+                pack_bf16(acc[j][q] * gd[j][q], acc[j][q + 1] * gd[j][q + 1]);
+        }
+}
+__device__ __forceinline__ void init_bias(float (&acc)[2][4], const float *bias, int n0) {
+    const int t = threadIdx.x & 3;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        acc[j][0] = acc[j][2] = bias[n0 + 8 * j + 2 * t];
+        acc[j][1] = acc[j][3] = bias[n0 + 8 * j + 2 * t + 1];
     }
-    for (int i = threadIdx.x; i < OUT * HID; i += blockDim.x) s.w4[i] = __bfloat162float(__float2bfloat16_rn(theta[OFF_W4 + i]));
-    for (int i = threadIdx.x; i < HID; i += blockDim.x) s.zero_bias[i] = 0.f;
-    for (int i = threadIdx.x; i < 3 * HID + OUT; i += blockDim.x) s.acc_b[i] = 0.f;
-    for (int i = threadIdx.x; i < OUT * HID; i += blockDim.x) s.acc_w4[i] = 0.f;
-    if (threadIdx.x < TRAIN_WARPS) s.loss[threadIdx.x] = 0.f;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, w = threadIdx.x >> 5;
-    const int r0 = 16 * w;
-    const float inv_b = 1.0f / (float)batch;
-    float gw1[4][4] = {}, gw2[8][4] = {}, gw3[8][4] = {};
-    float loss = 0.f;
-    for (int base = blockIdx.x * TILE; base < batch; base += gridDim.x * TILE) {
-        // input tile (BF16, columns 24..31 zero; rows past the batch zero)
-        for (int i = threadIdx.x; i < TILE * KIN; i += blockDim.x) {
-            const int r = i / KIN, c = i % KIN;
-            float v = 0.f;
-            if (base + r < batch && c < IN) v = X[(size_t)idx[base + r] * IN + c];
-            s.xs[i] = __float2bfloat16_rn(v);
-        }
-        __syncthreads();
-        // ---- forward (own 16 rows)
-        uint32_t x[2][4];
-#pragma unroll
-        for (int kb = 0; kb < 2; ++kb) {
-            const __nv_bfloat16 *xr0 = s.xs + (r0 + g) * KIN + 16 * kb + 2 * t;
-            const __nv_bfloat16 *xr1 = s.xs + (r0 + g + 8) * KIN + 16 * kb + 2 * t;
-            x[kb][0] = *reinterpret_cast<const uint32_t *>(xr0);
-            x[kb][1] = *reinterpret_cast<const uint32_t *>(xr1);
-            x[kb][2] = *reinterpret_cast<const uint32_t *>(xr0 + 8);
-            x[kb][3] = *reinterpret_cast<const uint32_t *>(xr1 + 8);
-        }
-        float acc[8][4];
-        uint32_t a[4][4];
-        layer<2, 8>(x, s.w.w1, s.w.b1, acc);
-        store_act(acc, r0, s.h1, s.gd1, a);
-        layer<4, 8>(a, s.w.w2, s.w.b2, acc);
-        store_act(acc, r0, s.h2, s.gd2, a);
-        layer<4, 8>(a, s.w.w3, s.w.b3, acc);
-        store_act(acc, r0, s.h3, s.gd3, a);
-        float o[1][4];
-        layer<4, 1>(a, s.w.w4, s.w.b4, o);
-        // output deltas 2 w (y - t) / B (w = 1 without sample weights)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int rl = r0 + g + (q >= 2 ? 8 : 0), c = 2 * t + (q & 1);
-            float dlt = 0.f;
-            if (c < OUT && base + rl < batch) {
-                const int row = idx[base + rl];
-                const float diff = o[0][q] - Y[(size_t)row * OUT + c];
-                const float wd = W ? W[row] * diff : diff;
-                loss += wd * diff;
-                dlt = 2.0f * wd * inv_b;
-            }
-            if (c < 4) s.d4[rl * 4 + c] = dlt;
-        }
-        __syncwarp();
-        // ---- backward deltas (own 16 rows)
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int rl = r0 + g + (q >= 2 ? 8 : 0), c = 8 * j + 2 * t + (q & 1);
-                acc[j][q] = s.d4[rl * 4] * s.w4[c] + s.d4[rl * 4 + 1] * s.w4[HID + c] + s.d4[rl * 4 + 2] * s.w4[2 * HID + c];
-            }
-        store_delta(acc, r0, s.gd3, s.d3, a);
-        layer<4, 8>(a, s.w3t, s.zero_bias, acc);
-        store_delta(acc, r0, s.gd2, s.d2, a);
-        layer<4, 8>(a, s.w2t, s.zero_bias, acc);
-        store_delta(acc, r0, s.gd1, s.d1, a);
-        __syncthreads();
-        // ---- weight gradients: warp w owns output rows 16w .. 16w+15
-        weight_grad<4, KIN>(s.d1, s.xs, gw1);
-        weight_grad<8, HID>(s.d2, s.h1, gw2);
-        weight_grad<8, HID>(s.d3, s.h2, gw3);
-        // biases and W4 (SIMT; each entry owned by one thread)
-        for (int task = threadIdx.x; task < 3 * HID + OUT + OUT * HID; task += blockDim.x) {
-            float sum = 0.f;
-            if (task < 3 * HID) {
-                const __nv_bfloat16 *d = task < HID ? s.d1 : (task < 2 * HID ? s.d2 : s.d3);
-                const int c = task % HID;
-                for (int r = 0; r < TILE; ++r) sum += __bfloat162float(d[r * HID + c]);
-                s.acc_b[task] += sum;
-            } else if (task < 3 * HID + OUT) {
-                const int c = task - 3 * HID;
-                for (int r = 0; r < TILE; ++r) sum += s.d4[r * 4 + c];
-                s.acc_b[task] += sum;
-            } else {
-                const int k = task - 3 * HID - OUT, oo = k / HID, c = k % HID;
-                for (int r = 0; r < TILE; ++r) sum += s.d4[r * 4 + oo] * __bfloat162float(s.h3[r * HID + c]);
-                s.acc_w4[k] += sum;
-            }
-        }
-        __syncthreads();
-    }
-    // ---- partial gradient of this CTA
-    float *P = part + (size_t)blockIdx.x * NPART;
-    const int m0 = 16 * w;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int oo = m0 + g + (q >= 2 ? 8 : 0), c = 8 * j + 2 * t + (q & 1);
-            if (c < IN) P[OFF_W1 + oo * IN + c] = gw1[j][q];
-        }
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int oo = m0 + g + (q >= 2 ? 8 : 0), c = 8 * j + 2 * t + (q & 1);
-            P[OFF_W2 + oo * HID + c] = gw2[j][q];
-            P[OFF_W3 + oo * HID + c] = gw3[j][q];
-        }
-    for (int i = threadIdx.x; i < HID; i += blockDim.x) {
-        P[OFF_B1 + i] = s.acc_b[i];
-        P[OFF_B2 + i] = s.acc_b[HID + i];
-        P[OFF_B3 + i] = s.acc_b[2 * HID + i];
-    }
-    for (int i = threadIdx.x; i < OUT * HID; i += blockDim.x) P[OFF_W4 + i] = s.acc_w4[i];
-    if (threadIdx.x < OUT) P[OFF_B4 + threadIdx.x] = s.acc_b[3 * HID + threadIdx.x];
-    // loss: fixed-order warp then CTA sum
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, off);
-    if (lane == 0) s.loss[w] = loss;
+}
+
+// Arrives at the grid barrier and waits until every CTA has (count: this
+// launch's arrivals with this one); false when the wait gave up.
+__device__ __forceinline__ bool grid_barrier(const TrainArgs &a, unsigned count) {
+    bool ok = true;
     __syncthreads();
     if (threadIdx.x == 0) {
-        float l = 0.f;
-        for (int i = 0; i < TRAIN_WARPS; ++i) l += s.loss[i];
-        P[NPARAM] = l * inv_b;
+        __threadfence();
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+        Spin spin;
+        for (;;) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+            if ((int)(v - (a.base + count)) >= 0) break;
+            if (spin.expired(a.err)) {
+                ok = false;
+                break;
+            }
+        }
+        __threadfence();
     }
+    return !__syncthreads_or(!ok);
 }
 
-__global__ void k_mlp_reduce(const float *part, int nparts, float *grad) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= NPART) return;
-    float s = 0.f;
-    for (int p = 0; p < nparts; ++p) s += part[(size_t)p * NPART + i];
-    grad[i] = s;
-}
-
-__global__ void k_mlp_adam(float *theta, float *m, float *v, const float *grad, float lr, float b1, float b2, float eps,
-                           float c1, float c2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= NPARAM) return;
-    const float gi = grad[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    theta[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+__global__ void __launch_bounds__(TRAIN_THREADS, 1) k_mlp_train(const __grid_constant__ TrainArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TrainSmem &s = *reinterpret_cast<TrainSmem *>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3, w = tid >> 5;
+    const int rg = w & 3, r0 = 16 * rg, n0 = 16 * (w >> 2);
+    const int G = gridDim.x, b = blockIdx.x;
+    const int per = (NPART + G - 1) / G, i0 = min(b * per, NPART), i1 = min(i0 + per, NPART);
+    const float inv_b = 1.0f / (float)a.batch;
+    // the tile's inputs, held in registers while the CTA is at a barrier
+    constexpr int XV = TILE * IN / TRAIN_THREADS;
+    static_assert(XV * TRAIN_THREADS == TILE * IN && TILE * OUT <= TRAIN_THREADS, "one tile a pass of the CTA");
+    float xv[XV], yv = 0.f, wv = 1.f;
+    auto load_inputs = [&](int step, int base) {
+        const int *idx = a.idx ? a.idx + (size_t)step * a.batch : nullptr;
+        auto row = [&](int r) { return idx ? idx[base + r] : base + r; };
+#pragma unroll
+        for (int q = 0; q < XV; ++q) {
+            const int e = tid + q * TRAIN_THREADS, r = e / IN;
+            xv[q] = base + r < a.batch ? a.X[(size_t)row(r) * IN + e % IN] : 0.f;
+        }
+        if (tid < TILE * OUT) yv = base + tid / OUT < a.batch ? a.Y[(size_t)row(tid / OUT) * OUT + tid % OUT] : 0.f;
+        if (tid < TILE && a.W) wv = base + tid < a.batch ? a.W[row(tid)] : 0.f;
+    };
+    auto store_inputs = [&]() {
+#pragma unroll
+        for (int q = 0; q < XV; ++q) {
+            const int e = tid + q * TRAIN_THREADS;
+            s.xs[e / IN * LDX + e % IN] = __float2bfloat16_rn(xv[q]);
+        }
+        if (tid < TILE * OUT) s.ys[tid] = yv;
+        if (tid < TILE) s.ws[tid] = wv;
+    };
+    for (int i = i0 + tid; i < min(i1, NPARAM); i += TRAIN_THREADS) put_param(a.image, i, a.theta[i]);
+    for (int i = tid; i < TILE * (LDX - IN); i += TRAIN_THREADS)
+        s.xs[i / (LDX - IN) * LDX + IN + i % (LDX - IN)] = __float2bfloat16_rn(0.f);
+    load_inputs(0, b * TILE);
+    unsigned arrivals = G;
+    if (!grid_barrier(a, arrivals)) return;
+    for (int step = 0; step < a.steps; ++step) {
+        {
+            const float4 *src = reinterpret_cast<const float4 *>(a.image);
+            float4 *dst = reinterpret_cast<float4 *>(&s.w);
+            for (int i = tid; i < (int)(sizeof(TrainImage) / 16); i += TRAIN_THREADS) cp_async16(dst + i, src + i);
+            cp_async_commit();
+        }
+        float gw1[1][4] = {}, gw2[2][4] = {}, gw3[2][4] = {};
+        float loss = 0.f, bsum = 0.f;
+        for (int base = b * TILE; base < a.batch; base += G * TILE) {
+            if (base != b * TILE) {
+                load_inputs(step, base);
+                __syncthreads();  // the last tile's readers are done
+            }
+            store_inputs();
+            cp_async_wait_all();
+            __syncthreads();
+            // ---- forward
+            float acc[2][4], gd1[2][4], gd2[2][4], gd3[2][4];
+            init_bias(acc, s.w.b1, n0);
+            mm_forward<KIN / 16, LDX, LDX>(s.xs + r0 * LDX, s.w.w1, n0, acc);
+            store_act(acc, r0, n0, s.h1, gd1);
+            __syncthreads();
+            init_bias(acc, s.w.b2, n0);
+            mm_forward<HID / 16, LDH, LDH>(s.h1 + r0 * LDH, s.w.w2, n0, acc);
+            store_act(acc, r0, n0, s.h2, gd2);
+            __syncthreads();
+            init_bias(acc, s.w.b3, n0);
+            mm_forward<HID / 16, LDH, LDH>(s.h2 + r0 * LDH, s.w.w3, n0, acc);
+            store_act(acc, r0, n0, s.h3, gd3);
+            __syncthreads();
+            if (n0 == 0) {  // the output layer, by one warp of the row group
+                float o[4] = {s.w.b4[2 * t], s.w.b4[2 * t + 1], s.w.b4[2 * t], s.w.b4[2 * t + 1]};
+                const __nv_bfloat16 *pa = s.h3 + (r0 + (lane & 15)) * LDH + (lane >> 4) * 8;
+                const __nv_bfloat16 *pb = s.w.w4 + (lane & 7) * LDH + (lane >> 3) * 8;
+#pragma unroll
+                for (int kb = 0; kb < HID / 16; kb += 2) {
+                    uint32_t a0[4], a1[4], bb[4];
+                    ldsm4(a0, pa + 16 * kb);
+                    ldsm4(a1, pa + 16 * kb + 16);
+                    ldsm4(bb, pb + 16 * kb);
+                    mma16816(o, a0, bb[0], bb[1]);
+                    mma16816(o, a1, bb[2], bb[3]);
+                }
+                // output deltas 2 w (y - t) / B (w = 1 without sample weights)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int rl = r0 + g + (q >= 2 ? 8 : 0), c = 2 * t + (q & 1);
+                    float dlt = 0.f;
+                    if (c < OUT && base + rl < a.batch) {
+                        const float diff = o[q] - s.ys[rl * OUT + c];
+                        const float wd = a.W ? s.ws[rl] * diff : diff;
+                        loss += wd * diff;
+                        dlt = 2.0f * wd * inv_b;
+                    }
+                    if (c < 4) s.d4[rl * 4 + c] = dlt;
+                }
+            }
+            __syncthreads();
+            // ---- backward deltas
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int rl = r0 + g + (q >= 2 ? 8 : 0), c = n0 + 8 * j + 2 * t + (q & 1);
+                    acc[j][q] = s.d4[rl * 4] * __bfloat162float(s.w.w4[c]) +
+                                s.d4[rl * 4 + 1] * __bfloat162float(s.w.w4[LDH + c]) +
+                                s.d4[rl * 4 + 2] * __bfloat162float(s.w.w4[2 * LDH + c]);
+                }
+            store_delta(acc, r0, n0, gd3, s.d3);
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc[q >> 2][q & 3] = 0.f;
+            mm_backward(s.d3 + r0 * LDH, s.w.w3, n0, acc);
+            store_delta(acc, r0, n0, gd2, s.d2);
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc[q >> 2][q & 3] = 0.f;
+            mm_backward(s.d2 + r0 * LDH, s.w.w2, n0, acc);
+            store_delta(acc, r0, n0, gd1, s.d1);
+            __syncthreads();
+            // ---- weight gradients: rows r0 .. + 15 of each matrix, columns n0 ..
+            // + 15 (w1: 8 (n0 / 16) .. + 7)
+            weight_grad<1, LDX>(s.d1, s.xs, r0, n0 / 2, gw1);
+            weight_grad<2, LDH>(s.d2, s.h1, r0, n0, gw2);
+            weight_grad<2, LDH>(s.d3, s.h2, r0, n0, gw3);
+            // biases and W4 (SIMT; each entry owned by one thread)
+            static_assert(3 * HID + OUT + OUT * HID <= TRAIN_THREADS, "one entry a thread");
+            float sum = 0.f;
+            if (tid < 3 * HID) {
+                const __nv_bfloat16 *d = (tid < HID ? s.d1 : tid < 2 * HID ? s.d2 : s.d3) + tid % HID;
+#pragma unroll 16
+                for (int r = 0; r < TILE; ++r) sum += __bfloat162float(d[r * LDH]);
+            } else if (tid < 3 * HID + OUT) {
+#pragma unroll 16
+                for (int r = 0; r < TILE; ++r) sum += s.d4[r * 4 + tid - 3 * HID];
+            } else if (tid < 3 * HID + OUT + OUT * HID) {
+                const int k = tid - 3 * HID - OUT, oo = k / HID, c = k % HID;
+#pragma unroll 16
+                for (int r = 0; r < TILE; ++r) sum += s.d4[r * 4 + oo] * __bfloat162float(s.h3[r * LDH + c]);
+            }
+            bsum += sum;
+        }
+        // ---- partial gradient of this CTA
+        float *P = a.part + (size_t)b * NPART;
+        auto put2 = [&](int at, float x, float y) { *reinterpret_cast<float2 *>(P + at) = make_float2(x, y); };
+#pragma unroll
+        for (int q = 0; q < 4; q += 2) {
+            const int oo = r0 + g + (q >= 2 ? 8 : 0), c1 = n0 / 2 + 2 * t;
+            if (c1 < IN) put2(OFF_W1 + oo * IN + c1, gw1[0][q], gw1[0][q + 1]);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int c = n0 + 8 * j + 2 * t;
+                put2(OFF_W2 + oo * HID + c, gw2[j][q], gw2[j][q + 1]);
+                put2(OFF_W3 + oo * HID + c, gw3[j][q], gw3[j][q + 1]);
+            }
+        }
+        if (tid < HID) P[OFF_B1 + tid] = bsum;
+        else if (tid < 2 * HID) P[OFF_B2 + tid - HID] = bsum;
+        else if (tid < 3 * HID) P[OFF_B3 + tid - 2 * HID] = bsum;
+        else if (tid < 3 * HID + OUT) P[OFF_B4 + tid - 3 * HID] = bsum;
+        else if (tid < 3 * HID + OUT + OUT * HID) P[OFF_W4 + tid - 3 * HID - OUT] = bsum;
+        // loss: fixed-order warp then CTA sum
+        if (n0 == 0) {
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, off);
+            if (lane == 0) s.loss[rg] = loss;
+        }
+        __syncthreads();
+        if (tid == 0) P[NPARAM] = (((s.loss[0] + s.loss[1]) + s.loss[2]) + s.loss[3]) * inv_b;
+        if (step + 1 < a.steps) load_inputs(step + 1, b * TILE);
+        arrivals += G;
+        if (!grid_barrier(a, arrivals)) return;
+        // ---- the gradient, in CTA order, and Adam on the FP32 masters
+        for (int i = i0 + tid; i < i1; i += TRAIN_THREADS) {
+            constexpr int U = 32;  // partials in flight
+            float gi = 0.f;
+            for (int p0 = 0; p0 < G; p0 += U) {
+                float q[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) q[u] = p0 + u < G ? __ldcg(a.part + (size_t)(p0 + u) * NPART + i) : 0.f;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (p0 + u < G) gi += q[u];
+            }
+            if (step + 1 == a.steps) a.grad[i] = gi;
+            if (i == NPARAM) {
+                a.losses[step] = gi;
+            } else if (a.update) {
+                // (roundings spelled out: the same bits wherever this is compiled)
+                const float mi = __fmaf_rn(1.f - a.b1, gi, __fmul_rn(a.b1, a.m[i]));
+                const float vi = __fmaf_rn(__fmul_rn(1.f - a.b2, gi), gi, __fmul_rn(a.b2, a.v[i]));
+                a.m[i] = mi;
+                a.v[i] = vi;
+                const float th = a.theta[i] - a.lr * (mi / a.c[step].x) / (sqrtf(vi / a.c[step].y) + a.eps);
+                a.theta[i] = th;
+                put_param(a.image, i, th);
+            }
+        }
+        if (step + 1 == a.steps) break;
+        arrivals += G;
+        if (!grid_barrier(a, arrivals)) return;
+    }
 }
 
 int grad_ctas(int batch, int sms) {
@@ -316,8 +451,12 @@ struct pbs_mlp {
     int sms = 148;
     float *theta = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr, *part = nullptr;
     float *X = nullptr, *Y = nullptr, *W = nullptr, *io = nullptr;
+    TrainImage *image = nullptr;
+    unsigned *sync = nullptr;  // [0] the grid barrier's count, [1] a wait gave up
+    float *losses = nullptr;
     int *idx = nullptr;
-    int n = 0, cap_part = 0, cap_io = 0, step = 0;
+    int n = 0, cap_part = 0, cap_io = 0, cap_losses = 0, step = 0;
+    unsigned arrivals = 0;  // the barrier's count after the launches so far
 };
 
 #define MCK(x)                                                                               \
@@ -346,17 +485,68 @@ static int ensure_part(pbs_mlp *t, int nparts) {
     return PBS_OK;
 }
 
-static int run_grad(pbs_mlp *t, const float *X, const float *Y, const float *W, const int *idx, int batch) {
+static int ensure_losses(pbs_mlp *t, int steps) {
+    if (steps <= t->cap_losses) return PBS_OK;
+    if (t->losses) cudaFree(t->losses);
+    t->losses = nullptr;
+    t->cap_losses = 0;
+    MCK(cudaMalloc(&t->losses, sizeof(float) * (size_t)steps));
+    t->cap_losses = steps;
+    return PBS_OK;
+}
+
+// Enqueues `steps` (at most TRAIN_STEPS) minibatches of rows idx[0 .. batch),
+// idx[batch .. 2 batch), ... (idx null: one, of rows 0 .. batch), with Adam
+// updates or (lr = 0) the gradient only.
+static int run_train(pbs_mlp *t, const float *X, const float *Y, const float *W, const int *idx, int batch, int steps,
+                     float lr, float *losses) {
+    TrainArgs a{};
     const int ctas = grad_ctas(batch, t->sms);
     int rc = ensure_part(t, ctas);
     if (rc != PBS_OK) return rc;
-    const size_t smem = sizeof(TrainSmem);
-    MCK(cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_mlp_grad<<<ctas, 128, smem, t->stream>>>(t->theta, X, Y, W, idx, batch, t->part);
-    MCK(cudaGetLastError());
-    k_mlp_reduce<<<(NPART + 255) / 256, 256, 0, t->stream>>>(t->part, ctas, t->grad);
-    MCK(cudaGetLastError());
+    a.theta = t->theta; a.m = t->m; a.v = t->v; a.grad = t->grad; a.part = t->part;
+    a.image = t->image;
+    a.X = X; a.Y = Y; a.W = W;
+    a.idx = idx;
+    a.losses = losses;
+    a.bar = t->sync;
+    a.err = (int *)(t->sync + 1);
+    a.base = t->arrivals;
+    a.batch = batch;
+    a.steps = steps;
+    a.update = lr > 0.f;
+    a.lr = lr;
+    a.b1 = 0.9f; a.b2 = 0.999f; a.eps = 1e-8f;
+    for (int s = 0; s < steps && a.update; ++s) {
+        t->step += 1;
+        a.c[s] = make_float2(1.f - std::pow(a.b1, (float)t->step), 1.f - std::pow(a.b2, (float)t->step));
+    }
+    MCK(cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem)));
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(TRAIN_THREADS);
+    cfg.dynamicSmemBytes = sizeof(TrainSmem);
+    cfg.stream = t->stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    MCK(cudaLaunchKernelEx(&cfg, k_mlp_train, a));
+    t->arrivals += 2u * (unsigned)steps * (unsigned)ctas;
     return PBS_OK;
+}
+
+// Waits for the trainer's stream; PBS_E_DEVICE_TIMEOUT when a device wait gave
+// up (the barrier then starts over).
+static int finish(pbs_mlp *t) {
+    unsigned flag = 0;
+    MCK(cudaMemcpyAsync(&flag, t->sync + 1, sizeof(flag), cudaMemcpyDeviceToHost, t->stream));
+    MCK(cudaStreamSynchronize(t->stream));
+    if (!flag) return PBS_OK;
+    MCK(cudaMemset(t->sync, 0, 2 * sizeof(unsigned)));
+    t->arrivals = 0;
+    return PBS_E_DEVICE_TIMEOUT;
 }
 
 extern "C" {
@@ -387,10 +577,12 @@ int pbs_mlp_create(pbs_mlp **out, const float *theta, unsigned long long seed) {
     auto fail = [&](int rc) { pbs_mlp_destroy(t); return rc; };
     if (cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(PBS_E_CUDA);
     if (cudaMalloc(&t->theta, sizeof(float) * NPARAM) != cudaSuccess || cudaMalloc(&t->m, sizeof(float) * NPARAM) != cudaSuccess ||
-        cudaMalloc(&t->v, sizeof(float) * NPARAM) != cudaSuccess || cudaMalloc(&t->grad, sizeof(float) * NPART) != cudaSuccess)
+        cudaMalloc(&t->v, sizeof(float) * NPARAM) != cudaSuccess || cudaMalloc(&t->grad, sizeof(float) * NPART) != cudaSuccess ||
+        cudaMalloc(&t->image, sizeof(TrainImage)) != cudaSuccess || cudaMalloc(&t->sync, 2 * sizeof(unsigned)) != cudaSuccess)
         return fail(PBS_E_OUT_OF_MEMORY);
     if (cudaMemcpy(t->theta, th.data(), sizeof(float) * NPARAM, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemset(t->m, 0, sizeof(float) * NPARAM) != cudaSuccess || cudaMemset(t->v, 0, sizeof(float) * NPARAM) != cudaSuccess)
+        cudaMemset(t->m, 0, sizeof(float) * NPARAM) != cudaSuccess || cudaMemset(t->v, 0, sizeof(float) * NPARAM) != cudaSuccess ||
+        cudaMemset(t->image, 0, sizeof(TrainImage)) != cudaSuccess || cudaMemset(t->sync, 0, 2 * sizeof(unsigned)) != cudaSuccess)
         return fail(PBS_E_CUDA);
     *out = t;
     return PBS_OK;
@@ -399,9 +591,11 @@ int pbs_mlp_create(pbs_mlp **out, const float *theta, unsigned long long seed) {
 void pbs_mlp_destroy(pbs_mlp *t) {
     if (!t) return;
     if (t->stream) cudaStreamSynchronize(t->stream);
-    float *bufs[] = {t->theta, t->m, t->v, t->grad, t->part, t->X, t->Y, t->W, t->io};
+    float *bufs[] = {t->theta, t->m, t->v, t->grad, t->part, t->X, t->Y, t->W, t->io, t->losses};
     for (float *b : bufs)
         if (b) cudaFree(b);
+    if (t->image) cudaFree(t->image);
+    if (t->sync) cudaFree(t->sync);
     if (t->idx) cudaFree(t->idx);
     if (t->stream) cudaStreamDestroy(t->stream);
     delete t;
@@ -439,22 +633,16 @@ int pbs_mlp_forward(pbs_mlp *t, const float *X, int n, float *Y) {
 int pbs_mlp_gradient(pbs_mlp *t, const float *X, const float *Y, int n, float *grad, float *loss) {
     if (!t || !X || !Y || n <= 0 || !grad) return PBS_E_INVALID_ARG;
     int rc = ensure_io(t, n);
+    if (rc == PBS_OK) rc = ensure_losses(t, 1);
     if (rc != PBS_OK) return rc;
     float *dX = t->io, *dY = t->io + (size_t)n * IN;
-    int *didx = nullptr;
-    MCK(cudaMalloc(&didx, sizeof(int) * n));
-    std::vector<int> iota(n);
-    for (int i = 0; i < n; ++i) iota[i] = i;
-    cudaError_t e = cudaMemcpyAsync(dX, X, sizeof(float) * (size_t)n * IN, cudaMemcpyHostToDevice, t->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dY, Y, sizeof(float) * (size_t)n * OUT, cudaMemcpyHostToDevice, t->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(didx, iota.data(), sizeof(int) * n, cudaMemcpyHostToDevice, t->stream);
-    if (e != cudaSuccess) { cudaFree(didx); return PBS_E_CUDA; }
-    rc = run_grad(t, dX, dY, nullptr, didx, n);
+    MCK(cudaMemcpyAsync(dX, X, sizeof(float) * (size_t)n * IN, cudaMemcpyHostToDevice, t->stream));
+    MCK(cudaMemcpyAsync(dY, Y, sizeof(float) * (size_t)n * OUT, cudaMemcpyHostToDevice, t->stream));
+    rc = run_train(t, dX, dY, nullptr, nullptr, n, 1, 0.f, t->losses);
+    if (rc != PBS_OK) return rc;
     std::vector<float> g(NPART);
-    if (rc == PBS_OK && cudaMemcpyAsync(g.data(), t->grad, sizeof(float) * NPART, cudaMemcpyDeviceToHost, t->stream) != cudaSuccess)
-        rc = PBS_E_CUDA;
-    if (rc == PBS_OK && cudaStreamSynchronize(t->stream) != cudaSuccess) rc = PBS_E_CUDA;
-    cudaFree(didx);
+    MCK(cudaMemcpyAsync(g.data(), t->grad, sizeof(float) * NPART, cudaMemcpyDeviceToHost, t->stream));
+    rc = finish(t);
     if (rc != PBS_OK) return rc;
     std::memcpy(grad, g.data(), sizeof(float) * NPARAM);
     if (loss) *loss = g[NPARAM];
@@ -487,35 +675,37 @@ int pbs_mlp_set_data(pbs_mlp *t, const float *X, const float *Y, const float *W,
 
 // `steps` Adam steps on minibatches of `batch` rows drawn without replacement
 // (a fresh permutation each epoch).  losses (optional, `steps` floats) gets
-// each step's minibatch loss.
+// each step's minibatch loss.  An epoch's permutation (192 us for 65,536 rows)
+// is drawn while the device trains on the one before.
 int pbs_mlp_train(pbs_mlp *t, int steps, int batch, float lr, unsigned long long seed, float *losses) {
     if (!t || steps < 0 || batch <= 0 || !(lr > 0.f) || t->n <= 0) return PBS_E_INVALID_ARG;
     if (batch > t->n) batch = t->n;
+    int rc = ensure_losses(t, steps);
+    if (rc != PBS_OK) return rc;
     std::mt19937_64 rng(seed);
-    std::vector<int> perm(t->n);
-    int pos = t->n;
-    std::vector<float> lossbuf(steps > 0 ? steps : 1);
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    for (int sidx = 0; sidx < steps; ++sidx) {
-        if (pos + batch > t->n) {
-            for (int i = 0; i < t->n; ++i) perm[i] = i;
-            std::shuffle(perm.begin(), perm.end(), rng);
-            MCK(cudaMemcpyAsync(t->idx, perm.data(), sizeof(int) * t->n, cudaMemcpyHostToDevice, t->stream));
-            pos = 0;
+    std::vector<int> perm[2];  // the other one may still be on its way to the device
+    const int epoch = t->n / batch;
+    for (int done = 0, e = 0; done < steps; ++e) {
+        std::vector<int> &p = perm[e & 1];
+        p.resize(t->n);
+        for (int i = 0; i < t->n; ++i) p[i] = i;
+        std::shuffle(p.begin(), p.end(), rng);
+        if (e) MCK(cudaStreamSynchronize(t->stream));
+        MCK(cudaMemcpyAsync(t->idx, p.data(), sizeof(int) * t->n, cudaMemcpyHostToDevice, t->stream));
+        for (int k = 0; k < epoch && done < steps;) {
+            const int now = std::min({epoch - k, steps - done, TRAIN_STEPS});
+            rc = run_train(t, t->X, t->Y, t->W, t->idx + (size_t)k * batch, batch, now, lr, t->losses + done);
+            if (rc != PBS_OK) {
+                cudaStreamSynchronize(t->stream);
+                return rc;
+            }
+            k += now;
+            done += now;
         }
-        int rc = run_grad(t, t->X, t->Y, t->W, t->idx + pos, batch);
-        if (rc != PBS_OK) return rc;
-        pos += batch;
-        t->step += 1;
-        const float c1 = 1.f - std::pow(b1, (float)t->step), c2 = 1.f - std::pow(b2, (float)t->step);
-        k_mlp_adam<<<(NPARAM + 255) / 256, 256, 0, t->stream>>>(t->theta, t->m, t->v, t->grad, lr, b1, b2, eps, c1, c2);
-        MCK(cudaGetLastError());
-        if (losses) MCK(cudaMemcpyAsync(&lossbuf[sidx], t->grad + NPARAM, sizeof(float), cudaMemcpyDeviceToHost, t->stream));
-        if (pos + batch > t->n) MCK(cudaStreamSynchronize(t->stream));  // perm is rewritten next step
     }
-    MCK(cudaStreamSynchronize(t->stream));
-    if (losses) std::memcpy(losses, lossbuf.data(), sizeof(float) * steps);
-    return PBS_OK;
+    if (losses && steps > 0)
+        MCK(cudaMemcpyAsync(losses, t->losses, sizeof(float) * steps, cudaMemcpyDeviceToHost, t->stream));
+    return finish(t);
 }
 
 }  // extern "C"

@@ -109,3 +109,38 @@ def test_training_reduces_loss():
     losses = t.train(400, batch=1024, lr=2e-3, seed=1)
     assert losses[-20:].mean() < 0.25 * losses[:5].mean(), (losses[:5], losses[-20:])
     t.close()
+
+
+# rows about the tile and grid lines: 1; a 16-row fragment's edge; one tile and
+# one row more; two steps a launch's limit apart; one tile a SM and one more
+# (152 x 64 = 9,728)
+@pytest.mark.parametrize("n,steps", [(1, 2), (17, 3), (64, 3), (65, 3), (300, 66), (9728, 2), (9729, 2)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_steps_of_one_launch_match_adam(n, steps, weighted):
+    """Steps on the whole set as one minibatch against FP64 Adam on the
+    gradients of the same parameters (weights of 2: twice the gradient).  The
+    bound: an FP32 update's rounding, and a gradient's (1e-5 of an update of at
+    most lr) where rows are summed in another order, a step."""
+    theta = OM.init_params(11).astype(np.float32)
+    X, Y = _data(n, 4)
+    a, b = MLPTrainer(theta), MLPTrainer(theta)
+    a.set_data(X, Y, np.full(n, 2.0, np.float32) if weighted else None)
+    b.set_data(X, Y)
+    ref, m, v = theta.astype(np.float64), np.zeros(a.n_params), np.zeros(a.n_params)
+    losses = a.train(steps, batch=n, lr=1e-3, seed=0)
+    scale = 2.0 if weighted else 1.0
+    if steps > 4:  # too long for the gradients' sensitivity: one launch against two
+        got = a.params
+        b.set_data(X, Y, np.full(n, 2.0, np.float32) if weighted else None)
+        lb = b.train(steps, batch=n, lr=1e-3, seed=0)
+        assert np.array_equal(got, b.params) and np.array_equal(losses, lb)
+        assert np.all(np.isfinite(losses)) and losses[-1] < losses[0]
+    else:
+        for k in range(steps):
+            b.params = ref.astype(np.float32)
+            loss, g = b.gradient(X, Y)
+            assert abs(losses[k] - scale * loss) <= 1e-4 * scale * loss
+            ref, m, v = OM.adam(ref, m, v, scale * g.astype(np.float64), k + 1, 1e-3)
+        assert np.abs(a.params - ref).max() < steps * (1e-6 + 1e-5 * np.abs(ref).max())
+    a.close()
+    b.close()
