@@ -81,21 +81,33 @@ __device__ __forceinline__ void corner_words(const ChunkView &v, const int lc[4]
     }
 }
 
+// A tet's constants.
+struct TetRows {
+    float4 r0, r1, r2;
+    uint4 cor;
+};
+__device__ __forceinline__ TetRows load_rows(const ChunkView &v, int lt) {
+    return TetRows{v.r0[lt], v.r1[lt], v.r2[lt], v.cor[lt]};
+}
+
 // Corner forces of the chunk's tets into the slots; on line-search passes
 // returns the thread's sum of clamped tet energies.
 // A near-inverted tet (full stress) gets its FP32 forces here and a mark in
 // its corner-0 slot's .w; *any_exact tells whether the thread marked one.
 // CHECK: a line-search pass (the tet energies too); the loop is compiled once
-// with and once without them.
-template <int MATERIAL, int THREADS, bool INC, bool PACK, bool CHECK>
+// with and once without them.  first: the constants of the thread's first tet,
+// where the caller loaded them ahead (PRE).
+template <int MATERIAL, int THREADS, bool INC, bool PACK, bool PRE, bool CHECK>
 __device__ __forceinline__ DFloat chunk_forces(const DevParams &p, const ChunkView &v, int nt, float4 *sf,
-                                               bool *any_exact) {
+                                               bool *any_exact, const TetRows &first) {
     DFloat e{0.f, 0.f};
     bool any = false;
+    TetRows rows = first;
     for (int lt = threadIdx.x; lt < nt; lt += THREADS) {
-        const float4 r0 = v.r0[lt], r1 = v.r1[lt], r2 = v.r2[lt];
+        if (!PRE || lt != threadIdx.x) rows = load_rows(v, lt);
+        const float4 r0 = rows.r0, r1 = rows.r1, r2 = rows.r2;
         int lc[4], sl[4];
-        unpack_cor(v.cor[lt], lc, sl);
+        unpack_cor(rows.cor, lc, sl);
         const float dinv[9] = {r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r2.x, r2.y, r2.z};
         Kin<float> kin;
         float f[12];
@@ -174,12 +186,12 @@ template <int THREADS, bool PART> __device__ __forceinline__ bool chunk_sync_or(
 
 // chunk_forces, then the FP64 stress of a chunk that has a near-inverted tet;
 // every (participating) thread sees the finished slots on return.
-template <int MATERIAL, int THREADS, bool INC, bool PACK, bool PART = false>
+template <int MATERIAL, int THREADS, bool INC, bool PACK, bool PRE, bool PART = false>
 __device__ __forceinline__ DFloat chunk_forces_all(const DevParams &p, const ChunkView &v, int nt, bool check,
-                                                   float4 *sf) {
+                                                   float4 *sf, const TetRows &first = TetRows()) {
     bool ex;
-    const DFloat e = check ? chunk_forces<MATERIAL, THREADS, INC, PACK, true>(p, v, nt, sf, &ex)
-                           : chunk_forces<MATERIAL, THREADS, INC, PACK, false>(p, v, nt, sf, &ex);
+    const DFloat e = check ? chunk_forces<MATERIAL, THREADS, INC, PACK, PRE, true>(p, v, nt, sf, &ex, first)
+                           : chunk_forces<MATERIAL, THREADS, INC, PACK, PRE, false>(p, v, nt, sf, &ex, first);
     if (INC) {
         chunk_sync<THREADS, PART>();
     } else if (chunk_sync_or<THREADS, PART>(ex)) {

@@ -319,12 +319,12 @@ __device__ __forceinline__ void chunk_line_search(const DevMesh &m, const DevPar
 // The whole of one chunk once its node words (and, with STAGE, its rows and
 // records) are in shared memory: forces, partials, the Jacobi diagonal every
 // hd_every passes, and the line-search tail.
-template <int MATERIAL, int THREADS, bool INC, bool PACK>
+template <int MATERIAL, int THREADS, bool INC, bool PACK, bool PRE>
 __device__ __forceinline__ void chunk_body(const DevMesh &m, const DevParams &p, const DevState &st, int c,
                                            int inst, int par, const PassView &pv, size_t cur, const ChunkView &v,
                                            const int4 *meta, int nt, int nl, float4 *sf, double *sh,
-                                           int *is_last) {
-    const DFloat e = chunk_forces_all<MATERIAL, THREADS, INC, PACK>(p, v, nt, pv.check, sf);
+                                           int *is_last, const TetRows &first = TetRows()) {
+    const DFloat e = chunk_forces_all<MATERIAL, THREADS, INC, PACK, PRE>(p, v, nt, pv.check, sf, first);
     chunk_partials<THREADS>(meta, nl, sf, st.part);
     if (pv.do_h) {
         __syncthreads();
@@ -340,7 +340,15 @@ __device__ __forceinline__ void chunk_body(const DevMesh &m, const DevParams &p,
     if (pv.check) chunk_line_search<THREADS>(m, p, st, c, inst, par, pv.k, cur, e, sh, is_last);
 }
 
-// One CTA per chunk.  STAGE: every thread first issues asynchronous copies of
+// One CTA per chunk.  What bounds it: with four CTAs of 256 threads a SM, each
+// of them two waits for memory and two barriers, the latency of its loads (the
+// shared-memory wavefronts take 39% of the active cycles at 512,000 tets).  The
+// constants of a thread's first node and first tet are therefore read before
+// the grid-dependency wait, and the first node's words beside the control block
+// instead of after it: 1M tets, full / incremental stress, 35.3 / 41.7 -> 34.1
+// / 38.1 us a pass; 256 boxes of 1K-41K tets 93.4 / 107 -> 90.2 / 99.6.  (Rows
+// of the second tet prefetched into L1 or L2 as well: no change.)
+// STAGE: every thread first issues asynchronous copies of
 // its tets' rows and corner records and of the chunk's local-node records into
 // shared memory -- before the grid-dependency wait, since they are constant --
 // and of the chunk's node words after it; one wait then covers all of them,
@@ -376,8 +384,18 @@ __global__ void __launch_bounds__(THREADS, PBS_INC_THREADS_PER_SM / THREADS)
     const int4 cd = m.chunk[c];
     const int inst = m.chunk_inst[c];
     const int tq0 = cd.x, nt = cd.y, l0 = cd.z, nl = cd.w;
-    // the chunk's reference node for the increments (incremental form)
+    // the chunk's reference node for the increments (incremental form), this
+    // thread's first node and its first tet's constants
     const int g_ref = INC && !STAGE ? m.lmeta[l0].x : 0;
+    int g_first = 0;
+    TetRows first;
+    if (!STAGE) {
+        if (threadIdx.x < nl) g_first = m.lmeta[l0 + threadIdx.x].x;
+        if (threadIdx.x < nt) {
+            const int q = tq0 + threadIdx.x;
+            first = TetRows{m.qrow0[q], m.qrow1[q], m.qrow2[q], m.qcor[q]};
+        }
+    }
     if (STAGE) {
         for (int lt = threadIdx.x; lt < nt; lt += THREADS) {
             const int q = tq0 + lt;
@@ -408,6 +426,15 @@ __global__ void __launch_bounds__(THREADS, PBS_INC_THREADS_PER_SM / THREADS)
         }
         cp_async_commit();
     }
+    // the first node's words, read while the control block is (a stopped
+    // instance's go unused)
+    float4 uh0, ul0, ub0, r_ref;
+    if (!STAGE && threadIdx.x < nl) {
+        uh0 = st.uh[cur + g_first];
+        ul0 = st.ul[cur + g_first];
+        if (INC) ub0 = st.ub[g_first];
+    }
+    if (!STAGE && INC) r_ref = st.uh[cur + g_ref];
     const PassView pv = pass_view(src, p);
     if (pv.skip) {
         // an instance that stopped: its first chunk carries the control block
@@ -428,13 +455,15 @@ __global__ void __launch_bounds__(THREADS, PBS_INC_THREADS_PER_SM / THREADS)
         }
     } else {
         // (the increments relative to the chunk's local node 0)
-        float4 r;
-        if (INC) r = st.uh[cur + g_ref];
         for (int j = threadIdx.x; j < nl; j += THREADS) {
-            const int g = meta[j].x;
-            const float4 uh = st.uh[cur + g], ul = st.ul[cur + g];
-            if (INC) pack_words(s_wa, s_wb, j, increment_rel(uh, ul, r), st.ub[g]);
-            else pack_words(s_wa, s_wb, j, uh, ul);
+            if (j != threadIdx.x) {
+                const int g = meta[j].x;
+                uh0 = st.uh[cur + g];
+                ul0 = st.ul[cur + g];
+                if (INC) ub0 = st.ub[g];
+            }
+            if (INC) pack_words(s_wa, s_wb, j, increment_rel(uh0, ul0, r_ref), ub0);
+            else pack_words(s_wa, s_wb, j, uh0, ul0);
         }
     }
     __syncthreads();
@@ -450,7 +479,8 @@ __global__ void __launch_bounds__(THREADS, PBS_INC_THREADS_PER_SM / THREADS)
     v.cor = STAGE ? s_cor : m.qcor + tq0;
     v.meta = meta;
     v.rest = m.rest;
-    chunk_body<MATERIAL, THREADS, INC, !STAGE>(m, p, st, c, inst, par, pv, cur, v, meta, nt, nl, s_f, sh, &is_last);
+    chunk_body<MATERIAL, THREADS, INC, !STAGE, !STAGE>(m, p, st, c, inst, par, pv, cur, v, meta, nt, nl, s_f, sh,
+                                                       &is_last, first);
 }
 
 // ------------------------------------------------------------ persistent, TMA-fed variant
@@ -665,7 +695,7 @@ __global__ void __launch_bounds__(THREADS, 768 / THREADS) k_tstream(DevMesh m, D
             v.cor = sb.cor;
             v.meta = sb.meta;
             v.rest = m.rest;
-            chunk_body<MATERIAL, THREADS, INC, false>(m, p, st, c, cur.inst, par, cur.pv, cur.cur, v, sb.meta, cur.nt,
+            chunk_body<MATERIAL, THREADS, INC, false, false>(m, p, st, c, cur.inst, par, cur.pv, cur.cur, v, sb.meta, cur.nt,
                                                cur.nl, s_f, sh, &is_last);
         }
         __syncthreads();  // buffer b and the slots are free again

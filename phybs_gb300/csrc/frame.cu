@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
                 v.cor = RES ? s_cor : m.qcor + cd.x;
                 v.meta = meta;
                 v.rest = m.rest;
-                const DFloat ec = chunk_forces_all<MATERIAL, THREADS, INC, true, true>(p, v, nt, check, s_f);
+                const DFloat ec = chunk_forces_all<MATERIAL, THREADS, INC, true, false, true>(p, v, nt, check, s_f);
                 publish_partials<THREADS>(meta, nl, s_f, st.part, tag);
                 if (do_h) {
                     chunk_sync<THREADS, true>();
