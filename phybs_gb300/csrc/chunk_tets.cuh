@@ -209,7 +209,7 @@ __device__ __forceinline__ DFloat chunk_forces_all(const DevParams &p, const Chu
 // was half as large, and one pull in ten to a residual of 1e-4 took another
 // rejection.  Called by whole warps.
 template <int THREADS> __device__ __forceinline__ float noise_square(const DevMesh &m, int nt, float e) {
-    const int lanes = m.noise_tets == 0 ? 1 : nt > THREADS ? m.noise_tets / 2 : m.noise_tets;
+    const int lanes = m.noise_tets == 0 || nt > 3 * THREADS ? 1 : nt > THREADS ? m.noise_tets / 2 : m.noise_tets;
     if (lanes > 1) e += __shfl_xor_sync(0xffffffffu, e, 1);
     if (lanes > 2) e += __shfl_xor_sync(0xffffffffu, e, 2);
     return e * e / (float)lanes;

@@ -201,30 +201,34 @@ void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<doubl
 }
 
 // Where the lines lie (96 passes of a 5-tet box, full / incremental stress, us;
-// "graph" the pass kernels at their best shape, "frame" the frame kernel):
+// "graph" the pass kernels at their best shape, "frame" the frame kernel, with
+// 128 threads a CTA):
 //   up to 4,096 tets: 128 a chunk (2,340 tets: 409 / 444, 256 a chunk 473 /
 //     507, graph 1003 / 1050; up to 8,192 a single instance gained 7% and the
 //     batch below lost 4%);
-//   up to 3 * sms * 256 (116,736): 256, up to three CTAs a SM of the frame
-//     kernel (24,500 tets: 501 / 548, 192 a chunk 493 / 540, graph 1059 / 1119;
-//     59,940: 631 / 673, graph 1122 / 1197; 100,800: 939 / 832, graph 1245 /
-//     1326).  Finer chunks cost a large batch, whose instances are of these
-//     sizes and which the pass kernels run, more partials than they save a
-//     single instance: 256 boxes of 1K-41K tets take 12.4 ms at 256 a chunk,
-//     14.5 at 128;
-//   up to 2 * sms * 512 (155,648): 512 tets, 256 threads, two CTAs a SM
-//     (149,445: 1183 / 1236, graph 1301 / 1387);
-//   beyond, the pass kernels: 384 tets up to 250,000 (203,205: 1463 / 1596,
-//     512 tets 1622 / 1731), then 512 (311,040: 1602 / 1770, 384 tets 1829 /
-//     2058; 1M tets, us a pass of the tet kernel: 35.0 / 40.9, 1,024 tets and
-//     512 threads 36.7 / 43.8).
-// (Measured with chunks of exactly these sizes; the pieces of a group of 1,024
-// are of 342 where this says 384.)
+//   up to 2 * sms * 256 (77,824): 256, up to two CTAs a SM of the frame kernel
+//     (24,500 tets: 491 / 534, 192 a chunk 497 / 539; 59,940: 616 / 655, 512 a
+//     chunk 649 / 712, graph 1114 / 1200).  Finer chunks cost a large batch,
+//     whose instances are of these sizes and which the pass kernels run, more
+//     partials than they save a single instance: 256 boxes of 1K-41K tets take
+//     12.4 ms at 256 a chunk, 14.5 at 128;
+//   up to 2 * sms * 342 (103,968): 384, which a group makes 342 (78,000: 694 /
+//     748, 256 a chunk 799 / 747; 100,800: 744 / 799, 256 a chunk and three
+//     CTAs a SM 917 / 838, 512 a chunk 839 / 879, graph 1226 / 1329);
+//   up to 2 * sms * 512 (155,648): 512 (125,000: 845 / 891, with 256 threads,
+//     whose registers spill at two CTAs a SM, 1120 / 1160; 154,980: 891 / 937,
+//     graph 1240 / 1360);
+//   beyond, the pass kernels (with 256 threads): 384 up to 250,000 (203,205:
+//     1372 / 1519, 512 a chunk 1458 / 1606; the frame kernel with 704 a chunk
+//     1291 / 1314, but a group has no pieces of that size), then 512 (311,040:
+//     1460 / 1653, 384 a chunk 1671 / 1946; 1M tets, us a pass of the tet
+//     kernel: 35.0 / 40.9, 1,024 tets and 512 threads 36.7 / 43.8).
 // The node limit leaves room for meshes with more nodes a tet than a box.
 ChunkLimits auto_chunk_limits(int tets, int sms) {
     int n;
     if (tets <= 4096) n = 128;
-    else if (tets <= 3 * 256 * sms) n = 256;
+    else if (tets <= 2 * 256 * sms) n = 256;
+    else if (tets <= 2 * 342 * sms) n = 384;
     else if (tets > 2 * 512 * sms && tets <= 250000) n = 384;
     else n = 512;
     return ChunkLimits{n, n == 512 ? 256 : 32 + n / 2 + n / 16};

@@ -228,7 +228,9 @@ struct FrameView {
 // PER_SM: CTAs a SM the registers are budgeted for.  A pass is bound by the
 // dependent chain of one tet, so a mesh that needs fewer CTAs a SM runs the
 // variant with more registers: on 24,500 tets 493 us a 96-pass step at one
-// CTA a SM (no spills), 523 at two, 650 at three.
+// CTA a SM (no spills), 523 at two, 650 at three.  For the same reason 128
+// threads take chunks of up to 512 tets, four a thread: 256 threads at two CTAs
+// a SM have 96 registers and spill (125,000 tets: 1120 us against 845).
 template <int MATERIAL, int THREADS, bool INC, bool RES, int PER_SM>
 __global__ void __launch_bounds__(THREADS + 32, PER_SM)
     k_frame(DevMesh m, DevParams p, DevState st, FrameAux fx) {
@@ -546,7 +548,7 @@ static cudaError_t launch_frame_v(cudaStream_t s, const DevMesh &m, const DevPar
 }
 
 // The register classes: resident 128-thread CTAs at one, two or three a SM,
-// 256-thread CTAs at two; walking five and three.
+// 256-thread CTAs (a caller's shape) at two; walking five and three.
 template <int MATERIAL, int THREADS, bool INC>
 static cudaError_t launch_frame_t(cudaStream_t s, const DevMesh &m, const DevParams &p, const DevState &st,
                                   const FrameAux &fx, const FramePlan &plan) {

@@ -250,7 +250,6 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
             ct = std::max(ct, limits[b].tets);
             cn = std::max(cn, limits[b].nodes);
         }
-        threads = ct > 256 ? 256 : 128;  // one or two tets a thread
     }
     const bool grouped = h->shape_auto;  // (a caller's own shape keeps a reference node a chunk)
     ChunkLayout cl;
@@ -261,6 +260,10 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
         build_chunks(h->Np, h->h_tets_pad, h->h_rest_pad, ctl, limits, grouped, false, cl);
     }
     const int nc = (int)cl.chunk.size();
+    // the pass kernels run chunks of more than 256 tets with two tets a thread;
+    // the frame kernel, where every chunk has its place on two CTAs a SM, with
+    // up to four (auto_chunk_limits has both sides)
+    if (threads == 0) threads = ct > 256 && nc > 2 * h->sms ? 256 : 128;
     const size_t L = cl.lmeta.size(), T = (size_t)h->T;
     h->chunk.release(); h->chunk_inst.release(); h->cpart.release(); h->qperm.release();
     h->lmeta.release(); h->pptr.release();
