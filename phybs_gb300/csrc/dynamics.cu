@@ -187,8 +187,8 @@ __device__ __forceinline__ void pbd_apply(const PbdView &v, const PbdTet &t, con
 // those of the next one, so it reads what the serial order gives it; and tets
 // of one step share no node.  L + (sweeps - 1) D steps instead of L sweeps:
 // the dependent chain of a level, which bounds a step, then serves several
-// sweeps at once.  On structured meshes D is 2-20% of L (the 1M-tet box: L
-// 2,320, D 44; the 24,000-tet bar 348 and 72), on meshes in arbitrary order up
+// sweeps at once.  On structured meshes D is 2-10% of L (the 1M-tet box: L
+// 2,325, D 39; the 24,000-tet bar 348 and 34), on meshes in arbitrary order up
 // to L, where the sweeps simply follow one another.
 struct PbdStep {
     int l0, L, D, sweeps, steps;

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -1687,32 +1688,51 @@ int pbs_backward_euler_step(pbs_handle *h, float dt, float alpha, float beta, co
 
 // ---- strain-based PBD and projective dynamics
 
-// Levels of the caller's tet order per instance (a tet one level above the
-// last earlier tet touching any of its nodes), the level-ordered tets, and
-// the step's rest data formed as the reference forms it (launch_pbd_rest).
+
+// Levels of the caller's tet order per instance (a tet above the last earlier
+// tet touching any of its nodes), the level-ordered tets, and the step's rest
+// data formed as the reference forms it (launch_pbd_rest).
 static int ensure_pbd(pbs_handle *h) {
     if (h->pbd_ready) return PBS_OK;
     const int B = h->B, Tp = h->Tp;
-    std::vector<int> level(Tp, -1), last(h->Np, -1), grp(B + 1, 0), nlev(B, 0), delay(B, 1);
+    std::vector<int> level(Tp, -1), second(Tp, -1), last(h->Np, -1), grp(B + 1, 0), delay(B, 1);
     for (int b = 0; b < B; ++b) {
-        int top = -1;
-        for (int tp = h->h_inst_tets[2 * b]; tp < h->h_inst_tets[2 * b + 1]; ++tp) {
-            const int4 q = h->h_tets_pad[tp];
-            if (q.x < 0) continue;
-            const int l = 1 + std::max(std::max(last[q.x], last[q.y]), std::max(last[q.z], last[q.w]));
-            level[tp] = l;
-            last[q.x] = last[q.y] = last[q.z] = last[q.w] = l;
-            top = std::max(top, l);
+        // levels of the instance's tets after the levels in `last`, from 0:
+        // {their number, the delay between sweeps}
+        auto levels = [&](std::vector<int> &lv) {
+            int lo = INT_MAX, top = -1, D = 1;
+            for (int tp = h->h_inst_tets[2 * b]; tp < h->h_inst_tets[2 * b + 1]; ++tp) {
+                const int4 q = h->h_tets_pad[tp];
+                if (q.x < 0) continue;
+                const int l = 1 + std::max(std::max(last[q.x], last[q.y]), std::max(last[q.z], last[q.w]));
+                lv[tp] = l;
+                last[q.x] = last[q.y] = last[q.z] = last[q.w] = l;
+                lo = std::min(lo, l);
+                top = std::max(top, l);
+            }
+            // (last: the highest level at each node)
+            for (int tp = h->h_inst_tets[2 * b]; tp < h->h_inst_tets[2 * b + 1]; ++tp) {
+                const int4 q = h->h_tets_pad[tp];
+                if (q.x < 0) continue;
+                const int up = std::max(std::max(last[q.x], last[q.y]), std::max(last[q.z], last[q.w]));
+                D = std::max(D, up - lv[tp] + 1);
+                lv[tp] -= lo;
+            }
+            return std::make_pair(top < 0 ? 0 : top - lo + 1, D);
+        };
+        // the earliest levels, or those that the tets have in a second sweep
+        // behind the first, where nothing is earlier than the next sweep needs
+        // it: about as many, and a smaller delay (the 24,000-tet bar 348 and 72
+        // against 348 and 34, the 1M-tet box 2,320 and 44 against 2,325 and 39).
+        // Whichever gives the reference's five sweeps fewer steps
+        const auto p1 = levels(level), p2 = levels(second);
+        auto best = p1;
+        if (p2.first + 4 * p2.second < p1.first + 4 * p1.second) {
+            best = p2;
+            for (int tp = h->h_inst_tets[2 * b]; tp < h->h_inst_tets[2 * b + 1]; ++tp) level[tp] = second[tp];
         }
-        nlev[b] = top + 1;
-        grp[b + 1] = grp[b] + nlev[b];
-        // the delay between sweeps (last: the highest level at each node)
-        for (int tp = h->h_inst_tets[2 * b]; tp < h->h_inst_tets[2 * b + 1]; ++tp) {
-            const int4 q = h->h_tets_pad[tp];
-            if (q.x < 0) continue;
-            const int up = std::max(std::max(last[q.x], last[q.y]), std::max(last[q.z], last[q.w]));
-            delay[b] = std::max(delay[b], up - level[tp] + 1);
-        }
+        delay[b] = best.second;
+        grp[b + 1] = grp[b] + best.first;
     }
     const int L = grp[B];
     std::vector<int> lvl(L + 1, 0);
