@@ -215,23 +215,27 @@ void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<doubl
 //   up to 2 * sms * 342 (103,968): 384, which a group makes 342 (78,000: 694 /
 //     748, 256 a chunk 799 / 747; 100,800: 744 / 799, 256 a chunk and three
 //     CTAs a SM 917 / 838, 512 a chunk 839 / 879, graph 1226 / 1329);
-//   up to 2 * sms * 512 (155,648): 512 (125,000: 845 / 891, with 256 threads,
-//     whose registers spill at two CTAs a SM, 1120 / 1160; 154,980: 891 / 937,
-//     graph 1240 / 1360);
-//   beyond, the pass kernels (with 256 threads): 384 up to 250,000 (203,205:
-//     1372 / 1519, 512 a chunk 1458 / 1606; the frame kernel with 704 a chunk
-//     1291 / 1314, but a group has no pieces of that size), then 512 (311,040:
-//     1460 / 1653, 384 a chunk 1671 / 1946; 1M tets, us a pass of the tet
-//     kernel: 35.0 / 40.9, 1,024 tets and 512 threads 36.7 / 43.8).
+//   up to sms * 1,024 (155,648): whole groups, one CTA of 256 threads a SM
+//     (125,000: 855 / 924, 512 a chunk, 128 threads and two CTAs a SM 849 /
+//     894, the same with 256 threads, which spill, 1120 / 1160; 154,980: 879 /
+//     950, graph 1240 / 1360).  Where they cost so little, whole groups are
+//     worth their sums: a node's partials are then the ones of every other
+//     machine width, and iterations to a tolerance stop at the same pass
+//     (pieces move one pull in 40 to a residual of 1e-4 by more than 2e-5 of
+//     its velocities);
+//   beyond, the pass kernels: 384 up to 250,000 (203,205, 256 threads: 1372 /
+//     1519, 512 a chunk 1458 / 1606; the frame kernel with 704 a chunk 1291 /
+//     1314, but a group has no pieces of that size), then whole groups on 512
+//     threads (1M tets, us a pass of both kernels: 48.6 / 54.9, 512 a chunk on
+//     256 threads 47.5 / 51.6).
 // The node limit leaves room for meshes with more nodes a tet than a box.
 ChunkLimits auto_chunk_limits(int tets, int sms) {
     int n;
     if (tets <= 4096) n = 128;
     else if (tets <= 2 * 256 * sms) n = 256;
-    else if (tets <= 2 * 342 * sms) n = 384;
-    else if (tets > 2 * 512 * sms && tets <= 250000) n = 384;
-    else n = 512;
-    return ChunkLimits{n, n == 512 ? 256 : 32 + n / 2 + n / 16};
+    else if (tets <= 2 * 342 * sms || (tets > CHUNK_GROUP_TETS * sms && tets <= 250000)) n = 384;
+    else return ChunkLimits{CHUNK_GROUP_TETS, CHUNK_GROUP_NODES};
+    return ChunkLimits{n, 32 + n / 2 + n / 16};
 }
 
 // ------------------------------------------------------------ device
@@ -263,7 +267,17 @@ __device__ __forceinline__ void chunk_line_search(const DevMesh &m, const DevPar
     InstCtl *dst = ctl_buf(st, par ^ 1) + inst;
     unsigned int *cnt = st.tcount + inst;
     __shared__ float shs[THREADS / 32];
-    float e2 = noise_square<THREADS>(m, m.chunk[c].y, e.hi);
+    float e2;
+    if (THREADS == 512 && m.noise_tets != 0 && m.chunk[c].y > THREADS) {
+        // two tets a thread: with those of the thread half a CTA away
+        __shared__ float s_e[THREADS / 2];
+        if (threadIdx.x >= THREADS / 2) s_e[threadIdx.x - THREADS / 2] = e.hi;
+        __syncthreads();
+        const float x = threadIdx.x < THREADS / 2 ? e.hi + s_e[threadIdx.x] : 0.f;
+        e2 = x * x;
+    } else {
+        e2 = noise_square<THREADS>(m, m.chunk[c].y, e.hi);
+    }
     const int cb = src->cblk_begin, ce = src->cblk_end;
     {
         const int nb = ce - cb;

@@ -228,9 +228,10 @@ struct FrameView {
 // PER_SM: CTAs a SM the registers are budgeted for.  A pass is bound by the
 // dependent chain of one tet, so a mesh that needs fewer CTAs a SM runs the
 // variant with more registers: on 24,500 tets 493 us a 96-pass step at one
-// CTA a SM (no spills), 523 at two, 650 at three.  For the same reason 128
-// threads take chunks of up to 512 tets, four a thread: 256 threads at two CTAs
-// a SM have 96 registers and spill (125,000 tets: 1120 us against 845).
+// CTA a SM (no spills), 523 at two, 650 at three.  For the same reason a group
+// of 1,024 tets runs on one CTA of 256 threads (168 registers), four tets a
+// thread: 256 threads at two CTAs a SM have 96 and spill (125,000 tets: 1120 us
+// against 855).
 template <int MATERIAL, int THREADS, bool INC, bool RES, int PER_SM>
 __global__ void __launch_bounds__(THREADS + 32, PER_SM)
     k_frame(DevMesh m, DevParams p, DevState st, FrameAux fx) {
@@ -548,14 +549,14 @@ static cudaError_t launch_frame_v(cudaStream_t s, const DevMesh &m, const DevPar
 }
 
 // The register classes: resident 128-thread CTAs at one, two or three a SM,
-// 256-thread CTAs (a caller's shape) at two; walking five and three.
+// 256-thread CTAs at one or two; walking five and three.
 template <int MATERIAL, int THREADS, bool INC>
 static cudaError_t launch_frame_t(cudaStream_t s, const DevMesh &m, const DevParams &p, const DevState &st,
                                   const FrameAux &fx, const FramePlan &plan) {
     constexpr int WALK = THREADS == 128 ? 5 : 3;
     if (!plan.resident) return launch_frame_v<MATERIAL, THREADS, INC, false, WALK>(s, m, p, st, fx, plan.grid);
+    if (plan.per_sm == 1) return launch_frame_v<MATERIAL, THREADS, INC, true, 1>(s, m, p, st, fx, plan.grid);
     if constexpr (THREADS == 128) {
-        if (plan.per_sm == 1) return launch_frame_v<MATERIAL, 128, INC, true, 1>(s, m, p, st, fx, plan.grid);
         if (plan.per_sm == 3) return launch_frame_v<MATERIAL, 128, INC, true, 3>(s, m, p, st, fx, plan.grid);
     }
     return launch_frame_v<MATERIAL, THREADS, INC, true, 2>(s, m, p, st, fx, plan.grid);
@@ -566,10 +567,8 @@ template <int MATERIAL, int THREADS, bool INC> static FramePlan frame_plan_t(con
     FramePlan r;
     r.resident = true;
     r.grid = m.n_chunks;
-    if constexpr (THREADS == 128) {
-        r.per_sm = 1;
-        if (frame_fit<MATERIAL, 128, INC, true, 1>(m, sms) >= m.n_chunks) return r;
-    }
+    r.per_sm = 1;
+    if (frame_fit<MATERIAL, THREADS, INC, true, 1>(m, sms) >= m.n_chunks) return r;
     r.per_sm = 2;
     if (frame_fit<MATERIAL, THREADS, INC, true, 2>(m, sms) >= m.n_chunks) return r;
     if constexpr (THREADS == 128) {

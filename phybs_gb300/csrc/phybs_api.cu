@@ -261,10 +261,14 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
         build_chunks(h->Np, h->h_tets_pad, h->h_rest_pad, ctl, limits, grouped, false, cl);
     }
     const int nc = (int)cl.chunk.size();
-    // the pass kernels run chunks of more than 256 tets with two tets a thread;
-    // the frame kernel, where every chunk has its place on two CTAs a SM, with
-    // up to four (auto_chunk_limits has both sides)
-    if (threads == 0) threads = ct > 256 && nc > 2 * h->sms ? 256 : 128;
+    // the pass kernels run chunks of more than 256 tets with two tets a thread
+    // (a packed batch's with 256 threads, which its smaller instances can use);
+    // the frame kernel, where every chunk has its place, with up to four
+    // (auto_chunk_limits has both sides)
+    if (threads == 0) {
+        if (ct == CHUNK_GROUP_TETS) threads = nc > h->sms && h->B == 1 ? 512 : 256;
+        else threads = ct > 256 && nc > 2 * h->sms ? 256 : 128;
+    }
     const size_t L = cl.lmeta.size(), T = (size_t)h->T;
     h->chunk.release(); h->chunk_inst.release(); h->cpart.release(); h->qperm.release();
     h->lmeta.release(); h->pptr.release();

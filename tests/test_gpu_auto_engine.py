@@ -32,7 +32,7 @@ def _box(nx, ny, nz):
 
 # one tet; one cube (5); one chunk and a few more (120, 130, 180); around the 128 / 256 line
 # (4,080, 4,160), 7,680, 8,320; one and two CTAs a SM of 256 tets (38,440, 60,000, 77,760); the
-# pieces of 342 (78,000, 102,060); the 512-tet class (104,780, 115,200, 119,000, 155,000); past
+# pieces of 342 (78,000, 102,060); whole groups (104,780, 115,200, 119,000, 155,000); past
 # the resident sizes (161,700: the pass kernels either way)
 BOXES = [(1, 1, 1), (2, 3, 4), (2, 1, 13), (3, 3, 4), (8, 8, 24), (8, 8, 26), (31, 31, 8), (20, 20, 30),
          (24, 24, 40), (28, 25, 34), (31, 25, 40), (33, 28, 35), (8, 6, 17), (8, 8, 13), (24, 24, 27),
@@ -123,13 +123,14 @@ def test_stretch_stress_without_svd(s):
     a.close()
 
 
-PULLS = [(3, 3, 5), (8, 7, 12), (12, 9, 13), (20, 17, 31), (22, 21, 40), (25, 25, 40), (31, 23, 46)]
+PULLS = [(3, 3, 5), (8, 7, 12), (12, 9, 13), (20, 17, 31), (22, 21, 40), (25, 25, 40), (31, 23, 46), (34, 33, 46)]
 
 
 @pytest.mark.parametrize("dims", PULLS, ids=[f"{5 * a * b * c}" for a, b, c in PULLS])
 def test_pull_takes_one_path_at_every_chunk_size(dims):
     """Two frames of a pull to a residual of 1e-4 on the automatic chunks (one
-    group and less, pieces of 128, 256, 342, 512, 342 tets) and on whole groups of 1,024:
+    group and less, pieces of 128, 256, 342, whole groups, pieces of 342,
+    whole groups) and on whole groups of 1,024:
     the tets' forces have the same bits, so that the passes and rejections are
     the same, and the positions to the sums' rounding."""
     m = M.box_mesh(*dims, edge=0.25 / max(dims[:2]), jitter=0.1, seed=7, young=1e5, pin="both")
