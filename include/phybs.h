@@ -54,7 +54,9 @@ extern "C" {
  *   Psi = mu/2 (I1 - 3) - mu ln J + lambda/2 (ln J)^2,
  * evaluated through the invariants (IsotropicNeohookeanMaterial.cpp:104)
  * or through the principal stretches of the modified SVD
- * (IsotropicMaterial.cpp:360-409, Xu et al. 2015). */
+ * (IsotropicMaterial.cpp:360-409, Xu et al. 2015).  The descent's passes take
+ * the stretch material's stress from the invariants too, which is the same
+ * stress, where the invariants show the tet to be away from inversion. */
 #define PBS_MATERIAL_NEOHOOKEAN 0
 #define PBS_MATERIAL_STRETCH 1
 
