@@ -768,9 +768,17 @@ static int ensure_graph(pbs_handle *h) {
 }
 
 // How the frame kernel runs the handle's current layout.
+// The mesh as the frame kernel takes it: automatic chunks that the pass kernels
+// run with 512 threads, which it has no variant for, with 256.
+static DevMesh frame_mesh(pbs_handle *h) {
+    DevMesh m = h->mesh();
+    if (h->shape_auto && m.chunk_threads == 512) m.chunk_threads = 256;
+    return m;
+}
+
 static const FramePlan &handle_frame_plan(pbs_handle *h) {
     if (!h->plan_valid) {
-        h->fplan = frame_plan(h->mesh(), h->material,
+        h->fplan = frame_plan(frame_mesh(h), h->material,
                               h->material == PBS_MATERIAL_NEOHOOKEAN && h->dparams.incremental, h->sms);
         h->plan_valid = true;
     }
@@ -819,7 +827,7 @@ static int launch_frame_step(pbs_handle *h, const DevParams &p, int max_passes) 
     fx.tag0 = h->frame_tag;
     fx.max_passes = max_passes;
     h->frame_clean = false;
-    CK(launch_frame(s, h->mesh(), p, h->state(), h->material, fx, plan));
+    CK(launch_frame(s, frame_mesh(h), p, h->state(), h->material, fx, plan));
     return PBS_OK;
 }
 

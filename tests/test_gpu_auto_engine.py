@@ -171,3 +171,24 @@ def test_shapes_without_room_for_padding(staged, threads, tets, nodes, inc):
         x.append(s.positions())
         s.close()
     assert np.array_equal(x[0], x[1])
+
+
+@pytest.mark.parametrize("inc", [0, 1])
+def test_frame_engine_on_automatic_chunks_beyond_residence(inc):
+    """A body whose automatic chunks run with 512 threads in the pass kernels
+    takes the frame engine too, with the same bits; a caller's 512-thread shape
+    stays refused."""
+    m = _box(34, 33, 46)
+    p = make_params("gpu_reference", h=1 / 30, max_iters=24, incremental_stress=inc)
+    x = []
+    for engine in ("graph", "frame"):
+        s = DescentSolver(m, params=p)
+        s.set_pass_engine(engine)
+        s.step()
+        x.append(s.positions())
+        if engine == "frame":
+            s.set_chunk_shape(512, 1024, 448)
+            with pytest.raises(L.PhybsError):
+                s.step()
+        s.close()
+    assert np.array_equal(x[0], x[1])
