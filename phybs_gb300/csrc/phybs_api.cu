@@ -403,19 +403,29 @@ static void setup_l2_residency(pbs_handle *h, const cudaDeviceProp &prop) {
     h->l2_hit = (float)std::min(1.0, (double)aside / (double)h->l2_window);
 }
 
+// Every tet's corners are four different nodes of its own instance.  Checked
+// before anything is built from them: the pass layout sorts a chunk's nodes by
+// their corner count, which a tet that repeats a node could raise past the
+// chunk's tets.
+static int check_tets(const int *tets, const std::vector<int> &nptr, const std::vector<int> &tptr) {
+    for (size_t b = 0; b + 1 < nptr.size(); ++b)
+        for (int t = tptr[b]; t < tptr[b + 1]; ++t) {
+            const int *q = tets + 4 * (size_t)t;
+            for (int c = 0; c < 4; ++c) {
+                if (q[c] < nptr[b] || q[c] >= nptr[b + 1]) return PBS_E_BAD_MESH;
+                for (int e = 0; e < c; ++e)
+                    if (q[c] == q[e]) return PBS_E_BAD_MESH;
+            }
+        }
+    return PBS_OK;
+}
+
 int pbs_create(const pbs_mesh_desc *d, pbs_handle **out) {
     if (!d || !out || d->n_nodes <= 0 || d->n_tets <= 0 || !d->rest || !d->tets || d->n_instances < 1 ||
         !(d->density > 0.f))
         return PBS_E_INVALID_ARG;
     if (d->n_instances > 1 && (!d->instance_node_ptr || !d->instance_tet_ptr)) return PBS_E_INVALID_ARG;
     *out = nullptr;
-    int dev = 0, ndev = 0;
-    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return PBS_E_NO_DEVICE;
-    if (cudaGetDevice(&dev) != cudaSuccess) return PBS_E_NO_DEVICE;
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return PBS_E_NO_DEVICE;
-    if (prop.major != 10 || prop.minor != 3) return PBS_E_NO_DEVICE;
-
     const int N = d->n_nodes, T = d->n_tets, B = d->n_instances;
     std::vector<int> nptr(B + 1), tptr(B + 1);
     if (B == 1) { nptr = {0, N}; tptr = {0, T}; }
@@ -426,6 +436,15 @@ int pbs_create(const pbs_mesh_desc *d, pbs_handle **out) {
     if (nptr[0] != 0 || tptr[0] != 0 || nptr[B] != N || tptr[B] != T) return PBS_E_INVALID_ARG;
     for (int b = 0; b < B; ++b)
         if (nptr[b + 1] < nptr[b] || tptr[b + 1] < tptr[b]) return PBS_E_INVALID_ARG;
+    int rc = check_tets(d->tets, nptr, tptr);
+    if (rc != PBS_OK) return rc;
+
+    int dev = 0, ndev = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return PBS_E_NO_DEVICE;
+    if (cudaGetDevice(&dev) != cudaSuccess) return PBS_E_NO_DEVICE;
+    cudaDeviceProp prop;
+    if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return PBS_E_NO_DEVICE;
+    if (prop.major != 10 || prop.minor != 3) return PBS_E_NO_DEVICE;
 
     pbs_handle *h = new (std::nothrow) pbs_handle();
     if (!h) return PBS_E_OUT_OF_MEMORY;
@@ -466,8 +485,7 @@ int pbs_create(const pbs_mesh_desc *d, pbs_handle **out) {
             double e[3][3];
             for (int c = 0; c < 3; ++c)
                 for (int k = 0; k < 3; ++k) {
-                    int a = q[c + 1], o = q[0];
-                    if (a < 0 || a >= N || o < 0 || o >= N) { delete h; return PBS_E_BAD_MESH; }
+                    const int a = q[c + 1], o = q[0];
                     e[c][k] = (double)d->rest[3 * (size_t)a + k] - d->rest[3 * (size_t)o + k];
                 }
             vs += std::fabs(e[0][0] * (e[1][1] * e[2][2] - e[1][2] * e[2][1]) - e[0][1] * (e[1][0] * e[2][2] - e[1][2] * e[2][0]) +
@@ -489,11 +507,7 @@ int pbs_create(const pbs_mesh_desc *d, pbs_handle **out) {
             int tp = tet_off[b] + (t - tptr[b]);
             h->h_tet_user[tp] = t;
             int id[4];
-            for (int c = 0; c < 4; ++c) {
-                int u = d->tets[4 * (size_t)t + c];
-                if (u < nptr[b] || u >= nptr[b + 1]) { delete h; return PBS_E_BAD_MESH; }
-                id[c] = h->user2pad[u];
-            }
+            for (int c = 0; c < 4; ++c) id[c] = h->user2pad[d->tets[4 * (size_t)t + c]];
             tets_pad[tp] = make_int4(id[0], id[1], id[2], id[3]);
         }
     }
@@ -570,10 +584,8 @@ int pbs_create(const pbs_mesh_desc *d, pbs_handle **out) {
     setup_l2_residency(h, prop);
     CKC(prepare_chunk_kernels());
     cudaStream_t s = h->stream;
-    {
-        const int rc = set_pass_layout(h, 0, 0, 0, 0, &ctl);
-        if (rc != PBS_OK) return fail(rc);
-    }
+    rc = set_pass_layout(h, 0, 0, 0, 0, &ctl);
+    if (rc != PBS_OK) return fail(rc);
     CKC(cudaMemcpyAsync(h->tets.p, tets_pad.data(), sizeof(int4) * Tp, cudaMemcpyHostToDevice, s));
     CKC(cudaMemcpyAsync(h->tslot.p, tslot.data(), sizeof(int4) * Tp, cudaMemcpyHostToDevice, s));
     CKC(cudaMemcpyAsync(h->inc_ptr.p, iptr.data(), sizeof(int) * (Np + 1), cudaMemcpyHostToDevice, s));
@@ -624,7 +636,7 @@ int pbs_create(const pbs_mesh_desc *d, pbs_handle **out) {
     // default material: TetMesh.cpp:185 (E = 5e5, nu = 0.45), the reference's Lame formula
     float mu, lam;
     pbs_lame(5e5f, 0.45f, 1, &mu, &lam);
-    int rc = pbs_set_material(h, PBS_MATERIAL_NEOHOOKEAN, &mu, &lam, 1);
+    rc = pbs_set_material(h, PBS_MATERIAL_NEOHOOKEAN, &mu, &lam, 1);
     if (rc != PBS_OK) return fail(rc);
     CKC(cudaStreamSynchronize(s));
     *out = h;

@@ -157,6 +157,20 @@ def test_create_rejects_bad_input_without_device(lib):
     assert lib.pbs_create(C.byref(d), C.byref(h)) == L.PBS_E_INVALID_ARG
 
 
+@pytest.mark.parametrize("tet", [(0, 1, 1, 2), (0, 1, 1, 1), (0, 1, 2, 0), (0, 0, 0, 0), (0, 1, 2, 4), (-1, 1, 2, 3)])
+def test_create_rejects_bad_tets_before_it_needs_a_device(lib, tet):
+    """A repeated or out-of-range corner is refused on the host, before a
+    layout is built from it."""
+    rest = np.float32([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1]])
+    tets = np.int32([[0, 1, 2, 3], tet])
+    for k in (0, 1):  # among others, and alone
+        t = np.ascontiguousarray(tets[k:])
+        h = C.c_void_p()
+        d = L.MeshDesc(4, rest.ctypes.data, None, len(t), t.ctypes.data, None, 1, None, None, 1000.0, 9.8)
+        assert lib.pbs_create(C.byref(d), C.byref(h)) == L.PBS_E_BAD_MESH
+        assert not h.value
+
+
 def test_params_validation(lib):
     p = L.default_params()
     p.h = 0.0
