@@ -402,9 +402,11 @@ __global__ void __launch_bounds__(THREADS, PBS_INC_THREADS_PER_SM / THREADS)
     const int4 cd = m.chunk[c];
     const int inst = m.chunk_inst[c];
     const int tq0 = cd.x, nt = cd.y, l0 = cd.z, nl = cd.w;
-    // the chunk's reference node for the increments (incremental form), this
-    // thread's first node and its first tet's constants
-    const int g_ref = INC && !STAGE ? m.lmeta[l0].x : 0;
+    // the chunk's reference node for the increments (incremental form; the
+    // chunk of an instance without tets has no local node: its first record
+    // may lie past the table), this thread's first node and its first tet's
+    // constants
+    const int g_ref = INC && !STAGE && nl > 0 ? m.lmeta[l0].x : 0;
     int g_first = 0;
     TetRows first;
     if (!STAGE) {
@@ -452,7 +454,7 @@ __global__ void __launch_bounds__(THREADS, PBS_INC_THREADS_PER_SM / THREADS)
         ul0 = st.ul[cur + g_first];
         if (INC) ub0 = st.ub[g_first];
     }
-    if (!STAGE && INC) r_ref = st.uh[cur + g_ref];
+    if (!STAGE && INC && nl > 0) r_ref = st.uh[cur + g_ref];
     const PassView pv = pass_view(src, p);
     if (pv.skip) {
         // an instance that stopped: its first chunk carries the control block

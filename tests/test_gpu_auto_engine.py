@@ -76,6 +76,35 @@ def test_default_engine_packed(n):
     b.close()
 
 
+@pytest.mark.parametrize("engine", [None, "graph"])
+@pytest.mark.parametrize("at", [0, 1, 2], ids=["first", "middle", "last"])
+@pytest.mark.parametrize("inc", [0, 1], ids=["full", "incremental"])
+def test_packed_instance_without_tets(engine, at, inc):
+    """A packed instance of three nodes and no tets changes nothing for the
+    others, wherever it lies (as the last one its chunk's records are past the
+    table's end)."""
+    m = M.batch_of_boxes(2, seed=4, nxy=(4, 6), nz=(8, 12))
+    cut = m.instance_node_ptr[at]
+    rest = np.insert(m.rest, [cut] * 3, [[9, 0, 0], [9, 1, 0], [9, 0, 1]], axis=0).astype(np.float32)
+    up = lambda i: np.where(i >= cut, i + 3, i)
+    nptr = np.insert(m.instance_node_ptr, at + 1, cut + 3)
+    nptr[at + 2:] += 3
+    tptr = np.insert(m.instance_tet_ptr, at + 1, m.instance_tet_ptr[at])
+    e = M.TetMeshData(rest, up(m.tets), up(m.pins), m.young, m.poisson, instance_node_ptr=nptr.astype(np.int32),
+                      instance_tet_ptr=tptr.astype(np.int32), name="with an empty instance")
+    p = make_params("gpu_reference", h=1 / 30, max_iters=40, incremental_stress=inc)
+    x = []
+    for mesh in (m, e):
+        s = DescentSolver(mesh, params=p)
+        if engine:
+            s.set_pass_engine(engine)
+        s.step()
+        s.step()
+        x.append(s.positions())
+        s.close()
+    assert np.array_equal(x[0], np.delete(x[1], np.arange(cut, cut + 3), axis=0))
+
+
 def test_single_tet_and_loose_nodes():
     """One tet, and nodes that no tet touches (more than a CTA has threads)."""
     x = np.random.default_rng(0).uniform(0, 1, (400, 3)).astype(np.float32)
