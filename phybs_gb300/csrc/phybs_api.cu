@@ -106,6 +106,7 @@ struct pbs_handle {
     DevBuf<CgState> cg_state;   // of the solves of a step
     DevBuf<unsigned> cg_ctl;    // [0] the last tag of the exchanged words, [1] a wait gave up
     CgState *h_cg = nullptr;    // pinned, CG_SOLVES of them, and the two control words
+    bool test_wait_error = false;  // TEST_WAIT_ERROR: the next solve's wait flag is set already
     DevBuf<double2> tpart;
     DevBuf<double> npart;
     DevBuf<float> npartf;
@@ -1066,6 +1067,15 @@ int pbs_set_guess(pbs_handle *h, const float *positions) {
     return PBS_OK;
 }
 
+// For the tests only (not in phybs.h).
+int pbs_test_hook(pbs_handle *h, int what, int value) {
+    if (!h) return PBS_E_INVALID_ARG;
+    switch (what) {
+        case TEST_WAIT_ERROR: h->test_wait_error = value != 0; return PBS_OK;
+        default: return PBS_E_INVALID_ARG;
+    }
+}
+
 int pbs_get_stream(pbs_handle *h, void **stream) {
     if (!h || !stream) return PBS_E_INVALID_ARG;
     *stream = (void *)h->stream;
@@ -1639,6 +1649,11 @@ static int ensure_bsr(pbs_handle *h) {
 // Enqueues one solve A x = b (slot: where its state goes).
 static cudaError_t enqueue_solve(pbs_handle *h, bool scalar, const float *val, const float *dinv, double tol2,
                                  int max_iters, int pnorm, int slot) {
+    if (h->test_wait_error) {
+        h->test_wait_error = false;
+        const cudaError_t e = cudaMemsetAsync(h->cg_ctl.p + 1, 1, sizeof(unsigned), h->stream);
+        if (e != cudaSuccess) return e;
+    }
     CgArgs a{};
     a.val = val;
     a.dinv = dinv;
@@ -1657,13 +1672,18 @@ static cudaError_t enqueue_solve(pbs_handle *h, bool scalar, const float *val, c
 }
 
 // The states of the last `count` solves on the host, and the exchanged words'
-// tags kept from wrapping (or, after a wait that gave up, made clean again).
+// tags kept from wrapping.  A solve takes its state from its first CTA, which
+// may have every word when another CTA's wait gave up (and wrote no rows), so
+// the flag of such a wait makes every one of these solves a timeout; the words
+// are then made clean again.
 static int read_solves(pbs_handle *h, int count) {
     cudaStream_t s = h->stream;
     unsigned *ctl = (unsigned *)(h->h_cg + CG_SOLVES);
     CK(cudaMemcpyAsync(h->h_cg, h->cg_state.p, sizeof(CgState) * count, cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(ctl, h->cg_ctl.p, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    if (ctl[1])
+        for (int k = 0; k < count; ++k) h->h_cg[k].status = PBS_E_DEVICE_TIMEOUT;
     if (ctl[0] > 0x40000000u || ctl[1]) {
         CK(cudaMemsetAsync(h->cg_xp.p, 0, sizeof(float4) * h->cg_xp.n, s));
         CK(cudaMemsetAsync(h->cg_red.p, 0, sizeof(float4) * h->cg_red.n, s));

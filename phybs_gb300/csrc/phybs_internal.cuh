@@ -138,6 +138,12 @@ inline double residual_ratio(const InstCtl &c) {
     return c.g0 > 0.0 ? __builtin_sqrt(c.r2) / c.g0 : 0.0;
 }
 
+// What pbs_test_hook presets, so that the tests reach states that only a fault
+// elsewhere or another device brings about.
+enum TestHook : int {
+    TEST_WAIT_ERROR = 0,  // the next solve finds its flag of a wait that gave up set
+};
+
 struct DevMesh {
     int Np, Tp, n_inst;
     int n_tblk, n_nblk;

@@ -173,3 +173,30 @@ def test_converted_inputs_outlive_the_call():
         s.update_positions(np.asfortranarray(x0.astype(np.float64)))
         assert np.array_equal(s.positions(), x0)
     s.close()
+
+
+TEST_WAIT_ERROR = 0  # pbs_test_hook
+
+
+@pytest.mark.parametrize("integrator", ["be", "pd"])
+def test_wait_that_gave_up_is_an_error(integrator):
+    """A set flag (a CTA whose wait ran out, whether or not the solve's first
+    CTA noticed) ends the step with PBS_E_DEVICE_TIMEOUT, the state as it was;
+    the next step is the one of a handle without it."""
+    m, x0, v0 = _moving(5, 9, 9, 9)
+    mu, lam = O.lame(m.young, m.poisson)
+    a, b = DescentSolver(m, positions=x0, mu=mu, lam=lam), DescentSolver(m, positions=x0, mu=mu, lam=lam)
+    step = lambda s: s.backward_euler_step(tol=1e-6) if integrator == "be" else s.pd_step()
+    a.write_velocities(v0, v0)
+    b.write_velocities(v0, v0)
+    assert L.lib().pbs_test_hook(a._h, TEST_WAIT_ERROR, 1) == 0
+    with pytest.raises(L.PhybsError) as e:
+        step(a)
+    assert e.value.code == L.PBS_E_DEVICE_TIMEOUT
+    assert np.array_equal(a.positions(), b.positions()) and np.array_equal(a.velocities()[0], b.velocities()[0])
+    for _ in range(2):
+        step(a)
+        step(b)
+        assert np.array_equal(a.positions(), b.positions()) and np.array_equal(a.velocities()[0], b.velocities()[0])
+    a.close()
+    b.close()
