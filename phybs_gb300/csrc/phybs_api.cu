@@ -106,7 +106,7 @@ struct pbs_handle {
     DevBuf<CgState> cg_state;   // of the solves of a step
     DevBuf<unsigned> cg_ctl;    // [0] the last tag of the exchanged words, [1] a wait gave up
     CgState *h_cg = nullptr;    // pinned, CG_SOLVES of them, and the two control words
-    bool test_wait_error = false;  // TEST_WAIT_ERROR: the next solve's wait flag is set already
+    bool test_wait_error = false;  // TEST_WAIT_ERROR: the next solve or step finds its wait flag set
     DevBuf<double2> tpart;
     DevBuf<double> npart;
     DevBuf<float> npartf;
@@ -132,7 +132,8 @@ struct pbs_handle {
     DevBuf<float> pd_val, pd_dinv, pd_cgval;
     DevBuf<float4> dyn_px, dyn_x0, dyn_s;
     // host pinned
-    int *h_active = nullptr;   // 2 slots: running counts of the host loop, or the bodies the loop ran
+    int *h_active = nullptr;   // 2 slots: running counts of the host loop; or the bodies the loop ran;
+                               // or, in the second, the frame kernel's flag of a wait that gave up
     InstCtl *h_ctl = nullptr;
     cudaEvent_t ev_start = nullptr, ev_end = nullptr, ev_chunk[2] = {nullptr, nullptr};
     cudaGraphExec_t graph = nullptr;
@@ -845,10 +846,15 @@ static int launch_frame_step(pbs_handle *h, const DevParams &p, int max_passes) 
 }
 
 // After a frame launch that ended with at most `passes` passes of any
-// instance: the tags it used are spent.
-static void frame_done(pbs_handle *h, int passes) {
+// instance; gave_up: the device's flag of a wait that ran out (st.active[1]).
+// Without it the tags the launch used are spent.  With it a CTA may have gone
+// further than the one that reports, so the words are not clean and every
+// instance's results are invalid, whatever its control block says.
+static int frame_done(pbs_handle *h, int passes, int gave_up) {
+    if (gave_up) return PBS_E_DEVICE_TIMEOUT;
     h->frame_tag += (unsigned)passes + 2u;
     h->frame_clean = true;
+    return PBS_OK;
 }
 
 int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
@@ -869,6 +875,10 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     CK(cudaEventRecord(h->ev_start, s));
     if (ext) CK(cudaMemcpyAsync(h->staging.p, ext, sizeof(float) * 3 * (size_t)h->N, cudaMemcpyHostToDevice, s));
     CK(cudaMemsetAsync(h->active.p, 0, 4 * sizeof(int), s));
+    if (h->test_wait_error) {
+        h->test_wait_error = false;
+        CK(cudaMemsetAsync(h->active.p + 1, 1, sizeof(int), s));
+    }
     CK(launch_init_ctl(s, h->B, h->dparams, st));
     CK(launch_prologue(s, m, h->dparams, st, ext ? h->staging.p : nullptr, h->pad2user.p));
     CK(launch_guess_check(s, m, h->dparams, st));
@@ -894,6 +904,7 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     if (frame) {
         rc = launch_frame_step(h, h->dparams, h->dparams.pass_cap);
         if (rc != PBS_OK) return rc;
+        CK(cudaMemcpyAsync(h->h_active + 1, h->active.p + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
     } else if (h->graph_loop) {
         CK(cudaGraphLaunch(h->graph, s));
         CK(cudaMemcpyAsync(h->h_active, h->active.p + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -918,10 +929,12 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     cudaEventElapsedTime(&ms, h->ev_start, h->ev_end);
     h->last_ms = ms;
     if (!frame && h->graph_loop) launched = h->h_active[0];
+    const bool gave_up = frame && h->h_active[1] != 0;
     pbs_stats S{};
     S.status = PBS_OK;
     for (int b = 0; b < h->B; ++b) {
-        const InstCtl &c = h->h_ctl[b];
+        InstCtl &c = h->h_ctl[b];
+        if (gave_up) c.status = PBS_E_DEVICE_TIMEOUT;
         S.passes = std::max(S.passes, c.passes);
         S.iterations = std::max(S.iterations, c.k);
         S.rejections += c.rejections;
@@ -940,7 +953,7 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     // the default engine counts in bodies whichever kernel ran its passes
     S.graph_launches = auto_frame ? std::max(1, (S.passes + CHUNK_PASSES - 1) / CHUNK_PASSES) : launched;
     h->stats = S;
-    if (frame) frame_done(h, S.passes);
+    if (frame) frame_done(h, S.passes, gave_up);
     if (iters_out) *iters_out = S.iterations;
     return S.status;
 }
@@ -1175,8 +1188,10 @@ static int time_frame(pbs_handle *h, int passes, double *pass_ms) {
     CK(e);
     if (rc != PBS_OK) return rc;
     InstCtl c;
+    int gave_up = 0;
     CK(cudaMemcpy(&c, h->ctl.p, sizeof(InstCtl), cudaMemcpyDeviceToHost));
-    frame_done(h, passes);
+    CK(cudaMemcpy(&gave_up, h->active.p + 1, sizeof(int), cudaMemcpyDeviceToHost));
+    if (frame_done(h, passes, gave_up) != PBS_OK) c.status = PBS_E_DEVICE_TIMEOUT;
     if (c.status != PBS_OK || c.passes < passes) {
         pbs_stats S{};
         S.passes = c.passes; S.iterations = c.k; S.rejections = c.rejections; S.converged = c.converged;

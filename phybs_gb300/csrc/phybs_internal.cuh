@@ -141,7 +141,7 @@ inline double residual_ratio(const InstCtl &c) {
 // What pbs_test_hook presets, so that the tests reach states that only a fault
 // elsewhere or another device brings about.
 enum TestHook : int {
-    TEST_WAIT_ERROR = 0,  // the next solve finds its flag of a wait that gave up set
+    TEST_WAIT_ERROR = 0,  // the next solve or step finds its flag of a wait that gave up set
 };
 
 struct DevMesh {

@@ -220,3 +220,35 @@ def test_profile_frame_runs_the_passes():
     print(f"frame engine {ms * 1e3:.1f} us a pass; graph engine kernels {tet * 1e3:.1f} + {node * 1e3:.1f} us")
     assert np.array_equal(s.positions(), x)  # the state is left as it was
     s.close()
+
+
+TEST_WAIT_ERROR = 0  # pbs_test_hook
+
+
+@pytest.mark.parametrize("engine", ["auto", "frame", "graph"])
+def test_wait_that_gave_up_is_an_error(engine):
+    """A set flag (a CTA whose wait ran out, whether or not the CTA that writes
+    the control block noticed) ends the step with PBS_E_DEVICE_TIMEOUT; the
+    steps after it are those of a handle without it."""
+    m = M.box_mesh(8, 7, 12, edge=0.03, seed=2, young=1e5)
+    p = make_params("gpu_reference", h=1 / 30, max_iters=24)
+    a, b = DescentSolver(m, params=p), DescentSolver(m, params=p)
+    if engine == "frame":
+        for s in (a, b):
+            s.set_chunk_shape(128, 256, 160)
+    if engine != "auto":
+        for s in (a, b):
+            s.set_pass_engine(engine)
+    a.step()
+    assert L.lib().pbs_test_hook(a._h, TEST_WAIT_ERROR, 1) == 0
+    with pytest.raises(L.PhybsError) as e:
+        a.step()
+    assert e.value.code == L.PBS_E_DEVICE_TIMEOUT
+    assert a.stats()["status"] == a.instance_stats(0)["status"] == L.PBS_E_DEVICE_TIMEOUT
+    a.reset()
+    for _ in range(3):
+        a.step()
+        b.step()
+        assert np.array_equal(a.positions(), b.positions())
+    a.close()
+    b.close()
