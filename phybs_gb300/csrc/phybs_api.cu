@@ -21,16 +21,31 @@ namespace {
 constexpr int CHUNK_PASSES = 16;  // passes per body of the step graph
 constexpr int CG_SOLVES = 64;     // solves of a step between two reads of their states
 
+// TEST_FAIL_ALLOC: the allocation of this thread that is to fail, from 1 (0: none)
+thread_local int test_fail_alloc = 0;
+
+// Device memory of n elements; p is null and n 0 without it, so that a call
+// whose allocation failed finds nothing to use and allocates again.
 template <typename T> struct DevBuf {
     T *p = nullptr;
     size_t n = 0;
     cudaError_t alloc(size_t count) {
+        release();
+        cudaError_t e = cudaErrorMemoryAllocation;
+        if (test_fail_alloc == 0 || --test_fail_alloc != 0)
+            e = cudaMalloc((void **)&p, std::max<size_t>(count, 1) * sizeof(T));
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();  // (the next launch's check is not to find it)
+            p = nullptr;
+            return e;
+        }
         n = count;
-        return cudaMalloc((void **)&p, std::max<size_t>(count, 1) * sizeof(T));
+        return cudaSuccess;
     }
     void release() {
         if (p) cudaFree(p);
         p = nullptr;
+        n = 0;
     }
 };
 
@@ -245,8 +260,8 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
         CK(cudaMemcpy(ctl.data(), h->ctl.p, sizeof(InstCtl) * h->B, cudaMemcpyDeviceToHost));
     }
     std::vector<ChunkLimits> limits(h->B, ChunkLimits{ct, cn});
-    h->shape_auto = threads == 0;
-    if (threads == 0) {
+    const bool automatic = threads == 0;
+    if (automatic) {
         ct = cn = 0;
         for (int b = 0; b < h->B; ++b) {
             limits[b] = auto_chunk_limits(ctl[b].tet_end - ctl[b].tet_begin, h->sms);
@@ -254,7 +269,7 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
             cn = std::max(cn, limits[b].nodes);
         }
     }
-    const bool grouped = h->shape_auto;  // (a caller's own shape keeps a reference node a chunk)
+    const bool grouped = automatic;  // (a caller's own shape keeps a reference node a chunk)
     ChunkLayout cl;
     const std::vector<InstCtl> ctl0 = ctl;
     build_chunks(h->Np, h->h_tets_pad, h->h_rest_pad, ctl, limits, grouped, true, cl);
@@ -267,18 +282,36 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
     // (a packed batch's with 256 threads, which its smaller instances can use);
     // the frame kernel, where every chunk has its place, with up to four
     // (auto_chunk_limits has both sides)
-    if (threads == 0) {
+    if (automatic) {
         if (ct == CHUNK_GROUP_TETS) threads = nc > h->sms && h->B == 1 ? 512 : 256;
         else threads = ct > 256 && nc > 2 * h->sms ? 256 : 128;
     }
     const size_t L = cl.lmeta.size(), T = (size_t)h->T;
-    h->chunk.release(); h->chunk_inst.release(); h->cpart.release(); h->qperm.release();
-    h->lmeta.release(); h->pptr.release();
-    h->part.release(); h->parth.release();
-    CK(h->chunk.alloc(nc)); CK(h->chunk_inst.alloc(nc)); CK(h->cpart.alloc(nc));
-    CK(h->qperm.alloc(T));
-    CK(h->lmeta.alloc(L)); CK(h->pptr.alloc(h->Np + 1));
-    CK(h->part.alloc(L)); CK(h->parth.alloc(L));
+    // all of the new layout's memory before the old one's is given up: a
+    // handle that runs out of it keeps the layout it had
+    DevBuf<int4> chunk, lmeta;
+    DevBuf<int> chunk_inst, qperm, pptr;
+    DevBuf<double2> cpart;
+    DevBuf<float4> part, parth;
+    cudaError_t ea = chunk.alloc(nc);
+    if (ea == cudaSuccess) ea = chunk_inst.alloc(nc);
+    if (ea == cudaSuccess) ea = cpart.alloc(nc);
+    if (ea == cudaSuccess) ea = qperm.alloc(T);
+    if (ea == cudaSuccess) ea = lmeta.alloc(L);
+    if (ea == cudaSuccess) ea = pptr.alloc(h->Np + 1);
+    if (ea == cudaSuccess) ea = part.alloc(L);
+    if (ea == cudaSuccess) ea = parth.alloc(L);
+    if (ea == cudaSuccess) {
+        std::swap(h->chunk, chunk); std::swap(h->lmeta, lmeta);
+        std::swap(h->chunk_inst, chunk_inst); std::swap(h->qperm, qperm); std::swap(h->pptr, pptr);
+        std::swap(h->cpart, cpart);
+        std::swap(h->part, part); std::swap(h->parth, parth);
+    }
+    chunk.release(); lmeta.release(); chunk_inst.release(); qperm.release(); pptr.release(); cpart.release();
+    part.release(); parth.release();
+    CK(ea);
+    h->shape_auto = automatic;
+    h->graph_valid = h->plan_valid = false;
     cudaStream_t s = h->stream;
     CK(cudaMemcpyAsync(h->chunk.p, cl.chunk.data(), sizeof(int4) * nc, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(h->chunk_inst.p, cl.chunk_inst.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, s));
@@ -302,7 +335,6 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
                             h->qrow2));
     }
     CK(cudaStreamSynchronize(s));
-    h->graph_valid = h->plan_valid = false;
     return PBS_OK;
 }
 
@@ -809,17 +841,16 @@ static int launch_frame_step(pbs_handle *h, const DevParams &p, int max_passes) 
     const FramePlan &plan = handle_frame_plan(h);
     if (plan.grid <= 0) return PBS_E_INVALID_ARG;
     cudaStream_t s = h->stream;
-    if (!h->fxh.p) {
+    // (each group is known by its last member)
+    if (!h->fxl.p) {
+        h->frame_clean = false;
         CK(h->fxh.alloc(h->Np));
         CK(h->fxl.alloc(h->Np));
-        h->frame_clean = false;
     }
-    if (h->fce.n < (size_t)plan.grid) {
-        h->fce.release();
-        h->fcr.release();
+    if (h->fcr.n < 2 * (size_t)plan.grid) {
+        h->frame_clean = false;
         CK(h->fce.alloc(plan.grid));
         CK(h->fcr.alloc(2 * (size_t)plan.grid));
-        h->frame_clean = false;
     }
     // tags only grow, so the words of earlier launches need no clearing; they
     // are cleared after a launch whose passes are not known, and long before
@@ -1085,6 +1116,7 @@ int pbs_test_hook(pbs_handle *h, int what, int value) {
     if (!h) return PBS_E_INVALID_ARG;
     switch (what) {
         case TEST_WAIT_ERROR: h->test_wait_error = value != 0; return PBS_OK;
+        case TEST_FAIL_ALLOC: test_fail_alloc = value; return PBS_OK;
         default: return PBS_E_INVALID_ARG;
     }
 }
@@ -1243,8 +1275,9 @@ int pbs_set_chunk_shape(pbs_handle *h, int threads, int chunk_tets, int chunk_no
             (size_t)CHUNK_MAX_SMEM)
         return PBS_E_INVALID_ARG;
     PBS_DEVICE_SCOPE(h->device);
-    h->node_npt = node_npt;
-    return set_pass_layout(h, threads, chunk_tets, chunk_nodes, staged, nullptr);
+    const int rc = set_pass_layout(h, threads, chunk_tets, chunk_nodes, staged, nullptr);
+    if (rc == PBS_OK) h->node_npt = node_npt;
+    return rc;
 }
 
 int pbs_autotune(pbs_handle *h, int passes, pbs_tune_result *out) {
@@ -1859,7 +1892,7 @@ static int ensure_pbd(pbs_handle *h) {
 }
 
 static int ensure_dyn_buffers(pbs_handle *h) {
-    if (h->dyn_px.p) return PBS_OK;
+    if (h->dyn_s.p) return PBS_OK;  // (the last of the three)
     CK(h->dyn_px.alloc(h->Np)); CK(h->dyn_x0.alloc(h->Np)); CK(h->dyn_s.alloc(h->Np));
     return PBS_OK;
 }
@@ -1919,7 +1952,7 @@ int pbs_pd_step(pbs_handle *h, float dt, float dt_matrix, float stiffness, int i
     A.ptr = h->bsr_ptr.p;
     A.col = h->bsr_col.p;
     A.scalar = 1;
-    if (!h->pd_val.p) {
+    if (!h->pd_dinv.p) {  // (the last of the three)
         int nnzb = 0;
         CK(cudaMemcpy(&nnzb, h->bsr_ptr.p + h->Np, sizeof(int), cudaMemcpyDeviceToHost));
         CK(h->pd_val.alloc((size_t)nnzb));

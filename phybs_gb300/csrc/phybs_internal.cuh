@@ -142,6 +142,7 @@ inline double residual_ratio(const InstCtl &c) {
 // elsewhere or another device brings about.
 enum TestHook : int {
     TEST_WAIT_ERROR = 0,  // the next solve or step finds its flag of a wait that gave up set
+    TEST_FAIL_ALLOC = 1,  // the value-th device allocation of this thread from now fails
 };
 
 struct DevMesh {
