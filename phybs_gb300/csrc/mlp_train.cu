@@ -457,6 +457,7 @@ struct pbs_mlp {
     int *idx = nullptr;
     int n = 0, cap_part = 0, cap_io = 0, cap_losses = 0, step = 0;
     unsigned arrivals = 0;  // the barrier's count after the launches so far
+    int launch_steps = TRAIN_STEPS;  // steps of a launch at most
 };
 
 #define MCK(x)                                                                               \
@@ -693,7 +694,7 @@ int pbs_mlp_train(pbs_mlp *t, int steps, int batch, float lr, unsigned long long
         if (e) MCK(cudaStreamSynchronize(t->stream));
         MCK(cudaMemcpyAsync(t->idx, p.data(), sizeof(int) * t->n, cudaMemcpyHostToDevice, t->stream));
         for (int k = 0; k < epoch && done < steps;) {
-            const int now = std::min({epoch - k, steps - done, TRAIN_STEPS});
+            const int now = std::min({epoch - k, steps - done, t->launch_steps});
             rc = run_train(t, t->X, t->Y, t->W, t->idx + (size_t)k * batch, batch, now, lr, t->losses + done);
             if (rc != PBS_OK) {
                 cudaStreamSynchronize(t->stream);
@@ -706,6 +707,13 @@ int pbs_mlp_train(pbs_mlp *t, int steps, int batch, float lr, unsigned long long
     if (losses && steps > 0)
         MCK(cudaMemcpyAsync(losses, t->losses, sizeof(float) * steps, cudaMemcpyDeviceToHost, t->stream));
     return finish(t);
+}
+
+// For the tests only (not in phybs.h): at most `steps` steps a launch.
+int pbs_mlp_test_launch_steps(pbs_mlp *t, int steps) {
+    if (!t || steps < 1 || steps > TRAIN_STEPS) return PBS_E_INVALID_ARG;
+    t->launch_steps = steps;
+    return PBS_OK;
 }
 
 }  // extern "C"

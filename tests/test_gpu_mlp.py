@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from oracle import mlp as OM
+from phybs_gb300 import _lib as L
 from phybs_gb300.warmstart import MLPTrainer
 
 pytestmark = pytest.mark.gpu
@@ -144,3 +145,43 @@ def test_steps_of_one_launch_match_adam(n, steps, weighted):
         assert np.abs(a.params - ref).max() < steps * (1e-6 + 1e-5 * np.abs(ref).max())
     a.close()
     b.close()
+
+
+# (rows, batch, steps): batches below a tile, not a multiple of it, beyond one
+# tile a SM; several epochs, rows left over in each; more steps an epoch than a
+# launch takes (64), once with rows left over
+@pytest.mark.parametrize("n,batch,steps", [(1000, 16, 130), (1000, 99, 25), (4097, 64, 70), (5000, 333, 31),
+                                           (30001, 9729, 7), (65, 64, 5)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_steps_of_one_launch_equal_single_steps(n, batch, steps, weighted):
+    """Minibatches of one launch (rows found on the device, weights carried from
+    step to step there) against the same ones a launch each: bit for bit."""
+    theta = OM.init_params(5).astype(np.float32)
+    X, Y = _data(n, 6)
+    W = np.random.default_rng(7).uniform(0.2, 3.0, n).astype(np.float32) if weighted else None
+    out = []
+    for cap in (64, 1):
+        t = MLPTrainer(theta)
+        assert L.lib().pbs_mlp_test_launch_steps(t._t, cap) == 0
+        t.set_data(X, Y, W)
+        out.append((t.train(steps, batch=batch, lr=1e-3, seed=9), t.params))
+        t.close()
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+    assert not np.array_equal(out[0][1], theta)
+
+
+@pytest.mark.parametrize("n,batch", [(6400, 100), (9600, 96), (4096, 1024)])
+def test_an_epoch_takes_every_row_once(n, batch):
+    """With a step too small to change a parameter (1e-30) the mean loss of an
+    epoch's minibatches is the loss of all rows.  Both are FP32 sums of n
+    positive terms: they agree to a few times 2^-24 sqrt(n), below 1e-5."""
+    theta = OM.init_params(5).astype(np.float32)
+    X, Y = _data(n, 8)
+    Y *= np.linspace(0.1, 3, n, dtype=np.float32)[:, None]  # no two rows weigh the same
+    t = MLPTrainer(theta)
+    full, _ = t.gradient(X, Y)
+    t.set_data(X, Y)
+    losses = t.train(n // batch, batch=batch, lr=1e-30, seed=3)
+    assert np.abs(t.params - theta).max() <= 1e-28
+    assert abs(losses.astype(np.float64).mean() - full) <= 1e-5 * full
+    t.close()
