@@ -94,8 +94,9 @@ __device__ __forceinline__ TetRows load_rows(const ChunkView &v, int lt) {
 // returns the thread's sum of clamped tet energies.
 // A near-inverted tet (full stress) gets its FP32 forces here and a mark in
 // its corner-0 slot's .w; *any_exact tells whether the thread marked one.
-// CHECK: a line-search pass (the tet energies too); the loop is compiled once
-// with and once without them.  first: the constants of the thread's first tet,
+// CHECK: a line-search pass (the tet energies too, each also in its corner-1
+// slot's .w for team_energy); the loop is compiled once with and once without
+// them.  first: the constants of the thread's first tet,
 // where the caller loaded them ahead (PRE).
 template <int MATERIAL, int THREADS, bool INC, bool PACK, bool PRE, bool CHECK>
 __device__ __forceinline__ DFloat chunk_forces(const DevParams &p, const ChunkView &v, int nt, float4 *sf,
@@ -120,9 +121,12 @@ __device__ __forceinline__ DFloat chunk_forces(const DevParams &p, const ChunkVi
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc)
             sts128(sf + sl[cc], f[3 * cc], f[3 * cc + 1], f[3 * cc + 2], cc == 0 && ex ? 1.f : 0.f);
-        if (CHECK)
-            e = df_add(e, search_energy(energy_density<float>(kin, r1.w, r2.w) * fabsf(r0.w), p.clamp_cpu,
-                                        p.control == PBS_CONTROL_RESTART));
+        if (CHECK) {
+            const float en = search_energy(energy_density<float>(kin, r1.w, r2.w) * fabsf(r0.w), p.clamp_cpu,
+                                           p.control == PBS_CONTROL_RESTART);
+            e = df_add(e, en);
+            sf[sl[1]].w = en;
+        }
     }
     *any_exact = any;
     return e;
@@ -161,8 +165,10 @@ __device__ __forceinline__ void chunk_exact(const ChunkView &v, int nt, float4 *
             pk1_exact_fp64(MATERIAL, CornerRest{v.rest, v.meta, {lc[0], lc[1], lc[2], lc[3]}}, x[0], x[1], x[2],
                            x[3], l[0], l[1], l[2], l[3], r0, r1, r2, r1.w, r2.w, P);
         corner_forces(P, dinv, r0.w, f);
+        const float en = lds128(sf + sl[1]).w;
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) sts128(sf + sl[cc], f[3 * cc], f[3 * cc + 1], f[3 * cc + 2]);
+        for (int cc = 0; cc < 4; ++cc)
+            sts128(sf + sl[cc], f[3 * cc], f[3 * cc + 1], f[3 * cc + 2], cc == 1 ? en : 0.f);
     }
 }
 
@@ -201,6 +207,34 @@ __device__ __forceinline__ DFloat chunk_forces_all(const DevParams &p, const Chu
     return e;
 }
 
+// Thread t's sum of the chunk's tet energies where the instance's team is not
+// the CTA's threads: the tets t, t + team, ..., from the slots that the tet loop
+// left them in (threads beyond the team: nothing).  Before anything else goes
+// into the slots.
+__device__ __forceinline__ DFloat team_energy(const ChunkView &v, int nt, int team, const float4 *sf) {
+    DFloat e{0.f, 0.f};
+    if (threadIdx.x < team)
+        for (int lt = threadIdx.x; lt < nt; lt += team) {
+            int lc[4], sl[4];
+            unpack_cor(v.cor[lt], lc, sl);
+            e = df_add(e, lds128(sf + sl[1]).w);
+        }
+    return e;
+}
+
+// The energy terms of the nodes [n, n1), every team-th, added to the thread's e
+// and their squares to e2.
+__device__ __forceinline__ void share_energy(const DevMesh &m, const DevParams &p, const DevState &st, size_t cur, int n,
+                                             int n1, int team, const float4 *base, DFloat &e, float &e2) {
+    for (int i = n; i < n1; i += team) {
+        const float4 info = m.info[i];
+        if (info.z != 0.f) continue;
+        const DFloat en = node_energy_df(st, info, st.uh[cur + i], st.ul[cur + i], i, p.h2inv, base);
+        e = df_add(e, en);
+        e2 = fmaf(en.hi, en.hi, e2);
+    }
+}
+
 // A thread's share of the line search's noise scale, from the sum e of its tet
 // energies: the scale adds the squares of the sums of m.noise_tets tets (four,
 // whose threads' sums are grouped by neighbouring lanes; 0: of each thread's
@@ -208,11 +242,24 @@ __device__ __forceinline__ DFloat chunk_forces_all(const DevParams &p, const Chu
 // chunk size.  With each thread's own at one or two tets a thread the allowance
 // was half as large, and one pull in ten to a residual of 1e-4 took another
 // rejection.  Called by whole warps.
-template <int THREADS> __device__ __forceinline__ float noise_square(const DevMesh &m, int nt, float e) {
-    const int lanes = m.noise_tets == 0 || nt > 3 * THREADS ? 1 : nt > THREADS ? m.noise_tets / 2 : m.noise_tets;
+__device__ __forceinline__ float noise_square(const DevMesh &m, int team, int nt, float e) {
+    const int lanes = m.noise_tets == 0 || nt > 3 * team ? 1 : nt > team ? m.noise_tets / 2 : m.noise_tets;
     if (lanes > 1) e += __shfl_xor_sync(0xffffffffu, e, 1);
     if (lanes > 2) e += __shfl_xor_sync(0xffffffffu, e, 2);
     return e * e / (float)lanes;
+}
+
+// A chunk's sums from the warps' (s_e, s_e2: team / 32 of them), by one warp;
+// valid in lane 0.
+__device__ __forceinline__ void join_warps(const float2 *s_e, const float *s_e2, int team, double &e, float &e2) {
+    const int warps = team >> 5, w = threadIdx.x & (warps - 1);
+    DFloat se{s_e[w].x, s_e[w].y};
+    e2 = s_e2[w];
+    for (int o = warps >> 1; o > 0; o >>= 1) {
+        se = df_add(se, DFloat{__shfl_down_sync(0xffffffffu, se.hi, o), __shfl_down_sync(0xffffffffu, se.lo, o)});
+        e2 += __shfl_down_sync(0xffffffffu, e2, o);
+    }
+    e = df_double(se);
 }
 
 // Jacobi-diagonal refresh: the same slots carry the 12 diagonal terms.

@@ -40,6 +40,7 @@
 
 #include "../../include/phybs.h"
 #include "chunk_tets.cuh"
+#include "exchange.cuh"
 #include "pass_ctl.cuh"
 #include "pass_math.cuh"
 #include "phybs_internal.cuh"
@@ -238,6 +239,8 @@ ChunkLimits auto_chunk_limits(int tets, int sms) {
     return ChunkLimits{n, 32 + n / 2 + n / 16};
 }
 
+int auto_team(int tets, int sms) { return tets <= 2 * 342 * sms ? 128 : 256; }
+
 // ------------------------------------------------------------ device
 __global__ void k_pass_rows(int T, const int *qperm, const float4 *row0, const float4 *row1, const float4 *row2,
                             float4 *q0, float4 *q1, float4 *q2) {
@@ -249,51 +252,54 @@ __global__ void k_pass_rows(int T, const int *qperm, const float4 *row0, const f
     q2[j] = row2[t];
 }
 
-// Line-search pass: adds the chunk's share of the instance's node energy terms
-// to the thread's tet energies e, stores the chunk's {sum e, sum e^2}, and in
-// the instance's last chunk to finish sums the chunks in order and decides
-// accept / reject (DescentOptimize.cpp:107-128) on dst, the control-block copy
-// the pass's node kernel reads (its first chunk settled the last pass into
-// it before counting itself in).  The sums run in double-float (e) and FP32
-// (e^2, a noise scale), the chunk totals and their sum in FP64.  Called by
-// every thread of the CTA; *is_last is a shared word.
+// Line-search pass: the chunk's {sum e, sum e^2} of its tets and of its share
+// of the instance's nodes -> st.cpart.  e: the thread's tet energies, where the
+// team is the CTA's threads.  Double-float (e) and FP32 (e^2, a noise scale),
+// in the order that phybs_internal.cuh gives.  Called by every thread, before
+// anything else goes into the slots.
+template <int THREADS>
+__device__ __forceinline__ void chunk_energy(const DevMesh &m, const DevParams &p, const DevState &st, int c, int inst,
+                                             int par, size_t cur, const ChunkView &v, int nt, const float4 *sf,
+                                             DFloat ec) {
+    __shared__ float2 s_e[THREADS / 32];
+    __shared__ float s_e2[THREADS / 32];
+    // (formed here, not carried through the tet loop: registers are short)
+    const InstCtl *src = ctl_buf(st, par) + inst;
+    const int team = src->team, cb = src->cblk_begin, n0 = src->node_begin;
+    if (team != THREADS) ec = team_energy(v, nt, team, sf);
+    DFloat e{0.f, 0.f};
+    float e2 = 0.f;
+    if (threadIdx.x < team) {
+        const int per = node_share(src->node_end - n0, src->cblk_end - cb), a = n0 + (c - cb) * per;
+        share_energy(m, p, st, cur, a + threadIdx.x, min(a + per, src->node_end), team,
+                     p.incremental ? st.ub : nullptr, e, e2);
+        e = warp_sum_df(df_add(e, ec));
+        e2 = warp_sum_f(e2 + noise_square(m, team, nt, ec.hi));
+        if ((threadIdx.x & 31) == 0) {
+            s_e[threadIdx.x >> 5] = make_float2(e.hi, e.lo);
+            s_e2[threadIdx.x >> 5] = e2;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    double d;
+    join_warps(s_e, s_e2, team, d, e2);
+    if (threadIdx.x == 0) st.cpart[c] = make_double2(d, (double)e2);
+}
+
+// Then counts the chunk in, and in the instance's last one sums the chunks and
+// decides accept / reject (DescentOptimize.cpp:107-128) on dst, the
+// control-block copy the pass's node kernel reads (its first chunk settled the
+// last pass into it before counting itself in).  The sum runs in FP64.  Called
+// by every thread of the CTA; *is_last is a shared word.
 template <int THREADS>
 __device__ __forceinline__ void chunk_line_search(const DevMesh &m, const DevParams &p, const DevState &st, int c,
-                                                  int inst, int par, int k, size_t cur, DFloat e, double *sh,
-                                                  int *is_last) {
-    __shared__ float2 shf[THREADS / 32];
-    // (formed here, not carried through the tet loop: registers are short)
+                                                  int inst, int par, int k, double *sh, int *is_last) {
     const InstCtl *src = ctl_buf(st, par) + inst;
     InstCtl *dst = ctl_buf(st, par ^ 1) + inst;
     unsigned int *cnt = st.tcount + inst;
-    __shared__ float shs[THREADS / 32];
-    float e2;
-    if (THREADS == 512 && m.noise_tets != 0 && m.chunk[c].y > THREADS) {
-        // two tets a thread: with those of the thread half a CTA away
-        __shared__ float s_e[THREADS / 2];
-        if (threadIdx.x >= THREADS / 2) s_e[threadIdx.x - THREADS / 2] = e.hi;
-        __syncthreads();
-        const float x = threadIdx.x < THREADS / 2 ? e.hi + s_e[threadIdx.x] : 0.f;
-        e2 = x * x;
-    } else {
-        e2 = noise_square<THREADS>(m, m.chunk[c].y, e.hi);
-    }
     const int cb = src->cblk_begin, ce = src->cblk_end;
-    {
-        const int nb = ce - cb;
-        const float4 *U = st.uh + cur;
-        for (int i = src->node_begin + (c - cb) * THREADS + threadIdx.x; i < src->node_end; i += nb * THREADS) {
-            const float4 info = m.info[i];
-            if (info.z != 0.f) continue;
-            const DFloat en = node_energy_df(st, info, U[i], st.ul[cur + i], i, p.h2inv, p.incremental ? st.ub : nullptr);
-            e = df_add(e, en);
-            e2 = fmaf(en.hi, en.hi, e2);
-        }
-    }
-    const DFloat se = block_sum_df(e, shf);
-    const float se2 = block_sum_f(e2, shs);
     if (threadIdx.x == 0) {
-        st.cpart[c] = make_double2(df_double(se), (double)se2);
         __threadfence();
         const unsigned int prev = atomicAdd(cnt, 1u);
         *is_last = (prev == (unsigned int)(ce - cb - 1));
@@ -301,26 +307,27 @@ __device__ __forceinline__ void chunk_line_search(const DevMesh &m, const DevPar
     __syncthreads();
     if (!*is_last) return;
     __threadfence();
-    // the instance's last chunk: fixed-order sums (each thread adds its chunks
-    // in ascending order, then the block tree), then accept / reject.  The
+    // the instance's last chunk: fixed-order sums, then accept / reject.  The
     // partials are loaded eight at a time ahead of their additions: this tail
     // runs on one CTA while the rest of the GPU waits, and one load round trip
     // per partial made it several microseconds
     constexpr int U = 8;
+    const int lanes = ce - cb <= SUM_CHUNKS ? 32 : THREADS < 256 ? THREADS : 256;
     double ea = 0.0, eb = 0.0;
-    for (int j0 = cb + threadIdx.x; j0 < ce; j0 += U * THREADS) {
-        double2 v[U];
+    if (threadIdx.x < lanes)
+        for (int j0 = cb + threadIdx.x; j0 < ce; j0 += U * lanes) {
+            double2 v[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int j = j0 + u * THREADS;
-            v[u] = j < ce ? __ldcg(st.cpart + j) : make_double2(0.0, 0.0);
-        }
+            for (int u = 0; u < U; ++u) {
+                const int j = j0 + u * lanes;
+                v[u] = j < ce ? __ldcg(st.cpart + j) : make_double2(0.0, 0.0);
+            }
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            ea += v[u].x;
-            eb += v[u].y;
+            for (int u = 0; u < U; ++u) {
+                ea += v[u].x;
+                eb += v[u].y;
+            }
         }
-    }
     const double E = block_sum(ea, sh);
     const double E2 = block_sum(eb, sh);
     if (threadIdx.x != 0) return;
@@ -344,6 +351,7 @@ __device__ __forceinline__ void chunk_body(const DevMesh &m, const DevParams &p,
                                            int *is_last, const TetRows &first = TetRows()) {
     const DFloat e = chunk_forces_all<MATERIAL, THREADS, INC, PACK, PRE>(p, v, nt, pv.check, sf, first);
     chunk_partials<THREADS>(meta, nl, sf, st.part);
+    if (pv.check) chunk_energy<THREADS>(m, p, st, c, inst, par, cur, v, nt, sf, e);
     if (pv.do_h) {
         __syncthreads();
         chunk_hdiag<MATERIAL, THREADS, INC, PACK>(v, nt, sf);
@@ -355,7 +363,7 @@ __device__ __forceinline__ void chunk_body(const DevMesh &m, const DevParams &p,
     // waiting), and before it counts itself into a line search
     const InstCtl *src = ctl_buf(st, par) + inst;
     if (c == src->cblk_begin) settle_pass<THREADS>(p, st, src, ctl_buf(st, par ^ 1) + inst, true);
-    if (pv.check) chunk_line_search<THREADS>(m, p, st, c, inst, par, pv.k, cur, e, sh, is_last);
+    if (pv.check) chunk_line_search<THREADS>(m, p, st, c, inst, par, pv.k, sh, is_last);
 }
 
 // One CTA per chunk.  What bounds it: with four CTAs of 256 threads a SM, each

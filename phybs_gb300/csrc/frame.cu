@@ -223,8 +223,9 @@ struct FrameView {
 //   workers   update their nodes and publish them; warp sums of |g|^2;
 //   (one CTA barrier)
 //   control   publishes the CTA's |g|^2.
-// The nodes of an instance are split evenly among its CTAs (27 a CTA on the
-// 24,000-tet bar), so that no CTA's node phase is longer than another's.
+// The nodes of an instance are split evenly among its CTAs, in whole warps (64
+// a CTA on the 24,000-tet bar), so that no CTA's node phase is longer than
+// another's and the sums are the pass kernels' (phybs_internal.cuh).
 // PER_SM: CTAs a SM the registers are budgeted for.  A pass is bound by the
 // dependent chain of one tet, so a mesh that needs fewer CTAs a SM runs the
 // variant with more registers: on 24,500 tets 493 us a 96-pass step at one
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
     __shared__ InstCtl sc;  // this CTA's copy of the instance's control block (the control warp's)
     __shared__ FrameView sv;
     __shared__ float2 s_e[WARPS];
-    __shared__ float s_e2[WARPS], s_g2[WARPS];
+    __shared__ float s_e2[WARPS], s_g2[SUM_GROUPS];
     const int b = blockIdx.x, tid = threadIdx.x;
     const bool worker = tid < THREADS;
     const int inst = RES ? m.chunk_inst[b] : 0;
@@ -277,7 +278,8 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
     const int bi = b - cb;
     int *err = st.active + 1;
     // this CTA's nodes [n0, n1), this thread's i0, i0 + THREADS, ...
-    const int per = (sc.node_end - sc.node_begin + G - 1) / G;
+    const int per = node_share(sc.node_end - sc.node_begin, G);
+    const int team = sc.team;
     const int n0 = min(sc.node_begin + bi * per, sc.node_end), n1 = min(n0 + per, sc.node_end);
     const int i0 = worker ? n0 + tid : n1;
     int pa0 = 0, pe0 = 0;
@@ -321,18 +323,9 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
                 nn.dd = st.dd[cur + i0];
                 nn.diag = st.diag[i0];
             }
-            if (check) {
-                // the CTA's share of the node energy terms, before the other
-                // CTAs' words arrive
-                for (int i = i0; i < n1; i += THREADS) {
-                    const float4 info = m.info[i];
-                    if (info.z != 0.f) continue;
-                    const DFloat en = node_energy_df(st, info, st.uh[cur + i], st.ul[cur + i], i, p.h2inv,
-                                                     INC ? st.ub : nullptr);
-                    e = df_add(e, en);
-                    e2 = fmaf(en.hi, en.hi, e2);
-                }
-            }
+            // the CTA's share of the node energy terms, before the other CTAs'
+            // words arrive
+            if (check && tid < team) share_energy(m, p, st, cur, i0, n1, team, INC ? st.ub : nullptr, e, e2);
             // ---- tet phase: this CTA's chunk, or the chunks b, b + G, ...
             for (int c = b; c < m.n_chunks; c += RES ? m.n_chunks : G) {
                 const int4 cd = m.chunk[c];
@@ -365,7 +358,8 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
                 v.cor = RES ? s_cor : m.qcor + cd.x;
                 v.meta = meta;
                 v.rest = m.rest;
-                const DFloat ec = chunk_forces_all<MATERIAL, THREADS, INC, true, false, true>(p, v, nt, check, s_f);
+                DFloat ec = chunk_forces_all<MATERIAL, THREADS, INC, true, false, true>(p, v, nt, check, s_f);
+                if (check && team != THREADS) ec = team_energy(v, nt, team, s_f);
                 publish_partials<THREADS>(meta, nl, s_f, st.part, tag);
                 if (do_h) {
                     chunk_sync<THREADS, true>();
@@ -373,9 +367,9 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
                     chunk_sync<THREADS, true>();
                     publish_partials<THREADS>(meta, nl, s_f, st.parth, tag);
                 }
-                if (check) {
+                if (check && tid < team) {
                     e = df_add(e, ec);
-                    e2 += noise_square<THREADS>(m, nt, ec.hi);
+                    e2 += noise_square(m, team, nt, ec.hi);
                 }
                 // the slots and node words are free for the next chunk (or pass)
                 if (!RES) chunk_sync<THREADS, true>();
@@ -397,7 +391,14 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
             if (!last) asm volatile("barrier.cta.sync 2, %0;" ::"n"(THREADS + 32) : "memory");
             DFloat R;
             ok = poll_r2(fx.cr + ((pass - 1) & 1) * gridDim.x + cb, G, tag - 1, R, err);
-            if (tid == THREADS) decide_pass(sc, p, sc.k, act, rho, omega, df_double(R));
+            if (tid == THREADS) {
+                decide_pass(sc, p, sc.k, act, rho, omega, df_double(R));
+                // (settle_pass's count of a void pass)
+                if (fx.count_void && !last && !sc.done && sc.force_check && !check && ++sc.passes >= p.pass_cap) {
+                    sc.done = 1;
+                    sc.status = PBS_E_ITER_CAP;
+                }
+            }
             __syncwarp();
         }
         if (check && !last) {
@@ -405,20 +406,12 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
             // CTA's
             __syncthreads();
             if (!worker && !sc.done) {
-                const int w = tid & (WARPS - 1);
-                DFloat se{s_e[w].x, s_e[w].y};
-                float se2 = s_e2[w];
-#pragma unroll
-                for (int o = WARPS / 2; o > 0; o >>= 1) {
-                    se = df_add(se, DFloat{__shfl_down_sync(0xffffffffu, se.hi, o),
-                                           __shfl_down_sync(0xffffffffu, se.lo, o)});
-                    se2 += __shfl_down_sync(0xffffffffu, se2, o);
-                }
-                if (tid == THREADS) {
-                    const double d = df_double(se);
+                double d;
+                float se2;
+                join_warps(s_e, s_e2, team, d, se2);
+                if (tid == THREADS)
                     st_word(fx.ce + b, (unsigned)__double2loint(d), (unsigned)__double2hiint(d),
                             __float_as_uint(se2), tag);
-                }
                 __syncwarp();
                 double E, E2;
                 ok = poll_energy(fx.ce + cb, G, tag, p.energy_slack != 0.f, E, E2, err) && ok;
@@ -466,32 +459,35 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
         ctx.omega = omega;
         ctx.cur = cur;
         ctx.nxt = (size_t)(1 - par) * m.Np;
-        float r2 = 0.f;
-        for (int i = i0; i < n1; i += THREADS) {
-            if (i != i0) {
-                nc.ch = st.ch[i];
-                nc.cl = st.cl[i];
-                nn.uh = st.uh[cur + i];
-                nn.ul = st.ul[cur + i];
-                nn.dd = st.dd[cur + i];
-                nn.diag = st.diag[i];
-                sum = NodeSums{make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f)};
-                ok = collect_partials(st, m.pptr[i], m.pptr[i + 1], do_h, tag, sum, err) && ok;
+        // (by whole warps: a warp's nodes are one group of 32)
+        for (int g = tid & ~31; worker && g < n1 - n0; g += THREADS) {
+            const int i = n0 + g + (tid & 31);
+            float r2 = 0.f;
+            if (i < n1) {
+                if (i != i0) {
+                    nc.ch = st.ch[i];
+                    nc.cl = st.cl[i];
+                    nn.uh = st.uh[cur + i];
+                    nn.ul = st.ul[cur + i];
+                    nn.dd = st.dd[cur + i];
+                    nn.diag = st.diag[i];
+                    sum = NodeSums{make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f)};
+                    ok = collect_partials(st, m.pptr[i], m.pptr[i + 1], do_h, tag, sum, err) && ok;
+                }
+                float4 x[2];
+                r2 = node_update(p, st, i, nc, nn, ctx, [&] { return sum; }, x);
+                st_word(fx.xh + i, make_float3(x[0].x, x[0].y, x[0].z), tag + 1);
+                st_word(fx.xl + i, make_float3(x[1].x, x[1].y, x[1].z), tag + 1);
             }
-            float4 x[2];
-            r2 += node_update(p, st, i, nc, nn, ctx, [&] { return sum; }, x);
-            st_word(fx.xh + i, make_float3(x[0].x, x[0].y, x[0].z), tag + 1);
-            st_word(fx.xl + i, make_float3(x[1].x, x[1].y, x[1].z), tag + 1);
-        }
-        if (worker) {
             r2 = warp_sum_f(r2);
-            if ((tid & 31) == 0) s_g2[tid >> 5] = r2;
+            // (beyond SUM_GROUPS groups the same warp's places again)
+            float *o = s_g2 + (g >> 5) % SUM_GROUPS;
+            if ((tid & 31) == 0) *o = (g >> 5) < SUM_GROUPS ? r2 : *o + r2;
         }
         __syncthreads();
         if (tid == THREADS) {
-            float s = s_g2[0];
-#pragma unroll
-            for (int w = 1; w < WARPS; ++w) s += s_g2[w];
+            float s = 0.f;
+            for (int g = 0; g < min((n1 - n0 + 31) >> 5, SUM_GROUPS); ++g) s += s_g2[g];
             st_pair(fx.cr + (pass & 1) * gridDim.x + b, __float_as_uint(s), tag);
         }
         __syncwarp();

@@ -259,14 +259,12 @@ __global__ void k_from_increment(DevMesh m, DevState st) {
 // grid-dependency wait, so no registers hold them across it.  With two nodes
 // a thread the kernel is held to 85 registers: six 128-thread CTAs fit an SM,
 // and the 1M-tet box's 823 node blocks run as one wave.  |g|^2 is summed in
-// FP32 within the block (256 positive terms: relative error < 1e-6); the
-// pass decision on the block sums (FP64 over the blocks) is taken by the
-// next pass's tet kernel or by k_settle, so the kernel ends with its blocks
-// and no CTA waits for the instance's last one.
+// FP32 within 32 nodes (a warp's); the pass decision on these sums
+// (instance_r2) is taken by the next pass's tet kernel or by k_settle, so the
+// kernel ends with its blocks and no CTA waits for the instance's last one.
 template <int NPT>
 __global__ void __launch_bounds__(BLOCK / NPT, NPT == 2 ? 6 : 0) k_node(DevMesh m, DevParams p, DevState st, int par) {
     constexpr int TH = BLOCK / NPT;
-    __shared__ float sh[TH / 32];
     __shared__ __align__(16) float4 s_c[2][BLOCK];  // c hi (.w = M/h^2), c lo (.w = state) of the block's nodes
     const int b = blockIdx.x;
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -329,17 +327,17 @@ __global__ void __launch_bounds__(BLOCK / NPT, NPT == 2 ? 6 : 0) k_node(DevMesh 
     ctx.omega = omega;
     ctx.cur = cur;
     ctx.nxt = nxt;
-    float r2 = 0.f;
 #pragma unroll
     for (int j = 0; j < NPT; ++j) {
         const int l = threadIdx.x + j * TH;
         NodeConst nc;
         nc.ch = s_c[0][l];
         nc.cl = s_c[1][l];
-        r2 += node_update(p, st, b * BLOCK + l, nc, in[j], ctx, [&] { return node_sums<NPRE>(st, in[j], fp[j], do_h); });
+        float r2 = node_update(p, st, b * BLOCK + l, nc, in[j], ctx, [&] { return node_sums<NPRE>(st, in[j], fp[j], do_h); });
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) r2 += __shfl_down_sync(0xffffffffu, r2, o);
+        if ((l & 31) == 0) st.npartf[(b * BLOCK + l) / 32] = r2;
     }
-    const float sr = block_sum_f(r2, sh);
-    if (threadIdx.x == 0) st.npartf[b] = sr;
 }
 
 // The pending pass decisions after the last pass of a run, one CTA an

@@ -152,10 +152,75 @@ __device__ __forceinline__ InstCtl load_ctl_cg(const InstCtl *p) {
     return c;
 }
 
+// Warp 0: the lane sums of |g|^2 in double-float (lane 0 has the total).
+__device__ __forceinline__ DFloat lane_tree_df(DFloat v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        v = df_add(v, DFloat{__shfl_down_sync(0xffffffffu, v.hi, o), __shfl_down_sync(0xffffffffu, v.lo, o)});
+    return v;
+}
+
+// |g|^2 of an instance from its nodes' groups (st.npartf), in the order that
+// phybs_internal.cuh gives.  Called by every thread; valid in thread 0.
+template <int THREADS>
+__device__ __forceinline__ DFloat instance_r2(const DevState &st, const InstCtl *src) {
+    const int nodes = src->node_end - src->node_begin, C = src->cblk_end - src->cblk_begin;
+    const float *g = st.npartf + src->node_begin / 32;
+    DFloat acc{0.f, 0.f};
+    if (sums_by_share(nodes, C)) {
+        // THREADS shares at a time: a share's groups by a thread, then the
+        // lanes' shares by warp 0
+        __shared__ float s_share[THREADS];
+        const int groups = (nodes + 31) / 32, per = node_share(nodes, C) / 32;
+        for (int j0 = 0; j0 < C; j0 += THREADS) {
+            const int j = j0 + (int)threadIdx.x, a = min(j * per, groups), e = min(a + per, groups);
+            float s = 0.f;
+            if (j < C) {
+                constexpr int U = 8;  // groups in flight
+                for (int q0 = a; q0 < e; q0 += U) {
+                    float v[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) v[u] = q0 + u < e ? __ldcg(g + q0 + u) : 0.f;
+#pragma unroll
+                    for (int u = 0; u < U; ++u) s += v[u];
+                }
+            }
+            s_share[threadIdx.x] = s;
+            __syncthreads();
+            if (threadIdx.x < 32)
+                for (int l = threadIdx.x; l < min(THREADS, C - j0); l += 32) acc = df_add(acc, s_share[l]);
+            __syncthreads();
+        }
+        return threadIdx.x < 32 ? lane_tree_df(acc) : acc;
+    }
+    // a block's eight groups as their lane tree, 256 threads of blocks
+    __shared__ float2 shf[THREADS / 32];
+    constexpr int LANES = THREADS < 256 ? THREADS : 256;
+    const float4 *g4 = reinterpret_cast<const float4 *>(g);
+    const int blocks = src->nblk_end - src->nblk_begin;
+    if (threadIdx.x < LANES) {
+        constexpr int U = 4;
+        for (int j0 = threadIdx.x; j0 < blocks; j0 += U * LANES) {
+            float4 v[U][2];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    v[u][q] = j0 + u * LANES < blocks ? __ldcg(g4 + 2 * (j0 + u * LANES) + q)
+                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (j0 + u * LANES < blocks)
+                    acc = df_add(acc, ((v[u][0].x + v[u][1].x) + (v[u][0].z + v[u][1].z)) +
+                                          ((v[u][0].y + v[u][1].y) + (v[u][0].w + v[u][1].w)));
+        }
+    }
+    return block_sum_df(acc, shf);
+}
+
 // The pass decision of the instance's last node update, taken by one CTA from
-// the control block src into dst: |g|^2 summed in double-float from the node
-// blocks' partials (each thread its blocks in ascending order, then the block
-// tree), then decide_pass with the action, rho and omega that update used.
+// the control block src into dst: |g|^2 (instance_r2), then decide_pass with
+// the action, rho and omega that update used.
 // in_pass: the first chunk CTA of a pass that already runs on the outcome
 // (pass_view); dst is then the copy this pass's line search and node kernel
 // read, its decision pending again, and a forced energy check at a k without
@@ -165,24 +230,11 @@ __device__ __forceinline__ InstCtl load_ctl_cg(const InstCtl *p) {
 template <int THREADS>
 __device__ __forceinline__ void settle_pass(const DevParams &p, const DevState &st, const InstCtl *src,
                                             InstCtl *dst, bool in_pass) {
-    __shared__ float2 shf[THREADS / 32];
     const bool pend = src->pending && !src->done;
-    const int nb0 = src->nblk_begin, nb1 = src->nblk_end;
-    DFloat acc{0.f, 0.f};
-    if (pend) {
-        // eight partials in flight a thread ahead of their additions
-        constexpr int U = 8;
-        for (int j0 = nb0 + (int)threadIdx.x; j0 < nb1; j0 += U * THREADS) {
-            float v[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) v[u] = j0 + u * THREADS < nb1 ? __ldcg(st.npartf + j0 + u * THREADS) : 0.f;
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (j0 + u * THREADS < nb1) acc = df_add(acc, v[u]);
-        }
-    }
-    // (its barriers also order every thread's reads of src before the store)
-    const DFloat R = block_sum_df(acc, shf);
+    DFloat R{0.f, 0.f};
+    if (pend) R = instance_r2<THREADS>(st, src);
+    // (every thread's reads of src come before the store)
+    __syncthreads();
     if (threadIdx.x != 0) return;
     InstCtl ci = *src;
     const bool was_done = ci.done != 0;

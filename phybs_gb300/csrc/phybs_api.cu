@@ -153,6 +153,7 @@ struct pbs_handle {
     cudaEvent_t ev_start = nullptr, ev_end = nullptr, ev_chunk[2] = {nullptr, nullptr};
     cudaGraphExec_t graph = nullptr;
     bool graph_valid = false;
+    bool share_sums = true;   // every instance's |g|^2 is summed by share (sums_by_share)
     bool shape_auto = true;   // no caller set the chunk shape (pbs_set_chunk_shape, pbs_autotune)
     bool engine_auto = true;  // nor the pass engine (pbs_set_pass_engine)
     bool plan_valid = false;  // fplan describes the current layout, material and stress
@@ -261,10 +262,15 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
     }
     std::vector<ChunkLimits> limits(h->B, ChunkLimits{ct, cn});
     const bool automatic = threads == 0;
+    int max_team = 0;
+    for (InstCtl &c : ctl) c.team = threads;
     if (automatic) {
         ct = cn = 0;
         for (int b = 0; b < h->B; ++b) {
-            limits[b] = auto_chunk_limits(ctl[b].tet_end - ctl[b].tet_begin, h->sms);
+            const int nt = ctl[b].tet_end - ctl[b].tet_begin;
+            limits[b] = auto_chunk_limits(nt, h->sms);
+            ctl[b].team = auto_team(nt, h->sms);
+            max_team = std::max(max_team, ctl[b].team);
             ct = std::max(ct, limits[b].tets);
             cn = std::max(cn, limits[b].nodes);
         }
@@ -285,7 +291,11 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
     if (automatic) {
         if (ct == CHUNK_GROUP_TETS) threads = nc > h->sms && h->B == 1 ? 512 : 256;
         else threads = ct > 256 && nc > 2 * h->sms ? 256 : 128;
+        threads = std::max(threads, max_team);
     }
+    bool share_sums = true;
+    for (const InstCtl &c : ctl)
+        share_sums = share_sums && sums_by_share(c.node_end - c.node_begin, c.cblk_end - c.cblk_begin);
     const size_t L = cl.lmeta.size(), T = (size_t)h->T;
     // all of the new layout's memory before the old one's is given up: a
     // handle that runs out of it keeps the layout it had
@@ -327,6 +337,7 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
     h->chunk_slots = cl.max_slots;
     h->chunk_nodes = cn;
     h->chunk_stage = stage;
+    h->share_sums = share_sums;
     if (host_ctl) {
         *host_ctl = ctl;
     } else {
@@ -605,7 +616,7 @@ int pbs_create(const pbs_mesh_desc *d, pbs_handle **out) {
     // slot-ordered hot-loop buffers (3 * 4T) also serve the per-tet probes (12 * Tp)
     CKC(h->tf.alloc(std::max(12 * (size_t)Tp, 16 * (size_t)T))); CKC(h->hd.alloc(std::max(12 * (size_t)Tp, 16 * (size_t)T)));
     CKC(h->staging.alloc(3 * (size_t)N)); CKC(h->staging2.alloc(12 * (size_t)Tp)); CKC(h->staging_ids.alloc(N));
-    CKC(h->tpart.alloc(h->n_tblk)); CKC(h->npart.alloc(h->n_nblk)); CKC(h->npartf.alloc(h->n_nblk));
+    CKC(h->tpart.alloc(h->n_tblk)); CKC(h->npart.alloc(h->n_nblk)); CKC(h->npartf.alloc(8 * (size_t)h->n_nblk));
     CKC(h->ctl.alloc(B)); CKC(h->ctl2.alloc(B)); CKC(h->tcount.alloc(B)); CKC(h->active.alloc(4));
     CKC(cudaMemsetAsync(h->ctl2.p, 0, sizeof(InstCtl) * B, h->stream));
     CKC(cudaMemsetAsync(h->tcount.p, 0, sizeof(unsigned int) * B, h->stream));
@@ -837,7 +848,7 @@ static bool frame_applies(pbs_handle *h) { return h->B == 1 && handle_frame_plan
 // Enqueues one frame-kernel launch of at most max_passes passes with params p;
 // frame_done must follow once the launch has ended.  PBS_E_INVALID_ARG when
 // the frame kernel does not apply to the handle's layout.
-static int launch_frame_step(pbs_handle *h, const DevParams &p, int max_passes) {
+static int launch_frame_step(pbs_handle *h, const DevParams &p, int max_passes, bool count_void) {
     const FramePlan &plan = handle_frame_plan(h);
     if (plan.grid <= 0) return PBS_E_INVALID_ARG;
     cudaStream_t s = h->stream;
@@ -871,6 +882,7 @@ static int launch_frame_step(pbs_handle *h, const DevParams &p, int max_passes) 
     fx.cr = h->fcr.p;
     fx.tag0 = h->frame_tag;
     fx.max_passes = max_passes;
+    fx.count_void = count_void;
     h->frame_clean = false;
     CK(launch_frame(s, frame_mesh(h), p, h->state(), h->material, fx, plan));
     return PBS_OK;
@@ -896,7 +908,8 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     // the caller chose neither an engine nor a shape: the frame kernel where
     // every chunk has a resident CTA of its own (auto_chunk_limits), which
     // spares a pass its two launches and its trips to memory
-    const bool auto_frame = !frame && h->engine_auto && h->shape_auto && handle_frame_plan(h).resident;
+    const bool auto_frame =
+        !frame && h->engine_auto && h->shape_auto && h->share_sums && handle_frame_plan(h).resident;
     frame |= auto_frame;
     int rc = frame ? PBS_OK : ensure_graph(h);
     if (rc != PBS_OK) return rc;
@@ -933,7 +946,7 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     const int max_chunks = frame || h->graph_loop ? 0 : max_runs(h);
     int launched = 0;
     if (frame) {
-        rc = launch_frame_step(h, h->dparams, h->dparams.pass_cap);
+        rc = launch_frame_step(h, h->dparams, h->dparams.pass_cap, auto_frame);
         if (rc != PBS_OK) return rc;
         CK(cudaMemcpyAsync(h->h_active + 1, h->active.p + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
     } else if (h->graph_loop) {
@@ -1211,7 +1224,7 @@ static int time_frame(pbs_handle *h, int passes, double *pass_ms) {
     if (e == cudaSuccess) e = launch_to_increment(s, m, p, st);
     if (e == cudaSuccess) e = cudaEventRecord(ev[0], s);
     int rc = PBS_OK;
-    if (e == cudaSuccess) rc = launch_frame_step(h, p, passes);
+    if (e == cudaSuccess) rc = launch_frame_step(h, p, passes, false);
     if (e == cudaSuccess && rc == PBS_OK) e = cudaEventRecord(ev[1], s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     float ms = 0.f;

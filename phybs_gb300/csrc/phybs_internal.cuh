@@ -47,7 +47,7 @@
 //   cpart       double2[n_chunks]  per chunk {sum e, sum e^2}
 //   rslot       double[3][4T]      per-step FP64 corner forces at the base, by gather slot
 //   npart       double[n_nblk]     per node-block |g|^2 (warm-start reference)
-//   npartf      float[n_nblk]      per node-block |g|^2 of a pass (FP32 block sums)
+//   npartf      float[8*n_nblk]    |g|^2 of a pass per 32 nodes (FP32 sums)
 //   ctl         InstCtl[n_inst]    per-instance descent state
 #pragma once
 #include <cuda_runtime.h>
@@ -129,8 +129,36 @@ struct __align__(16) InstCtl {
     // non-finite forces an energy check the pass's tet kernel did not make)
     int pending, void_pass;
     double g1;                             // |g| at the learned candidate (extrapolation base)
-    double pad6;
+    int team;  // threads whose sums make up a chunk's energy (chunk_energy)
+    int pad6;
 };
+
+// How an instance's line-search energy and |g|^2 are summed does not depend on
+// the kernel that sums them, its threads or the instance's company: an instance
+// takes one path alone (the frame kernel), packed (the pass kernels) and at
+// any CTA size.  With T = team threads, C chunks and 32-node groups:
+//   energy   of a chunk: thread t adds the terms of the nodes t, t + T, ... of the
+//            chunk's share, then those of its tets t, t + T, ...; a lane tree,
+//            then the warps' sums in a lane tree;
+//            of the instance: FP64, 32 lanes, each its chunks in ascending
+//            order, then the lane tree;
+//   |g|^2    of a group: a lane tree; of a share: its groups in ascending order;
+//            of the instance: 32 lanes of double-float, each its shares in
+//            ascending order, then the lane tree.
+// Beyond SUM_CHUNKS chunks, where the serial chains would be long and no frame
+// kernel is resident, 256 threads take the place of the 32 lanes, and |g|^2 is
+// summed by 256-node blocks instead of shares.
+constexpr int SUM_CHUNKS = 512, SUM_GROUPS = 256;  // (groups of a share that the frame kernel keeps)
+
+// Nodes of a chunk's share: the instance's, in whole groups of 32, evenly over
+// its chunks.
+__host__ __device__ inline int node_share(int nodes, int chunks) {
+    const int groups = (nodes + 31) / 32;
+    return chunks > 0 ? (groups + chunks - 1) / chunks * 32 : 0;
+}
+__host__ __device__ inline bool sums_by_share(int nodes, int chunks) {
+    return chunks <= SUM_CHUNKS && node_share(nodes, chunks) <= 32 * SUM_GROUPS;
+}
 
 // |g| / |g0| of an instance's last pass (-1 before the first pass).
 inline double residual_ratio(const InstCtl &c) {
@@ -264,6 +292,9 @@ struct ChunkLimits {
 // The chunk limits of an instance whose shape no caller set, from its own tet
 // count only: a packed batch then chunks an instance as it is chunked alone.
 ChunkLimits auto_chunk_limits(int tets, int sms);
+// The team of such an instance: the threads of the frame kernel's CTA where it
+// has one to a chunk, else 256.
+int auto_team(int tets, int sms);
 // limits: per instance.  grouped: the chunks are even pieces of groups of at
 // most CHUNK_GROUP_TETS tets and CHUNK_GROUP_NODES nodes, and every chunk of a
 // group holds the group's lowest node (without corners, where it has none of
@@ -289,11 +320,14 @@ int stream_grid(const DevMesh &m, int material, bool inc, int sms);
 // (FP64), sum e^2} of a check pass; cr: per-CTA |g|^2, two buffers of grid
 // pairs; the partials part / parth carry tags in .w.  A launch uses the tags
 // tag0 + 1 .. tag0 + 1 + passes; no word may hold one of them before it.
+// count_void: a pass redone for a forced energy check counts as a pass, as it
+// does in the pass kernels (DescentSolver's default, whichever kernel runs).
 struct FrameAux {
     float4 *xh, *xl, *ce;
     uint2 *cr;
     unsigned tag0;
     int max_passes;
+    int count_void;
 };
 // How the frame kernel runs a mesh: grid CTAs (0: it does not apply), each
 // with a chunk of its own (resident) or walking several (one instance only).

@@ -76,6 +76,70 @@ def test_default_engine_packed(n):
     b.close()
 
 
+def _pack(meshes):
+    """Meshes as one packed handle's, in place (instances do not meet)."""
+    nptr = np.cumsum([0] + [m.n_nodes for m in meshes]).astype(np.int32)
+    tptr = np.cumsum([0] + [m.n_tets for m in meshes]).astype(np.int32)
+    cat = lambda f: np.concatenate([f(m, int(o)) for m, o in zip(meshes, nptr)])
+    return M.TetMeshData(cat(lambda m, o: m.rest), cat(lambda m, o: m.tets + o), cat(lambda m, o: m.pins + o),
+                         cat(lambda m, o: np.broadcast_to(np.float32(m.young), m.n_tets)),
+                         cat(lambda m, o: np.broadcast_to(np.float32(m.poisson), m.n_tets)),
+                         instance_node_ptr=nptr, instance_tet_ptr=tptr, name="packed")
+
+
+# bodies whose automatic chunks are of 128, 256 and 342 tets, whole groups
+# (104,780; 260,100) and pieces of 342 beyond residence (161,700); what is said
+# of a company is the pass kernels' CTA.  Copies keep a company from being resident
+SMALL = [(2, 1, 13), (3, 5, 9), (8, 8, 12), (9, 8, 13), (12, 12, 20), (14, 13, 27)]
+COMPANIES = {
+    "resident": (SMALL, 1),
+    "128 threads": (SMALL + [(24, 24, 27)], 12),
+    "256 threads, pieces": (SMALL + [(24, 24, 28)], 8),
+    "256 threads, groups": (SMALL + [(28, 25, 34), (26, 26, 31)], 3),
+    "few groups": ([(26, 26, 31), (3, 5, 9)], 2),
+    "largest": ([(34, 30, 51), (8, 8, 12), (33, 28, 35)], 1),
+}
+
+
+@pytest.mark.parametrize("company", COMPANIES)
+@pytest.mark.parametrize("control", ["stop", "budget"])
+@pytest.mark.parametrize("material,inc", [(0, 1), (0, 0), (1, 0)], ids=["incremental", "full", "stretch"])
+def test_packed_instance_equals_the_body_alone(company, control, material, inc):
+    """A body takes the same steps alone (the frame kernel, where its chunks are
+    resident) and in any company (the pass kernels, at the company's CTA size):
+    decisions, sums and positions bit for bit, with a stop on the residual and
+    with the reference's line search at an iteration budget."""
+    dims, copies = COMPANIES[company]
+    meshes = [_box(*d) for d in dims]
+    if control == "stop":
+        p = make_params("gpu_reference", h=1 / 30, tol=3e-2, max_iters=2000, control=L.PBS_CONTROL_RESTART,
+                        energy_slack=16.0, alpha0=0.45, alpha_grow=1.2, incremental_stress=inc,
+                        profile=((5, 0.99), (25, 0.999), (100, 0.9999)))
+    else:
+        p = make_params("gpu_reference", h=1 / 30, max_iters=72, alpha0=0.6, profile=((10, 0.9999),),
+                        incremental_stress=inc)
+    packed = _pack(meshes * copies)
+    s = DescentSolver(packed, params=p, material=material)
+    keys = KEYS[:8] + ("energy", "residual_ratio")
+    got = []
+    for f in range(2):
+        s.step(raise_on_error=False)
+        x = s.positions()
+        got.append([(s.instance_stats(i), x[packed.instance_node_ptr[i]:packed.instance_node_ptr[i + 1]])
+                    for i in range(packed.n_instances)])
+    s.close()
+    for j, m in enumerate(meshes):
+        a = DescentSolver(m, params=p, material=material)
+        for f in range(2):
+            a.step(raise_on_error=False)
+            st, x = a.stats(), a.positions()
+            for i in range(j, packed.n_instances, len(meshes)):
+                sp, xp = got[f][i]
+                assert repr([sp[k] for k in keys]) == repr([st[k] for k in keys]), (dims[j], f, i)
+                assert np.array_equal(x, xp, equal_nan=True), (dims[j], f, i)
+        a.close()
+
+
 @pytest.mark.parametrize("engine", [None, "graph"])
 @pytest.mark.parametrize("at", [0, 1, 2], ids=["first", "middle", "last"])
 @pytest.mark.parametrize("inc", [0, 1], ids=["full", "incremental"])
