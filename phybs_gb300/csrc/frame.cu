@@ -207,10 +207,17 @@ __device__ __forceinline__ bool collect_partials(const DevState &st, int pa, int
     return ok;
 }
 
-// What the workers need of a pass's decisions.
+// What the workers need of a pass's decisions, and the next pass's decision of
+// this one's update.
 struct FrameView {
-    int done, force_check, action;
-    float alpha, rho, omega;  // rho, omega: the pass's own (chebyshev_schedule)
+    int done, force_check, action;  // action: what the node update does
+    float alpha, rho, omega;        // rho, omega: the pass's own (chebyshev_schedule)
+};
+
+// What a CTA owns of its instance; in shared memory, so that no register holds
+// it through the tets.
+struct FrameOwn {
+    int n0, n1, team;  // its share of the nodes, the instance's team (at most THREADS)
 };
 
 // THREADS workers and one control warp a CTA.  A pass:
@@ -249,6 +256,7 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
     int4 *s_meta = reinterpret_cast<int4 *>(s_cor + CT);
     __shared__ InstCtl sc;  // this CTA's copy of the instance's control block (the control warp's)
     __shared__ FrameView sv;
+    __shared__ FrameOwn own;
     __shared__ float2 s_e[WARPS];
     __shared__ float s_e2[WARPS], s_g2[SUM_GROUPS];
     const int b = blockIdx.x, tid = threadIdx.x;
@@ -278,20 +286,25 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
     const int bi = b - cb;
     int *err = st.active + 1;
     // this CTA's nodes [n0, n1), this thread's i0, i0 + THREADS, ...
-    const int per = node_share(sc.node_end - sc.node_begin, G);
-    const int team = sc.team;
-    const int n0 = min(sc.node_begin + bi * per, sc.node_end), n1 = min(n0 + per, sc.node_end);
-    const int i0 = worker ? n0 + tid : n1;
+    if (tid == 0) {
+        const int per = node_share(sc.node_end - sc.node_begin, G);
+        own.n0 = min(sc.node_begin + bi * per, sc.node_end);
+        own.n1 = min(own.n0 + per, sc.node_end);
+        own.team = sc.team;
+    }
+    __syncthreads();
+    // this thread's first node: mine() whether it has one
+    auto mine = [&] { return worker && own.n0 + tid < own.n1; };
     int pa0 = 0, pe0 = 0;
-    if (i0 < n1) {
-        pa0 = m.pptr[i0];
-        pe0 = m.pptr[i0 + 1];
+    if (mine()) {
+        pa0 = m.pptr[own.n0 + tid];
+        pe0 = m.pptr[own.n0 + tid + 1];
     }
     int k = sc.k, par = sc.par;
     bool force = sc.force_check != 0;
     {
         const size_t cur = (size_t)par * m.Np;
-        for (int i = i0; i < n1; i += THREADS) {
+        for (int i = own.n0 + tid; worker && i < own.n1; i += THREADS) {
             const float4 h = st.uh[cur + i], l = st.ul[cur + i];
             st_word(fx.xh + i, make_float3(h.x, h.y, h.z), fx.tag0 + 1);
             st_word(fx.xl + i, make_float3(l.x, l.y, l.z), fx.tag0 + 1);
@@ -300,8 +313,6 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
     __syncthreads();    // sc is the control warp's from here
     bool ok = true;     // no wait of this thread gave up
     bool pend = false;  // the pass decision of the last node update is not taken yet
-    int act = ACT_STEP;
-    float rho = 0.f, omega = 1.f;
     for (int pass = 0;;) {
         const unsigned tag = fx.tag0 + 1 + (unsigned)pass;
         // the pass runs on the foreseen outcome of the pending decision
@@ -317,7 +328,8 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
             DFloat e{0.f, 0.f};
             float e2 = 0.f;
             // the words of this thread's first node, only ever written by itself
-            if (i0 < n1) {
+            if (mine()) {
+                const int i0 = own.n0 + tid;
                 nn.uh = st.uh[cur + i0];
                 nn.ul = st.ul[cur + i0];
                 nn.dd = st.dd[cur + i0];
@@ -325,7 +337,8 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
             }
             // the CTA's share of the node energy terms, before the other CTAs'
             // words arrive
-            if (check && tid < team) share_energy(m, p, st, cur, i0, n1, team, INC ? st.ub : nullptr, e, e2);
+            if (check && tid < own.team)
+                share_energy(m, p, st, cur, own.n0 + tid, own.n1, own.team, INC ? st.ub : nullptr, e, e2);
             // ---- tet phase: this CTA's chunk, or the chunks b, b + G, ...
             for (int c = b; c < m.n_chunks; c += RES ? m.n_chunks : G) {
                 const int4 cd = m.chunk[c];
@@ -359,7 +372,7 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
                 v.meta = meta;
                 v.rest = m.rest;
                 DFloat ec = chunk_forces_all<MATERIAL, THREADS, INC, true, false, true>(p, v, nt, check, s_f);
-                if (check && team != THREADS) ec = team_energy(v, nt, team, s_f);
+                if (THREADS > 128 && check && own.team != THREADS) ec = team_energy(v, nt, own.team, s_f);
                 publish_partials<THREADS>(meta, nl, s_f, st.part, tag);
                 if (do_h) {
                     chunk_sync<THREADS, true>();
@@ -367,9 +380,9 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
                     chunk_sync<THREADS, true>();
                     publish_partials<THREADS>(meta, nl, s_f, st.parth, tag);
                 }
-                if (check && tid < team) {
+                if (check && tid < own.team) {
                     e = df_add(e, ec);
-                    e2 += noise_square(m, team, nt, ec.hi);
+                    e2 += noise_square(m, own.team, nt, ec.hi);
                 }
                 // the slots and node words are free for the next chunk (or pass)
                 if (!RES) chunk_sync<THREADS, true>();
@@ -392,7 +405,7 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
             DFloat R;
             ok = poll_r2(fx.cr + ((pass - 1) & 1) * gridDim.x + cb, G, tag - 1, R, err);
             if (tid == THREADS) {
-                decide_pass(sc, p, sc.k, act, rho, omega, df_double(R));
+                decide_pass(sc, p, sc.k, sv.action, sv.rho, sv.omega, df_double(R));
                 // (settle_pass's count of a void pass)
                 if (fx.count_void && !last && !sc.done && sc.force_check && !check && ++sc.passes >= p.pass_cap) {
                     sc.done = 1;
@@ -408,7 +421,7 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
             if (!worker && !sc.done) {
                 double d;
                 float se2;
-                join_warps(s_e, s_e2, team, d, se2);
+                join_warps(s_e, s_e2, own.team, d, se2);
                 if (tid == THREADS)
                     st_word(fx.ce + b, (unsigned)__double2loint(d), (unsigned)__double2hiint(d),
                             __float_as_uint(se2), tag);
@@ -422,20 +435,20 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
             if (tid == THREADS) {
                 sv.done = sc.done;
                 sv.force_check = sc.force_check;
-                sv.action = sc.action;
+                sv.action = check ? sc.action : ACT_STEP;
                 sv.alpha = sc.alpha;
                 float r = sc.rho, o = sc.omega;
                 chebyshev_schedule(p, k - sc.k_restart, r, o);
                 sv.rho = r;
                 sv.omega = o;
             }
-        } else if (!last && i0 < n1) {
+        } else if (!last && mine()) {
             // the partials of this thread's first node.  Every partial is
             // waited for whether or not the update needs it (pinned nodes, a
             // restore): the chunks have then read the state word that the
             // update overwrites
-            nc.ch = st.ch[i0];
-            nc.cl = st.cl[i0];
+            nc.ch = st.ch[own.n0 + tid];
+            nc.cl = st.cl[own.n0 + tid];
             ok = collect_partials(st, pa0, pe0, do_h, tag, sum, err) && ok;
         }
         ok = !__syncthreads_or(!ok);
@@ -449,22 +462,19 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
         }
         // ---- node phase
         force = false;
-        act = check ? sv.action : ACT_STEP;
-        rho = sv.rho;
-        omega = sv.omega;
         PassCtx ctx;
-        ctx.action = act;
+        ctx.action = sv.action;
         ctx.do_h = do_h;
         ctx.alpha = sv.alpha;
-        ctx.omega = omega;
+        ctx.omega = sv.omega;
         ctx.cur = cur;
         ctx.nxt = (size_t)(1 - par) * m.Np;
         // (by whole warps: a warp's nodes are one group of 32)
-        for (int g = tid & ~31; worker && g < n1 - n0; g += THREADS) {
-            const int i = n0 + g + (tid & 31);
+        for (int g = tid & ~31; worker && g < own.n1 - own.n0; g += THREADS) {
+            const int i = own.n0 + g + (tid & 31);
             float r2 = 0.f;
-            if (i < n1) {
-                if (i != i0) {
+            if (i < own.n1) {
+                if (g >= THREADS) {
                     nc.ch = st.ch[i];
                     nc.cl = st.cl[i];
                     nn.uh = st.uh[cur + i];
@@ -487,12 +497,19 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
         __syncthreads();
         if (tid == THREADS) {
             float s = 0.f;
-            for (int g = 0; g < min((n1 - n0 + 31) >> 5, SUM_GROUPS); ++g) s += s_g2[g];
+            const int groups = min((own.n1 - own.n0 + 31) >> 5, SUM_GROUPS);
+            for (int g = 0; g < groups; g += WARPS) {
+                float v[WARPS];
+#pragma unroll
+                for (int w = 0; w < WARPS; ++w) v[w] = g + w < groups ? s_g2[g + w] : 0.f;
+#pragma unroll
+                for (int w = 0; w < WARPS; ++w) s += v[w];
+            }
             st_pair(fx.cr + (pass & 1) * gridDim.x + b, __float_as_uint(s), tag);
         }
         __syncwarp();
         pend = true;
-        if (act != ACT_RESTORE) ++k;
+        if (sv.action != ACT_RESTORE) ++k;
         par ^= 1;
         ++pass;
     }
