@@ -55,8 +55,8 @@ extern "C" {
  * evaluated through the invariants (IsotropicNeohookeanMaterial.cpp:104)
  * or through the principal stretches of the modified SVD
  * (IsotropicMaterial.cpp:360-409, Xu et al. 2015).  The descent's passes take
- * the stretch material's stress from the invariants too, which is the same
- * stress, where the invariants show the tet to be away from inversion. */
+ * the stretch material's stress from the strain F^T F - I, without an SVD,
+ * where the invariants show the tet to be away from inversion. */
 #define PBS_MATERIAL_NEOHOOKEAN 0
 #define PBS_MATERIAL_STRETCH 1
 

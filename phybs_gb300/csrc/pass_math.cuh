@@ -220,12 +220,14 @@ __device__ __forceinline__ bool pass_forces_c(const float4 &x0, const float4 &x1
                              f4add(f4sub(x3, x0), f4sub(l3, l0)), dinv, kin.G);
         kinematics(kin);
         // near inversion (det F < 1e-3): the FP64 stress from the absolute
-        // positions.  The stretch-based material is the same energy, so an
-        // uninverted tet takes its stress from the invariants too, without an
-        // SVD, unless its smallest singular value may be below 0.3
-        // (stretch_needs_svd)
+        // positions.  The stretch-based stress comes from the strain's
+        // invariants, without an SVD, unless the smallest singular value may be
+        // below 0.3 (stretch_needs_svd)
         exact = 1.0f + kin.d < 1e-3f || (MATERIAL == PBS_MATERIAL_STRETCH && stretch_needs_svd(kin));
-        if (!exact) pk1_neohookean<float>(kin, mu, lambda, P);
+        if (!exact) {
+            if (MATERIAL == PBS_MATERIAL_STRETCH) stretch_pk1_strain(kin.G, mu, lambda, P);
+            else pk1_neohookean<float>(kin, mu, lambda, P);
+        }
         if (MATERIAL == PBS_MATERIAL_STRETCH && !DEFER && exact && 1.0f + kin.d >= 1e-3f)
             exact = !stretch_pk1<float>(kin.G, mu, lambda, P);
         if (exact && !DEFER)

@@ -386,16 +386,56 @@ template <typename T> __device__ __forceinline__ bool stretch_pk1(const T G[9], 
 // (sigma_1^2 + sigma_2^2) / 2 <= |F|^2 / 2, hence sigma_3 = det F / (sigma_1
 // sigma_2) >= 2 det F / |F|^2, and 0.31 leaves 3% for rounding.  At rest the
 // bound is 0.67; a tet stretched by 2 along one axis at constant volume has 0.4.
-// P = mu (F - F^-T) + lambda ln J F^-T is U diag(P^) V^T exactly, and its
-// cancellation-free form (pk1_neohookean) carries less rounding than the
-// rotations; four Jacobi sweeps and the QR of every tet were 80% of a
-// stretch-material pass.
+// (four Jacobi sweeps and the QR of every tet were 80% of a stretch-material
+// pass.)
 __device__ __forceinline__ bool stretch_needs_svd(const Kin<float> &k) {
     float g2 = 0.f;
 #pragma unroll
     for (int i = 0; i < 9; ++i) g2 += k.G[i] * k.G[i];
     // |F|^2 = 3 + 2 tr G + |G|^2; a NaN needs the SVD
     return !(2.f * (1.f + k.d) >= 0.31f * (3.f + 2.f * k.tr + g2));
+}
+
+// The stretch-based stress of such a tet without singular values.  U diag(P^)
+// V^T = mu (F - F^-T) + lambda ln J F^-T = F S with the symmetric
+//   S = mu (I - C^-1) + lambda ln J C^-1,  C = F^T F = I + E,
+//   J^2 (I - C^-1) = E + (c2 + c3) I - cof E,   J^2 C^-1 = (1 + tr E) I - E + cof E,
+//   J^2 = 1 + q,  q = tr E + c2 + c3,  ln J = log1p(q) / 2   (c2, c3: E's invariants),
+// from E = G + G^T + G^T G, the matrix whose eigenvalues the SVD takes.  A
+// rotation leaves E small, where in the form with F^-T (pk1_neohookean) terms
+// of order 1 cancel: on the tets of an ellipsoid twisted by 63 degrees and
+// turned about a random axis that one was off by 3.1e-6 to 5.8e-6 mu (the SVD
+// 0.5e-6 to 1.7e-6, this 0.4e-6 to 0.8e-6), and by up to 3.6e-7 mu in the
+// antisymmetric part of P F^T (the SVD 2e-8, this 1.5e-8).
+__device__ __forceinline__ void stretch_pk1_strain(const float G[9], float mu, float lambda, float P[9]) {
+    // (every rounding spelled out: the same bits in every kernel)
+    auto dot3 = [](float c, float a0, float b0, float a1, float b1, float a2, float b2) {
+        return __fmaf_rn(a2, b2, __fmaf_rn(a1, b1, __fmaf_rn(a0, b0, c)));
+    };
+    auto minor = [](float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); };
+    auto sum3 = [](float a, float b, float c) { return __fadd_rn(__fadd_rn(a, b), c); };
+    const float e00 = dot3(2.f * G[0], G[0], G[0], G[3], G[3], G[6], G[6]);
+    const float e11 = dot3(2.f * G[4], G[4], G[4], G[1], G[1], G[7], G[7]);
+    const float e22 = dot3(2.f * G[8], G[8], G[8], G[2], G[2], G[5], G[5]);
+    const float e01 = dot3(__fadd_rn(G[1], G[3]), G[0], G[1], G[3], G[4], G[6], G[7]);
+    const float e02 = dot3(__fadd_rn(G[2], G[6]), G[0], G[2], G[3], G[5], G[6], G[8]);
+    const float e12 = dot3(__fadd_rn(G[5], G[7]), G[1], G[2], G[4], G[5], G[7], G[8]);
+    const float k00 = minor(e11, e22, e12, e12), k11 = minor(e00, e22, e02, e02), k22 = minor(e00, e11, e01, e01);
+    const float k01 = minor(e12, e02, e01, e22), k02 = minor(e01, e12, e11, e02), k12 = minor(e02, e01, e00, e12);
+    const float tr = sum3(e00, e11, e22);
+    const float c23 = dot3(sum3(k00, k11, k22), e00, k00, e01, k01, e02, k02);
+    const float q = __fadd_rn(tr, c23), r = __fdiv_rn(1.f, __fadd_rn(1.f, q));
+    const float lg = __fmul_rn(lambda, 0.5f * log1pf(q));
+    const float d = __fmaf_rn(mu, c23, __fmaf_rn(lg, tr, lg)), m = __fsub_rn(mu, lg);
+    auto entry = [&](float c, float e, float k) { return __fmul_rn(__fmaf_rn(m, __fsub_rn(e, k), c), r); };
+    const float s00 = entry(d, e00, k00), s11 = entry(d, e11, k11), s22 = entry(d, e22, k22);
+    const float s01 = entry(0.f, e01, k01), s02 = entry(0.f, e02, k02), s12 = entry(0.f, e12, k12);
+    const float S[9] = {s00, s01, s02, s01, s11, s12, s02, s12, s22};
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            P[3 * i + j] = dot3(S[3 * i + j], G[3 * i], S[j], G[3 * i + 1], S[3 + j], G[3 * i + 2], S[6 + j]);
 }
 
 // Where a tet's four rest positions are: rest[meta[id[c]].x] (chunk-local

@@ -216,6 +216,45 @@ def test_stretch_stress_without_svd(s):
     a.close()
 
 
+def test_stretch_stress_under_rotation():
+    """One iteration of the stretch material (lambda = 100 mu) from 48 bodies
+    turned about random axes and strained by up to 1.4% at constant volume,
+    against the FP64 restatement; the velocities' error in units of the ln J
+    that makes it (from a second restatement, of the body scaled by 1.001).
+    Grid, deformation and G are exact in FP32.  What rounds at the size of the
+    rotation are the nine terms of tr E, 2^-25 / sqrt(3) each and half of it in
+    ln J: 2.6e-8 together, and the bound on the root mean square over the bodies
+    is twice that.  A det F - 1 summed from G's invariants is off by 1.3e-7."""
+    from scipy.spatial.transform import Rotation
+    cube = M.box_mesh(4, 4, 5, edge=0.0625, jitter=0.0, seed=3, young=1e7, poisson=0.49, pin="bottom")
+    x = []
+    for k in range(48):
+        s = 1 + (k % 7 + 1) / 512
+        F = np.round(2**14 * Rotation.random(random_state=k).as_matrix() @ np.diag([s, 1 / s, 1])) / 2**14
+        x.append((cube.rest.astype(np.float64) @ F.T).astype(np.float32))
+        assert np.array_equal(x[-1], cube.rest.astype(np.float64) @ F.T)
+    p = make_params("gpu_reference", h=1 / 30, max_iters=1, alpha0=0.05)
+    a = DescentSolver(_pack([cube] * 48), positions=np.concatenate(x), material=L.PBS_MATERIAL_STRETCH, params=p)
+    a.step()
+    v = a.velocities()[0].reshape(48, -1, 3)
+    a.close()
+    pm = cube.pin_mask()
+    r64 = O.rest(cube.rest, cube.tets, pm, prec=64)
+
+    def exact(x0):
+        st = O.StepState(x0)
+        O.step(st, O.make_params(h=1 / 30, max_iters=1, alpha0=0.05, body_force_scale=1.0, energy_clamp=1, material=1,
+                                 hessian_closed=1), cube.tets, r64, *O.lame(cube.young, cube.poisson), pm, prec=64)
+        return st.v[pm == 0]
+
+    err = []
+    for k in range(48):
+        e = exact(x[k])
+        per_ln_j = np.abs(exact(np.float32(1.001) * x[k]) - e).max() / 3e-3
+        err.append(np.abs(v[k][pm == 0] - e).max() / per_ln_j)
+    assert np.sqrt(np.square(err).mean()) <= 2 * 2.6e-8, np.sqrt(np.square(err).mean())
+
+
 PULLS = [(3, 3, 5), (8, 7, 12), (12, 9, 13), (20, 17, 31), (22, 21, 40), (25, 25, 40), (31, 23, 46), (34, 33, 46)]
 
 
