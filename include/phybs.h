@@ -350,6 +350,11 @@ int pbs_set_pass_engine(pbs_handle *h, int engine);
  * do not depend on it.  No counterpart in the reference. */
 int pbs_set_l2_residency(pbs_handle *h, int enable);
 int pbs_get_pass_engine(pbs_handle *h, int *engine);
+/* The engine that ran the passes of the last pbs_step: the set one, or for a
+ * handle that set neither an engine nor a chunk shape the one it took by
+ * itself.  PBS_ENGINE_GRAPH before the first step.  No counterpart in the
+ * reference. */
+int pbs_get_step_engine(pbs_handle *h, int *engine);
 /* pbs_profile_kernels for the frame engine: one frame launch of `passes`
  * passes from the current state (left as it was), timed with CUDA events;
  * returns the mean milliseconds per pass.  Fails as pbs_profile_kernels does,

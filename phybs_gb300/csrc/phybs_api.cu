@@ -161,6 +161,7 @@ struct pbs_handle {
     bool graph_loop = false;  // graph is the WHILE node over the pass body (else the body alone)
     // persistent frame kernel: its exchanged words
     int engine = PBS_ENGINE_GRAPH;
+    int step_engine = PBS_ENGINE_GRAPH;  // what ran the last pbs_step's passes
     DevBuf<float4> fxh, fxl, fce;
     DevBuf<uint2> fcr;
     unsigned frame_tag = 0;     // the last tag any word may hold
@@ -997,6 +998,7 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     // the default engine counts in bodies whichever kernel ran its passes
     S.graph_launches = auto_frame ? std::max(1, (S.passes + CHUNK_PASSES - 1) / CHUNK_PASSES) : launched;
     h->stats = S;
+    h->step_engine = frame ? PBS_ENGINE_FRAME : PBS_ENGINE_GRAPH;
     if (frame) frame_done(h, S.passes, gave_up);
     if (iters_out) *iters_out = S.iterations;
     return S.status;
@@ -1263,6 +1265,12 @@ int pbs_set_pass_engine(pbs_handle *h, int engine) {
 int pbs_get_pass_engine(pbs_handle *h, int *engine) {
     if (!h || !engine) return PBS_E_INVALID_ARG;
     *engine = h->engine;
+    return PBS_OK;
+}
+
+int pbs_get_step_engine(pbs_handle *h, int *engine) {
+    if (!h || !engine) return PBS_E_INVALID_ARG;
+    *engine = h->step_engine;
     return PBS_OK;
 }
 

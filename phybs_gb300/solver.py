@@ -172,6 +172,12 @@ class DescentSolver:
         L.check(L.lib().pbs_get_pass_engine(self._h, C.byref(e)), "pbs_get_pass_engine")
         return "frame" if e.value == L.PBS_ENGINE_FRAME else "graph"
 
+    def step_engine(self) -> str:
+        """The engine that ran the last step's passes (pass_engine is the set one)."""
+        e = C.c_int()
+        L.check(L.lib().pbs_get_step_engine(self._h, C.byref(e)), "pbs_get_step_engine")
+        return "frame" if e.value == L.PBS_ENGINE_FRAME else "graph"
+
     def autotune(self, passes: int = 32) -> dict:
         """Pick the pass kernels' chunk shape by timing candidates on this mesh."""
         r = L.TuneResult()

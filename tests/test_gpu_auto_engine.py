@@ -57,6 +57,20 @@ def test_default_engine_equals_pass_kernels(dims, material, inc):
     b.close()
 
 
+def test_step_engine_is_the_one_that_ran():
+    """What ran the passes, where the set engine (pass_engine) and the count of
+    graph bodies do not tell."""
+    for dims, want in (((8, 8, 24), "frame"), ((34, 34, 54), "graph")):
+        s = DescentSolver(_box(*dims), params=make_params("gpu_reference", h=1 / 30, max_iters=8))
+        assert s.step_engine() == s.pass_engine() == "graph"
+        s.step()
+        assert (s.step_engine(), s.pass_engine()) == (want, "graph") and s.stats()["graph_launches"] > 0
+        s.set_pass_engine("graph")
+        s.step()
+        assert s.step_engine() == "graph"
+        s.close()
+
+
 @pytest.mark.parametrize("n", [2, 5, 24])
 def test_default_engine_packed(n):
     """Packed uneven boxes: resident (2, 5) and beyond (24); the iteration
