@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstdint>
@@ -50,6 +51,34 @@ template <typename T> struct DevBuf {
 };
 
 int round_up(int x, int a) { return (x + a - 1) / a * a; }
+
+// Default steps now running on a device whose frame kernel takes more than half
+// of its SMs, over all handles and threads of the process.  Such kernels run
+// one after the other, while the pass kernels of several handles overlap.  From
+// the third on a step therefore runs the pass kernels, which give the same
+// bits.  Steps of 1 / 2 / 4 / 8 threads, one handle each, us a step of all:
+//   24,000 tets    frame 536 / 464 / 466 / 464   pass kernels 1097 / 623 / 340 / 248
+//   60,000         653 / 574 / 574 / 572         1207 / 722 / 391 / 290
+//   125,000        889 / 800 / 798 / 804         1406 / 861 / 506 / 458
+// Smaller ones share the device as frame kernels too (16,000 tets 518 / 275 /
+// 231 / 232, pass kernels 1087 / 590 / 325 / 228; 8,000 at eight threads 121 and
+// 204).
+std::atomic<int> large_steps[64];
+
+class LargeStep {
+  public:
+    // Counts this step in; the others that run.
+    int enter(int device) {
+        count_ = &large_steps[device & 63];
+        return count_->fetch_add(1);
+    }
+    ~LargeStep() {
+        if (count_) count_->fetch_sub(1);
+    }
+
+  private:
+    std::atomic<int> *count_ = nullptr;
+};
 
 }  // namespace
 
@@ -909,8 +938,12 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     // the caller chose neither an engine nor a shape: the frame kernel where
     // every chunk has a resident CTA of its own (auto_chunk_limits), which
     // spares a pass its two launches and its trips to memory
-    const bool auto_frame =
-        !frame && h->engine_auto && h->shape_auto && h->share_sums && handle_frame_plan(h).resident;
+    bool auto_frame = !frame && h->engine_auto && h->shape_auto && h->share_sums && handle_frame_plan(h).resident;
+    LargeStep large;
+    if (auto_frame) {
+        const FramePlan &plan = handle_frame_plan(h);
+        if ((plan.per_sm > 1 || 2 * plan.grid > h->sms) && large.enter(h->device) >= 2) auto_frame = false;
+    }
     frame |= auto_frame;
     int rc = frame ? PBS_OK : ensure_graph(h);
     if (rc != PBS_OK) return rc;
@@ -1132,6 +1165,7 @@ int pbs_test_hook(pbs_handle *h, int what, int value) {
     switch (what) {
         case TEST_WAIT_ERROR: h->test_wait_error = value != 0; return PBS_OK;
         case TEST_FAIL_ALLOC: test_fail_alloc = value; return PBS_OK;
+        case TEST_LARGE_STEPS: large_steps[h->device & 63] += value; return PBS_OK;
         default: return PBS_E_INVALID_ARG;
     }
 }

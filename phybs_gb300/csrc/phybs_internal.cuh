@@ -171,6 +171,7 @@ inline double residual_ratio(const InstCtl &c) {
 enum TestHook : int {
     TEST_WAIT_ERROR = 0,  // the next solve or step finds its flag of a wait that gave up set
     TEST_FAIL_ALLOC = 1,  // the value-th device allocation of this thread from now fails
+    TEST_LARGE_STEPS = 2,  // value more large default steps count as running
 };
 
 struct DevMesh {

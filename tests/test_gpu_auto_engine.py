@@ -71,6 +71,68 @@ def test_step_engine_is_the_one_that_ran():
         s.close()
 
 
+TEST_LARGE_STEPS = 2  # pbs_test_hook
+
+
+def test_default_step_beside_others():
+    """A step whose frame kernel takes more than half of the SMs runs the pass
+    kernels when two such steps run already, with the same bits; smaller ones
+    and a chosen engine stay."""
+    p = make_params("gpu_reference", h=1 / 30, max_iters=24)
+    small, half, large = _box(8, 8, 12), _box(16, 14, 18), _box(20, 20, 30)  # 15, 79 and two CTAs a SM
+    for m, others, want in ((small, 0, "frame"), (small, 7, "frame"), (half, 1, "frame"), (half, 2, "graph"),
+                            (large, 1, "frame"), (large, 2, "graph")):
+        a, b = DescentSolver(m, params=p), DescentSolver(m, params=p)
+        b.set_pass_engine("graph")
+        L.lib().pbs_test_hook(a._h, TEST_LARGE_STEPS, others)
+        try:
+            a.step()
+        finally:
+            L.lib().pbs_test_hook(a._h, TEST_LARGE_STEPS, -others)
+        b.step()
+        assert a.step_engine() == want
+        assert np.array_equal(a.positions(), b.positions()) and a.stats()["energy"] == b.stats()["energy"]
+        a.step()
+        assert a.step_engine() == "frame"  # nothing is left counted
+        a.close()
+        b.close()
+
+
+@pytest.mark.parametrize("threads,tets", [(2, (9, 8, 13)), (8, (2, 1, 13)), (6, (12, 12, 20)), (4, (20, 20, 30)),
+                                          (3, (28, 25, 34))])
+def test_handles_stepped_from_threads(threads, tets):
+    """Handles stepped from several threads at once, one each: every one's steps
+    are those it takes by itself, whichever engine a step finds room for."""
+    import threading
+    p = make_params("gpu_reference", h=1 / 30, max_iters=40)
+    meshes = [M.box_mesh(*tets, edge=0.25 / max(tets[:2]), jitter=0.1, seed=k, young=1e5) for k in range(threads)]
+    want = []
+    for m in meshes:
+        s = DescentSolver(m, params=p)
+        for _ in range(12):
+            s.step()
+        want.append((s.positions(), s.stats()["energy"]))
+        s.close()
+    got = [None] * threads
+    start = threading.Barrier(threads)
+
+    def run(k):
+        s = DescentSolver(meshes[k], params=p)
+        start.wait()
+        for _ in range(12):
+            s.step()
+        got[k] = (s.positions(), s.stats()["energy"])
+        s.close()
+
+    ts = [threading.Thread(target=run, args=(k,)) for k in range(threads)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for g, w in zip(got, want):
+        assert g is not None and np.array_equal(g[0], w[0]) and g[1] == w[1]
+
+
 @pytest.mark.parametrize("n", [2, 5, 24])
 def test_default_engine_packed(n):
     """Packed uneven boxes: resident (2, 5) and beyond (24); the iteration
