@@ -207,18 +207,18 @@ __device__ __forceinline__ DFloat chunk_forces_all(const DevParams &p, const Chu
     return e;
 }
 
-// Thread t's sum of the chunk's tet energies where the instance's team is not
-// the CTA's threads: the tets t, t + team, ..., from the slots that the tet loop
-// left them in (threads beyond the team: nothing).  Before anything else goes
-// into the slots.
-__device__ __forceinline__ DFloat team_energy(const ChunkView &v, int nt, int team, const float4 *sf) {
+// Thread t's sum of a piece's tet energies where the tet loop did not form it
+// (the instance's team is not the CTA's threads, or the chunk has several
+// pieces): the tets t, t + team, ... of the nt whose corner records start at
+// cor, from the slots that the tet loop left them in.  Before anything else
+// goes into the slots.
+__device__ __forceinline__ DFloat team_energy(const uint4 *cor, int nt, int t, int team, const float4 *sf) {
     DFloat e{0.f, 0.f};
-    if (threadIdx.x < team)
-        for (int lt = threadIdx.x; lt < nt; lt += team) {
-            int lc[4], sl[4];
-            unpack_cor(v.cor[lt], lc, sl);
-            e = df_add(e, lds128(sf + sl[1]).w);
-        }
+    for (int lt = t; lt < nt; lt += team) {
+        int lc[4], sl[4];
+        unpack_cor(cor[lt], lc, sl);
+        e = df_add(e, lds128(sf + sl[1]).w);
+    }
     return e;
 }
 

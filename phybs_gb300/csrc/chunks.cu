@@ -50,7 +50,8 @@ namespace pbs {
 
 // ------------------------------------------------------------ host: layout
 void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<double> &rest, std::vector<InstCtl> &ctl,
-                  const std::vector<ChunkLimits> &limits, bool grouped, bool pad_slots, ChunkLayout &out) {
+                  const std::vector<ChunkLimits> &limits, bool grouped, int join_tets, bool pad_slots,
+                  ChunkLayout &out) {
     out = ChunkLayout();
     std::vector<int> stamp(Np, -1), lidx(Np, 0), n_part(Np, 0);
     int mark = -1;
@@ -62,6 +63,7 @@ void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<doubl
         const int chunk_tets = limits[b].tets, chunk_nodes = limits[b].nodes;
         const int group_tets = grouped ? CHUNK_GROUP_TETS : 0, group_nodes = CHUNK_GROUP_NODES;
         C.cblk_begin = (int)out.chunk.size();
+        C.pblk_begin = (int)out.piece.size();
         double lo[3], hi[3];
         for (int d = 0; d < 3; ++d) {
             lo[d] = std::numeric_limits<double>::max();
@@ -96,7 +98,9 @@ void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<doubl
         }
         std::sort(order.begin(), order.end());
         if (order.empty()) {  // an instance without tets still needs a CTA for its line-search decisions
+            out.cpiece.push_back((int)out.piece.size());
             out.chunk.push_back(make_int4(tq, 0, (int)lnode_all.size(), 0));
+            out.piece.push_back(make_int2(tq, 0));
             out.chunk_inst.push_back((int)b);
         }
         // the tets from pos on, up to end, that fit the limits -> ctets; their
@@ -128,9 +132,11 @@ void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<doubl
             }
         };
         size_t pos = 0, group_end = 0;
-        int ref = -1, piece = chunk_tets;
+        int ref = -1, piece = chunk_tets, slot = 0;  // slot: of the chunk so far
         while (pos < order.size()) {
+            bool join = join_tets > 0;
             if (group_tets && pos == group_end) {
+                join = false;
                 // a new group, cut into pieces of even size
                 take(pos, order.size(), group_tets, group_nodes, -1);
                 group_end = pos + ctets.size();
@@ -144,12 +150,19 @@ void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<doubl
             // share sectors
             std::sort(lnodes.begin(), lnodes.end());
             const int nl = (int)lnodes.size(), nt = (int)ctets.size();
+            if (!(join && out.chunk.back().y + nt <= join_tets)) {
+                out.cpiece.push_back((int)out.piece.size());
+                out.chunk.push_back(make_int4(tq, 0, (int)lnode_all.size(), 0));
+                out.chunk_inst.push_back((int)b);
+                slot = 0;
+            }
+            int4 &cd = out.chunk.back();
+            const int l0 = cd.w;  // the chunk's local nodes so far
             for (int j = 0; j < nl; ++j) lidx[lnodes[j]] = j;
             scount.assign(nl + 1, 0);
             first.resize(nl);
             for (int t : ctets)
                 for (int c = 0; c < 4; ++c) scount[lidx[(&tets[t].x)[c]] + 1]++;
-            const int l0 = (int)lnode_all.size();
             // slot runs: the nodes with the most corners first (a counting sort),
             // so that a warp's partial-sum loops end together; runs of even
             // length padded to odd, so that eight neighbouring lanes read eight
@@ -161,7 +174,6 @@ void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<doubl
             for (int k = 0; k <= nt; ++k) by_count[k + 1] += by_count[k];
             run_of.resize(nl);
             for (int j = 0; j < nl; ++j) run_of[by_count[nt - scount[j + 1]]++] = j;
-            int slot = 0;
             for (int r = 0; r < nl; ++r) {
                 const int j = run_of[r], cnt = scount[j + 1];
                 first[j] = slot;
@@ -176,27 +188,31 @@ void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<doubl
                 const int *q = &tets[ctets[lt]].x;
                 unsigned loc[4], sl[4];
                 for (int c = 0; c < 4; ++c) {
-                    loc[c] = (unsigned)lidx[q[c]];
-                    sl[c] = (unsigned)first[loc[c]]++;
+                    const int j = lidx[q[c]];
+                    loc[c] = (unsigned)(l0 + j);
+                    sl[c] = (unsigned)first[j]++;
                 }
                 out.qcor.push_back(make_uint4(loc[0] | loc[1] << 16, loc[2] | loc[3] << 16, sl[0] | sl[1] << 16,
                                               sl[2] | sl[3] << 16));
                 out.qperm.push_back(ctets[lt]);
             }
-            out.chunk.push_back(make_int4(tq, nt, l0, nl));
-            out.chunk_inst.push_back((int)b);
-            out.max_local = std::max(out.max_local, nl);
+            out.piece.push_back(make_int2(tq, nt));
+            cd.y += nt;
+            cd.w += nl;
+            out.max_local = std::max(out.max_local, cd.w);
             out.max_slots = std::max(out.max_slots, slot);
             tq += nt;
         }
         C.cblk_end = (int)out.chunk.size();
+        C.pblk_end = (int)out.piece.size();
     }
-    // node -> partials, in chunk order
+    out.cpiece.push_back((int)out.piece.size());
+    // node -> partials, in piece order
     out.pptr.assign(Np + 1, 0);
     for (int i = 0; i < Np; ++i) out.pptr[i + 1] = out.pptr[i] + n_part[i];
     std::vector<int> fill(out.pptr.begin(), out.pptr.end() - 1);
     out.lmeta.resize(lnode_all.size());
-    // (a chunk's runs are of its own nodes: each node's places go up by chunk)
+    // (a piece's runs are of its own nodes: each node's places go up by piece)
     for (size_t j = 0; j < lnode_all.size(); ++j)
         out.lmeta[j] = make_int4(lnode_all[j], lsptr_all[j], lsend_all[j], fill[lrun_all[j]]++);
 }
@@ -252,12 +268,18 @@ __global__ void k_pass_rows(int T, const int *qperm, const float4 *row0, const f
     q2[j] = row2[t];
 }
 
-// Line-search pass: the chunk's {sum e, sum e^2} of its tets and of its share
-// of the instance's nodes -> st.cpart.  e: the thread's tet energies, where the
-// team is the CTA's threads.  Double-float (e) and FP32 (e^2, a noise scale),
-// in the order that phybs_internal.cuh gives.  Called by every thread, before
-// anything else goes into the slots.
-template <int THREADS>
+// Line-search pass: the {sum e, sum e^2} of each of the chunk's pieces, of its
+// tets and of its share of the instance's nodes -> st.cpart.  ec: the thread's
+// tet energies, where the chunk is one piece and the team is the CTA's threads.
+// Double-float (e) and FP32 (e^2, a noise scale), in the order that
+// phybs_internal.cuh gives.  Called by every thread, before anything else goes
+// into the slots.
+// TEAMS: the layout has chunks of several pieces or a team that is not the
+// CTA's threads (then by the slots, one team a piece at a time); without it
+// every chunk is one piece and every thread in its team, and the kernel keeps
+// its registers (two bodies of 150,000 tets, 96 passes without a line search:
+// 1460 us, and 1470 when one kernel held both).
+template <int THREADS, bool TEAMS>
 __device__ __forceinline__ void chunk_energy(const DevMesh &m, const DevParams &p, const DevState &st, int c, int inst,
                                              int par, size_t cur, const ChunkView &v, int nt, const float4 *sf,
                                              DFloat ec) {
@@ -265,26 +287,40 @@ __device__ __forceinline__ void chunk_energy(const DevMesh &m, const DevParams &
     __shared__ float s_e2[THREADS / 32];
     // (formed here, not carried through the tet loop: registers are short)
     const InstCtl *src = ctl_buf(st, par) + inst;
-    const int team = src->team, cb = src->cblk_begin, n0 = src->node_begin;
-    if (team != THREADS) ec = team_energy(v, nt, team, sf);
-    DFloat e{0.f, 0.f};
-    float e2 = 0.f;
-    if (threadIdx.x < team) {
-        const int per = node_share(src->node_end - n0, src->cblk_end - cb), a = n0 + (c - cb) * per;
-        share_energy(m, p, st, cur, a + threadIdx.x, min(a + per, src->node_end), team,
-                     p.incremental ? st.ub : nullptr, e, e2);
-        e = warp_sum_df(df_add(e, ec));
-        e2 = warp_sum_f(e2 + noise_square(m, team, nt, ec.hi));
-        if ((threadIdx.x & 31) == 0) {
-            s_e[threadIdx.x >> 5] = make_float2(e.hi, e.lo);
-            s_e2[threadIdx.x >> 5] = e2;
+    const int pb = src->pblk_begin, n0 = src->node_begin, n1 = src->node_end, per = src->share;
+    const float4 *base = p.incremental ? st.ub : nullptr;
+    const int team = TEAMS ? src->team : THREADS, tid = threadIdx.x & (team - 1), side = threadIdx.x / team;
+    const int p0 = TEAMS ? m.cpiece[c] : pb + c - src->cblk_begin, p1 = TEAMS ? m.cpiece[c + 1] : p0 + 1;
+    const bool own = !TEAMS || (team == THREADS && p1 - p0 == 1);
+    const int t0 = own ? 0 : m.piece[p0].x;
+    for (int q0 = p0; q0 < p1; q0 += THREADS / team) {
+        const int q = q0 + side;
+        if (q < p1) {
+            const int2 pc = own ? make_int2(0, nt) : m.piece[q];
+            if (!own) ec = team_energy(v.cor + (pc.x - t0), pc.y, tid, team, sf);
+            DFloat e{0.f, 0.f};
+            float e2 = 0.f;
+            const int a = n0 + (q - pb) * per;
+            share_energy(m, p, st, cur, a + tid, min(a + per, n1), team, base, e, e2);
+            e = warp_sum_df(df_add(e, ec));
+            e2 = warp_sum_f(e2 + noise_square(m, team, pc.y, ec.hi));
+            if ((tid & 31) == 0) {
+                s_e[threadIdx.x >> 5] = make_float2(e.hi, e.lo);
+                s_e2[threadIdx.x >> 5] = e2;
+            }
         }
+        __syncthreads();
+        if (q < p1 && tid < 32) {
+            double d;
+            float e2;
+            join_warps(s_e + side * (team >> 5), s_e2 + side * (team >> 5), team, d, e2);
+            if (tid == 0) {
+                st.cpart[q] = make_double2(d, (double)e2);
+                if (TEAMS) __threadfence();  // (thread 0 counts the chunk in for every team)
+            }
+        }
+        if (TEAMS) __syncthreads();
     }
-    __syncthreads();
-    if (threadIdx.x >= 32) return;
-    double d;
-    join_warps(s_e, s_e2, team, d, e2);
-    if (threadIdx.x == 0) st.cpart[c] = make_double2(d, (double)e2);
 }
 
 // Then counts the chunk in, and in the instance's last one sums the chunks and
@@ -293,16 +329,16 @@ __device__ __forceinline__ void chunk_energy(const DevMesh &m, const DevParams &
 // last pass into it before counting itself in).  The sum runs in FP64.  Called
 // by every thread of the CTA; *is_last is a shared word.
 template <int THREADS>
-__device__ __forceinline__ void chunk_line_search(const DevMesh &m, const DevParams &p, const DevState &st, int c,
-                                                  int inst, int par, int k, double *sh, int *is_last) {
+__device__ __forceinline__ void chunk_line_search(const DevParams &p, const DevState &st, int inst, int par, int k,
+                                                  double *sh, int *is_last) {
     const InstCtl *src = ctl_buf(st, par) + inst;
     InstCtl *dst = ctl_buf(st, par ^ 1) + inst;
     unsigned int *cnt = st.tcount + inst;
-    const int cb = src->cblk_begin, ce = src->cblk_end;
+    const int pb = src->pblk_begin, pe = src->pblk_end;
     if (threadIdx.x == 0) {
         __threadfence();
         const unsigned int prev = atomicAdd(cnt, 1u);
-        *is_last = (prev == (unsigned int)(ce - cb - 1));
+        *is_last = (prev == (unsigned int)(src->cblk_end - src->cblk_begin - 1));
     }
     __syncthreads();
     if (!*is_last) return;
@@ -312,15 +348,15 @@ __device__ __forceinline__ void chunk_line_search(const DevMesh &m, const DevPar
     // runs on one CTA while the rest of the GPU waits, and one load round trip
     // per partial made it several microseconds
     constexpr int U = 8;
-    const int lanes = ce - cb <= SUM_CHUNKS ? 32 : THREADS < 256 ? THREADS : 256;
+    const int lanes = pe - pb <= SUM_PIECES ? 32 : THREADS < 256 ? THREADS : 256;
     double ea = 0.0, eb = 0.0;
     if (threadIdx.x < lanes)
-        for (int j0 = cb + threadIdx.x; j0 < ce; j0 += U * lanes) {
+        for (int j0 = pb + threadIdx.x; j0 < pe; j0 += U * lanes) {
             double2 v[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int j = j0 + u * lanes;
-                v[u] = j < ce ? __ldcg(st.cpart + j) : make_double2(0.0, 0.0);
+                v[u] = j < pe ? __ldcg(st.cpart + j) : make_double2(0.0, 0.0);
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -344,14 +380,14 @@ __device__ __forceinline__ void chunk_line_search(const DevMesh &m, const DevPar
 // The whole of one chunk once its node words (and, with STAGE, its rows and
 // records) are in shared memory: forces, partials, the Jacobi diagonal every
 // hd_every passes, and the line-search tail.
-template <int MATERIAL, int THREADS, bool INC, bool PACK, bool PRE>
+template <int MATERIAL, int THREADS, bool INC, bool PACK, bool PRE, bool TEAMS>
 __device__ __forceinline__ void chunk_body(const DevMesh &m, const DevParams &p, const DevState &st, int c,
                                            int inst, int par, const PassView &pv, size_t cur, const ChunkView &v,
                                            const int4 *meta, int nt, int nl, float4 *sf, double *sh,
                                            int *is_last, const TetRows &first = TetRows()) {
     const DFloat e = chunk_forces_all<MATERIAL, THREADS, INC, PACK, PRE>(p, v, nt, pv.check, sf, first);
     chunk_partials<THREADS>(meta, nl, sf, st.part);
-    if (pv.check) chunk_energy<THREADS>(m, p, st, c, inst, par, cur, v, nt, sf, e);
+    if (pv.check) chunk_energy<THREADS, TEAMS>(m, p, st, c, inst, par, cur, v, nt, sf, e);
     if (pv.do_h) {
         __syncthreads();
         chunk_hdiag<MATERIAL, THREADS, INC, PACK>(v, nt, sf);
@@ -363,7 +399,7 @@ __device__ __forceinline__ void chunk_body(const DevMesh &m, const DevParams &p,
     // waiting), and before it counts itself into a line search
     const InstCtl *src = ctl_buf(st, par) + inst;
     if (c == src->cblk_begin) settle_pass<THREADS>(p, st, src, ctl_buf(st, par ^ 1) + inst, true);
-    if (pv.check) chunk_line_search<THREADS>(m, p, st, c, inst, par, pv.k, sh, is_last);
+    if (pv.check) chunk_line_search<THREADS>(p, st, inst, par, pv.k, sh, is_last);
 }
 
 // One CTA per chunk.  What bounds it: with four CTAs of 256 threads a SM, each
@@ -387,7 +423,7 @@ __device__ __forceinline__ void chunk_body(const DevMesh &m, const DevParams &p,
 // against 49.7 us a pass on the 1M-tet box at 85 registers).  The full stress
 // of either material needs 64 on its tet loop; the bound keeps the out-of-line
 // calls of near-inverted tets, after the loop, from raising it.
-template <int MATERIAL, int THREADS, bool INC, bool STAGE>
+template <int MATERIAL, int THREADS, bool INC, bool STAGE, bool TEAMS>
 __global__ void __launch_bounds__(THREADS, PBS_INC_THREADS_PER_SM / THREADS)
     k_tchunk(DevMesh m, DevParams p, DevState st, int par) {
     extern __shared__ float4 smem4[];
@@ -507,8 +543,8 @@ __global__ void __launch_bounds__(THREADS, PBS_INC_THREADS_PER_SM / THREADS)
     v.cor = STAGE ? s_cor : m.qcor + tq0;
     v.meta = meta;
     v.rest = m.rest;
-    chunk_body<MATERIAL, THREADS, INC, !STAGE, !STAGE>(m, p, st, c, inst, par, pv, cur, v, meta, nt, nl, s_f, sh,
-                                                       &is_last, first);
+    chunk_body<MATERIAL, THREADS, INC, !STAGE, !STAGE, TEAMS>(m, p, st, c, inst, par, pv, cur, v, meta, nt, nl, s_f, sh,
+                                                              &is_last, first);
 }
 
 // ------------------------------------------------------------ persistent, TMA-fed variant
@@ -723,8 +759,8 @@ __global__ void __launch_bounds__(THREADS, 768 / THREADS) k_tstream(DevMesh m, D
             v.cor = sb.cor;
             v.meta = sb.meta;
             v.rest = m.rest;
-            chunk_body<MATERIAL, THREADS, INC, false, false>(m, p, st, c, cur.inst, par, cur.pv, cur.cur, v, sb.meta, cur.nt,
-                                               cur.nl, s_f, sh, &is_last);
+            chunk_body<MATERIAL, THREADS, INC, false, false, false>(m, p, st, c, cur.inst, par, cur.pv, cur.cur, v, sb.meta,
+                                                                    cur.nt, cur.nl, s_f, sh, &is_last);
         }
         __syncthreads();  // buffer b and the slots are free again
         if (threadIdx.x == 0 && j + 2 < nj) stage_chunk_bulk(m, c + 2 * G, sb, &bar[b]);
@@ -733,8 +769,8 @@ __global__ void __launch_bounds__(THREADS, 768 / THREADS) k_tstream(DevMesh m, D
 }
 
 // ------------------------------------------------------------ launchers
-template <int MATERIAL, int THREADS, bool INC, bool STAGE> static cudaError_t allow_smem() {
-    return cudaFuncSetAttribute(k_tchunk<MATERIAL, THREADS, INC, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+template <int MATERIAL, int THREADS, bool INC, bool STAGE, bool TEAMS = false> static cudaError_t allow_smem() {
+    return cudaFuncSetAttribute(k_tchunk<MATERIAL, THREADS, INC, STAGE, TEAMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 CHUNK_MAX_SMEM);
 }
 
@@ -745,7 +781,8 @@ template <int MATERIAL, int THREADS, bool INC> static cudaError_t allow_smem_str
 
 template <int MATERIAL, bool INC> static cudaError_t allow_smem_all() {
     const cudaError_t e[] = {allow_smem<MATERIAL, 128, INC, false>(), allow_smem<MATERIAL, 256, INC, false>(),
-                             allow_smem<MATERIAL, 512, INC, false>()};
+                             allow_smem<MATERIAL, 512, INC, false>(), allow_smem<MATERIAL, 256, INC, false, true>(),
+                             allow_smem<MATERIAL, 512, INC, false, true>()};
     for (cudaError_t x : e)
         if (x != cudaSuccess) return x;
     return cudaSuccess;
@@ -805,13 +842,13 @@ static cudaLaunchConfig_t chunk_config(cudaStream_t s, int grid, int threads, si
     return cfg;
 }
 
-template <int MATERIAL, int THREADS, bool INC, bool STAGE>
+template <int MATERIAL, int THREADS, bool INC, bool STAGE, bool TEAMS = false>
 static cudaError_t launch_tchunk_t(cudaStream_t s, const DevMesh &m, const DevParams &p, const DevState &st, int par,
                                    bool pdl) {
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = chunk_config(s, m.n_chunks, THREADS,
                                           chunk_smem(m.chunk_tets, m.chunk_nodes, m.chunk_slots, INC, STAGE ? 1 : 0), pdl, at, m);
-    return cudaLaunchKernelEx(&cfg, k_tchunk<MATERIAL, THREADS, INC, STAGE>, m, p, st, par);
+    return cudaLaunchKernelEx(&cfg, k_tchunk<MATERIAL, THREADS, INC, STAGE, TEAMS>, m, p, st, par);
 }
 
 template <int MATERIAL, int THREADS, bool INC>
@@ -828,6 +865,9 @@ template <int MATERIAL, bool INC>
 static cudaError_t launch_tchunk(cudaStream_t s, const DevMesh &m, const DevParams &p, const DevState &st, int par,
                                  bool pdl) {
     if (m.chunk_threads == 128) return launch_tchunk_t<MATERIAL, 128, INC, false>(s, m, p, st, par, pdl);
+    if (m.teams)  // (automatic layouts: no team is of more threads than the CTA)
+        return m.chunk_threads == 512 ? launch_tchunk_t<MATERIAL, 512, INC, false, true>(s, m, p, st, par, pdl)
+                                      : launch_tchunk_t<MATERIAL, 256, INC, false, true>(s, m, p, st, par, pdl);
     if (m.chunk_threads == 512) return launch_tchunk_t<MATERIAL, 512, INC, false>(s, m, p, st, par, pdl);
     return launch_tchunk_t<MATERIAL, 256, INC, false>(s, m, p, st, par, pdl);
 }

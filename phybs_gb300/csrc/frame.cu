@@ -293,18 +293,24 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
         own.team = sc.team;
     }
     __syncthreads();
-    // this thread's first node: mine() whether it has one
-    auto mine = [&] { return worker && own.n0 + tid < own.n1; };
+    // (the variant with registers to spare keeps its nodes in them)
+    constexpr bool REGS = THREADS == 128 && PER_SM == 1;
+    const int rn0 = own.n0, rn1 = own.n1;
+    auto n0 = [&] { return REGS ? rn0 : own.n0; };
+    auto n1 = [&] { return REGS ? rn1 : own.n1; };
+    auto team = [&] { return THREADS == 128 ? 128 : own.team; };  // (no team is smaller than 128)
+    // this thread's first node is n0() + tid: mine() whether it has one
+    auto mine = [&] { return worker && n0() + tid < n1(); };
     int pa0 = 0, pe0 = 0;
     if (mine()) {
-        pa0 = m.pptr[own.n0 + tid];
-        pe0 = m.pptr[own.n0 + tid + 1];
+        pa0 = m.pptr[n0() + tid];
+        pe0 = m.pptr[n0() + tid + 1];
     }
     int k = sc.k, par = sc.par;
     bool force = sc.force_check != 0;
     {
         const size_t cur = (size_t)par * m.Np;
-        for (int i = own.n0 + tid; worker && i < own.n1; i += THREADS) {
+        for (int i = n0() + tid; worker && i < n1(); i += THREADS) {
             const float4 h = st.uh[cur + i], l = st.ul[cur + i];
             st_word(fx.xh + i, make_float3(h.x, h.y, h.z), fx.tag0 + 1);
             st_word(fx.xl + i, make_float3(l.x, l.y, l.z), fx.tag0 + 1);
@@ -329,7 +335,7 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
             float e2 = 0.f;
             // the words of this thread's first node, only ever written by itself
             if (mine()) {
-                const int i0 = own.n0 + tid;
+                const int i0 = n0() + tid;
                 nn.uh = st.uh[cur + i0];
                 nn.ul = st.ul[cur + i0];
                 nn.dd = st.dd[cur + i0];
@@ -337,8 +343,8 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
             }
             // the CTA's share of the node energy terms, before the other CTAs'
             // words arrive
-            if (check && tid < own.team)
-                share_energy(m, p, st, cur, own.n0 + tid, own.n1, own.team, INC ? st.ub : nullptr, e, e2);
+            if (check && tid < team())
+                share_energy(m, p, st, cur, n0() + tid, n1(), team(), INC ? st.ub : nullptr, e, e2);
             // ---- tet phase: this CTA's chunk, or the chunks b, b + G, ...
             for (int c = b; c < m.n_chunks; c += RES ? m.n_chunks : G) {
                 const int4 cd = m.chunk[c];
@@ -372,7 +378,7 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
                 v.meta = meta;
                 v.rest = m.rest;
                 DFloat ec = chunk_forces_all<MATERIAL, THREADS, INC, true, false, true>(p, v, nt, check, s_f);
-                if (THREADS > 128 && check && own.team != THREADS) ec = team_energy(v, nt, own.team, s_f);
+                if (check && team() != THREADS && tid < team()) ec = team_energy(v.cor, nt, tid, team(), s_f);
                 publish_partials<THREADS>(meta, nl, s_f, st.part, tag);
                 if (do_h) {
                     chunk_sync<THREADS, true>();
@@ -380,9 +386,9 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
                     chunk_sync<THREADS, true>();
                     publish_partials<THREADS>(meta, nl, s_f, st.parth, tag);
                 }
-                if (check && tid < own.team) {
+                if (check && tid < team()) {
                     e = df_add(e, ec);
-                    e2 += noise_square(m, own.team, nt, ec.hi);
+                    e2 += noise_square(m, team(), nt, ec.hi);
                 }
                 // the slots and node words are free for the next chunk (or pass)
                 if (!RES) chunk_sync<THREADS, true>();
@@ -421,7 +427,7 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
             if (!worker && !sc.done) {
                 double d;
                 float se2;
-                join_warps(s_e, s_e2, own.team, d, se2);
+                join_warps(s_e, s_e2, team(), d, se2);
                 if (tid == THREADS)
                     st_word(fx.ce + b, (unsigned)__double2loint(d), (unsigned)__double2hiint(d),
                             __float_as_uint(se2), tag);
@@ -447,8 +453,8 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
             // waited for whether or not the update needs it (pinned nodes, a
             // restore): the chunks have then read the state word that the
             // update overwrites
-            nc.ch = st.ch[own.n0 + tid];
-            nc.cl = st.cl[own.n0 + tid];
+            nc.ch = st.ch[n0() + tid];
+            nc.cl = st.cl[n0() + tid];
             ok = collect_partials(st, pa0, pe0, do_h, tag, sum, err) && ok;
         }
         ok = !__syncthreads_or(!ok);
@@ -470,10 +476,10 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
         ctx.cur = cur;
         ctx.nxt = (size_t)(1 - par) * m.Np;
         // (by whole warps: a warp's nodes are one group of 32)
-        for (int g = tid & ~31; worker && g < own.n1 - own.n0; g += THREADS) {
-            const int i = own.n0 + g + (tid & 31);
+        for (int g = tid & ~31; worker && g < n1() - n0(); g += THREADS) {
+            const int i = n0() + g + (tid & 31);
             float r2 = 0.f;
-            if (i < own.n1) {
+            if (i < n1()) {
                 if (g >= THREADS) {
                     nc.ch = st.ch[i];
                     nc.cl = st.cl[i];
@@ -497,7 +503,7 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
         __syncthreads();
         if (tid == THREADS) {
             float s = 0.f;
-            const int groups = min((own.n1 - own.n0 + 31) >> 5, SUM_GROUPS);
+            const int groups = min((n1() - n0() + 31) >> 5, SUM_GROUPS);
             for (int g = 0; g < groups; g += WARPS) {
                 float v[WARPS];
 #pragma unroll

@@ -164,18 +164,19 @@ __device__ __forceinline__ DFloat lane_tree_df(DFloat v) {
 // phybs_internal.cuh gives.  Called by every thread; valid in thread 0.
 template <int THREADS>
 __device__ __forceinline__ DFloat instance_r2(const DevState &st, const InstCtl *src) {
-    const int nodes = src->node_end - src->node_begin, C = src->cblk_end - src->cblk_begin;
+    const int C = src->pblk_end - src->pblk_begin;
     const float *g = st.npartf + src->node_begin / 32;
     DFloat acc{0.f, 0.f};
-    if (sums_by_share(nodes, C)) {
+    if (src->by_share) {
         // THREADS shares at a time: a share's groups by a thread, then the
         // lanes' shares by warp 0
         __shared__ float s_share[THREADS];
-        const int groups = (nodes + 31) / 32, per = node_share(nodes, C) / 32;
+        const int groups = (src->node_end - src->node_begin + 31) / 32, per = src->share / 32;
         for (int j0 = 0; j0 < C; j0 += THREADS) {
-            const int j = j0 + (int)threadIdx.x, a = min(j * per, groups), e = min(a + per, groups);
-            float s = 0.f;
+            const int j = j0 + (int)threadIdx.x;
             if (j < C) {
+                const int a = j * per, e = min(a + per, groups);
+                float s = 0.f;
                 constexpr int U = 8;  // groups in flight
                 for (int q0 = a; q0 < e; q0 += U) {
                     float v[U];
@@ -184,12 +185,14 @@ __device__ __forceinline__ DFloat instance_r2(const DevState &st, const InstCtl 
 #pragma unroll
                     for (int u = 0; u < U; ++u) s += v[u];
                 }
+                s_share[threadIdx.x] = s;
             }
-            s_share[threadIdx.x] = s;
             __syncthreads();
-            if (threadIdx.x < 32)
-                for (int l = threadIdx.x; l < min(THREADS, C - j0); l += 32) acc = df_add(acc, s_share[l]);
-            __syncthreads();
+            if (threadIdx.x < 32) {
+                const int n = min(THREADS, C - j0);
+                for (int l = threadIdx.x; l < n; l += 32) acc = df_add(acc, s_share[l]);
+            }
+            if (j0 + THREADS < C) __syncthreads();
         }
         return threadIdx.x < 32 ? lane_tree_df(acc) : acc;
     }

@@ -104,7 +104,8 @@ struct pbs_handle {
     std::vector<int4> h_tets_pad;
     std::vector<double> h_rest_pad;
     DevBuf<int4> chunk;
-    DevBuf<int> chunk_inst, qperm, pptr;
+    DevBuf<int2> piece;
+    DevBuf<int> chunk_inst, cpiece, qperm, pptr;
     uint4 *qcor = nullptr;  // in qrows, after the three row arrays
     DevBuf<int4> lmeta;
     // the pass tets' rows and corner records, one allocation (4 x 16 B a tet):
@@ -182,6 +183,8 @@ struct pbs_handle {
     cudaEvent_t ev_start = nullptr, ev_end = nullptr, ev_chunk[2] = {nullptr, nullptr};
     cudaGraphExec_t graph = nullptr;
     bool graph_valid = false;
+    bool teams = false;       // DevMesh::teams
+    bool joined = false;      // chunks of several pieces: for the pass kernels only
     bool share_sums = true;   // every instance's |g|^2 is summed by share (sums_by_share)
     bool shape_auto = true;   // no caller set the chunk shape (pbs_set_chunk_shape, pbs_autotune)
     bool engine_auto = true;  // nor the pass engine (pbs_set_pass_engine)
@@ -205,8 +208,10 @@ struct pbs_handle {
         m.inc_ptr = inc_ptr.p; m.inc = inc.p; m.tslot = tslot.p; m.info = info.p; m.rest = rest4.p;
         m.tblk_inst = tblk_inst.p; m.nblk_inst = nblk_inst.p;
         m.n_chunks = n_chunks; m.chunk = chunk.p; m.chunk_inst = chunk_inst.p;
+        m.piece = piece.p; m.cpiece = cpiece.p;
         m.chunk_tets = chunk_tets; m.chunk_nodes = chunk_nodes; m.chunk_threads = chunk_threads;
         m.chunk_slots = chunk_slots;
+        m.teams = teams;
         m.noise_tets = shape_auto ? CHUNK_NOISE_TETS : 0;
         m.chunk_stage = chunk_stage;
         m.node_npt = node_npt;
@@ -240,8 +245,8 @@ struct pbs_handle {
                              &staging_ids};
         for (auto b : ii) b->release();
         ws_theta.release(); ws_stats.release();
-        chunk.release(); lmeta.release(); cpart.release(); rslot.release();
-        DevBuf<int> *ci[] = {&chunk_inst, &qperm, &pptr};
+        chunk.release(); piece.release(); lmeta.release(); cpart.release(); rslot.release();
+        DevBuf<int> *ci[] = {&chunk_inst, &cpiece, &qperm, &pptr};
         for (auto b : ci) b->release();
         DevBuf<float4> *cf[] = {&qrows, &part, &parth};
         for (auto b : cf) b->release();
@@ -306,36 +311,63 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
         }
     }
     const bool grouped = automatic;  // (a caller's own shape keeps a reference node a chunk)
-    ChunkLayout cl;
-    const std::vector<InstCtl> ctl0 = ctl;
-    build_chunks(h->Np, h->h_tets_pad, h->h_rest_pad, ctl, limits, grouped, true, cl);
-    if (chunk_smem(ct, cn, cl.max_slots, true, stage) > (size_t)CHUNK_MAX_SMEM) {  // no room to pad slot runs
-        ctl = ctl0;
-        build_chunks(h->Np, h->h_tets_pad, h->h_rest_pad, ctl, limits, grouped, false, cl);
-    }
-    const int nc = (int)cl.chunk.size();
-    // the pass kernels run chunks of more than 256 tets with two tets a thread
+    // The pass kernels run chunks of more than 256 tets with two tets a thread
     // (a packed batch's with 256 threads, which its smaller instances can use);
     // the frame kernel, where every chunk has its place, with up to four
-    // (auto_chunk_limits has both sides)
+    // (auto_chunk_limits has both sides).  In a batch that 256 threads run and
+    // that is too large to be resident, the smaller instances' pieces are joined
+    // up to the largest one's chunk: every CTA takes the shared memory of that,
+    // and alone in it a piece of 128 tets kept half of its threads idle (96
+    // passes, full / incremental stress, us: a body of 300,000 tets and 100 of
+    // 2,000 2925 / 3312 joined, 3516 / 3889 in pieces; 120,000 and 60 of 2,000-10,000
+    // 2874 / 3255 and 3329 / 3698; 90,000 and 100 of 2,000-4,000 2135 / 2418 and
+    // 2541 / 2844).
+    size_t est = 0;  // pieces at least
+    for (int b = 0; automatic && b < h->B; ++b)
+        est += (ctl[b].tet_end - ctl[b].tet_begin + limits[b].tets - 1) / limits[b].tets;
+    const bool wide = ct == CHUNK_GROUP_TETS || (ct > 256 && est > 2 * (size_t)h->sms);
+    int join = automatic && h->B > 1 && wide && est > 2 * (size_t)h->sms ? ct : 0;
+    ChunkLayout cl;
+    const std::vector<InstCtl> ctl0 = ctl;
+    auto build = [&](bool pad) {
+        ctl = ctl0;
+        build_chunks(h->Np, h->h_tets_pad, h->h_rest_pad, ctl, limits, grouped, join, pad, cl);
+        const int nodes = join ? std::max(cn, cl.max_local) : cn;
+        return chunk_smem(ct, nodes, cl.max_slots, true, stage) <= (size_t)CHUNK_MAX_SMEM;
+    };
+    // (no room to pad slot runs, nor for the joined ones)
+    if (!build(true) && !build(false) && join) {
+        join = 0;
+        if (!build(true)) build(false);
+    }
+    if (join) cn = std::max(cn, cl.max_local);
+    const int nc = (int)cl.chunk.size();
     if (automatic) {
         if (ct == CHUNK_GROUP_TETS) threads = nc > h->sms && h->B == 1 ? 512 : 256;
-        else threads = ct > 256 && nc > 2 * h->sms ? 256 : 128;
+        else threads = wide || (ct > 256 && nc > 2 * h->sms) ? 256 : 128;
         threads = std::max(threads, max_team);
     }
-    bool share_sums = true;
-    for (const InstCtl &c : ctl)
-        share_sums = share_sums && sums_by_share(c.node_end - c.node_begin, c.cblk_end - c.cblk_begin);
+    bool share_sums = true, teams = join > 0;
+    for (InstCtl &c : ctl) {
+        const int nodes = c.node_end - c.node_begin, pieces = c.pblk_end - c.pblk_begin;
+        c.share = node_share(nodes, pieces);
+        c.by_share = sums_by_share(nodes, pieces);
+        share_sums = share_sums && c.by_share;
+        teams = teams || c.team != threads;
+    }
     const size_t L = cl.lmeta.size(), T = (size_t)h->T;
     // all of the new layout's memory before the old one's is given up: a
     // handle that runs out of it keeps the layout it had
     DevBuf<int4> chunk, lmeta;
-    DevBuf<int> chunk_inst, qperm, pptr;
+    DevBuf<int2> piece;
+    DevBuf<int> chunk_inst, cpiece, qperm, pptr;
     DevBuf<double2> cpart;
     DevBuf<float4> part, parth;
     cudaError_t ea = chunk.alloc(nc);
     if (ea == cudaSuccess) ea = chunk_inst.alloc(nc);
-    if (ea == cudaSuccess) ea = cpart.alloc(nc);
+    if (ea == cudaSuccess) ea = piece.alloc(cl.piece.size());
+    if (ea == cudaSuccess) ea = cpiece.alloc(cl.cpiece.size());
+    if (ea == cudaSuccess) ea = cpart.alloc(cl.piece.size());
     if (ea == cudaSuccess) ea = qperm.alloc(T);
     if (ea == cudaSuccess) ea = lmeta.alloc(L);
     if (ea == cudaSuccess) ea = pptr.alloc(h->Np + 1);
@@ -344,16 +376,19 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
     if (ea == cudaSuccess) {
         std::swap(h->chunk, chunk); std::swap(h->lmeta, lmeta);
         std::swap(h->chunk_inst, chunk_inst); std::swap(h->qperm, qperm); std::swap(h->pptr, pptr);
-        std::swap(h->cpart, cpart);
+        std::swap(h->cpart, cpart); std::swap(h->piece, piece); std::swap(h->cpiece, cpiece);
         std::swap(h->part, part); std::swap(h->parth, parth);
     }
     chunk.release(); lmeta.release(); chunk_inst.release(); qperm.release(); pptr.release(); cpart.release();
+    piece.release(); cpiece.release();
     part.release(); parth.release();
     CK(ea);
     h->shape_auto = automatic;
     h->graph_valid = h->plan_valid = false;
     cudaStream_t s = h->stream;
     CK(cudaMemcpyAsync(h->chunk.p, cl.chunk.data(), sizeof(int4) * nc, cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(h->piece.p, cl.piece.data(), sizeof(int2) * cl.piece.size(), cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(h->cpiece.p, cl.cpiece.data(), sizeof(int) * cl.cpiece.size(), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(h->chunk_inst.p, cl.chunk_inst.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(h->qperm.p, cl.qperm.data(), sizeof(int) * T, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(h->qcor, cl.qcor.data(), sizeof(uint4) * T, cudaMemcpyHostToDevice, s));
@@ -368,6 +403,8 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
     h->chunk_nodes = cn;
     h->chunk_stage = stage;
     h->share_sums = share_sums;
+    h->joined = join > 0;
+    h->teams = teams;
     if (host_ctl) {
         *host_ctl = ctl;
     } else {
@@ -938,7 +975,7 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     // the caller chose neither an engine nor a shape: the frame kernel where
     // every chunk has a resident CTA of its own (auto_chunk_limits), which
     // spares a pass its two launches and its trips to memory
-    bool auto_frame = !frame && h->engine_auto && h->shape_auto && h->share_sums && handle_frame_plan(h).resident;
+    bool auto_frame = !frame && h->engine_auto && h->shape_auto && h->share_sums && !h->joined && handle_frame_plan(h).resident;
     LargeStep large;
     if (auto_frame) {
         const FramePlan &plan = handle_frame_plan(h);

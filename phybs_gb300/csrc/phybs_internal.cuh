@@ -42,9 +42,13 @@
 //                                  per slot run of the chunk (as many, in order of length), .y the
 //                                  first slot, .z the end slot, .w where the partial of the run's
 //                                  node goes
-//   pptr        int[Np+1]          node i's partials: part[pptr[i] .. pptr[i+1]-1], by chunk
-//   part, parth float4[L]          per (node, chunk) partial force / Jacobi-diagonal sums
-//   cpart       double2[n_chunks]  per chunk {sum e, sum e^2}
+//   pptr        int[Np+1]          node i's partials: part[pptr[i] .. pptr[i+1]-1], by piece
+//   part, parth float4[L]          per (node, piece) partial force / Jacobi-diagonal sums
+//   piece       int2[n_pieces]     {first pass tet, tet count}: the tets whose forces and energies
+//                                  are summed together.  A chunk is one piece, or several of a
+//                                  group that one CTA takes together (build_chunks, join_tets)
+//   cpiece      int[n_chunks+1]    chunk c's pieces: cpiece[c] .. cpiece[c+1]-1
+//   cpart       double2[n_pieces]  per piece {sum e, sum e^2}
 //   rslot       double[3][4T]      per-step FP64 corner forces at the base, by gather slot
 //   npart       double[n_nblk]     per node-block |g|^2 (warm-start reference)
 //   npartf      float[8*n_nblk]    |g|^2 of a pass per 32 nodes (FP32 sums)
@@ -129,35 +133,38 @@ struct __align__(16) InstCtl {
     // non-finite forces an energy check the pass's tet kernel did not make)
     int pending, void_pass;
     double g1;                             // |g| at the learned candidate (extrapolation base)
-    int team;  // threads whose sums make up a chunk's energy (chunk_energy)
-    int pad6;
+    int team;  // threads whose sums make up a piece's energy (chunk_energy)
+    int pblk_begin, pblk_end;  // the instance's pieces
+    int share;     // nodes of a piece's share (node_share)
+    int by_share;  // |g|^2 is summed by share (sums_by_share)
+    int pad;
 };
 
 // How an instance's line-search energy and |g|^2 are summed does not depend on
 // the kernel that sums them, its threads or the instance's company: an instance
 // takes one path alone (the frame kernel), packed (the pass kernels) and at
-// any CTA size.  With T = team threads, C chunks and 32-node groups:
-//   energy   of a chunk: thread t adds the terms of the nodes t, t + T, ... of the
-//            chunk's share, then those of its tets t, t + T, ...; a lane tree,
+// any CTA size.  With T = team threads, C pieces and 32-node groups:
+//   energy   of a piece: thread t adds the terms of the nodes t, t + T, ... of the
+//            piece's share, then those of its tets t, t + T, ...; a lane tree,
 //            then the warps' sums in a lane tree;
-//            of the instance: FP64, 32 lanes, each its chunks in ascending
+//            of the instance: FP64, 32 lanes, each its pieces in ascending
 //            order, then the lane tree;
 //   |g|^2    of a group: a lane tree; of a share: its groups in ascending order;
 //            of the instance: 32 lanes of double-float, each its shares in
 //            ascending order, then the lane tree.
-// Beyond SUM_CHUNKS chunks, where the serial chains would be long and no frame
+// Beyond SUM_PIECES pieces, where the serial chains would be long and no frame
 // kernel is resident, 256 threads take the place of the 32 lanes, and |g|^2 is
 // summed by 256-node blocks instead of shares.
-constexpr int SUM_CHUNKS = 512, SUM_GROUPS = 256;  // (groups of a share that the frame kernel keeps)
+constexpr int SUM_PIECES = 512, SUM_GROUPS = 256;  // (groups of a share that the frame kernel keeps)
 
-// Nodes of a chunk's share: the instance's, in whole groups of 32, evenly over
-// its chunks.
-__host__ __device__ inline int node_share(int nodes, int chunks) {
+// Nodes of a piece's share: the instance's, in whole groups of 32, evenly over
+// its pieces.
+__host__ __device__ inline int node_share(int nodes, int pieces) {
     const int groups = (nodes + 31) / 32;
-    return chunks > 0 ? (groups + chunks - 1) / chunks * 32 : 0;
+    return pieces > 0 ? (groups + pieces - 1) / pieces * 32 : 0;
 }
-__host__ __device__ inline bool sums_by_share(int nodes, int chunks) {
-    return chunks <= SUM_CHUNKS && node_share(nodes, chunks) <= 32 * SUM_GROUPS;
+__host__ __device__ inline bool sums_by_share(int nodes, int pieces) {
+    return pieces <= SUM_PIECES && node_share(nodes, pieces) <= 32 * SUM_GROUPS;
 }
 
 // |g| / |g0| of an instance's last pass (-1 before the first pass).
@@ -185,10 +192,12 @@ struct DevMesh {
     const int *tblk_inst, *nblk_inst;
     // pass layout
     int n_chunks, chunk_tets, chunk_nodes, chunk_slots, chunk_threads, chunk_stage;
+    int teams;       // a chunk has several pieces, or a team is not the CTA's threads (chunk_energy)
     int noise_tets;  // tets whose energies the noise scale adds before squaring (noise_square)
     int node_npt;
     const int4 *chunk;
-    const int *chunk_inst;
+    const int2 *piece;
+    const int *chunk_inst, *cpiece;
     const float4 *qrow0, *qrow1, *qrow2;
     const uint4 *qcor;
     const int4 *lmeta;
@@ -281,7 +290,8 @@ inline uint32_t spread10(uint32_t v) {
 // instances' node / tet ranges, whose cblk ranges are filled in.
 struct ChunkLayout {
     std::vector<int4> chunk;
-    std::vector<int> chunk_inst, qperm, pptr;
+    std::vector<int2> piece;
+    std::vector<int> chunk_inst, cpiece, qperm, pptr;
     std::vector<uint4> qcor;
     std::vector<int4> lmeta;
     int max_local = 0, max_slots = 0;
@@ -303,11 +313,14 @@ int auto_team(int tets, int sms);
 // stress: the tet forces then have the same bits at every chunk limit, and an
 // iteration to a tolerance takes the same path.  With a reference node a chunk
 // the count of passes to a residual of 1e-4 moved by up to 1%, and the
-// velocities with it by up to 5e-5.  pad_slots: see the slot runs.
+// velocities with it by up to 5e-5.  join_tets: consecutive pieces of a group
+// make one chunk of at most so many tets (0: each its own), whose partials,
+// energies and bits stay those of its pieces.  pad_slots: see the slot runs.
 constexpr int CHUNK_GROUP_TETS = 1024, CHUNK_GROUP_NODES = 448;
 constexpr int CHUNK_NOISE_TETS = 4;
 void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<double> &rest, std::vector<InstCtl> &ctl,
-                  const std::vector<ChunkLimits> &limits, bool grouped, bool pad_slots, ChunkLayout &out);
+                  const std::vector<ChunkLimits> &limits, bool grouped, int join_tets, bool pad_slots,
+                  ChunkLayout &out);
 cudaError_t launch_pass_rows(cudaStream_t s, int T, const int *qperm, const float4 *row0, const float4 *row1,
                              const float4 *row2, float4 *q0, float4 *q1, float4 *q2);
 cudaError_t prepare_chunk_kernels();
