@@ -157,7 +157,7 @@ struct pbs_handle {
     DevBuf<float> npartf;
     DevBuf<InstCtl> ctl, ctl2;  // ctl2: the pass graph's second control-block copy
     DevBuf<unsigned int> tcount;
-    DevBuf<int> active;  // [0] instances running, [1] a device wait gave up
+    int *active = nullptr;  // DevState::active, behind the control blocks: one copy brings both to the host
     // strain-based PBD (levels built on first use) and projective dynamics
     // (its matrix built per (dt_matrix, stiffness)); dyn_* are their per-step
     // positions, start positions and right-hand-side base
@@ -177,8 +177,7 @@ struct pbs_handle {
     DevBuf<float> pd_val, pd_dinv, pd_cgval;
     DevBuf<float4> dyn_px, dyn_x0, dyn_s;
     // host pinned
-    int *h_active = nullptr;   // 2 slots: running counts of the host loop; or the bodies the loop ran;
-                               // or, in the second, the frame kernel's flag of a wait that gave up
+    int *h_active = nullptr;   // 2 slots: running counts of the host loop, or the bodies the loop ran
     InstCtl *h_ctl = nullptr;
     cudaEvent_t ev_start = nullptr, ev_end = nullptr, ev_chunk[2] = {nullptr, nullptr};
     cudaGraphExec_t graph = nullptr;
@@ -228,7 +227,7 @@ struct pbs_handle {
         s.uh = uh.p; s.ul = ul.p; s.dd = dd.p; s.oh = oh.p; s.ol = ol.p; s.u0h = u0h.p; s.u0l = u0l.p;
         s.th = th.p; s.tl = tl.p; s.v = v.p; s.vold = vold.p; s.ext = ext.p; s.diag = diag.p;
         s.hist1 = hist1.p; s.hist2 = hist2.p; s.bh = bh.p; s.bl = bl.p; s.ub = ub.p; s.ch = ch.p; s.cl = cl.p;
-        s.tf = tf.p; s.hd = hd.p; s.tpart = tpart.p; s.npart = npart.p; s.npartf = npartf.p; s.ctl = ctl.p; s.active = active.p;
+        s.tf = tf.p; s.hd = hd.p; s.tpart = tpart.p; s.npart = npart.p; s.npartf = npartf.p; s.ctl = ctl.p; s.active = active;
         s.ctl2 = ctl2.p; s.tcount = tcount.p;
         s.cpart = cpart.p; s.part = part.p; s.parth = parth.p; s.rslot = rslot.p;
         return s;
@@ -241,7 +240,7 @@ struct pbs_handle {
         DevBuf<float4> *f4[] = {&row0, &row1, &row2, &info, &rest4, &uh, &ul, &dd, &oh, &ol, &u0h, &u0l, &th, &tl,
                                 &v, &vold, &ext, &diag, &hist1, &hist2, &bh, &bl, &ub, &ch, &cl};
         for (auto b : f4) b->release();
-        DevBuf<int> *ii[] = {&inc_ptr, &inc, &tblk_inst, &nblk_inst, &pad2user, &tet_user, &node_state, &bad, &active,
+        DevBuf<int> *ii[] = {&inc_ptr, &inc, &tblk_inst, &nblk_inst, &pad2user, &tet_user, &node_state, &bad,
                              &staging_ids};
         for (auto b : ii) b->release();
         ws_theta.release(); ws_stats.release();
@@ -667,8 +666,8 @@ int pbs_create(const pbs_mesh_desc *d, pbs_handle **out) {
     CKC(cudaEventCreateWithFlags(&h->ev_chunk[0], cudaEventDisableTiming));
     CKC(cudaEventCreateWithFlags(&h->ev_chunk[1], cudaEventDisableTiming));
     CKC(cudaMallocHost((void **)&h->h_active, 2 * sizeof(int)));
-    CKC(cudaMallocHost((void **)&h->h_ctl, B * sizeof(InstCtl)));
-    std::memset(h->h_ctl, 0, B * sizeof(InstCtl));
+    CKC(cudaMallocHost((void **)&h->h_ctl, (B + 1) * sizeof(InstCtl)));
+    std::memset(h->h_ctl, 0, (B + 1) * sizeof(InstCtl));
     CKC(h->tets.alloc(Tp)); CKC(h->tslot.alloc(Tp)); CKC(h->row0.alloc(Tp)); CKC(h->row1.alloc(Tp)); CKC(h->row2.alloc(Tp));
     CKC(h->info.alloc(Np)); CKC(h->inc_ptr.alloc(Np + 1)); CKC(h->inc.alloc(4 * (size_t)T));
     CKC(h->tblk_inst.alloc(h->n_tblk)); CKC(h->nblk_inst.alloc(h->n_nblk));
@@ -684,10 +683,11 @@ int pbs_create(const pbs_mesh_desc *d, pbs_handle **out) {
     CKC(h->tf.alloc(std::max(12 * (size_t)Tp, 16 * (size_t)T))); CKC(h->hd.alloc(std::max(12 * (size_t)Tp, 16 * (size_t)T)));
     CKC(h->staging.alloc(3 * (size_t)N)); CKC(h->staging2.alloc(12 * (size_t)Tp)); CKC(h->staging_ids.alloc(N));
     CKC(h->tpart.alloc(h->n_tblk)); CKC(h->npart.alloc(h->n_nblk)); CKC(h->npartf.alloc(8 * (size_t)h->n_nblk));
-    CKC(h->ctl.alloc(B)); CKC(h->ctl2.alloc(B)); CKC(h->tcount.alloc(B)); CKC(h->active.alloc(4));
+    CKC(h->ctl.alloc(B + 1)); CKC(h->ctl2.alloc(B)); CKC(h->tcount.alloc(B));
+    h->active = reinterpret_cast<int *>(h->ctl.p + B);
     CKC(cudaMemsetAsync(h->ctl2.p, 0, sizeof(InstCtl) * B, h->stream));
     CKC(cudaMemsetAsync(h->tcount.p, 0, sizeof(unsigned int) * B, h->stream));
-    CKC(cudaMemsetAsync(h->active.p, 0, 4 * sizeof(int), h->stream));
+    CKC(cudaMemsetAsync(h->active, 0, 4 * sizeof(int), h->stream));
     CKC(h->qrows.alloc(4 * (size_t)T)); CKC(h->rslot.alloc(12 * (size_t)T));
     h->qrow0 = h->qrows.p;
     h->qrow1 = h->qrows.p + (size_t)T;
@@ -989,10 +989,10 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     DevState st = h->state();
     CK(cudaEventRecord(h->ev_start, s));
     if (ext) CK(cudaMemcpyAsync(h->staging.p, ext, sizeof(float) * 3 * (size_t)h->N, cudaMemcpyHostToDevice, s));
-    CK(cudaMemsetAsync(h->active.p, 0, 4 * sizeof(int), s));
+    CK(cudaMemsetAsync(h->active, 0, 4 * sizeof(int), s));
     if (h->test_wait_error) {
         h->test_wait_error = false;
-        CK(cudaMemsetAsync(h->active.p + 1, 1, sizeof(int), s));
+        CK(cudaMemsetAsync(h->active + 1, 1, sizeof(int), s));
     }
     CK(launch_init_ctl(s, h->B, h->dparams, st));
     CK(launch_prologue(s, m, h->dparams, st, ext ? h->staging.p : nullptr, h->pad2user.p));
@@ -1019,15 +1019,14 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     if (frame) {
         rc = launch_frame_step(h, h->dparams, h->dparams.pass_cap, auto_frame);
         if (rc != PBS_OK) return rc;
-        CK(cudaMemcpyAsync(h->h_active + 1, h->active.p + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
     } else if (h->graph_loop) {
         CK(cudaGraphLaunch(h->graph, s));
-        CK(cudaMemcpyAsync(h->h_active, h->active.p + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(h->h_active, h->active + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
     }
     for (int j = 0; j < max_chunks; ++j) {
         ++launched;
         CK(cudaGraphLaunch(h->graph, s));
-        CK(cudaMemcpyAsync(h->h_active + (j & 1), h->active.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(h->h_active + (j & 1), h->active, sizeof(int), cudaMemcpyDeviceToHost, s));
         CK(cudaEventRecord(h->ev_chunk[j & 1], s));
         if (j >= 1) {
             CK(cudaEventSynchronize(h->ev_chunk[(j - 1) & 1]));
@@ -1036,7 +1035,7 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     }
     CK(launch_from_increment(s, m, h->dparams, st));
     CK(launch_epilogue(s, m, h->dparams, st, h->pad2user.p));
-    CK(cudaMemcpyAsync(h->h_ctl, h->ctl.p, sizeof(InstCtl) * h->B, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(h->h_ctl, h->ctl.p, sizeof(InstCtl) * h->B + 4 * sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaEventRecord(h->ev_end, s));
     CK(cudaMemsetAsync(h->ext.p, 0, sizeof(float4) * h->Np, s));  // fvm.cpp:188 resetExternalForce
     CK(cudaStreamSynchronize(s));
@@ -1044,7 +1043,7 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     cudaEventElapsedTime(&ms, h->ev_start, h->ev_end);
     h->last_ms = ms;
     if (!frame && h->graph_loop) launched = h->h_active[0];
-    const bool gave_up = frame && h->h_active[1] != 0;
+    const bool gave_up = frame && reinterpret_cast<const int *>(h->h_ctl + h->B)[1] != 0;
     pbs_stats S{};
     S.status = PBS_OK;
     for (int b = 0; b < h->B; ++b) {
@@ -1169,7 +1168,7 @@ int pbs_warm_start_features(pbs_handle *h, const float *ext, float *features, fl
     DevMesh m = h->mesh();
     DevState st = h->state();
     if (ext) CK(cudaMemcpyAsync(h->staging.p, ext, sizeof(float) * 3 * (size_t)h->N, cudaMemcpyHostToDevice, s));
-    CK(cudaMemsetAsync(h->active.p, 0, 4 * sizeof(int), s));
+    CK(cudaMemsetAsync(h->active, 0, 4 * sizeof(int), s));
     CK(launch_init_ctl(s, h->B, h->dparams, st));
     CK(launch_prologue(s, m, h->dparams, st, ext ? h->staging.p : nullptr, h->pad2user.p));
     DevBuf<float> out;
@@ -1232,7 +1231,7 @@ static int time_passes(pbs_handle *h, int passes, double *tet_ms, double *node_m
     DevState st = h->state();
     std::vector<cudaEvent_t> ev(2 * passes + 1, nullptr);
     for (auto &e : ev) CK(cudaEventCreate(&e));
-    cudaError_t e = cudaMemsetAsync(h->active.p, 0, 4 * sizeof(int), s);
+    cudaError_t e = cudaMemsetAsync(h->active, 0, 4 * sizeof(int), s);
     if (e == cudaSuccess) e = launch_init_ctl(s, h->B, p, st);
     if (e == cudaSuccess) e = launch_prologue(s, m, p, st, nullptr, h->pad2user.p);
     if (e == cudaSuccess) e = launch_guess_check(s, m, p, st);
@@ -1289,7 +1288,7 @@ static int time_frame(pbs_handle *h, int passes, double *pass_ms) {
     DevState st = h->state();
     cudaEvent_t ev[2] = {nullptr, nullptr};
     for (auto &e : ev) CK(cudaEventCreate(&e));
-    cudaError_t e = cudaMemsetAsync(h->active.p, 0, 4 * sizeof(int), s);
+    cudaError_t e = cudaMemsetAsync(h->active, 0, 4 * sizeof(int), s);
     if (e == cudaSuccess) e = launch_init_ctl(s, h->B, p, st);
     if (e == cudaSuccess) e = launch_prologue(s, m, p, st, nullptr, h->pad2user.p);
     if (e == cudaSuccess) e = launch_guess_check(s, m, p, st);
@@ -1308,7 +1307,7 @@ static int time_frame(pbs_handle *h, int passes, double *pass_ms) {
     InstCtl c;
     int gave_up = 0;
     CK(cudaMemcpy(&c, h->ctl.p, sizeof(InstCtl), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(&gave_up, h->active.p + 1, sizeof(int), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(&gave_up, h->active + 1, sizeof(int), cudaMemcpyDeviceToHost));
     if (frame_done(h, passes, gave_up) != PBS_OK) c.status = PBS_E_DEVICE_TIMEOUT;
     if (c.status != PBS_OK || c.passes < passes) {
         pbs_stats S{};
