@@ -563,7 +563,7 @@ int pbs_mlp_create(pbs_mlp **out, const float *theta, unsigned long long seed) {
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess || prop.major != 10 || prop.minor != 3) return PBS_E_NO_DEVICE;
     pbs_mlp *t = new pbs_mlp();
-    t->sms = prop.multiProcessorCount;
+    t->sms = pbs::context_sms(prop);
     std::vector<float> th(NPARAM, 0.f);
     if (theta) {
         std::memcpy(th.data(), theta, sizeof(float) * NPARAM);

@@ -1,5 +1,6 @@
 // Host side of the C ABI (include/phybs.h): mesh packing, device memory,
 // the graph-captured pass loop and parity/debug entry points.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -126,7 +127,8 @@ struct pbs_handle {
     bool ws_enabled = false;
     int ws_base = 0;  // 0: corrections to the plain guess, 1: to the extrapolation u0 + 2 d1 - d2
     bool guess_pending = false;  // parity 1 holds a caller guess for the next step
-    int sms = 148;
+    int sms = 148;      // the device's: what layouts are chosen by
+    int ctx_sms = 148;  // the context's: what cooperative launches may fill
     DevBuf<float> tf, hd, staging, staging2;
     int last_fp64_svd = 0;  // tets of the last pbs_eval_tets whose stretch stress took the FP64 SVD
     // boundary surface for picking and drag forces: faces and rings in padded
@@ -151,6 +153,7 @@ struct pbs_handle {
     DevBuf<CgState> cg_state;   // of the solves of a step
     DevBuf<unsigned> cg_ctl;    // [0] the last tag of the exchanged words, [1] a wait gave up
     CgState *h_cg = nullptr;    // pinned, CG_SOLVES of them, and the two control words
+    bool test_refuse_frame = false;  // TEST_REFUSE_FRAME
     bool test_wait_error = false;  // TEST_WAIT_ERROR: the next solve or step finds its wait flag set
     DevBuf<double2> tpart;
     DevBuf<double> npart;
@@ -219,7 +222,7 @@ struct pbs_handle {
         m.l2_bytes = l2_window;
         m.l2_hit = l2_hit;
         m.pptr = pptr.p;
-        m.stream_grid = stream_grid(m, material, dparams.incremental != 0, sms);
+        m.stream_grid = stream_grid(m, material, dparams.incremental != 0, ctx_sms);
         return m;
     }
     DevState state() const {
@@ -415,6 +418,24 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
     return PBS_OK;
 }
 
+int pbs::context_sms(const cudaDeviceProp &prop) {
+    // (through the runtime: the library does not link the driver's)
+    void *get = nullptr, *current = nullptr;
+    cudaDriverEntryPointQueryResult st;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetDevResource", &get, 12040, cudaEnableDefault, &st) != cudaSuccess ||
+        cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &current, 4000, cudaEnableDefault, &st) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return prop.multiProcessorCount;
+    }
+    CUcontext ctx = nullptr;
+    CUdevResource res = {};
+    if (!get || !current || reinterpret_cast<decltype(&cuCtxGetCurrent)>(current)(&ctx) != CUDA_SUCCESS || !ctx ||
+        reinterpret_cast<decltype(&cuCtxGetDevResource)>(get)(ctx, &res, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS ||
+        res.sm.smCount == 0)
+        return prop.multiProcessorCount;
+    return std::min((int)res.sm.smCount, prop.multiProcessorCount);
+}
+
 static void to_dev_params(const pbs_step_params &p, DevParams &d) {
     d.h = p.h;
     d.h2inv = 1.0f / (p.h * p.h);
@@ -561,6 +582,7 @@ int pbs_create(const pbs_mesh_desc *d, pbs_handle **out) {
     if (!h) return PBS_E_OUT_OF_MEMORY;
     h->device = dev;
     h->sms = prop.multiProcessorCount;
+    h->ctx_sms = context_sms(prop);
     h->N = N; h->T = T; h->B = B;
     h->density = d->density; h->gravity = d->gravity;
     pbs_default_params(&h->params);
@@ -903,7 +925,7 @@ static DevMesh frame_mesh(pbs_handle *h) {
 static const FramePlan &handle_frame_plan(pbs_handle *h) {
     if (!h->plan_valid) {
         h->fplan = frame_plan(frame_mesh(h), h->material,
-                              h->material == PBS_MATERIAL_NEOHOOKEAN && h->dparams.incremental, h->sms);
+                              h->material == PBS_MATERIAL_NEOHOOKEAN && h->dparams.incremental, h->ctx_sms);
         h->plan_valid = true;
     }
     return h->fplan;
@@ -914,8 +936,10 @@ static bool frame_applies(pbs_handle *h) { return h->B == 1 && handle_frame_plan
 
 // Enqueues one frame-kernel launch of at most max_passes passes with params p;
 // frame_done must follow once the launch has ended.  PBS_E_INVALID_ARG when
-// the frame kernel does not apply to the handle's layout.
-static int launch_frame_step(pbs_handle *h, const DevParams &p, int max_passes, bool count_void) {
+// the frame kernel does not apply to the handle's layout.  *refused: the launch
+// was refused because its CTAs cannot be resident together; nothing ran.
+static int launch_frame_step(pbs_handle *h, const DevParams &p, int max_passes, bool count_void, bool *refused) {
+    *refused = false;
     const FramePlan &plan = handle_frame_plan(h);
     if (plan.grid <= 0) return PBS_E_INVALID_ARG;
     cudaStream_t s = h->stream;
@@ -951,7 +975,11 @@ static int launch_frame_step(pbs_handle *h, const DevParams &p, int max_passes, 
     fx.max_passes = max_passes;
     fx.count_void = count_void;
     h->frame_clean = false;
-    CK(launch_frame(s, frame_mesh(h), p, h->state(), h->material, fx, plan));
+    const cudaError_t e = h->test_refuse_frame ? cudaErrorCooperativeLaunchTooLarge
+                                               : launch_frame(s, frame_mesh(h), p, h->state(), h->material, fx, plan);
+    *refused = e == cudaErrorCooperativeLaunchTooLarge;
+    if (*refused) (void)cudaGetLastError();
+    CK(e);
     return PBS_OK;
 }
 
@@ -979,7 +1007,7 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     LargeStep large;
     if (auto_frame) {
         const FramePlan &plan = handle_frame_plan(h);
-        if ((plan.per_sm > 1 || 2 * plan.grid > h->sms) && large.enter(h->device) >= 2) auto_frame = false;
+        if ((plan.per_sm > 1 || 2 * plan.grid > h->ctx_sms) && large.enter(h->device) >= 2) auto_frame = false;
     }
     frame |= auto_frame;
     int rc = frame ? PBS_OK : ensure_graph(h);
@@ -1014,11 +1042,19 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     // idles on the poll (body j may then find every instance done).  The frame
     // engine: one launch runs every pass of the step (its pass cap ends it at
     // the latest).
+    if (frame) {
+        bool refused = false;
+        rc = launch_frame_step(h, h->dparams, h->dparams.pass_cap, auto_frame, &refused);
+        if (refused && auto_frame) {  // this step's own choice: the pass kernels run it as well
+            frame = auto_frame = false;
+            rc = ensure_graph(h);
+        }
+        if (rc != PBS_OK) return rc;
+    }
     const int max_chunks = frame || h->graph_loop ? 0 : max_runs(h);
     int launched = 0;
     if (frame) {
-        rc = launch_frame_step(h, h->dparams, h->dparams.pass_cap, auto_frame);
-        if (rc != PBS_OK) return rc;
+        // (enqueued)
     } else if (h->graph_loop) {
         CK(cudaGraphLaunch(h->graph, s));
         CK(cudaMemcpyAsync(h->h_active, h->active + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1201,6 +1237,7 @@ int pbs_test_hook(pbs_handle *h, int what, int value) {
     switch (what) {
         case TEST_WAIT_ERROR: h->test_wait_error = value != 0; return PBS_OK;
         case TEST_FAIL_ALLOC: test_fail_alloc = value; return PBS_OK;
+        case TEST_REFUSE_FRAME: h->test_refuse_frame = value != 0; return PBS_OK;
         case TEST_LARGE_STEPS: large_steps[h->device & 63] += value; return PBS_OK;
         default: return PBS_E_INVALID_ARG;
     }
@@ -1296,7 +1333,8 @@ static int time_frame(pbs_handle *h, int passes, double *pass_ms) {
     if (e == cudaSuccess) e = launch_to_increment(s, m, p, st);
     if (e == cudaSuccess) e = cudaEventRecord(ev[0], s);
     int rc = PBS_OK;
-    if (e == cudaSuccess) rc = launch_frame_step(h, p, passes, false);
+    bool refused = false;
+    if (e == cudaSuccess) rc = launch_frame_step(h, p, passes, false, &refused);
     if (e == cudaSuccess && rc == PBS_OK) e = cudaEventRecord(ev[1], s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     float ms = 0.f;
@@ -1633,7 +1671,7 @@ static int ensure_bsr(pbs_handle *h) {
     const int n = (int)order.size();
     // one CTA a SM, but no fewer than CG_MIN_ROWS rows each: more CTAs shorten
     // the row loops, fewer the sums every CTA waits for
-    const int G = std::max(1, std::min(h->sms, (n + CG_MIN_ROWS - 1) / CG_MIN_ROWS));
+    const int G = std::max(1, std::min(h->ctx_sms, (n + CG_MIN_ROWS - 1) / CG_MIN_ROWS));
     std::vector<int> cta_slice(G + 1, 0), cta_rows(G), cta_halo(G + 1, 0), cta_send(G + 1, 0);
     std::vector<int> srow, rlen, soff(1, 0), soff_local, halo, send;
     std::vector<int> place_of(np, -1), owner(np, -1), stamp(np, -1), lidx(np, 0), key;

@@ -173,12 +173,18 @@ inline double residual_ratio(const InstCtl &c) {
     return c.g0 > 0.0 ? __builtin_sqrt(c.r2) / c.g0 : 0.0;
 }
 
+// SMs that a kernel launched from the calling thread's current context can
+// have: the device's, or a green context's share of them.  The grids of
+// cooperative launches are sized by it.
+int context_sms(const cudaDeviceProp &prop);
+
 // What pbs_test_hook presets, so that the tests reach states that only a fault
 // elsewhere or another device brings about.
 enum TestHook : int {
     TEST_WAIT_ERROR = 0,  // the next solve or step finds its flag of a wait that gave up set
     TEST_FAIL_ALLOC = 1,  // the value-th device allocation of this thread from now fails
     TEST_LARGE_STEPS = 2,  // value more large default steps count as running
+    TEST_REFUSE_FRAME = 3,  // the frame kernel's launches are refused (value 0: no more)
 };
 
 struct DevMesh {

@@ -7,6 +7,8 @@ kernels' (set_pass_engine("graph") on the same automatic chunks) bit for bit:
 the residual stop is off and the regrouped energy sums do not flip a
 line-search test on these meshes.
 """
+import os
+
 import numpy as np
 import pytest
 
@@ -96,6 +98,108 @@ def test_default_step_beside_others():
         assert a.step_engine() == "frame"  # nothing is left counted
         a.close()
         b.close()
+
+
+TEST_REFUSE_FRAME = 3  # pbs_test_hook
+
+
+def test_refused_frame_kernel_leaves_the_pass_kernels():
+    """A default step whose frame kernel cannot be resident after all runs the
+    pass kernels; one that chose the frame engine reports the refusal."""
+    p = make_params("gpu_reference", h=1 / 30, max_iters=24)
+    a, b = (DescentSolver(_box(8, 8, 12), params=p) for _ in range(2))
+    for f in range(3):
+        L.lib().pbs_test_hook(a._h, TEST_REFUSE_FRAME, int(f == 1))
+        a.step()
+        b.step()
+        assert (a.step_engine(), b.step_engine()) == ("graph" if f == 1 else "frame", "frame")
+        assert np.array_equal(a.positions(), b.positions()) and a.stats()["energy"] == b.stats()["energy"]
+    a.set_pass_engine("frame")
+    L.lib().pbs_test_hook(a._h, TEST_REFUSE_FRAME, 1)
+    with pytest.raises(L.PhybsError):
+        a.step()
+    a.close()
+    b.close()
+
+
+IN_GREEN_CONTEXT = """
+import ctypes as C, sys
+cu = C.CDLL("libcuda.so.1")
+def ok(rc):
+    if rc:
+        print("unavailable", rc)
+        sys.exit(0)
+dev, n = C.c_int(), C.c_uint(1)
+full, part, rest = (C.create_string_buffer(144) for _ in range(3))  # CUdevResource
+desc, green, ctx = C.c_void_p(), C.c_void_p(), C.c_void_p()
+ok(cu.cuInit(0)); ok(cu.cuDeviceGet(C.byref(dev), 0))
+ok(cu.cuDeviceGetDevResource(dev, full, 1))                                 # CU_DEV_RESOURCE_TYPE_SM
+ok(cu.cuDevSmResourceSplitByCount(part, C.byref(n), full, rest, 0, 32))
+ok(cu.cuDevResourceGenerateDesc(C.byref(desc), part, 1))
+ok(cu.cuGreenCtxCreate(C.byref(green), desc, dev, 1))                       # CU_GREEN_CTX_DEFAULT_STREAM
+ok(cu.cuCtxFromGreenCtx(C.byref(ctx), green)); ok(cu.cuCtxSetCurrent(ctx))
+sms = int.from_bytes(part.raw[96:100], "little")
+import numpy as np
+from phybs_gb300 import meshes as M
+from phybs_gb300.solver import DescentSolver, make_params
+from phybs_gb300.warmstart import MLPTrainer
+p = make_params("gpu_reference", h=1 / 30, max_iters=24)
+out = {"sms": sms}
+for name, n in (("small", (5, 4, 6)), ("large", (20, 20, 30))):
+    m = M.box_mesh(*n, edge=0.25 / max(n[:2]), jitter=0.1, seed=2, young=1e5, pin="bottom")
+    s = DescentSolver(m, params=p)
+    s.step()
+    out[name] = s.positions()
+    out[name + "_engine"] = s.step_engine()
+    s.backward_euler_step()
+    out[name + "_be"] = s.positions()
+    s.pd_step()
+    out[name + "_pd"] = s.positions()
+    s.close()
+x = np.random.default_rng(0).standard_normal((9000, 24)).astype(np.float32)
+t = MLPTrainer(seed=3)
+t.set_data(x, np.tanh(x[:, :3]))
+out["losses"] = t.train(4, batch=4096, seed=1)
+t.close()
+np.savez(sys.argv[1], **out)
+print("done", sms)
+"""
+
+
+def test_in_a_context_with_fewer_sms(tmp_path):
+    """Every default path in a green context of some of the SMs: grids fit it
+    (the frame kernel where it does, else the pass kernels), and the results are
+    those of the whole device: the descent's bit for bit, the solves' and the
+    training's to the rounding of sums over another number of CTAs."""
+    import subprocess
+    import sys as _sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    f = str(tmp_path / "green.npz")
+    r = subprocess.run([_sys.executable, "-c", IN_GREEN_CONTEXT, f], cwd=root, capture_output=True, text=True,
+                       timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+    if r.stdout.startswith("unavailable"):
+        pytest.skip("no green context here: " + r.stdout)
+    g = np.load(f)
+    assert 0 < g["sms"] < 152
+    assert (str(g["small_engine"]), str(g["large_engine"])) == ("frame", "graph")
+    p = make_params("gpu_reference", h=1 / 30, max_iters=24)
+    for name, n in (("small", (5, 4, 6)), ("large", (20, 20, 30))):
+        m = M.box_mesh(*n, edge=0.25 / max(n[:2]), jitter=0.1, seed=2, young=1e5, pin="bottom")
+        s = DescentSolver(m, params=p)
+        s.step()
+        assert np.array_equal(s.positions(), g[name])
+        s.backward_euler_step()
+        assert np.abs(s.positions() - g[name + "_be"]).max() <= 1e-5 * m.bbox_diagonal()
+        s.pd_step()
+        assert np.abs(s.positions() - g[name + "_pd"]).max() <= 1e-5 * m.bbox_diagonal()
+        s.close()
+    from phybs_gb300.warmstart import MLPTrainer
+    x = np.random.default_rng(0).standard_normal((9000, 24)).astype(np.float32)
+    t = MLPTrainer(seed=3)
+    t.set_data(x, np.tanh(x[:, :3]))
+    assert np.abs(t.train(4, batch=4096, seed=1) / g["losses"] - 1).max() <= 1e-5
+    t.close()
 
 
 @pytest.mark.parametrize("threads,tets", [(2, (9, 8, 13)), (8, (2, 1, 13)), (6, (12, 12, 20)), (4, (20, 20, 30)),
