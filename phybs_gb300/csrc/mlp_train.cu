@@ -458,6 +458,7 @@ struct pbs_mlp {
     int n = 0, cap_part = 0, cap_io = 0, cap_losses = 0, step = 0;
     unsigned arrivals = 0;  // the barrier's count after the launches so far
     int launch_steps = TRAIN_STEPS;  // steps of a launch at most
+    bool refuse_launch = false;      // (tests) the next launch fails
 };
 
 #define MCK(x)                                                                               \
@@ -519,8 +520,8 @@ static int run_train(pbs_mlp *t, const float *X, const float *Y, const float *W,
     a.lr = lr;
     a.b1 = 0.9f; a.b2 = 0.999f; a.eps = 1e-8f;
     for (int s = 0; s < steps && a.update; ++s) {
-        t->step += 1;
-        a.c[s] = make_float2(1.f - std::pow(a.b1, (float)t->step), 1.f - std::pow(a.b2, (float)t->step));
+        const float n = (float)(t->step + 1 + s);
+        a.c[s] = make_float2(1.f - std::pow(a.b1, n), 1.f - std::pow(a.b2, n));
     }
     MCK(cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem)));
     cudaLaunchAttribute at[1];
@@ -533,7 +534,12 @@ static int run_train(pbs_mlp *t, const float *X, const float *Y, const float *W,
     cfg.stream = t->stream;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    if (t->refuse_launch) {
+        t->refuse_launch = false;
+        return PBS_E_CUDA;
+    }
     MCK(cudaLaunchKernelEx(&cfg, k_mlp_train, a));
+    if (a.update) t->step += steps;  // (a launch that failed took no step)
     t->arrivals += 2u * (unsigned)steps * (unsigned)ctas;
     return PBS_OK;
 }
@@ -713,6 +719,13 @@ int pbs_mlp_train(pbs_mlp *t, int steps, int batch, float lr, unsigned long long
 int pbs_mlp_test_launch_steps(pbs_mlp *t, int steps) {
     if (!t || steps < 1 || steps > TRAIN_STEPS) return PBS_E_INVALID_ARG;
     t->launch_steps = steps;
+    return PBS_OK;
+}
+
+// For the tests only: the next launch fails.
+int pbs_mlp_test_refuse(pbs_mlp *t) {
+    if (!t) return PBS_E_INVALID_ARG;
+    t->refuse_launch = true;
     return PBS_OK;
 }
 

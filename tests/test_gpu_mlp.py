@@ -186,3 +186,21 @@ def test_an_epoch_takes_every_row_once(n, batch):
     assert np.array_equal(t.params[theta != 0], theta[theta != 0])
     assert abs(losses.astype(np.float64).mean() - full) <= 1e-5 * full
     t.close()
+
+
+def test_failed_launch_takes_no_adam_step():
+    """Training after a launch that failed is training from where it was: the
+    step count of Adam's bias correction goes on from the steps taken."""
+    X, Y = _data(500, 3)
+    out = []
+    for fail in (False, True):
+        t = MLPTrainer(seed=4)
+        t.set_data(X, Y)
+        t.train(3, batch=100, seed=0)
+        if fail:
+            assert L.lib().pbs_mlp_test_refuse(t._t) == 0
+            with pytest.raises(L.PhybsError):
+                t.train(4, batch=100, seed=1)
+        out.append((t.train(2, batch=100, seed=2), t.params))
+        t.close()
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
