@@ -304,7 +304,10 @@ typedef struct pbs_tune_result {
  * the persistent double-buffered kernel), times
  * `passes` passes of it from the current state (then the node kernel with 1
  * and 2 nodes per thread) with
- * CUDA events and keeps the fastest.  Forces stay deterministic for a given
+ * CUDA events and keeps the fastest.  A handle that chose no engine and whose
+ * default steps would run the frame kernel (pbs_set_pass_engine) keeps that,
+ * with its automatic chunks, when it is faster than every shape; out then
+ * describes the fastest shape of the pass kernels all the same.  Forces stay deterministic for a given
  * shape; another shape changes the order the corner forces are summed in, so
  * results can differ in the last bits.  Call between steps (it recaptures the
  * step graph).  No counterpart in the reference, whose launch shapes are

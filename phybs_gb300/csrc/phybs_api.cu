@@ -931,6 +931,12 @@ static const FramePlan &handle_frame_plan(pbs_handle *h) {
     return h->fplan;
 }
 
+// A handle whose caller chose neither an engine nor a shape, and whose chunks
+// all have resident CTAs.
+static bool auto_frame_applies(pbs_handle *h) {
+    return h->engine_auto && h->shape_auto && h->share_sums && !h->joined && handle_frame_plan(h).resident;
+}
+
 // The frame engine as the caller selects it: one instance.
 static bool frame_applies(pbs_handle *h) { return h->B == 1 && handle_frame_plan(h).grid > 0; }
 
@@ -1003,7 +1009,7 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     // the caller chose neither an engine nor a shape: the frame kernel where
     // every chunk has a resident CTA of its own (auto_chunk_limits), which
     // spares a pass its two launches and its trips to memory
-    bool auto_frame = !frame && h->engine_auto && h->shape_auto && h->share_sums && !h->joined && handle_frame_plan(h).resident;
+    bool auto_frame = !frame && auto_frame_applies(h);
     LargeStep large;
     if (auto_frame) {
         const FramePlan &plan = handle_frame_plan(h);
@@ -1342,12 +1348,15 @@ static int time_frame(pbs_handle *h, int passes, double *pass_ms) {
     for (auto &x : ev) cudaEventDestroy(x);
     CK(e);
     if (rc != PBS_OK) return rc;
-    InstCtl c;
+    std::vector<InstCtl> ctl(h->B);
     int gave_up = 0;
-    CK(cudaMemcpy(&c, h->ctl.p, sizeof(InstCtl), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(ctl.data(), h->ctl.p, sizeof(InstCtl) * h->B, cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(&gave_up, h->active + 1, sizeof(int), cudaMemcpyDeviceToHost));
-    if (frame_done(h, passes, gave_up) != PBS_OK) c.status = PBS_E_DEVICE_TIMEOUT;
-    if (c.status != PBS_OK || c.passes < passes) {
+    const bool ok = frame_done(h, passes, gave_up) == PBS_OK;
+    for (InstCtl &c : ctl) {
+        if (c.tet_end == c.tet_begin) continue;
+        if (!ok) c.status = PBS_E_DEVICE_TIMEOUT;
+        if (c.status == PBS_OK && c.passes >= passes) continue;
         pbs_stats S{};
         S.passes = c.passes; S.iterations = c.k; S.rejections = c.rejections; S.converged = c.converged;
         S.status = c.status; S.alpha = c.alpha; S.rho = c.rho; S.omega = c.omega; S.energy = c.energy;
@@ -1448,7 +1457,18 @@ int pbs_autotune(pbs_handle *h, int passes, pbs_tune_result *out) {
             bi = i;
         }
     }
-    int rc = set_pass_layout(h, shapes[bi][0], shapes[bi][1], shapes[bi][2], shapes[bi][3], nullptr);
+    // the frame kernel on the automatic layout, where a default step would run
+    // it: kept when it beats every shape of the pass kernels
+    int rc = PBS_OK;
+    bool keep_frame = false;
+    if (h->engine_auto) {
+        rc = set_pass_layout(h, 0, 0, 0, 0, nullptr);
+        if (rc != PBS_OK) return rc;
+        double f = 0.0;
+        keep_frame = auto_frame_applies(h) && time_frame(h, passes, &f) == PBS_OK &&
+                     time_frame(h, passes, &f) == PBS_OK && f <= best;
+    }
+    rc = set_pass_layout(h, shapes[bi][0], shapes[bi][1], shapes[bi][2], shapes[bi][3], nullptr);
     if (rc != PBS_OK) return rc;
     // the node kernel: 1 or 2 nodes per thread (independent of the chunk shape)
     double node_ms[2] = {0.0, 0.0};
@@ -1476,7 +1496,7 @@ int pbs_autotune(pbs_handle *h, int passes, pbs_tune_result *out) {
         out->pass_ms = best;
         out->default_pass_ms = first;
     }
-    return PBS_OK;
+    return keep_frame ? set_pass_layout(h, 0, 0, 0, 0, nullptr) : PBS_OK;
 }
 
 int pbs_read_velocities(pbs_handle *h, float *v, float *v_old) {

@@ -73,6 +73,33 @@ def test_step_engine_is_the_one_that_ran():
         s.close()
 
 
+@pytest.mark.parametrize("n", [1, 3])
+def test_autotune_keeps_the_frame_kernel_where_it_is_faster(n):
+    """A tuned handle of a size that the frame kernel steps in half the pass
+    kernels' time goes on running it, with the bits of an untuned one; a chosen
+    engine stays, and a body beyond residence gets a shape."""
+    p = make_params("gpu_reference", h=1 / 30, max_iters=24)
+    m = _pack([_box(12, 12, 20)] * n)
+    a, b = DescentSolver(m, params=p), DescentSolver(m, params=p)
+    r = a.autotune(16)
+    assert r["n_tried"] == 20 and 0 < r["pass_ms"] <= r["default_pass_ms"]
+    for _ in range(2):
+        a.step()
+        b.step()
+        assert a.step_engine() == "frame" and np.array_equal(a.positions(), b.positions())
+    a.set_pass_engine("graph")
+    a.autotune(4)
+    a.step()
+    assert a.step_engine() == "graph"
+    a.close()
+    b.close()
+    s = DescentSolver(_box(34, 33, 46), params=p)
+    s.autotune(4)
+    s.step()
+    assert s.step_engine() == "graph"
+    s.close()
+
+
 TEST_LARGE_STEPS = 2  # pbs_test_hook
 
 
