@@ -49,8 +49,10 @@ __device__ __forceinline__ float4 f4(float x, float y, float z) { return make_fl
 
 // ------------------------------------------------------------ pattern
 // Row i's columns: itself and every node it shares a tet with, ascending.
-// Selected one after the other as the smallest beyond the last: no scratch
-// and no limit on a row's length.
+// Selected one after the other as the smallest beyond the last, without scratch:
+// quadratic in the incident tets, so the rows of nodes with more than
+// BSR_HUB_TETS of them are left to the host, which sorts (a node of 12,000 tets
+// would take one thread seconds).
 __device__ __forceinline__ int next_col(const DevMesh &m, int i, int last) {
     int best = i > last ? i : INT_MAX;
     for (int j = m.inc_ptr[i]; j < m.inc_ptr[i + 1]; ++j) {
@@ -67,13 +69,16 @@ __global__ void k_bsr_count(DevMesh m, int *cnt) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.Np) return;
     int n = 0;
-    for (int c = next_col(m, i, -1); c != INT_MAX; c = next_col(m, i, c)) ++n;
+    if (m.inc_ptr[i + 1] - m.inc_ptr[i] > BSR_HUB_TETS) n = -1;
+    else
+        for (int c = next_col(m, i, -1); c != INT_MAX; c = next_col(m, i, c)) ++n;
     cnt[i] = n;
 }
 
 __global__ void k_bsr_fill(DevMesh m, const int *ptr, int *col) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.Np) return;
+    if (m.inc_ptr[i + 1] - m.inc_ptr[i] > BSR_HUB_TETS) return;
     int k = ptr[i];
     for (int c = next_col(m, i, -1); c != INT_MAX; c = next_col(m, i, c)) col[k++] = c;
 }

@@ -1657,12 +1657,35 @@ static int ensure_bsr(pbs_handle *h) {
     CK(launch_bsr_count(s, h->mesh(), h->bsr_ptr.p + 1));
     CK(cudaMemcpyAsync(ptr.data() + 1, h->bsr_ptr.p + 1, sizeof(int) * np, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    // the rows of nodes with many tets, which the kernels leave out (-1)
+    std::vector<std::vector<int>> hub;  // a node, then its row's columns
+    std::vector<int> hub_of;
+    for (size_t i = 0; i < np; ++i)
+        if (ptr[i + 1] < 0) {
+            hub_of.resize(np, -1);
+            hub_of[i] = (int)hub.size();
+            hub.push_back({(int)i});
+        }
+    if (!hub.empty())
+        for (const int4 &q : h->h_tets_pad)
+            for (int c = 0; c < 4 && q.x >= 0; ++c) {
+                const int r = hub_of[(&q.x)[c]];
+                if (r >= 0) hub[r].insert(hub[r].end(), &q.x, &q.x + 4);
+            }
+    for (auto &r : hub) {
+        std::sort(r.begin() + 1, r.end());
+        r.erase(std::unique(r.begin() + 1, r.end()), r.end());
+    }
+    for (const auto &r : hub) ptr[r[0] + 1] = (int)r.size() - 1;
     for (size_t i = 0; i < np; ++i) ptr[i + 1] += ptr[i];
     const size_t nnzb = (size_t)ptr[np];
     std::vector<int> col(nnzb);
     CK(h->bsr_col.alloc(nnzb));
     CK(cudaMemcpyAsync(h->bsr_ptr.p, ptr.data(), sizeof(int) * (np + 1), cudaMemcpyHostToDevice, s));
     CK(launch_bsr_fill(s, h->mesh(), h->bsr_ptr.p, h->bsr_col.p));
+    for (const auto &r : hub)
+        CK(cudaMemcpyAsync(h->bsr_col.p + ptr[r[0]], r.data() + 1, sizeof(int) * (r.size() - 1), cudaMemcpyHostToDevice,
+                           s));
     CK(cudaMemcpyAsync(col.data(), h->bsr_col.p, sizeof(int) * nnzb, cudaMemcpyDeviceToHost, s));
     // rows: (instance, Morton code) order, on the host meanwhile
     std::vector<std::pair<uint64_t, int>> order;

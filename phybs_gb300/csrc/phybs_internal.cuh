@@ -505,6 +505,7 @@ struct CgPlanView {
     int off_p, off_r, off_q, off_x, off_val, off_col, off_node, off_rlen, off_small, off_dinv;
 };
 constexpr int CG_MIN_ROWS = 128;
+constexpr int BSR_HUB_TETS = 256;  // incident tets of a node whose row's columns the device finds
 constexpr int CG_MAX_SMEM = 225 * 1024;
 constexpr int CG_COPIES = 8;  // places a CTA writes its share of a sum to
 struct CgArgs {

@@ -200,3 +200,41 @@ def test_wait_that_gave_up_is_an_error(integrator):
         assert np.array_equal(a.positions(), b.positions()) and np.array_equal(a.velocities()[0], b.velocities()[0])
     a.close()
     b.close()
+
+
+def _fan(n):
+    """n tets around one edge, its two nodes in all of them."""
+    a = np.linspace(0, 2 * np.pi, n, endpoint=False)
+    rest = np.concatenate([[[0, 0, 0], [0, 0, 1]], np.stack([np.cos(a), np.sin(a), 0.5 + 0.1 * np.cos(3 * a)], 1)])
+    i = np.arange(n)
+    tets = np.stack([np.zeros(n), np.ones(n), 2 + i, 2 + (i + 1) % n], 1).astype(np.int64)
+    tets = M.orient_positive(rest, tets)
+    return M.TetMeshData(rest.astype(np.float32), tets, np.array([0, 1]), 1e5, 0.3)
+
+
+# rows on both sides of the line between the device's columns and the host's (256 incident tets)
+@pytest.mark.parametrize("n", [40, 255, 256, 257, 600])
+def test_rows_of_nodes_with_many_tets(n):
+    m = _fan(n)
+    mu, lam = O.lame(m.young, m.poisson)
+    v0 = (0.1 * np.sin(7 * m.rest[:, [1, 2, 0]])).astype(np.float32)
+    v0[m.pins] = 0.0
+    s = DescentSolver(m, mu=mu, lam=lam)
+    s.write_velocities(v0, v0)
+    xo, vo, _, _ = I.backward_euler_step(s.positions(), v0, m.rest, m.tets, m.pin_mask(), mu, lam)
+    it, res = s.backward_euler_step(tol=1e-6)
+    assert res <= 1e-6
+    assert np.abs(s.positions() - xo).max() / m.bbox_diagonal() < POS_TOL
+    assert np.abs(s.velocities()[0] - vo).max() <= 1e-3 * np.abs(vo).max()
+    s.close()
+
+
+def test_pattern_time_at_a_node_of_many_tets():
+    """The pattern of a node with 6,000 tets: sorted, not selected (36 million
+    tets read one after the other, a second and more, against milliseconds)."""
+    import time
+    s = DescentSolver(_fan(6000))
+    t = time.perf_counter()
+    s.backward_euler_step(max_iters=1, raise_on_cap=False)
+    assert time.perf_counter() - t < 0.5
+    s.close()
