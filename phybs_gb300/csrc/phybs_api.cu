@@ -153,6 +153,8 @@ struct pbs_handle {
     DevBuf<CgState> cg_state;   // of the solves of a step
     DevBuf<unsigned> cg_ctl;    // [0] the last tag of the exchanged words, [1] a wait gave up
     CgState *h_cg = nullptr;    // pinned, CG_SOLVES of them, and the two control words
+    int test_solve_smem = -1;        // TEST_SOLVE_SMEM
+    bool test_solve_col32 = false;   // TEST_SOLVE_COL32
     bool test_refuse_frame = false;  // TEST_REFUSE_FRAME
     bool test_wait_error = false;  // TEST_WAIT_ERROR: the next solve or step finds its wait flag set
     DevBuf<double2> tpart;
@@ -1243,6 +1245,8 @@ int pbs_test_hook(pbs_handle *h, int what, int value) {
     switch (what) {
         case TEST_WAIT_ERROR: h->test_wait_error = value != 0; return PBS_OK;
         case TEST_FAIL_ALLOC: test_fail_alloc = value; return PBS_OK;
+        case TEST_SOLVE_SMEM: h->test_solve_smem = value; return PBS_OK;
+        case TEST_SOLVE_COL32: h->test_solve_col32 = value != 0; return PBS_OK;
         case TEST_REFUSE_FRAME: h->test_refuse_frame = value != 0; return PBS_OK;
         case TEST_LARGE_STEPS: large_steps[h->device & 63] += value; return PBS_OK;
         default: return PBS_E_INVALID_ARG;
@@ -1803,7 +1807,7 @@ static int ensure_bsr(pbs_handle *h) {
     CK(h->cg_plan.alloc(total));
     for (auto &p : part)
         CK(cudaMemcpyAsync(h->cg_plan.p + p.at, p.v->data(), sizeof(int) * p.v->size(), cudaMemcpyHostToDevice, s));
-    const bool col32 = max_local > 0xffff;
+    const bool col32 = max_local > 0xffff || h->test_solve_col32;
     std::vector<uint16_t> lcol16;
     if (!col32) lcol16.assign(lcol.begin(), lcol.end());
     const void *src = col32 ? (const void *)lcol.data() : (const void *)lcol16.data();
@@ -1821,6 +1825,7 @@ static int ensure_bsr(pbs_handle *h) {
     v.cta_send = base + part[8].at; v.send = base + part[9].at;
     v.scol = h->cg_col.p;
     v.col32 = col32;
+    const size_t budget = h->test_solve_smem >= 0 ? h->test_solve_smem : CG_MAX_SMEM;
     for (int kind = 0; kind < 2; ++kind) {
         // what fits shared memory, the most often read first
         CgPlanView &w = h->cgp[kind];
@@ -1828,7 +1833,7 @@ static int ensure_bsr(pbs_handle *h) {
         w.smem = 0;
         auto place = [&](size_t bytes) {
             bytes = (bytes + 127) / 128 * 128;
-            if (w.smem + bytes > (size_t)CG_MAX_SMEM) return -1;
+            if (w.smem + bytes > budget) return -1;
             const int at = w.smem;
             w.smem += (int)bytes;
             return at;
@@ -1842,7 +1847,7 @@ static int ensure_bsr(pbs_handle *h) {
         w.off_r = place(sizeof(float4) * max_rows);
         w.off_val = w.off_col = -1;
         const size_t vb = (size_t)max_entries * 128 * nv, cb = (size_t)max_entries * 32 * (col32 ? 4 : 2);
-        if (w.smem + vb + cb + 256 <= (size_t)CG_MAX_SMEM) {
+        if (w.smem + vb + cb + 256 <= budget) {
             w.off_val = place(vb);
             w.off_col = place(cb);
         }

@@ -185,6 +185,8 @@ enum TestHook : int {
     TEST_FAIL_ALLOC = 1,  // the value-th device allocation of this thread from now fails
     TEST_LARGE_STEPS = 2,  // value more large default steps count as running
     TEST_REFUSE_FRAME = 3,  // the frame kernel's launches are refused (value 0: no more)
+    TEST_SOLVE_SMEM = 4,    // the solves keep at most value bytes in shared memory (-1: as many as fit)
+    TEST_SOLVE_COL32 = 5,   // the solves' columns have 32 bits (both: before the handle's first solve)
 };
 
 struct DevMesh {

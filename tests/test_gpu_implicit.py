@@ -238,3 +238,34 @@ def test_pattern_time_at_a_node_of_many_tets():
     s.backward_euler_step(max_iters=1, raise_on_cap=False)
     assert time.perf_counter() - t < 0.5
     s.close()
+
+
+TEST_SOLVE_SMEM, TEST_SOLVE_COL32 = 4, 5  # pbs_test_hook
+
+
+@pytest.mark.parametrize("integrator", ["be", "pd"])
+@pytest.mark.parametrize("split,nx,ny,nz", [(5, 1, 1, 2), (5, 3, 3, 7), (6, 10, 6, 6), (5, 9, 14, 19)])
+def test_solve_with_vectors_in_global_memory(integrator, split, nx, ny, nz):
+    """What does not fit a CTA's shared memory on large meshes (the solution from
+    0.3 million nodes, then the residual, q, the direction) stays in global
+    memory, and columns beyond 65,535 take 32 bits: here under a smaller budget,
+    bit for bit as with everything in shared memory."""
+    m, x0, v0 = _moving(split, nx, ny, nz)
+    mu, lam = O.lame(m.young, m.poisson)
+
+    def solve(smem, wide):
+        s = DescentSolver(m, positions=x0, mu=mu, lam=lam)
+        s.write_velocities(v0, v0)
+        L.lib().pbs_test_hook(s._h, TEST_SOLVE_SMEM, smem)
+        L.lib().pbs_test_hook(s._h, TEST_SOLVE_COL32, wide)
+        its = [s.backward_euler_step(tol=1e-6) if integrator == "be" else s.pd_step() for _ in range(2)]
+        out = its, s.positions(), s.velocities()[0]
+        s.close()
+        return out
+
+    want = solve(-1, 0)
+    # nothing; the rows' records; the direction; q; r; all but the matrix; all but the inverses and x
+    for smem in (0, 1536, 6144, 8192, 10240, 12288, 16384, 65536):
+        for wide in (0, 1):
+            got = solve(smem, wide)
+            assert got[0] == want[0] and np.array_equal(got[1], want[1]) and np.array_equal(got[2], want[2]), (smem, wide)
