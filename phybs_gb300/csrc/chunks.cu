@@ -252,17 +252,21 @@ void build_chunks(int Np, const std::vector<int4> &tets, const std::vector<doubl
 //     machine width, and iterations to a tolerance stop at the same pass
 //     (pieces move one pull in 40 to a residual of 1e-4 by more than 2e-5 of
 //     its velocities);
-//   beyond, the pass kernels: 384 up to 250,000 (203,205, 256 threads: 1372 /
-//     1519, 512 a chunk 1458 / 1606; the frame kernel with 704 a chunk 1291 /
-//     1314, but a group has no pieces of that size), then whole groups on 512
-//     threads (1M tets, us a pass of both kernels: 48.6 / 54.9, 512 a chunk on
-//     256 threads 47.5 / 51.6).
+//   beyond, the pass kernels: 384 with 256 threads up to 1,600 a SM (243,200),
+//     else whole groups with 512 (384 / groups, full, then incremental stress:
+//     160,720 tets 1331 / 1403, 1453 / 1568; 203,205 1309 / 1505, 1444 / 1675;
+//     221,030 1429 / 1482, 1607 / 1670; 234,135 1476 / 1493, 1651 / 1686;
+//     248,540 1514 / 1490, 1690 / 1685; 298,080 and 400,000 equal within 0.5%;
+//     the frame kernel with 704 a chunk took 1291 / 1314 at 203,205, but a group
+//     has no pieces of that size).  1M tets, us a pass of both kernels: 48.6 /
+//     54.9, 512 a chunk on 256 threads 47.5 / 51.6: the groups' one path to a
+//     residual is worth that.
 // The node limit leaves room for meshes with more nodes a tet than a box.
 ChunkLimits auto_chunk_limits(int tets, int sms) {
     int n;
     if (tets <= 4096) n = 128;
     else if (tets <= 2 * 256 * sms) n = 256;
-    else if (tets <= 2 * 342 * sms || (tets > CHUNK_GROUP_TETS * sms && tets <= 250000)) n = 384;
+    else if (tets <= 2 * 342 * sms || (tets > CHUNK_GROUP_TETS * sms && tets <= 1600 * sms)) n = 384;
     else return ChunkLimits{CHUNK_GROUP_TETS, CHUNK_GROUP_NODES};
     return ChunkLimits{n, 32 + n / 2 + n / 16};
 }
