@@ -124,10 +124,9 @@ typedef struct pbs_step_params {
 } pbs_step_params;
 
 typedef struct pbs_stats {
-    int passes;               /* iterations executed, including redone ones (max over instances); the
-                                 graph engine's pass kernels also count a pass that carried the
-                                 state over unchanged because a non-finite residual forced an
-                                 energy check */
+    int passes;               /* iterations executed, including redone ones (max over instances);
+                                 without PBS_ENGINE_FRAME also those that carried the state over
+                                 unchanged because a non-finite residual forced an energy check */
     int iterations;           /* accepted iterations k at exit (max over instances) */
     int rejections;           /* line-search rejections (sum over instances)      */
     int converged;            /* instances that met tol                          */
@@ -137,7 +136,8 @@ typedef struct pbs_stats {
     double energy;            /* instance 0 energy at its last check             */
     double residual_ratio;    /* instance 0 |g_k| / |g_0|                         */
     double device_ms;         /* device time of the last pbs_step (CUDA events)   */
-    int graph_launches;       /* 16-pass bodies the last step ran (0: PBS_ENGINE_FRAME) */
+    int graph_launches;       /* 16-pass bodies the last step's passes fill (0: PBS_ENGINE_FRAME;
+                                 pbs_get_step_engine tells what ran them) */
     int warm_start_used;      /* instances whose step started from the learned guess */
     int guess_fallbacks;      /* RESTART control: instances whose inertial guess inverted a
                                  tet, started from the step's start positions instead */
@@ -323,19 +323,22 @@ int pbs_set_chunk_shape(pbs_handle *h, int threads, int chunk_tets, int chunk_no
 /* Pass engine of pbs_step.  PBS_ENGINE_GRAPH (the default): each pass is a
  * per-tet and a per-node kernel, 16 passes to the body of a captured CUDA
  * graph's loop.  A handle whose caller set neither an engine (this call) nor a
- * chunk shape (pbs_set_chunk_shape, pbs_autotune) runs the frame kernel
- * instead where every chunk has a resident CTA (up to ~155,000 tets; any
- * number of instances), which is faster there; its steps report
- * graph_launches as the 16-pass bodies the passes fill.
+ * chunk shape (pbs_set_chunk_shape, or an outcome of pbs_autotune) runs the
+ * frame kernel instead where every chunk has a resident CTA (up to ~155,000
+ * tets on a whole device; any number of instances), which is faster there,
+ * unless steps of two other handles already run frame kernels of more than half
+ * of the device.  Its results, energies and residuals included, are the same
+ * bits either way, alone and packed; its steps report graph_launches as the
+ * 16-pass bodies the passes fill (pbs_get_step_engine: what ran them).
  * PBS_ENGINE_FRAME: one cooperative launch runs all the passes of a step; its
  * CTAs stay resident for the whole step and hand each other the node words
  * and force sums of a pass as tagged 16-byte words, and every CTA takes the
  * line-search and stop decisions from the same sums.  For one-instance handles whose chunk shape
  * is unstaged (staged 0) with 128 or 256 threads; PBS_E_INVALID_ARG
  * otherwise, and from pbs_step when a later shape or parameter change leaves
- * the handle outside that set.  The instance's energy and residual sums are
- * grouped per CTA instead of per chunk, so results agree with the graph
- * engine's to rounding; they are bit-reproducible run to run.  A wait for
+ * the handle outside that set.  Where the chunks outnumber the resident CTAs
+ * the energy and residual sums are grouped per CTA, and results agree with the
+ * graph engine's to rounding; they are bit-reproducible run to run.  A wait for
  * another CTA's words that runs out (2 s) ends the step with
  * PBS_E_DEVICE_TIMEOUT.
  * pbs_stats.graph_launches is 0 for a frame-engine step.  No counterpart in

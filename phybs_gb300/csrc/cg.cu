@@ -30,7 +30,8 @@
 //
 // Dot products run in double-float on vectors scaled by powers of two (GB300's
 // FP64 pipe took longer for them than memory for the matrix): products exact,
-// sums to about 2^-44.  The scales bring the largest |b| and |D^-1 b| to [1, 2),
+// sums to about 2^-44.  With FP64 sums the outputs' errors against 64 bits were
+// the same to four digits on twenty systems of 300 to 37,000 rows.  The scales bring the largest |b| and |D^-1 b| to [1, 2),
 // so that no square leaves FP32's range.
 #include <climits>
 

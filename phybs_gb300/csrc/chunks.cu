@@ -16,7 +16,7 @@
 // The node kernel adds a node's partials in chunk order.  No atomics touch a
 // force, so results are bit-reproducible run to run, and instances are
 // chunked on their own, so a packed batch gives each instance the bits it gets
-// alone.  Against one thread per tet writing 4 global slots, this moves the
+// alone (the order of the energy and |g|^2 sums: phybs_internal.cuh).  Against one thread per tet writing 4 global slots, this moves the
 // corner forces through shared memory instead of HBM (64 B written and read
 // back per tet per pass) and replaces 4 gathers of 3 node words per tet with
 // one staged read per touched node.

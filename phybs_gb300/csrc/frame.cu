@@ -24,9 +24,10 @@
 // control warp beside the workers, so its sums leave the critical path.
 //
 // The arithmetic of a tet, a chunk's slot sums and a node's update is that of
-// the pass kernels, so the positions are theirs bit for bit; the instance's
-// energy and |g|^2 sums are grouped by CTA instead of by chunk and node block,
-// agree to rounding and are bit-reproducible run to run.
+// the pass kernels, and in the resident layout the order of every sum too
+// (phybs_internal.cuh): positions, decisions and stats are theirs bit for bit.
+// Walking CTAs add the energies of several chunks, so the walking layout's
+// energy and |g|^2 agree with them to rounding (and are bit-reproducible).
 //
 // Two layouts (RES):
 //   resident  every chunk has its own CTA, all of them co-resident; the
@@ -236,10 +237,12 @@ struct FrameOwn {
 // PER_SM: CTAs a SM the registers are budgeted for.  A pass is bound by the
 // dependent chain of one tet, so a mesh that needs fewer CTAs a SM runs the
 // variant with more registers: on 24,500 tets 493 us a 96-pass step at one
-// CTA a SM (no spills), 523 at two, 650 at three.  For the same reason a group
-// of 1,024 tets runs on one CTA of 256 threads (168 registers), four tets a
-// thread: 256 threads at two CTAs a SM have 96 and spill (125,000 tets: 1120 us
-// against 855).
+// CTA a SM (up to 246 registers, no spills), 523 at two (168: 200 bytes stored
+// and 290 loaded with the full stress, 22 and 52 with the incremental, 306 and
+// 408 with the stretch material), 650 at three (128: 440, 262 and 520 stored).
+// For the same reason a group of 1,024 tets runs on one CTA of 256 threads,
+// four tets a thread, with those 168 registers: at two CTAs a SM they have 96
+// and store 608 to 780 bytes (125,000 tets: 1120 us against 855).
 template <int MATERIAL, int THREADS, bool INC, bool RES, int PER_SM>
 __global__ void __launch_bounds__(THREADS + 32, PER_SM)
     k_frame(DevMesh m, DevParams p, DevState st, FrameAux fx) {

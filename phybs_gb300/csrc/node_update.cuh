@@ -1,7 +1,7 @@
 // The per-node update of a descent pass (the Jacobi step with Chebyshev
 // extrapolation, or the line search's restore / save), shared by the node
 // kernel of the graph path (kernels.cu) and the persistent frame kernel
-// (chunks.cu).
+// (frame.cu).
 #pragma once
 #include "../../include/phybs.h"
 #include "pass_math.cuh"

@@ -915,7 +915,6 @@ static int ensure_graph(pbs_handle *h) {
     return PBS_OK;
 }
 
-// How the frame kernel runs the handle's current layout.
 // The mesh as the frame kernel takes it: automatic chunks that the pass kernels
 // run with 512 threads, which it has no variant for, with 256.
 static DevMesh frame_mesh(pbs_handle *h) {
@@ -924,6 +923,7 @@ static DevMesh frame_mesh(pbs_handle *h) {
     return m;
 }
 
+// How the frame kernel runs the handle's current layout.
 static const FramePlan &handle_frame_plan(pbs_handle *h) {
     if (!h->plan_valid) {
         h->fplan = frame_plan(frame_mesh(h), h->material,

@@ -15,7 +15,7 @@ per axis), with the bottom face at its frame --frame position:
 3. With --warm: one warm-started step with the committed model (k_ws_*
    kernels once each, and a whole frame of passes).
 4. With --train-steps N: N Adam steps of the warm-start network on random
-   data (k_mlp_grad, k_mlp_reduce, k_mlp_adam per step).
+   data (k_mlp_train: up to 64 steps a launch).
 
 Prints one JSON line with the CUDA-event times.  A profiler's kernel filter
 and launch skip select the launches (for example `-k regex:k_tchunk -s 8 -c
