@@ -271,7 +271,7 @@ ChunkLimits auto_chunk_limits(int tets, int sms) {
     return ChunkLimits{n, 32 + n / 2 + n / 16};
 }
 
-int auto_team(int tets, int sms) { return tets <= 2 * 342 * sms ? 128 : 256; }
+int auto_team(int tets, int sms) { return tets <= 2 * 342 * sms ? 128 : tets <= 1600 * sms ? 256 : 512; }
 
 // ------------------------------------------------------------ device
 __global__ void k_pass_rows(int T, const int *qperm, const float4 *row0, const float4 *row1, const float4 *row2,
@@ -289,53 +289,99 @@ __global__ void k_pass_rows(int T, const int *qperm, const float4 *row0, const f
 // tet energies, where the chunk is one piece and the team is the CTA's threads.
 // Double-float (e) and FP32 (e^2, a noise scale), in the order that
 // phybs_internal.cuh gives.  Called by every thread, before anything else goes
-// into the slots.
-// TEAMS: the layout has chunks of several pieces or a team that is not the
-// CTA's threads (then by the slots, one team a piece at a time); without it
-// every chunk is one piece and every thread in its team, and the kernel keeps
-// its registers (two bodies of 150,000 tets, 96 passes without a line search:
-// 1460 us, and 1470 when one kernel held both).
-template <int THREADS, bool TEAMS>
+// into the slots.  (Its values are formed here, not carried through the tet
+// loop: registers are short.)
+template <int THREADS>
 __device__ __forceinline__ void chunk_energy(const DevMesh &m, const DevParams &p, const DevState &st, int c, int inst,
-                                             int par, size_t cur, const ChunkView &v, int nt, const float4 *sf,
-                                             DFloat ec) {
+                                             int par, size_t cur, int nt, DFloat ec) {
     __shared__ float2 s_e[THREADS / 32];
     __shared__ float s_e2[THREADS / 32];
-    // (formed here, not carried through the tet loop: registers are short)
     const InstCtl *src = ctl_buf(st, par) + inst;
-    const int pb = src->pblk_begin, n0 = src->node_begin, n1 = src->node_end, per = src->share;
-    const float4 *base = p.incremental ? st.ub : nullptr;
-    const int team = TEAMS ? src->team : THREADS, tid = threadIdx.x & (team - 1), side = threadIdx.x / team;
-    const int p0 = TEAMS ? m.cpiece[c] : pb + c - src->cblk_begin, p1 = TEAMS ? m.cpiece[c + 1] : p0 + 1;
-    const bool own = !TEAMS || (team == THREADS && p1 - p0 == 1);
-    const int t0 = own ? 0 : m.piece[p0].x;
-    for (int q0 = p0; q0 < p1; q0 += THREADS / team) {
+    const int q = src->pblk_begin + c - src->cblk_begin, a = src->node_begin + (c - src->cblk_begin) * src->share;
+    float noise;
+    if (THREADS == 512 && m.noise_tets != 0 && nt > THREADS) {
+        // two tets a thread: with those of the thread half a CTA away
+        __shared__ float s_x[THREADS / 2];
+        if (threadIdx.x >= THREADS / 2) s_x[threadIdx.x - THREADS / 2] = ec.hi;
+        __syncthreads();
+        const float x = threadIdx.x < THREADS / 2 ? ec.hi + s_x[threadIdx.x] : 0.f;
+        noise = x * x;
+    } else {
+        noise = noise_square(m, THREADS, nt, ec.hi);
+    }
+    DFloat e{0.f, 0.f};
+    float e2 = 0.f;
+    share_energy(m, p, st, cur, a + threadIdx.x, min(a + src->share, src->node_end), THREADS,
+                 p.incremental ? st.ub : nullptr, e, e2);
+    e = warp_sum_df(df_add(e, ec));
+    e2 = warp_sum_f(e2 + noise);
+    if ((threadIdx.x & 31) == 0) {
+        s_e[threadIdx.x >> 5] = make_float2(e.hi, e.lo);
+        s_e2[threadIdx.x >> 5] = e2;
+    }
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    double d;
+    join_warps(s_e, s_e2, THREADS, d, e2);
+    if (threadIdx.x == 0) st.cpart[q] = make_double2(d, (double)e2);
+}
+
+// The same where the layout has chunks of several pieces or teams that are not
+// the CTA's threads (a packed batch's), from the energies in the slots: teams
+// of fewer threads take a piece each at a time, one of 512 takes two rounds.
+// In kernels of their own, so that the others keep their registers (two bodies
+// of 150,000 tets, 96 passes without a line search: 1460 us, and 1470 when one
+// kernel held both).
+template <int THREADS>
+__device__ __forceinline__ void chunk_energy_teams(const DevMesh &m, const DevParams &p, const DevState &st, int c,
+                                                   int inst, int par, size_t cur, const ChunkView &v,
+                                                   const float4 *sf) {
+    constexpr int MAX_TEAM = 512;
+    __shared__ float2 s_e[MAX_TEAM / 32];
+    __shared__ float s_e2[MAX_TEAM / 32];
+    const InstCtl *src = ctl_buf(st, par) + inst;
+    const int pb = src->pblk_begin, per = src->share, p0 = m.cpiece[c], p1 = m.cpiece[c + 1], t0 = m.piece[p0].x;
+    const int team = src->team, width = min(team, THREADS), sides = THREADS / width;
+    const int tid = threadIdx.x & (width - 1), side = threadIdx.x / width;
+    for (int q0 = p0; q0 < p1; q0 += sides) {
         const int q = q0 + side;
         if (q < p1) {
-            const int2 pc = own ? make_int2(0, nt) : m.piece[q];
-            if (!own) ec = team_energy(v.cor + (pc.x - t0), pc.y, tid, team, sf);
-            DFloat e{0.f, 0.f};
-            float e2 = 0.f;
-            const int a = n0 + (q - pb) * per;
-            share_energy(m, p, st, cur, a + tid, min(a + per, n1), team, base, e, e2);
-            e = warp_sum_df(df_add(e, ec));
-            e2 = warp_sum_f(e2 + noise_square(m, team, pc.y, ec.hi));
-            if ((tid & 31) == 0) {
-                s_e[threadIdx.x >> 5] = make_float2(e.hi, e.lo);
-                s_e2[threadIdx.x >> 5] = e2;
+            const int2 pc = m.piece[q];
+            const int a = src->node_begin + (q - pb) * per, n1 = min(a + per, src->node_end);
+            const uint4 *cor = v.cor + (pc.x - t0);
+            float x = 0.f;  // (a team of 512 with two tets a thread: those of the threads t and t + 256)
+            for (int r = team - width; r >= 0; r -= width) {
+                const DFloat ec = team_energy(cor, pc.y, r + tid, team, sf);
+                float noise;
+                if (team == MAX_TEAM && m.noise_tets != 0 && pc.y > team) {
+                    x = r > 0 ? ec.hi : ec.hi + x;
+                    noise = r > 0 ? 0.f : x * x;
+                } else {
+                    noise = noise_square(m, team, pc.y, ec.hi);
+                }
+                DFloat e{0.f, 0.f};
+                float e2 = 0.f;
+                share_energy(m, p, st, cur, a + r + tid, n1, team, p.incremental ? st.ub : nullptr, e, e2);
+                e = warp_sum_df(df_add(e, ec));
+                e2 = warp_sum_f(e2 + noise);
+                if ((tid & 31) == 0) {
+                    const int w = side * (width >> 5) + ((r + tid) >> 5);
+                    s_e[w] = make_float2(e.hi, e.lo);
+                    s_e2[w] = e2;
+                }
             }
         }
         __syncthreads();
         if (q < p1 && tid < 32) {
             double d;
             float e2;
-            join_warps(s_e + side * (team >> 5), s_e2 + side * (team >> 5), team, d, e2);
+            join_warps(s_e + side * (width >> 5), s_e2 + side * (width >> 5), team, d, e2);
             if (tid == 0) {
                 st.cpart[q] = make_double2(d, (double)e2);
-                if (TEAMS) __threadfence();  // (thread 0 counts the chunk in for every team)
+                __threadfence();  // (thread 0 counts the chunk in for every team)
             }
         }
-        if (TEAMS) __syncthreads();
+        __syncthreads();
     }
 }
 
@@ -364,7 +410,7 @@ __device__ __forceinline__ void chunk_line_search(const DevParams &p, const DevS
     // runs on one CTA while the rest of the GPU waits, and one load round trip
     // per partial made it several microseconds
     constexpr int U = 8;
-    const int lanes = pe - pb <= SUM_PIECES ? 32 : THREADS < 256 ? THREADS : 256;
+    const int lanes = src->by_share ? 32 : min(src->team, 256);
     double ea = 0.0, eb = 0.0;
     if (threadIdx.x < lanes)
         for (int j0 = pb + threadIdx.x; j0 < pe; j0 += U * lanes) {
@@ -403,7 +449,10 @@ __device__ __forceinline__ void chunk_body(const DevMesh &m, const DevParams &p,
                                            int *is_last, const TetRows &first = TetRows()) {
     const DFloat e = chunk_forces_all<MATERIAL, THREADS, INC, PACK, PRE>(p, v, nt, pv.check, sf, first);
     chunk_partials<THREADS>(meta, nl, sf, st.part);
-    if (pv.check) chunk_energy<THREADS, TEAMS>(m, p, st, c, inst, par, cur, v, nt, sf, e);
+    if (pv.check) {
+        if (TEAMS) chunk_energy_teams<THREADS>(m, p, st, c, inst, par, cur, v, sf);
+        else chunk_energy<THREADS>(m, p, st, c, inst, par, cur, nt, e);
+    }
     if (pv.do_h) {
         __syncthreads();
         chunk_hdiag<MATERIAL, THREADS, INC, PACK>(v, nt, sf);
@@ -797,8 +846,7 @@ template <int MATERIAL, int THREADS, bool INC> static cudaError_t allow_smem_str
 
 template <int MATERIAL, bool INC> static cudaError_t allow_smem_all() {
     const cudaError_t e[] = {allow_smem<MATERIAL, 128, INC, false>(), allow_smem<MATERIAL, 256, INC, false>(),
-                             allow_smem<MATERIAL, 512, INC, false>(), allow_smem<MATERIAL, 256, INC, false, true>(),
-                             allow_smem<MATERIAL, 512, INC, false, true>()};
+                             allow_smem<MATERIAL, 512, INC, false>(), allow_smem<MATERIAL, 256, INC, false, true>()};
     for (cudaError_t x : e)
         if (x != cudaSuccess) return x;
     return cudaSuccess;
@@ -881,9 +929,9 @@ template <int MATERIAL, bool INC>
 static cudaError_t launch_tchunk(cudaStream_t s, const DevMesh &m, const DevParams &p, const DevState &st, int par,
                                  bool pdl) {
     if (m.chunk_threads == 128) return launch_tchunk_t<MATERIAL, 128, INC, false>(s, m, p, st, par, pdl);
-    if (m.teams)  // (automatic layouts: no team is of more threads than the CTA)
-        return m.chunk_threads == 512 ? launch_tchunk_t<MATERIAL, 512, INC, false, true>(s, m, p, st, par, pdl)
-                                      : launch_tchunk_t<MATERIAL, 256, INC, false, true>(s, m, p, st, par, pdl);
+    if (m.teams)  // (packed automatic layouts, with 256 threads)
+        return m.chunk_threads == 256 ? launch_tchunk_t<MATERIAL, 256, INC, false, true>(s, m, p, st, par, pdl)
+                                      : cudaErrorInvalidConfiguration;
     if (m.chunk_threads == 512) return launch_tchunk_t<MATERIAL, 512, INC, false>(s, m, p, st, par, pdl);
     return launch_tchunk_t<MATERIAL, 256, INC, false>(s, m, p, st, par, pdl);
 }

@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(THREADS + 32, PER_SM)
         const int per = node_share(sc.node_end - sc.node_begin, G);
         own.n0 = min(sc.node_begin + bi * per, sc.node_end);
         own.n1 = min(own.n0 + per, sc.node_end);
-        own.team = sc.team;
+        own.team = RES ? sc.team : THREADS;
     }
     __syncthreads();
     // (the variant with registers to spare keeps its nodes in them)

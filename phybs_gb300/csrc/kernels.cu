@@ -259,8 +259,8 @@ __global__ void k_from_increment(DevMesh m, DevState st) {
 // grid-dependency wait, so no registers hold them across it.  With two nodes
 // a thread the kernel is held to 85 registers: six 128-thread CTAs fit an SM,
 // and the 1M-tet box's 823 node blocks run as one wave.  |g|^2 is summed in
-// FP32 within 32 nodes (a warp's); the pass decision on these sums
-// (instance_r2) is taken by the next pass's tet kernel or by k_settle, so the
+// FP32 within 32 nodes (a warp's), or the block (instances that are not summed
+// by share); the pass decision on these sums (instance_r2) is taken by the next pass's tet kernel or by k_settle, so the
 // kernel ends with its blocks and no CTA waits for the instance's last one.
 template <int NPT>
 __global__ void __launch_bounds__(BLOCK / NPT, NPT == 2 ? 6 : 0) k_node(DevMesh m, DevParams p, DevState st, int par) {
@@ -327,6 +327,8 @@ __global__ void __launch_bounds__(BLOCK / NPT, NPT == 2 ? 6 : 0) k_node(DevMesh 
     ctx.omega = omega;
     ctx.cur = cur;
     ctx.nxt = nxt;
+    const bool by_share = cp->by_share != 0;
+    __shared__ float s_g[8];
 #pragma unroll
     for (int j = 0; j < NPT; ++j) {
         const int l = threadIdx.x + j * TH;
@@ -336,8 +338,15 @@ __global__ void __launch_bounds__(BLOCK / NPT, NPT == 2 ? 6 : 0) k_node(DevMesh 
         float r2 = node_update(p, st, b * BLOCK + l, nc, in[j], ctx, [&] { return node_sums<NPRE>(st, in[j], fp[j], do_h); });
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) r2 += __shfl_down_sync(0xffffffffu, r2, o);
-        if ((l & 31) == 0) st.npartf[(b * BLOCK + l) / 32] = r2;
+        if ((l & 31) == 0) {
+            if (by_share) st.npartf[(b * BLOCK + l) / 32] = r2;
+            else s_g[l / 32] = r2;
+        }
     }
+    if (by_share) return;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        st.npartf[b * (BLOCK / 32)] = ((s_g[0] + s_g[4]) + (s_g[2] + s_g[6])) + ((s_g[1] + s_g[5]) + (s_g[3] + s_g[7]));
 }
 
 // The pending pass decisions after the last pass of a run, one CTA an

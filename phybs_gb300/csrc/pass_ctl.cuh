@@ -196,28 +196,19 @@ __device__ __forceinline__ DFloat instance_r2(const DevState &st, const InstCtl 
         }
         return threadIdx.x < 32 ? lane_tree_df(acc) : acc;
     }
-    // a block's eight groups as their lane tree, 256 threads of blocks
+    // node blocks, by at most 256 threads (as many whatever the CTA's)
     __shared__ float2 shf[THREADS / 32];
-    constexpr int LANES = THREADS < 256 ? THREADS : 256;
-    const float4 *g4 = reinterpret_cast<const float4 *>(g);
-    const int blocks = src->nblk_end - src->nblk_begin;
-    if (threadIdx.x < LANES) {
-        constexpr int U = 4;
-        for (int j0 = threadIdx.x; j0 < blocks; j0 += U * LANES) {
-            float4 v[U][2];
+    constexpr int U = 8;
+    const int blocks = src->nblk_end - src->nblk_begin, lanes = min(src->team, 256);
+    if (threadIdx.x < lanes)
+        for (int j0 = threadIdx.x; j0 < blocks; j0 += U * lanes) {
+            float v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = j0 + u * lanes < blocks ? __ldcg(g + 8 * (j0 + u * lanes)) : 0.f;
 #pragma unroll
             for (int u = 0; u < U; ++u)
-#pragma unroll
-                for (int q = 0; q < 2; ++q)
-                    v[u][q] = j0 + u * LANES < blocks ? __ldcg(g4 + 2 * (j0 + u * LANES) + q)
-                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (j0 + u * LANES < blocks)
-                    acc = df_add(acc, ((v[u][0].x + v[u][1].x) + (v[u][0].z + v[u][1].z)) +
-                                          ((v[u][0].y + v[u][1].y) + (v[u][0].w + v[u][1].w)));
+                if (j0 + u * lanes < blocks) acc = df_add(acc, v[u]);
         }
-    }
     return block_sum_df(acc, shf);
 }
 

@@ -189,7 +189,7 @@ struct pbs_handle {
     bool graph_valid = false;
     bool teams = false;       // DevMesh::teams
     bool joined = false;      // chunks of several pieces: for the pass kernels only
-    bool share_sums = true;   // every instance's |g|^2 is summed by share (sums_by_share)
+    bool share_sums = true;   // every instance's |g|^2 is summed by share (InstCtl::by_share)
     bool shape_auto = true;   // no caller set the chunk shape (pbs_set_chunk_shape, pbs_autotune)
     bool engine_auto = true;  // nor the pass engine (pbs_set_pass_engine)
     bool plan_valid = false;  // fplan describes the current layout, material and stress
@@ -349,13 +349,15 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
     if (automatic) {
         if (ct == CHUNK_GROUP_TETS) threads = nc > h->sms && h->B == 1 ? 512 : 256;
         else threads = wide || (ct > 256 && nc > 2 * h->sms) ? 256 : 128;
-        threads = std::max(threads, max_team);
+        if (h->B == 1) threads = std::max(threads, max_team);
+        else if (threads < max_team) threads = 256;  // (teams of 512 take two rounds)
     }
     bool share_sums = true, teams = join > 0;
     for (InstCtl &c : ctl) {
         const int nodes = c.node_end - c.node_begin, pieces = c.pblk_end - c.pblk_begin;
         c.share = node_share(nodes, pieces);
-        c.by_share = sums_by_share(nodes, pieces);
+        c.by_share = c.tet_end - c.tet_begin <= CHUNK_GROUP_TETS * h->sms && pieces <= SUM_PIECES &&
+                     c.share <= 32 * SUM_GROUPS;
         share_sums = share_sums && c.by_share;
         teams = teams || c.team != threads;
     }

@@ -51,7 +51,8 @@
 //   cpart       double2[n_pieces]  per piece {sum e, sum e^2}
 //   rslot       double[3][4T]      per-step FP64 corner forces at the base, by gather slot
 //   npart       double[n_nblk]     per node-block |g|^2 (warm-start reference)
-//   npartf      float[8*n_nblk]    |g|^2 of a pass per 32 nodes (FP32 sums)
+//   npartf      float[8*n_nblk]    |g|^2 of a pass per 32 nodes (FP32 sums), or of an instance that
+//                                  is not summed by share per node block (every eighth)
 //   ctl         InstCtl[n_inst]    per-instance descent state
 #pragma once
 #include <cuda_runtime.h>
@@ -136,7 +137,7 @@ struct __align__(16) InstCtl {
     int team;  // threads whose sums make up a piece's energy (chunk_energy)
     int pblk_begin, pblk_end;  // the instance's pieces
     int share;     // nodes of a piece's share (node_share)
-    int by_share;  // |g|^2 is summed by share (sums_by_share)
+    int by_share;  // |g|^2 is summed by share, else by node block
     int pad;
 };
 
@@ -152,9 +153,10 @@ struct __align__(16) InstCtl {
 //   |g|^2    of a group: a lane tree; of a share: its groups in ascending order;
 //            of the instance: 32 lanes of double-float, each its shares in
 //            ascending order, then the lane tree.
-// Beyond SUM_PIECES pieces, where the serial chains would be long and no frame
-// kernel is resident, 256 threads take the place of the 32 lanes, and |g|^2 is
-// summed by 256-node blocks instead of shares.
+// An instance of more than CHUNK_GROUP_TETS tets a SM, for which no frame kernel
+// is resident, is not summed so (InstCtl::by_share): |g|^2 by 256-node blocks
+// instead of shares, and min(T, 256) threads in place of the 32 lanes, whose
+// chains cost its pass kernels 0.3-0.5 us a pass.
 constexpr int SUM_PIECES = 512, SUM_GROUPS = 256;  // (groups of a share that the frame kernel keeps)
 
 // Nodes of a piece's share: the instance's, in whole groups of 32, evenly over
@@ -163,10 +165,6 @@ __host__ __device__ inline int node_share(int nodes, int pieces) {
     const int groups = (nodes + 31) / 32;
     return pieces > 0 ? (groups + pieces - 1) / pieces * 32 : 0;
 }
-__host__ __device__ inline bool sums_by_share(int nodes, int pieces) {
-    return pieces <= SUM_PIECES && node_share(nodes, pieces) <= 32 * SUM_GROUPS;
-}
-
 // |g| / |g0| of an instance's last pass (-1 before the first pass).
 inline double residual_ratio(const InstCtl &c) {
     if (c.r2 < 0.0 || c.g0 < 0.0) return -1.0;
@@ -311,8 +309,8 @@ struct ChunkLimits {
 // The chunk limits of an instance whose shape no caller set, from its own tet
 // count only: a packed batch then chunks an instance as it is chunked alone.
 ChunkLimits auto_chunk_limits(int tets, int sms);
-// The team of such an instance: the threads of the frame kernel's CTA where it
-// has one to a chunk, else 256.
+// The team of such an instance: the threads of the CTA that runs its chunks
+// when it is alone.
 int auto_team(int tets, int sms);
 // limits: per instance.  grouped: the chunks are even pieces of groups of at
 // most CHUNK_GROUP_TETS tets and CHUNK_GROUP_NODES nodes, and every chunk of a
