@@ -467,8 +467,6 @@ __global__ void __launch_bounds__(512, 1) k_cg_solve(CgPlanView pl, CgArgs a) {
 }
 
 template <int NV, typename COL> cudaError_t launch_solve_t(cudaStream_t s, const CgPlanView &pl, const CgArgs &a) {
-    cudaError_t e = cudaFuncSetAttribute(k_cg_solve<NV, COL>, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem);
-    if (e != cudaSuccess) return e;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
@@ -498,6 +496,13 @@ cudaError_t launch_cg_pack(cudaStream_t s, const CgPlanView &pl, const BsrView &
     if (A.scalar) k_cg_pack<1><<<g, 256, 0, s>>>(pl, A, dinv9, out, dinv);
     else k_cg_pack<9><<<g, 256, 0, s>>>(pl, A, dinv9, out, dinv);
     return cudaGetLastError();
+}
+cudaError_t prepare_cg_kernels() {
+    const cudaError_t e[] = {allow_all_smem(k_cg_solve<1, int>), allow_all_smem(k_cg_solve<9, int>),
+                             allow_all_smem(k_cg_solve<1, unsigned short>), allow_all_smem(k_cg_solve<9, unsigned short>)};
+    for (cudaError_t x : e)
+        if (x != cudaSuccess) return x;
+    return cudaSuccess;
 }
 cudaError_t launch_cg_solve(cudaStream_t s, const CgPlanView &pl, const CgArgs &a, bool scalar) {
     if (pl.col32) return scalar ? launch_solve_t<1, int>(s, pl, a) : launch_solve_t<9, int>(s, pl, a);

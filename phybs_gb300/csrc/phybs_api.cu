@@ -1656,6 +1656,7 @@ int pbs_drag_face_ring(pbs_handle *h, int face, const float *drag, float *ext) {
 // that its rows multiply) and the rows of its own that are in others' halos.
 static int ensure_bsr(pbs_handle *h) {
     if (h->bsr_ready) return PBS_OK;
+    CK(prepare_cg_kernels());
     cudaStream_t s = h->stream;
     const size_t np = (size_t)h->Np;
     std::vector<int> ptr(np + 1, 0);

@@ -281,6 +281,21 @@ __device__ __forceinline__ int node_ctl_ws(const DevMesh &m, const DevState &st,
     return st.ctl[m.nblk_inst[i / BLOCK]].ws_used;
 }
 
+// Raises a kernel's limit of dynamic shared memory to all that the device has
+// beside its static part.  The limit is the function's, for every thread of the
+// process: set to what one launch needs, it refused the larger launch of another
+// thread in between.
+template <class Kernel> inline cudaError_t allow_all_smem(Kernel kernel) {
+    int dev = 0, all = 0;
+    cudaFuncAttributes a;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&all, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, all - (int)a.sharedSizeBytes);
+    return e;
+}
+
 // 10 bits -> every third bit of 30 (Morton codes).
 inline uint32_t spread10(uint32_t v) {
     v &= 0x3ffu;
@@ -527,6 +542,7 @@ cudaError_t launch_bsr_count(cudaStream_t s, const DevMesh &m, int *cnt);
 cudaError_t launch_bsr_fill(cudaStream_t s, const DevMesh &m, const int *ptr, int *col);
 cudaError_t launch_cg_pack(cudaStream_t s, const CgPlanView &pl, const BsrView &A, const float *dinv9, float *out,
                            float *dinv);
+cudaError_t prepare_cg_kernels();  // before a context's first solve
 cudaError_t launch_cg_solve(cudaStream_t s, const CgPlanView &pl, const CgArgs &a, bool scalar);
 cudaError_t launch_be_assemble(cudaStream_t s, const DevMesh &m, const DevState &st, int material, const BsrView &A,
                                float dt, float alpha, float beta, const float4 *ext, float4 *b, float4 *x,

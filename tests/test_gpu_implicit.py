@@ -269,3 +269,51 @@ def test_solve_with_vectors_in_global_memory(integrator, split, nx, ny, nz):
         for wide in (0, 1):
             got = solve(smem, wide)
             assert got[0] == want[0] and np.array_equal(got[1], want[1]) and np.array_equal(got[2], want[2]), (smem, wide)
+
+
+@pytest.mark.parametrize("integrator", ["be", "pd", "pbd"])
+def test_solves_of_several_threads(integrator):
+    """Handles of different sizes stepped from threads of their own: every one's
+    steps are those it takes by itself, and none is refused (the shared memory
+    that a launch may have is set per kernel, not per handle)."""
+    import threading
+    sizes = [(9, 14, 19), (3, 3, 7), (12, 12, 24), (6, 9, 9), (14, 14, 20), (9, 9, 9)]
+    ms = [_moving(5, *n) for n in sizes]
+
+    def steps(k, n):
+        m, x0, v0 = ms[k]
+        s = DescentSolver(m, positions=x0)
+        s.write_velocities(v0, v0)
+        out = []
+        for _ in range(n):
+            s.update_positions(x0)
+            s.write_velocities(v0, v0)
+            if integrator == "be":
+                s.backward_euler_step(tol=1e-6)
+            elif integrator == "pd":
+                s.pd_step()
+            else:
+                s.pbd_step()
+            out.append(s.positions())
+        s.close()
+        return out
+
+    want = [steps(k, 1)[0] for k in range(len(sizes))]
+    got, bad = [None] * len(sizes), []
+    start = threading.Barrier(len(sizes))
+
+    def run(k):
+        try:
+            start.wait()
+            got[k] = steps(k, 60)
+        except Exception as e:  # noqa: BLE001
+            bad.append((k, repr(e)))
+
+    ts = [threading.Thread(target=run, args=(k,)) for k in range(len(sizes))]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad, bad
+    for g, w in zip(got, want):
+        assert all(np.array_equal(x, w) for x in g)
