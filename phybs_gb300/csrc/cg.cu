@@ -253,8 +253,8 @@ template <int NV, typename COL> struct Rows {
     }
 };
 
-template <int NV, typename COL>
-__global__ void __launch_bounds__(512, 1) k_cg_solve(CgPlanView pl, CgArgs a) {
+template <int NV, typename COL, int PER_SM>
+__global__ void __launch_bounds__(512, PER_SM) k_cg_solve(CgPlanView pl, CgArgs a) {
     extern __shared__ float4 smem4[];
     __shared__ Reduce sh;
     char *sm = reinterpret_cast<char *>(smem4);
@@ -466,7 +466,8 @@ __global__ void __launch_bounds__(512, 1) k_cg_solve(CgPlanView pl, CgArgs a) {
     }
 }
 
-template <int NV, typename COL> cudaError_t launch_solve_t(cudaStream_t s, const CgPlanView &pl, const CgArgs &a) {
+template <int NV, typename COL, int PER_SM>
+cudaError_t launch_solve_t(cudaStream_t s, const CgPlanView &pl, const CgArgs &a) {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
@@ -477,7 +478,11 @@ template <int NV, typename COL> cudaError_t launch_solve_t(cudaStream_t s, const
     cfg.stream = s;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_cg_solve<NV, COL>, pl, a);
+    return cudaLaunchKernelEx(&cfg, k_cg_solve<NV, COL, PER_SM>, pl, a);
+}
+
+template <int NV, typename COL> cudaError_t launch_solve_p(cudaStream_t s, const CgPlanView &pl, const CgArgs &a) {
+    return pl.light ? launch_solve_t<NV, COL, 2>(s, pl, a) : launch_solve_t<NV, COL, 1>(s, pl, a);
 }
 
 }  // namespace
@@ -498,15 +503,18 @@ cudaError_t launch_cg_pack(cudaStream_t s, const CgPlanView &pl, const BsrView &
     return cudaGetLastError();
 }
 cudaError_t prepare_cg_kernels() {
-    const cudaError_t e[] = {allow_all_smem(k_cg_solve<1, int>), allow_all_smem(k_cg_solve<9, int>),
-                             allow_all_smem(k_cg_solve<1, unsigned short>), allow_all_smem(k_cg_solve<9, unsigned short>)};
+    const cudaError_t e[] = {
+        allow_all_smem(k_cg_solve<1, int, 1>),            allow_all_smem(k_cg_solve<9, int, 1>),
+        allow_all_smem(k_cg_solve<1, unsigned short, 1>), allow_all_smem(k_cg_solve<9, unsigned short, 1>),
+        allow_all_smem(k_cg_solve<1, int, 2>),            allow_all_smem(k_cg_solve<9, int, 2>),
+        allow_all_smem(k_cg_solve<1, unsigned short, 2>), allow_all_smem(k_cg_solve<9, unsigned short, 2>)};
     for (cudaError_t x : e)
         if (x != cudaSuccess) return x;
     return cudaSuccess;
 }
 cudaError_t launch_cg_solve(cudaStream_t s, const CgPlanView &pl, const CgArgs &a, bool scalar) {
-    if (pl.col32) return scalar ? launch_solve_t<1, int>(s, pl, a) : launch_solve_t<9, int>(s, pl, a);
-    return scalar ? launch_solve_t<1, unsigned short>(s, pl, a) : launch_solve_t<9, unsigned short>(s, pl, a);
+    if (pl.col32) return scalar ? launch_solve_p<1, int>(s, pl, a) : launch_solve_p<9, int>(s, pl, a);
+    return scalar ? launch_solve_p<1, unsigned short>(s, pl, a) : launch_solve_p<9, unsigned short>(s, pl, a);
 }
 
 }  // namespace pbs

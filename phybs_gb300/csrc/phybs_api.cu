@@ -66,14 +66,19 @@ int round_up(int x, int a) { return (x + a - 1) / a * a; }
 // 204).
 std::atomic<int> large_steps[64];
 
-class LargeStep {
+// The same for backward-Euler and projective-dynamics steps whose solve has a
+// CTA on more than half of the SMs: from the third on the solves take half a SM
+// each, so that two of them run side by side, with the same bits.
+std::atomic<int> large_solves[64];
+
+class LargeCount {
   public:
-    // Counts this step in; the others that run.
-    int enter(int device) {
-        count_ = &large_steps[device & 63];
+    // Counts this call in; the others that run.
+    int enter(std::atomic<int> *counts, int device) {
+        count_ = &counts[device & 63];
         return count_->fetch_add(1);
     }
-    ~LargeStep() {
+    ~LargeCount() {
         if (count_) count_->fetch_sub(1);
     }
 
@@ -148,7 +153,8 @@ struct pbs_handle {
     DevBuf<float4> cg_b, cg_x, cg_xp, cg_red, cg_ws;
     DevBuf<int> cg_plan;
     DevBuf<unsigned char> cg_col;
-    CgPlanView cgp[2]{};        // of the two matrix kinds: nine values a block, one value
+    CgPlanView cgp[2][2]{};     // of the two matrix kinds (nine values a block, one), for a SM and for half of one
+    bool solve_light = false;   // the running step's solves take half a SM (LargeCount)
     size_t cg_entries = 0, cg_rows_pad = 0, cg_halo = 0;
     DevBuf<CgState> cg_state;   // of the solves of a step
     DevBuf<unsigned> cg_ctl;    // [0] the last tag of the exchanged words, [1] a wait gave up
@@ -1014,10 +1020,11 @@ int pbs_step(pbs_handle *h, const float *ext, int *iters_out) {
     // every chunk has a resident CTA of its own (auto_chunk_limits), which
     // spares a pass its two launches and its trips to memory
     bool auto_frame = !frame && auto_frame_applies(h);
-    LargeStep large;
+    LargeCount large;
     if (auto_frame) {
         const FramePlan &plan = handle_frame_plan(h);
-        if ((plan.per_sm > 1 || 2 * plan.grid > h->ctx_sms) && large.enter(h->device) >= 2) auto_frame = false;
+        if ((plan.per_sm > 1 || 2 * plan.grid > h->ctx_sms) && large.enter(large_steps, h->device) >= 2)
+            auto_frame = false;
     }
     frame |= auto_frame;
     int rc = frame ? PBS_OK : ensure_graph(h);
@@ -1250,7 +1257,10 @@ int pbs_test_hook(pbs_handle *h, int what, int value) {
         case TEST_SOLVE_SMEM: h->test_solve_smem = value; return PBS_OK;
         case TEST_SOLVE_COL32: h->test_solve_col32 = value != 0; return PBS_OK;
         case TEST_REFUSE_FRAME: h->test_refuse_frame = value != 0; return PBS_OK;
-        case TEST_LARGE_STEPS: large_steps[h->device & 63] += value; return PBS_OK;
+        case TEST_LARGE_STEPS:
+            large_steps[h->device & 63] += value;
+            large_solves[h->device & 63] += value;
+            return PBS_OK;
         default: return PBS_E_INVALID_ARG;
     }
 }
@@ -1828,11 +1838,13 @@ static int ensure_bsr(pbs_handle *h) {
     v.cta_send = base + part[8].at; v.send = base + part[9].at;
     v.scol = h->cg_col.p;
     v.col32 = col32;
-    const size_t budget = h->test_solve_smem >= 0 ? h->test_solve_smem : CG_MAX_SMEM;
-    for (int kind = 0; kind < 2; ++kind) {
+    for (int kind = 0; kind < 2; ++kind)
+    for (int light = 0; light < 2; ++light) {
         // what fits shared memory, the most often read first
-        CgPlanView &w = h->cgp[kind];
+        const size_t budget = h->test_solve_smem >= 0 ? h->test_solve_smem : light ? CG_LIGHT_SMEM : CG_MAX_SMEM;
+        CgPlanView &w = h->cgp[kind][light];
         w = v;
+        w.light = light != 0;
         w.smem = 0;
         auto place = [&](size_t bytes) {
             bytes = (bytes + 127) / 128 * 128;
@@ -1874,6 +1886,11 @@ static int ensure_bsr(pbs_handle *h) {
     return PBS_OK;
 }
 
+// Before a step's solves: how much of a SM they take.
+static void enter_solves(pbs_handle *h, LargeCount &large) {
+    h->solve_light = 2 * h->cgp[0][0].grid > h->ctx_sms && large.enter(large_solves, h->device) >= 2;
+}
+
 // Enqueues one solve A x = b (slot: where its state goes).
 static cudaError_t enqueue_solve(pbs_handle *h, bool scalar, const float *val, const float *dinv, double tol2,
                                  int max_iters, int pnorm, int slot) {
@@ -1896,7 +1913,7 @@ static cudaError_t enqueue_solve(pbs_handle *h, bool scalar, const float *val, c
     a.tol2 = tol2;
     a.max_iters = max_iters;
     a.pnorm = pnorm;
-    return launch_cg_solve(h->stream, h->cgp[scalar ? 1 : 0], a, scalar);
+    return launch_cg_solve(h->stream, h->cgp[scalar ? 1 : 0][h->solve_light], a, scalar);
 }
 
 // The states of the last `count` solves on the host, and the exchanged words'
@@ -1931,6 +1948,8 @@ int pbs_backward_euler_step(pbs_handle *h, float dt, float alpha, float beta, co
         rc = upload_user(h, ext, h->ext.p);
         if (rc != PBS_OK) return rc;
     }
+    LargeCount large;
+    enter_solves(h, large);
     cudaStream_t s = h->stream;
     const DevMesh m = h->mesh();
     const DevState st = h->state();
@@ -1943,7 +1962,7 @@ int pbs_backward_euler_step(pbs_handle *h, float dt, float alpha, float beta, co
     float *cgd = h->cg_val.p + 9 * 32 * h->cg_entries;  // the inverses by row
     CK(launch_be_assemble(s, m, st, h->material, A, dt, alpha, beta, ext ? h->ext.p : nullptr, h->cg_b.p, h->cg_x.p,
                           h->cg_dinv.p));
-    CK(launch_cg_pack(s, h->cgp[0], A, h->cg_dinv.p, h->cg_val.p, cgd));
+    CK(launch_cg_pack(s, h->cgp[0][0], A, h->cg_dinv.p, h->cg_val.p, cgd));
     CK(enqueue_solve(h, false, h->cg_val.p, cgd, tol2, max_iters, 0, 0));
     rc = read_solves(h, 1);
     if (rc != PBS_OK) return rc;
@@ -2125,6 +2144,8 @@ int pbs_pd_step(pbs_handle *h, float dt, float dt_matrix, float stiffness, int i
     if (rc == PBS_OK) rc = ensure_dyn_buffers(h);
     if (rc == PBS_OK && ext) rc = upload_user(h, ext, h->ext.p);
     if (rc != PBS_OK) return rc;
+    LargeCount large;
+    enter_solves(h, large);
     cudaStream_t s = h->stream;
     const DevMesh m = h->mesh();
     const DevState st = h->state();
@@ -2142,7 +2163,7 @@ int pbs_pd_step(pbs_handle *h, float dt, float dt_matrix, float stiffness, int i
     A.val = h->pd_val.p;
     if (!h->pd_ready || h->pd_dtm != dtm || h->pd_k != stiffness) {
         CK(launch_pd_assemble(s, m, A, dtm, stiffness, h->pd_dinv.p));
-        CK(launch_cg_pack(s, h->cgp[1], A, h->pd_dinv.p, h->pd_cgval.p, h->pd_cgval.p + 32 * h->cg_entries));
+        CK(launch_cg_pack(s, h->cgp[1][0], A, h->pd_dinv.p, h->pd_cgval.p, h->pd_cgval.p + 32 * h->cg_entries));
         h->pd_ready = true;
         h->pd_dtm = dtm;
         h->pd_k = stiffness;

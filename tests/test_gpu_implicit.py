@@ -271,6 +271,30 @@ def test_solve_with_vectors_in_global_memory(integrator, split, nx, ny, nz):
             assert got[0] == want[0] and np.array_equal(got[1], want[1]) and np.array_equal(got[2], want[2]), (smem, wide)
 
 
+TEST_LARGE_STEPS = 2
+
+
+@pytest.mark.parametrize("integrator", ["be", "pd"])
+@pytest.mark.parametrize("nx,ny,nz", [(20, 20, 24), (24, 26, 40)])
+def test_solve_beside_others(integrator, nx, ny, nz):
+    """The solve of half a SM, which a step takes when two large ones run
+    already (84 CTAs; one on every SM): bit for bit the one of a whole SM."""
+    m, x0, v0 = _moving(5, nx, ny, nz)
+    out = []
+    for others in (0, 2):
+        s = DescentSolver(m, positions=x0)
+        s.write_velocities(v0, v0)
+        L.lib().pbs_test_hook(s._h, TEST_LARGE_STEPS, others)
+        try:
+            its = [s.backward_euler_step(tol=1e-6) if integrator == "be" else s.pd_step() for _ in range(2)]
+        finally:
+            L.lib().pbs_test_hook(s._h, TEST_LARGE_STEPS, -others)
+        out.append((its, s.positions(), s.velocities()[0]))
+        s.close()
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
+
+
 @pytest.mark.parametrize("integrator", ["be", "pd", "pbd"])
 def test_solves_of_several_threads(integrator):
     """Handles of different sizes stepped from threads of their own: every one's
