@@ -466,6 +466,14 @@ __global__ void __launch_bounds__(512, PER_SM) k_cg_solve(CgPlanView pl, CgArgs 
     }
 }
 
+// CTAs a SM of the solve beside others (CgPlanView::light).  Eight threads, one
+// handle each, us a step of all, in turn / two a SM with 110 KB / three with 73:
+// projective dynamics of 100,000 tets 2250 / 2143 / 1842, 200,000 5800 / 4383 /
+// 3960, 500,000 (10,430) / 8245 / 7629; backward Euler, two a SM with 110 KB /
+// with 55 (the matrix from L2) / three with 73: 100,000 3054 / 2373 / 2612,
+// 200,000 5342 / 5256 / 5993.
+template <int NV> constexpr int LIGHT_PER_SM = NV == 1 ? 3 : 2;
+
 template <int NV, typename COL, int PER_SM>
 cudaError_t launch_solve_t(cudaStream_t s, const CgPlanView &pl, const CgArgs &a) {
     cudaLaunchAttribute at[1];
@@ -482,7 +490,7 @@ cudaError_t launch_solve_t(cudaStream_t s, const CgPlanView &pl, const CgArgs &a
 }
 
 template <int NV, typename COL> cudaError_t launch_solve_p(cudaStream_t s, const CgPlanView &pl, const CgArgs &a) {
-    return pl.light ? launch_solve_t<NV, COL, 2>(s, pl, a) : launch_solve_t<NV, COL, 1>(s, pl, a);
+    return pl.light ? launch_solve_t<NV, COL, LIGHT_PER_SM<NV>>(s, pl, a) : launch_solve_t<NV, COL, 1>(s, pl, a);
 }
 
 }  // namespace
@@ -502,12 +510,13 @@ cudaError_t launch_cg_pack(cudaStream_t s, const CgPlanView &pl, const BsrView &
     else k_cg_pack<9><<<g, 256, 0, s>>>(pl, A, dinv9, out, dinv);
     return cudaGetLastError();
 }
+template <int NV, typename COL> static cudaError_t allow_cg() {
+    const cudaError_t e = allow_all_smem(k_cg_solve<NV, COL, 1>);
+    return e != cudaSuccess ? e : allow_all_smem(k_cg_solve<NV, COL, LIGHT_PER_SM<NV>>);
+}
 cudaError_t prepare_cg_kernels() {
-    const cudaError_t e[] = {
-        allow_all_smem(k_cg_solve<1, int, 1>),            allow_all_smem(k_cg_solve<9, int, 1>),
-        allow_all_smem(k_cg_solve<1, unsigned short, 1>), allow_all_smem(k_cg_solve<9, unsigned short, 1>),
-        allow_all_smem(k_cg_solve<1, int, 2>),            allow_all_smem(k_cg_solve<9, int, 2>),
-        allow_all_smem(k_cg_solve<1, unsigned short, 2>), allow_all_smem(k_cg_solve<9, unsigned short, 2>)};
+    const cudaError_t e[] = {allow_cg<1, int>(), allow_cg<9, int>(), allow_cg<1, unsigned short>(),
+                             allow_cg<9, unsigned short>()};
     for (cudaError_t x : e)
         if (x != cudaSuccess) return x;
     return cudaSuccess;

@@ -67,8 +67,8 @@ int round_up(int x, int a) { return (x + a - 1) / a * a; }
 std::atomic<int> large_steps[64];
 
 // The same for backward-Euler and projective-dynamics steps whose solve has a
-// CTA on more than half of the SMs: from the third on the solves take half a SM
-// each, so that two of them run side by side, with the same bits.
+// CTA on more than half of the SMs: from the third on the solves take a part of
+// a SM each, so that two or three of them run side by side, with the same bits.
 std::atomic<int> large_solves[64];
 
 class LargeCount {
@@ -153,8 +153,8 @@ struct pbs_handle {
     DevBuf<float4> cg_b, cg_x, cg_xp, cg_red, cg_ws;
     DevBuf<int> cg_plan;
     DevBuf<unsigned char> cg_col;
-    CgPlanView cgp[2][2]{};     // of the two matrix kinds (nine values a block, one), for a SM and for half of one
-    bool solve_light = false;   // the running step's solves take half a SM (LargeCount)
+    CgPlanView cgp[2][2]{};     // of the two matrix kinds (nine values a block, one), for a SM and for a part of one
+    bool solve_light = false;   // the running step's solves take a part of a SM (LargeCount)
     size_t cg_entries = 0, cg_rows_pad = 0, cg_halo = 0;
     DevBuf<CgState> cg_state;   // of the solves of a step
     DevBuf<unsigned> cg_ctl;    // [0] the last tag of the exchanged words, [1] a wait gave up
@@ -1841,7 +1841,7 @@ static int ensure_bsr(pbs_handle *h) {
     for (int kind = 0; kind < 2; ++kind)
     for (int light = 0; light < 2; ++light) {
         // what fits shared memory, the most often read first
-        const size_t budget = h->test_solve_smem >= 0 ? h->test_solve_smem : light ? CG_LIGHT_SMEM : CG_MAX_SMEM;
+        const size_t budget = h->test_solve_smem >= 0 ? h->test_solve_smem : light ? CG_LIGHT_SMEM[kind] : CG_MAX_SMEM;
         CgPlanView &w = h->cgp[kind][light];
         w = v;
         w.light = light != 0;

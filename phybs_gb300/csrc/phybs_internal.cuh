@@ -516,13 +516,13 @@ struct CgPlanView {
     const int *send;           // local rows that other CTAs' halos hold
     const void *scol;          // columns by entry and lane: own rows, then the halo (16 bits, or 32 with col32)
     bool col32;
-    bool light;  // half a SM: two solves can be on it, with the same bits (CG_LIGHT_SMEM)
+    bool light;  // a part of a SM: several solves can be on it, with the same bits (CG_LIGHT_SMEM)
     // byte offsets into the CTA's shared memory, -1: in global memory
     int off_p, off_r, off_q, off_x, off_val, off_col, off_node, off_rlen, off_small, off_dinv;
 };
 constexpr int CG_MIN_ROWS = 128;
 constexpr int BSR_HUB_TETS = 256;  // incident tets of a node whose row's columns the device finds
-constexpr int CG_MAX_SMEM = 225 * 1024, CG_LIGHT_SMEM = 110 * 1024;
+constexpr int CG_MAX_SMEM = 225 * 1024, CG_LIGHT_SMEM[2] = {55 * 1024, 73 * 1024};  // (by matrix kind)
 constexpr int CG_COPIES = 8;  // places a CTA writes its share of a sum to
 struct CgArgs {
     const float *val, *dinv;  // by entry, and the diagonal blocks' inverses by row (launch_cg_pack)

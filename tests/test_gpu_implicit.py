@@ -277,7 +277,7 @@ TEST_LARGE_STEPS = 2
 @pytest.mark.parametrize("integrator", ["be", "pd"])
 @pytest.mark.parametrize("nx,ny,nz", [(20, 20, 24), (24, 26, 40)])
 def test_solve_beside_others(integrator, nx, ny, nz):
-    """The solve of half a SM, which a step takes when two large ones run
+    """The solve of a part of a SM, which a step takes when two large ones run
     already (84 CTAs; one on every SM): bit for bit the one of a whole SM."""
     m, x0, v0 = _moving(5, nx, ny, nz)
     out = []
