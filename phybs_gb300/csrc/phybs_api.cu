@@ -353,7 +353,7 @@ static int set_pass_layout(pbs_handle *h, int threads, int ct, int cn, int stage
     if (join) cn = std::max(cn, cl.max_local);
     const int nc = (int)cl.chunk.size();
     if (automatic) {
-        if (ct == CHUNK_GROUP_TETS) threads = nc > h->sms && h->B == 1 ? 512 : 256;
+        if (ct == CHUNK_GROUP_TETS) threads = max_team == 512 && h->B == 1 ? 512 : 256;
         else threads = wide || (ct > 256 && nc > 2 * h->sms) ? 256 : 128;
         if (h->B == 1) threads = std::max(threads, max_team);
         else if (threads < max_team) threads = 256;  // (teams of 512 take two rounds)

@@ -59,6 +59,26 @@ def test_default_engine_equals_pass_kernels(dims, material, inc):
     b.close()
 
 
+@pytest.mark.parametrize("cells", [820, 15560, 20790, 22000, 49000])
+def test_meshes_with_many_nodes_a_tet(cells):
+    """Strips one cell thick (0.8 nodes a tet): their chunks end at the node
+    limits, so that there are more of them than of a box's at every line."""
+    m = M.box_mesh(cells, 1, 1, edge=0.01, seed=2, young=1e5, pin="bottom")
+    p = make_params("gpu_reference", h=1 / 30, max_iters=24)
+    alone, graph = DescentSolver(m, params=p), DescentSolver(m, params=p)
+    graph.set_pass_engine("graph")
+    packed = DescentSolver(_pack([_box(2, 1, 13), m, _box(8, 8, 12)]), params=p)
+    n0 = 3 * 2 * 14
+    for _ in range(2):
+        for s in (alone, graph, packed):
+            s.step(raise_on_error=False)
+        assert np.array_equal(alone.positions(), graph.positions())
+        assert np.array_equal(alone.positions(), packed.positions()[n0:n0 + m.n_nodes])
+        assert alone.stats()["energy"] == graph.stats()["energy"] == packed.instance_stats(1)["energy"]
+    for s in (alone, graph, packed):
+        s.close()
+
+
 def test_step_engine_is_the_one_that_ran():
     """What ran the passes, where the set engine (pass_engine) and the count of
     graph bodies do not tell."""
